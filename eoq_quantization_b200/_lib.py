@@ -184,6 +184,22 @@ def lib() -> C.CDLL:
     return L
 
 
+_NATIVE = None
+
+
+def native():
+    """The torch-facing front of the library (csrc/torch_native.cpp): the modules' forward calls in one C call each."""
+    global _NATIVE
+    if _NATIVE is None:
+        lib()
+        if not os.path.exists(os.path.join(_HERE, "_native.so")):
+            from . import build as _build
+            _build.build()
+        from . import _native
+        _NATIVE = _native
+    return _NATIVE
+
+
 def check(code: int, where: str = "") -> None:
     if code != EOQ_OK:
         raise EOQError(code, where)

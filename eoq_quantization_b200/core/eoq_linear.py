@@ -18,7 +18,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..eoq_file import EOQTensorRecord, fusable, read_eoq
-from ..fused import EOQWeight, require_cuda
+from ..fused import EOQWeight
 from .quantized_linear import get_model_memory, replace_linear_with_quantized
 
 
@@ -58,8 +58,7 @@ class EOQLinear(nn.Module):
     _dequantize = _dequantize_weight
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        require_cuda(x, "EOQLinear.forward")
-        return self.eoq.linear(x, self.bias_param)
+        return self.eoq.linear(x, self._buffers["bias_param"] if "bias_param" in self._buffers else self.bias_param)
 
     def memory_bytes(self) -> dict:
         info = self.eoq.info

@@ -12,6 +12,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from .. import _lib
 from ..fused import GEMM_MAX_ROWS, EOQWeight, dequant_packed, fused_rows, gemv_packed, PACKED_TENSOR_ROWS, packed_gemv_rows, require_cuda
 
 
@@ -127,6 +128,14 @@ class QuantizedLinear(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """x of shape (..., in_features), any float dtype -> (..., out_features) in x.dtype."""
+        buffers = self._buffers                 # not through nn.Module.__getattr__, which costs as much as the call
+        bias = buffers["bias_param"] if "bias_param" in buffers else self.bias_param
+        most = packed_gemv_rows(self.in_features, self.bits, self.block_size)
+        if most == PACKED_TENSOR_ROWS or not self._fusable():
+            y = _lib.native().packed_linear(buffers["packed_weight"], buffers["scales"], self.out_features, self.in_features, self.bits,
+                                            self.block_size, most if most == PACKED_TENSOR_ROWS else 0, x, bias)
+            if y is not None:
+                return y
         require_cuda(x, "QuantizedLinear.forward")
         require_cuda(self.packed_weight, "QuantizedLinear.forward")
         rows = x.numel() // max(self.in_features, 1)

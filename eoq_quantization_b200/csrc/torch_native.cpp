@@ -1,0 +1,197 @@
+// The modules' forward calls without the interpreter in between: one C function per route takes the module's tensors,
+// checks them, allocates the output and calls the library's C ABI.
+//
+// What a small call costs is the host, not the kernel: through ctypes, with tensor views and device guards made in
+// Python, EOQLinear took 25 us of host time around a 12 us kernel (4096 x 4096, one row) and the seven packed linears
+// of a 7B-shape block 160 us around 49 us of kernels.
+//
+// Every function returns None where anything is out of the ordinary (another device current, a subclass, gradients or
+// autocast asked for, a shape or type the route does not take, no rows): the caller then runs its Python path, which
+// handles those cases and raises the errors.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
+#include <ATen/core/LegacyTypeDispatch.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/ops/linear.h>
+#include <c10/core/GradMode.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/eoq_b200.h"
+
+namespace {
+
+using at::Tensor;
+
+int dtype_code(at::ScalarType t)
+{
+    return t == at::kHalf ? EOQ_B200_F16 : t == at::kBFloat16 ? EOQ_B200_BF16 : t == at::kFloat ? EOQ_B200_F32 : -1;
+}
+
+const Tensor *tensor_of(PyObject *o) { return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+// Nothing is going to watch or rewrite this call: no gradient through x, no autocast, no dispatch mode.
+bool plain_call(const Tensor &x)
+{
+    return !(x.requires_grad() && c10::GradMode::is_enabled()) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
+           !c10::impl::TorchDispatchModeTLS::any_modes_set();
+}
+
+// x is a dense tensor [..., K] on the current device, 16-byte aligned, of a type the kernels take; gives its rows.
+bool activations(const Tensor &x, int64_t K, int &code, int64_t &rows)
+{
+    if (!x.is_cuda() || x.layout() != at::kStrided || x.dim() < 1 || x.size(-1) != K || K <= 0 || !plain_call(x)) return false;
+    code = dtype_code(x.scalar_type());
+    if (code < 0 || !x.is_contiguous() || (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u)) return false;
+    if (x.get_device() != c10::cuda::current_device()) return false;
+    rows = x.numel() / K;
+    return rows > 0 && rows <= 0x7fffffff;
+}
+
+bool resident(const Tensor *t, const Tensor &x, at::ScalarType type)
+{
+    return t && t->is_cuda() && t->get_device() == x.get_device() && t->scalar_type() == type && t->is_contiguous();
+}
+
+// `bias` (None or an fp32 vector of N values beside x) as the kernels take it; false if it is anything else.
+bool bias_ptr(PyObject *o, const Tensor &x, int64_t N, const float *&b)
+{
+    b = nullptr;
+    if (o == Py_None) return true;
+    const Tensor *t = tensor_of(o);
+    if (!resident(t, x, at::kFloat) || t->numel() != N) return false;
+    b = static_cast<const float *>(t->data_ptr());
+    return true;
+}
+
+Tensor result(const Tensor &x, int64_t N, at::ScalarType type)
+{
+    auto sizes = x.sizes();
+    if (sizes.size() == 2) return at::detail::empty_cuda({sizes[0], N}, type, x.device(), std::nullopt);
+    c10::SmallVector<int64_t, 6> s(sizes.begin(), sizes.end());
+    s.back() = N;
+    return at::detail::empty_cuda(s, type, x.device(), std::nullopt);
+}
+
+void *stream_of(const Tensor &x) { return c10::cuda::getCurrentCUDAStream(x.get_device()).stream(); }
+
+// A call of the C ABI: None where the library says that it does not take the arguments (the Python path reports it).
+PyObject *done(eoq_error_t rc, Tensor &&y)
+{
+    if (rc != EOQ_OK) Py_RETURN_NONE;
+    return THPVariable_Wrap(std::move(y));
+}
+
+#define GUARD_BEGIN try {
+#define GUARD_END                                                        \
+    } catch (const std::exception &e) {                                  \
+        PyErr_SetString(PyExc_RuntimeError, e.what());                   \
+        return nullptr;                                                  \
+    }
+
+// weight_linear(handle, device, N, K, rows16, rows32, x, bias): EOQWeight.linear.  Up to rows16 (rows32 for fp32) rows by
+// the fused decode + GEMV, more by one decode to a dense matrix and a library GEMM.
+PyObject *weight_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
+{
+    if (n != 8) { PyErr_SetString(PyExc_TypeError, "weight_linear takes 8 arguments"); return nullptr; }
+    GUARD_BEGIN
+    const Tensor *x = tensor_of(a[6]);
+    const int64_t dev = PyLong_AsLongLong(a[1]), N = PyLong_AsLongLong(a[2]), K = PyLong_AsLongLong(a[3]);
+    int code;
+    int64_t rows;
+    const float *b;
+    if (!x || !activations(*x, K, code, rows) || x->get_device() != dev || !bias_ptr(a[7], *x, N, b)) Py_RETURN_NONE;
+    eoq_b200_weight_t *w = static_cast<eoq_b200_weight_t *>(PyLong_AsVoidPtr(a[0]));
+    void *st = stream_of(*x);
+    if (rows <= PyLong_AsLongLong(a[code == EOQ_B200_F32 ? 5 : 4])) {
+        if (rows > 8) Py_RETURN_NONE;
+        Tensor y = result(*x, N, x->scalar_type());
+        return done(eoq_b200_gemv(w, x->data_ptr(), code, (uint32_t)rows, y.data_ptr(), code, b, st), std::move(y));
+    }
+    Tensor dense = at::detail::empty_cuda({N, K}, x->scalar_type(), x->device(), std::nullopt);
+    if (eoq_b200_weight_decode(w, nullptr, 0, dense.data_ptr(), code, st) != EOQ_OK) Py_RETURN_NONE;
+    at::AutoDispatchBelowADInplaceOrView guard;
+    std::optional<Tensor> bias;
+    if (b) bias = THPVariable_Unpack(a[7]).to(x->scalar_type());
+    return THPVariable_Wrap(at::linear(*x, dense, bias));
+    GUARD_END
+}
+
+// packed_linear(packed, scales, N, K, bits, group, rows, x, bias): QuantizedLinear.forward.  Up to `rows` rows straight
+// from the packed codes, more by one dequantisation and a library GEMM.
+PyObject *packed_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
+{
+    if (n != 9) { PyErr_SetString(PyExc_TypeError, "packed_linear takes 9 arguments"); return nullptr; }
+    GUARD_BEGIN
+    const Tensor *pk = tensor_of(a[0]), *sc = tensor_of(a[1]), *x = tensor_of(a[7]);
+    const int64_t N = PyLong_AsLongLong(a[2]), K = PyLong_AsLongLong(a[3]), bits = PyLong_AsLongLong(a[4]),
+                  group = PyLong_AsLongLong(a[5]), most = PyLong_AsLongLong(a[6]);
+    int code;
+    int64_t rows;
+    const float *b;
+    if (!x || !pk || !activations(*x, K, code, rows) || !bias_ptr(a[8], *x, N, b) || group <= 0) Py_RETURN_NONE;
+    const at::ScalarType pt = bits == 4 || bits == 2 ? at::kByte : at::kChar;
+    const int64_t row_bytes = bits == 4 ? (K + 1) / 2 : bits == 2 ? (K + 3) / 4 : K;
+    if (!resident(pk, *x, pt) || !resident(sc, *x, at::kHalf) || pk->numel() != N * row_bytes || sc->numel() < (N * K + group - 1) / group)
+        Py_RETURN_NONE;
+    void *st = stream_of(*x);
+    const uint8_t *codes = static_cast<const uint8_t *>(pk->data_ptr());
+    const uint16_t *scales = static_cast<const uint16_t *>(sc->data_ptr());
+    if (rows <= most) {
+        Tensor y = result(*x, N, x->scalar_type()), scratch;
+        // fp32 activations on the tensor cores: room for their two fp16 halves
+        if (code == EOQ_B200_F32) scratch = at::detail::empty_cuda({rows, K}, at::kFloat, x->device(), std::nullopt);
+        return done(eoq_b200_gemv_packed(codes, scales, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)group, x->data_ptr(), code,
+                                         (uint32_t)rows, scratch.defined() ? scratch.data_ptr() : nullptr, y.data_ptr(), code, b, st),
+                    std::move(y));
+    }
+    Tensor dense = at::detail::empty_cuda({N, K}, x->scalar_type(), x->device(), std::nullopt);
+    if (eoq_b200_dequant_packed(codes, scales, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)group, 0, (uint32_t)N, dense.data_ptr(),
+                                code, st) != EOQ_OK)
+        Py_RETURN_NONE;
+    at::AutoDispatchBelowADInplaceOrView guard;
+    std::optional<Tensor> bias;
+    if (b) bias = THPVariable_Unpack(a[8]).to(x->scalar_type());
+    return THPVariable_Wrap(at::linear(*x, dense, bias));
+    GUARD_END
+}
+
+// polar_linear(codes, norms, centroids, N, K, bits, block, x): the product of PolarLinear.forward as fp16, without bias,
+// up to 32 rows (8 for blocks below 64 columns) straight from the byte codes.
+PyObject *polar_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
+{
+    if (n != 8) { PyErr_SetString(PyExc_TypeError, "polar_linear takes 8 arguments"); return nullptr; }
+    GUARD_BEGIN
+    const Tensor *cd = tensor_of(a[0]), *nr = tensor_of(a[1]), *ct = tensor_of(a[2]), *x = tensor_of(a[7]);
+    const int64_t N = PyLong_AsLongLong(a[3]), K = PyLong_AsLongLong(a[4]), bits = PyLong_AsLongLong(a[5]), block = PyLong_AsLongLong(a[6]);
+    int code;
+    int64_t rows;
+    if (!x || !activations(*x, K, code, rows) || block < 16 || (block & (block - 1)) || K % block || bits < 1 || bits > 8) Py_RETURN_NONE;
+    if (rows > (block >= 64 ? 32 : 8) || !resident(cd, *x, at::kChar) || !resident(nr, *x, at::kHalf) || !resident(ct, *x, at::kFloat) ||
+        cd->numel() < N * K || nr->numel() < N * K / block || ct->numel() < (1 << bits))
+        Py_RETURN_NONE;
+    Tensor y = result(*x, N, at::kHalf), scratch = at::detail::empty_cuda({rows, K}, at::kFloat, x->device(), std::nullopt);
+    return done(eoq_b200_gemv_polar_codes(static_cast<const uint8_t *>(cd->data_ptr()), static_cast<const uint16_t *>(nr->data_ptr()),
+                                          static_cast<const float *>(ct->data_ptr()), (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)block,
+                                          x->data_ptr(), code, (uint32_t)rows, scratch.data_ptr(), y.data_ptr(), EOQ_B200_F16, nullptr, -1,
+                                          stream_of(*x)),
+                std::move(y));
+    GUARD_END
+}
+
+PyMethodDef methods[] = {
+    {"weight_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(weight_linear)), METH_FASTCALL, nullptr},
+    {"packed_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(packed_linear)), METH_FASTCALL, nullptr},
+    {"polar_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(polar_linear)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&module); }

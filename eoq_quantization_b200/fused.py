@@ -57,6 +57,9 @@ class EOQWeight:
         _lib.check(_lib.lib().eoq_b200_weight_info(self._h, C.byref(info)), "eoq_b200_weight_info")
         self.info = info
         self.rows, self.cols = info.rows, info.cols
+        # what the native front of `linear` needs to know of this weight, in its argument order
+        self._linear = _lib.native().weight_linear
+        self._linear_args = (handle, self.device.index if self.device is not None else -1, self.rows, self.cols)
 
     def __del__(self):
         h, self._h = getattr(self, "_h", None), None
@@ -239,6 +242,9 @@ class EOQWeight:
         fused decode + GEMV; beyond, the weight is decoded to a dense matrix once (fused decode + dequantise kernel)
         for a library GEMM.  (Were GEMM_MAX_ROWS raised above 8, 16-bit activations on 4-bit weights would take the
         fused decode + tensor-core kernel, `gemm`, up to that many rows.)"""
+        y = self._linear(*self._linear_args, GEMV_MAX_ROWS[torch.float16], GEMV_MAX_ROWS[torch.float32], x, bias)
+        if y is not None:
+            return y
         require_cuda(x, "EOQWeight.linear")
         rows = x.numel() // max(self.cols, 1)
         if rows >= 1 and x.dtype in _DTYPES:
