@@ -39,7 +39,7 @@ EXPORTS = [
     "eoq_cuda_decode_tensor", "eoq_cuda_decode_tensor_device",
     "eoq_cuda_batch_init", "eoq_cuda_batch_create", "eoq_cuda_batch_prepare_tensor", "eoq_cuda_batch_launch",
     "eoq_cuda_batch_sync_and_free", "eoq_cuda_batch_destroy",
-    "eoq_b200_decode_blocked", "eoq_b200_encode_blocked",
+    "eoq_b200_decode_blocked", "eoq_b200_decode_blocked_as", "eoq_b200_encode_blocked", "eoq_b200_count_symbols", "eoq_b200_wire_encode", "eoq_b200_wire_take",
     "eoq_b200_tiles_build", "eoq_b200_tiles_view", "eoq_b200_tiles_free",
     "eoq_b200_weight_from_tiles", "eoq_b200_weight_from_symbols", "eoq_b200_weight_from_device_symbols", "eoq_b200_weight_from_rans", "eoq_b200_weight_destroy",
     "eoq_b200_weight_info", "eoq_b200_gemv", "eoq_b200_gemm",
@@ -144,6 +144,12 @@ def lib() -> C.CDLL:
                                               C.c_uint32, vp, C.c_int, C.c_int, vp]),
         "eoq_b200_encode_blocked": (C.c_int, [vp, C.c_uint32, C.c_uint32, vp, C.c_uint32, C.c_uint32, vp,
                                               C.POINTER(C.c_size_t), vp]),
+        "eoq_b200_decode_blocked_as": (C.c_int, [vp, C.c_uint32, C.c_uint32, vp, C.c_size_t, vp, C.c_uint32, C.c_uint32, C.c_uint32, vp,
+                                                 C.c_int, C.c_int64, vp]),
+        "eoq_b200_count_symbols": (C.c_int, [vp, C.c_int, C.c_size_t, C.c_int64, C.c_int, C.c_uint32, vp, vp]),
+        "eoq_b200_wire_encode": (C.c_int, [vp, C.c_int, C.c_uint32, C.c_int64, C.c_int, vp, C.c_uint32, C.c_uint32, C.c_uint32, C.POINTER(vp),
+                                           C.POINTER(C.c_size_t)]),
+        "eoq_b200_wire_take": (None, [vp, vp, vp]),
         "eoq_b200_tiles_build": (C.c_int, [vp, C.POINTER(WeightOpts), C.POINTER(vp)]),
         "eoq_b200_tiles_view": (C.c_int, [vp, C.POINTER(TilesView)]),
         "eoq_b200_tiles_free": (None, [vp]),

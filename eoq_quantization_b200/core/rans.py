@@ -10,14 +10,40 @@ import numpy as np
 from .. import _lib
 
 
+#: integer types the library reads symbols in and writes them in, where they lie
+_ELEMENTS = {np.dtype(np.int8): 0, np.dtype(np.uint8): 1, np.dtype(np.int16): 2, np.dtype(np.uint16): 3,
+             np.dtype(np.int32): 4, np.dtype(np.uint32): 5, np.dtype(np.int64): 6}
+
+
+def _native(result, where: str):
+    """A result of the native front, or its error code raised."""
+    if isinstance(result, int):
+        _lib.check(result, where)
+    return result
+
+
+def readable(symbols: np.ndarray) -> bool:
+    return symbols.dtype in _ELEMENTS and symbols.flags.c_contiguous and symbols.dtype.isnative
+
+
+def count_symbols(symbols: np.ndarray, alphabet_size: int, shift: int = 0, clamp: bool = False):
+    """(int64 counts, least, greatest) of value + shift over an array of one of the types above."""
+    counts, lo, hi = _native(_lib.native().count_symbols(symbols, _ELEMENTS[symbols.dtype], shift, int(clamp), alphabet_size), "count_symbols")
+    return np.array(counts, dtype=np.int64), lo, hi
+
+
 def compute_frequency_table(symbols: np.ndarray, alphabet_size: int) -> np.ndarray:
     """Histogram of symbol values (core/rans.py:32-55); ValueError if out of range."""
     symbols = np.asarray(symbols).ravel()
     if symbols.size == 0:
         return np.zeros(alphabet_size, dtype=np.int64)
-    if symbols.min() < 0 or symbols.max() >= alphabet_size:
-        raise ValueError(f"Symbols must be in [0, {alphabet_size}), got range [{symbols.min()}, {symbols.max()}]")
-    return np.bincount(symbols, minlength=alphabet_size).astype(np.int64)[:alphabet_size]
+    if readable(symbols) and 0 < alphabet_size <= 1 << 20:
+        counts, lo, hi = count_symbols(symbols, alphabet_size)
+    else:
+        counts, lo, hi = None, symbols.min(), symbols.max()
+    if lo < 0 or hi >= alphabet_size:
+        raise ValueError(f"Symbols must be in [0, {alphabet_size}), got range [{lo}, {hi}]")
+    return np.bincount(symbols, minlength=alphabet_size).astype(np.int64)[:alphabet_size] if counts is None else counts
 
 
 def estimate_compressed_size(freq_table: np.ndarray, num_symbols: int) -> int:
@@ -51,14 +77,17 @@ def _normalize_frequencies(raw_freq: np.ndarray, precision_bits: int):
     raw = np.maximum(raw, 1)
     scaled = np.maximum((raw.astype(np.float64) / raw.sum() * M).astype(np.int64), 1)
     residual = int(M - scaled.sum())
-    if residual:
+    if residual > 0:                        # nobody is passed over: whole rounds, then one more for the first ones
+        order = np.argsort(-scaled)
+        scaled += residual // a
+        scaled[order[:residual % a]] += 1
+    elif residual:
         order = np.argsort(-scaled)
         at = 0
         while residual:
-            step = 1 if residual > 0 else -1
-            if scaled[order[at]] + step >= 1:
-                scaled[order[at]] += step
-                residual -= step
+            if scaled[order[at]] > 1:
+                scaled[order[at]] -= 1
+                residual += 1
             at = (at + 1) % a
     cdf = np.zeros(a + 1, dtype=np.int64)
     np.cumsum(scaled, out=cdf[1:])
@@ -72,10 +101,14 @@ def _check_precision(p: int) -> None:
 
 def encode_blocks(freq_norm: np.ndarray, precision_bits: int, symbols: np.ndarray, block_size: int):
     """Host encoder of the library -> (bytes, offsets), wire format of core/rans.py:210-276."""
-    sym = np.ascontiguousarray(np.asarray(symbols).ravel().astype(np.uint32))
+    sym = np.asarray(symbols).ravel()
     if sym.size == 0:
         return b"", []
     f = np.ascontiguousarray(freq_norm, dtype=np.uint32)
+    if precision_bits <= 16 and readable(sym):
+        return _native(_lib.native().encode_symbols(sym, _ELEMENTS[sym.dtype], 0, 0, f, precision_bits, block_size, None, None),
+                       "eoq_b200_wire_encode")
+    sym = np.ascontiguousarray(sym.astype(np.uint32))
     nb = (sym.size + block_size - 1) // block_size
     cap = C.c_size_t(3 * sym.size + 16 * nb + 64)
     out = np.empty(cap.value, np.uint8)
@@ -86,23 +119,31 @@ def encode_blocks(freq_norm: np.ndarray, precision_bits: int, symbols: np.ndarra
     return out[:cap.value].tobytes(), offs.astype(np.int64).tolist()
 
 
-def decode_blocks(freq_norm: np.ndarray, precision_bits: int, data: bytes, offsets, block_size: int, n: int) -> np.ndarray:
-    """GPU decode of wire-format blocks -> int64 symbols (core/rans.py:368-419 per block)."""
+def encode_container(symbols: np.ndarray, shift: int, freq_norm: np.ndarray, precision_bits: int, block_size: int, head: bytes,
+                     counts: np.ndarray) -> bytes:
+    """A whole `RANS` container (core/rans_blocked.py:176-214) of value + shift, clipped to the alphabet: `head` up to the
+    data size, the counts, the offsets and the blocks."""
+    table = np.asarray(counts).astype("<u4")
+    if symbols.size == 0:
+        return head + b"\0\0\0\0" + table.tobytes()
+    return _native(_lib.native().encode_symbols(symbols, _ELEMENTS[symbols.dtype], shift, 1, np.ascontiguousarray(freq_norm, dtype=np.uint32),
+                                                precision_bits, block_size, head, table), "eoq_b200_wire_encode")
+
+
+def decode_blocks(freq_norm: np.ndarray, precision_bits: int, data: bytes, offsets, block_size: int, n: int,
+                  dtype=np.int64, shift: int = 0) -> np.ndarray:
+    """GPU decode of wire-format blocks -> symbols + shift (core/rans.py:368-419 per block), int64 unless asked otherwise."""
     if n == 0 or len(data) == 0:
-        return np.empty(0, dtype=np.int64)
+        return np.empty(0, dtype=dtype)
     if precision_bits > 16:
         raise NotImplementedError("the GPU decoder keeps a 32-bit state: precision_bits must be <= 16")
     f = np.ascontiguousarray(freq_norm, dtype=np.uint32)
     if f.size > 65536:
         raise NotImplementedError("alphabets above 65536 symbols are not supported")
-    buf = np.frombuffer(data, dtype=np.uint8)
-    offs = np.ascontiguousarray(np.asarray(offsets, dtype=np.uint32))
-    width = 1 if f.size <= 256 else 2
-    out = np.empty(n, np.uint8 if width == 1 else np.uint16)
-    _lib.check(_lib.lib().eoq_b200_decode_blocked(f.ctypes.data, f.size, precision_bits, buf.ctypes.data, buf.size,
-                                                  offs.ctypes.data, offs.size, block_size, n, out.ctypes.data, width, 0, None),
-               "eoq_b200_decode_blocked")
-    return out.astype(np.int64)
+    out = np.empty(n, dtype)
+    offs = offsets if type(offsets) is list else np.ascontiguousarray(np.asarray(offsets, dtype=np.uint32))
+    _native(_lib.native().decode_symbols(f, precision_bits, data, offs, block_size, out, _ELEMENTS[out.dtype], shift), "eoq_b200_decode_blocked")
+    return out
 
 
 class RANSEncoder:

@@ -10,7 +10,9 @@ from typing import Callable, Dict, Optional, Tuple
 import numpy as np
 import torch
 
-from .rans_blocked import (BlockedRANSDecoder, BlockedRANSEncoder, deserialize_blocked_rans, serialize_blocked_rans)
+from .rans import RANSEncoder, _normalize_frequencies, count_symbols, decode_blocks, encode_container, readable
+from .rans_blocked import (BlockedRANSDecoder, BlockedRANSEncoder, container_head, deserialize_blocked_rans,  # noqa: F401
+                           open_container, serialize_blocked_rans)  # noqa: F401
 from .utils import QuantizedTensor, dequantize, quantize_absmax
 
 
@@ -33,12 +35,17 @@ def compress_tensor_rans(name: str, codes: torch.Tensor, scales: torch.Tensor, b
     """Signed codes -> symbols code+qmax -> blocked rANS with 256-symbol blocks at 14-bit precision;
     scales stored as fp16 (core/rans_bitpacked.py:62-123)."""
     n = codes.numel()
-    flat = codes.detach().cpu().flatten().numpy().astype(np.int64)
+    flat = codes.detach().cpu().flatten().numpy()
+    if not readable(flat):
+        flat = flat.astype(np.int64)
     qmax = (1 << (bits - 1)) - 1
     alphabet = 2 * qmax + 1
-    unsigned = np.clip(flat + qmax, 0, alphabet - 1)
-    blocked = BlockedRANSEncoder(block_size=256, precision_bits=14).encode(unsigned, alphabet)
-    rans_bytes = serialize_blocked_rans(blocked)
+    block, precision = 256, 14
+    # counted and encoded where they lie, code + qmax clipped to the alphabet on the way
+    counts = count_symbols(flat, alphabet, qmax, True)[0] if n else np.zeros(alphabet, np.int64)
+    enc = RANSEncoder(counts, precision_bits=precision)
+    head = container_head(n, block, (n + block - 1) // block, alphabet, precision)
+    rans_bytes = encode_container(flat, qmax, enc.freq, precision, block, head, counts)
     scales_bytes = scales.detach().cpu().float().numpy().astype(np.float16).tobytes()
     return CompressedTensorData(name=name, shape=shape, bits=bits, block_size=block_size, scales_bytes=scales_bytes,
                                 rans_bytes=rans_bytes, n_elements=n, original_size=n * 2,
@@ -47,11 +54,13 @@ def compress_tensor_rans(name: str, codes: torch.Tensor, scales: torch.Tensor, b
 
 def decompress_tensor_rans(data: CompressedTensorData) -> Tuple[torch.Tensor, torch.Tensor]:
     """(int8 signed codes, float32 scales of fp16 precision) (core/rans_bitpacked.py:126-154)."""
-    unsigned = BlockedRANSDecoder().decode_all(deserialize_blocked_rans(data.rans_bytes))
     qmax = (1 << (data.bits - 1)) - 1
-    signed = unsigned.astype(np.int64) - qmax
+    n, block, _, _, precision, counts, offsets, stream = open_container(data.rans_bytes)
+    signed = np.empty(0, np.int8)
+    if n:
+        signed = decode_blocks(_normalize_frequencies(counts, precision)[0], precision, stream, offsets, block, n, np.int8, -qmax)
     scales = np.frombuffer(data.scales_bytes, dtype=np.float16).copy()
-    return torch.from_numpy(signed.astype(np.int8)).to(torch.int8), torch.from_numpy(scales.astype(np.float32))
+    return torch.from_numpy(signed), torch.from_numpy(scales.astype(np.float32))
 
 
 def compress_model_rans(model, bits_fn: Callable, block_size: int = 128,

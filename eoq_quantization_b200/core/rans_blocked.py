@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import math
 import struct
+from array import array
 from dataclasses import dataclass
 
 import numpy as np
@@ -88,26 +89,41 @@ def serialize_blocked_rans(data: BlockedRANSData) -> bytes:
     """`RANS` container of core/rans_blocked.py:176-214: magic, seven little-endian u32
     (version, num_symbols, block_size, num_blocks, alphabet_size, precision_bits, data_size),
     u32 freq_table[], u32 block_offsets[], data."""
-    head = _MAGIC + struct.pack("<7I", _VERSION, data.num_symbols, data.block_size, data.num_blocks,
-                                data.alphabet_size, data.precision_bits, len(data.compressed_blocks))
-    return (head + np.asarray(data.freq_table).astype("<u4").tobytes()
-            + np.asarray(data.block_offsets, dtype=np.int64).astype("<u4").tobytes() + bytes(data.compressed_blocks))
+    offsets = data.block_offsets
+    try:
+        offsets = array("I", offsets).tobytes() if type(offsets) is list and array("I").itemsize == 4 else None
+    except (OverflowError, TypeError):
+        offsets = None
+    if offsets is None:
+        offsets = np.asarray(data.block_offsets, dtype=np.int64).astype("<u4").tobytes()
+    return b"".join((container_head(data.num_symbols, data.block_size, data.num_blocks, data.alphabet_size, data.precision_bits),
+                     struct.pack("<I", len(data.compressed_blocks)), np.asarray(data.freq_table).astype("<u4").tobytes(), offsets,
+                     bytes(data.compressed_blocks)))
 
 
-def deserialize_blocked_rans(raw: bytes) -> BlockedRANSData:
-    """core/rans_blocked.py:217-259; ValueError on bad magic or version."""
+def container_head(num_symbols: int, block_size: int, num_blocks: int, alphabet_size: int, precision_bits: int) -> bytes:
+    """The container up to its data size."""
+    return _MAGIC + struct.pack("<6I", _VERSION, num_symbols, block_size, num_blocks, alphabet_size, precision_bits)
+
+
+def open_container(raw: bytes):
+    """(num_symbols, block_size, num_blocks, alphabet, precision, frequencies, offsets, data) of a container, the last three
+    as views of it; ValueError on bad magic or version."""
     magic = raw[:4]
     if magic != _MAGIC:
         raise ValueError(f"Invalid magic: {magic!r}")
     version, n, bs, nb, a, p, dsz = struct.unpack_from("<7I", raw, 4)
     if version != _VERSION:
         raise ValueError(f"Unsupported version: {version}")
-    at = 32
-    freq = np.frombuffer(raw, "<u4", a, at).astype(np.int64)
-    at += 4 * a
-    offsets = np.frombuffer(raw, "<u4", nb, at).astype(np.int64).tolist()
-    at += 4 * nb
-    return BlockedRANSData(compressed_blocks=bytes(raw[at:at + dsz]), block_offsets=offsets, freq_table=freq,
+    at = 32 + 4 * a
+    return (n, bs, nb, a, p, np.frombuffer(raw, "<u4", a, 32), np.frombuffer(raw, "<u4", nb, at),
+            memoryview(raw)[at + 4 * nb:at + 4 * nb + dsz])
+
+
+def deserialize_blocked_rans(raw: bytes) -> BlockedRANSData:
+    """core/rans_blocked.py:217-259; ValueError on bad magic or version."""
+    n, bs, nb, a, p, freq, offsets, data = open_container(raw)
+    return BlockedRANSData(compressed_blocks=bytes(data), block_offsets=offsets.tolist(), freq_table=freq.astype(np.int64),
                            num_symbols=n, block_size=bs, num_blocks=nb, alphabet_size=a, precision_bits=p)
 
 

@@ -4,12 +4,14 @@
 #include "eoq_internal.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <cuda_runtime.h>
 #include <memory>
 #include <mutex>
+#include <thread>
 #include <unistd.h>
 
 using namespace eoq;
@@ -37,8 +39,72 @@ struct DeviceBuf {
     DeviceBuf() = default;
     DeviceBuf(const DeviceBuf &) = delete;
     DeviceBuf &operator=(const DeviceBuf &) = delete;
-    ~DeviceBuf() { if (p) cudaFree(p); }
+    ~DeviceBuf() { release(); }
     cudaError_t alloc(size_t n) { return cudaMalloc(&p, n ? n : 1); }
+    // Out of this library's own memory pool: a model load allocates and a replaced layer releases without the driver mapping
+    // and unmapping memory each time (cudaMalloc and cudaFree of the 24 MB of a layer: 0.5 to 10 ms).  The pool keeps at
+    // most 256 MB that nobody uses; what is beyond goes back to the driver.
+    cudaError_t alloc_pooled(size_t n)
+    {
+        cudaMemPool_t pool;
+        cudaError_t e = cudaGetDevice(&device);
+        if (e == cudaSuccess) e = weight_pool(device, pool);
+        if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&p, n ? n : 1, pool, nullptr);
+        pooled = e == cudaSuccess;
+        if (!pooled) p = nullptr;
+        return e;
+    }
+    void take(DeviceBuf &o)
+    {
+        p = o.p; pooled = o.pooled; device = o.device;
+        o.p = nullptr;
+    }
+    void release()
+    {
+        if (!p) return;
+        if (pooled) {
+            int cur = device;
+            cudaGetDevice(&cur);
+            if (cur != device) cudaSetDevice(device);
+            cudaDeviceSynchronize();                 // as cudaFree does: whatever stream still reads it
+            cudaFreeAsync(p, nullptr);
+            if (cur != device) cudaSetDevice(cur);
+        } else {
+            cudaFree(p);
+        }
+        p = nullptr;
+    }
+
+  private:
+    bool pooled = false;
+    int device = 0;
+    static cudaError_t weight_pool(int dev, cudaMemPool_t &out)
+    {
+        static std::mutex *mu = new std::mutex();
+        static cudaMemPool_t pools[64] = {};
+        if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+        std::lock_guard<std::mutex> lock(*mu);
+        if (!pools[dev]) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            cudaError_t e = cudaMemPoolCreate(&pools[dev], &props);
+            uint64_t keep = 256ull << 20;
+            if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+            if (e != cudaSuccess) { pools[dev] = nullptr; return e; }
+        }
+        out = pools[dev];
+        return cudaSuccess;
+    }
+
+  public:
+    template <typename T> T *as() const { return reinterpret_cast<T *>(p); }
+};
+
+// A part of somebody else's allocation.
+struct DeviceView {
+    void *p = nullptr;
     template <typename T> T *as() const { return reinterpret_cast<T *>(p); }
 };
 
@@ -152,6 +218,69 @@ class DeviceArena {
     Block cur_;
 };
 
+constexpr size_t kPinnedChunk = 256u << 10, kPinnedThreads = 16, kPinnedBytes = 2 * kPinnedChunk * kPinnedThreads;
+
+// Page-locked staging memory (8 MB a block), kept between calls: at most two blocks, the rest is given back at once.
+class PinnedBlock {
+  public:
+    PinnedBlock() = default;
+    PinnedBlock(const PinnedBlock &) = delete;
+    PinnedBlock &operator=(const PinnedBlock &) = delete;
+    cudaError_t acquire()
+    {
+        {
+            std::lock_guard<std::mutex> lock(cache().mu);
+            if (!cache().free_list.empty()) { p_ = cache().free_list.back(); cache().free_list.pop_back(); return cudaSuccess; }
+        }
+        return cudaHostAlloc(reinterpret_cast<void **>(&p_), kPinnedBytes, cudaHostAllocPortable);
+    }
+    ~PinnedBlock()
+    {
+        if (!p_) return;
+        std::lock_guard<std::mutex> lock(cache().mu);
+        if (cache().free_list.size() < 2) cache().free_list.push_back(p_);
+        else cudaFreeHost(p_);
+    }
+    uint8_t *chunk(size_t i) const { return p_ + i * kPinnedChunk; }
+
+  private:
+    struct Cache { std::mutex mu; std::vector<uint8_t *> free_list; };
+    static Cache &cache() { static Cache *c = new Cache(); return *c; }      // never destroyed: no CUDA call after main
+    uint8_t *p_ = nullptr;
+};
+
+// `bytes` of pageable host memory to the device.  The driver stages a pageable copy on one core (some 9 GB/s); from a few
+// megabytes on several threads stage it, each through two chunks of its own.  The source has been read when this returns.
+cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t st)
+{
+    const size_t chunks = (bytes + kPinnedChunk - 1) / kPinnedChunk, hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t threads = std::min<size_t>({kPinnedThreads / 2, hw, chunks / 4});
+    PinnedBlock pinned;
+    if (threads < 2 || pinned.acquire() != cudaSuccess) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    std::atomic<int> failed{(int)cudaSuccess};
+    parallel_for(threads, [&](size_t t) {
+        cudaEvent_t free_again[2] = {nullptr, nullptr};
+        cudaError_t r = cudaSetDevice(device);
+        for (cudaEvent_t &ev : free_again) if (r == cudaSuccess) r = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        int slot = 0;
+        for (size_t c = t; r == cudaSuccess && c < chunks; c += threads, slot ^= 1) {
+            const size_t lo = c * kPinnedChunk, cnt = std::min(kPinnedChunk, bytes - lo);
+            r = cudaEventSynchronize(free_again[slot]);              // never recorded: complete
+            if (r != cudaSuccess) break;
+            std::memcpy(pinned.chunk(2 * t + slot), static_cast<const uint8_t *>(src) + lo, cnt);
+            r = cudaMemcpyAsync(static_cast<uint8_t *>(dst) + lo, pinned.chunk(2 * t + slot), cnt, cudaMemcpyHostToDevice, st);
+            if (r == cudaSuccess) r = cudaEventRecord(free_again[slot], st);
+        }
+        for (cudaEvent_t ev : free_again)
+            if (ev) { cudaEventSynchronize(ev); cudaEventDestroy(ev); }      // the staging memory is another call's from here on
+        if (r != cudaSuccess) failed.store((int)r);
+    }, threads);
+    return (cudaError_t)failed.load();
+}
+
 // One tensor of a decode call.
 struct V1Job {
     Payload pl;                         // validated host views of the payload
@@ -242,7 +371,7 @@ eoq_error_t decode_jobs(V1Job **jobs, size_t n, cudaStream_t st, DeviceArena &ar
     CU_TRY(cudaMemcpyAsync(d, blob.data(), meta, cudaMemcpyHostToDevice, st));
     for (size_t i = 0; i < n; i++) {
         V1Job &j = *jobs[i];
-        if (j.pl.stream_bytes) CU_TRY(cudaMemcpyAsync(d + j.at_stream, j.pl.stream, j.pl.stream_bytes, cudaMemcpyHostToDevice, st));
+        if (j.pl.stream_bytes) CU_TRY(upload(d + j.at_stream, j.pl.stream, j.pl.stream_bytes, st));
     }
     if (!tasks.empty()) {
         int e = launch_decode_v1_lanes(reinterpret_cast<const V1Task *>(d + at_tasks), reinterpret_cast<const uint32_t *>(d + at_cta), grid,
@@ -610,13 +739,12 @@ extern "C" void eoq_cuda_batch_destroy(eoq_cuda_batch_ctx_t *ctx)
 // Part 2: Python-facing codec entry points and the fused path
 // =========================================================================
 
-extern "C" eoq_error_t eoq_b200_decode_blocked(const uint32_t *freq, uint32_t alphabet, uint32_t precision_bits,
-                                               const uint8_t *data, size_t data_len, const uint32_t *offsets,
-                                               uint32_t num_blocks, uint32_t block_size, uint32_t num_symbols,
-                                               void *out, int out_elem_bytes, int out_on_device, void *stream)
+// Validates a blocked stream on the host, as the reference's decoders do block by block, and makes it a job.
+static eoq_error_t blocked_job(const uint32_t *freq, uint32_t alphabet, uint32_t precision_bits, const uint8_t *data, size_t data_len,
+                               const uint32_t *offsets, uint32_t num_blocks, uint32_t block_size, uint32_t num_symbols,
+                               int out_elem_bytes, V1Job &job)
 {
-    if (num_symbols == 0) return EOQ_OK;
-    if (!freq || !data || !offsets || !out) return EOQ_ERR_NULL_PTR;
+    if (!freq || !data || !offsets) return EOQ_ERR_NULL_PTR;
     if (alphabet == 0 || block_size == 0) return EOQ_ERR_INVALID_HEADER;
     if (precision_bits < 1 || precision_bits > 16) return EOQ_ERR_UNSUPPORTED;   // 32-bit device state
     if (out_elem_bytes != 1 && out_elem_bytes != 2) return EOQ_ERR_UNSUPPORTED;
@@ -635,9 +763,6 @@ extern "C" eoq_error_t eoq_b200_decode_blocked(const uint32_t *freq, uint32_t al
         if (sizes[b] && 1u + data[lo] > sizes[b]) return EOQ_ERR_CORRUPT_STREAM;
         if (sizes[b] && data[lo] > 4) return EOQ_ERR_UNSUPPORTED;                  // state wider than 32 bits
     }
-    if (!have_device()) return EOQ_ERR_CUDA;
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    V1Job job;
     job.pl.alphabet = alphabet; job.pl.p = precision_bits; job.pl.block = block_size; job.pl.total = num_symbols;
     job.pl.nblocks = num_blocks; job.pl.stream = data; job.pl.stream_bytes = (uint32_t)data_len;
     job.pl.offsets.assign(offsets, offsets + num_blocks);
@@ -645,12 +770,116 @@ extern "C" eoq_error_t eoq_b200_decode_blocked(const uint32_t *freq, uint32_t al
     job.freq = std::move(f);
     job.cdf = std::move(cdf);
     job.out_elem_bytes = (uint32_t)out_elem_bytes;
+    return EOQ_OK;
+}
+
+extern "C" eoq_error_t eoq_b200_decode_blocked(const uint32_t *freq, uint32_t alphabet, uint32_t precision_bits,
+                                               const uint8_t *data, size_t data_len, const uint32_t *offsets,
+                                               uint32_t num_blocks, uint32_t block_size, uint32_t num_symbols,
+                                               void *out, int out_elem_bytes, int out_on_device, void *stream)
+{
+    if (num_symbols == 0) return EOQ_OK;
+    if (!out) return EOQ_ERR_NULL_PTR;
+    V1Job job;
+    eoq_error_t rc = blocked_job(freq, alphabet, precision_bits, data, data_len, offsets, num_blocks, block_size, num_symbols, out_elem_bytes, job);
+    if (rc != EOQ_OK) return rc;
+    if (!have_device()) return EOQ_ERR_CUDA;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (out_on_device) job.dev_out = out; else job.host_out = out;
     V1Job *one = &job;
     DeviceArena arena;
-    eoq_error_t rc = decode_jobs(&one, 1, st, arena);
+    rc = decode_jobs(&one, 1, st, arena);
     if (rc != EOQ_OK) return rc;
     CU_TRY(cudaStreamSynchronize(st));   // the staging arena goes back to the cache on return
+    return EOQ_OK;
+}
+
+// -- symbols from the device to a host array of another integer type ------------
+//
+// The decoder leaves one or two bytes per symbol; the Python interface wants int64 (or int8 codes).  Copying the bytes to
+// pageable memory and converting them on one core took 22 of the 24 ms of a 4096 x 4096 container: here a few threads
+// each move chunks through page-locked memory of their own (two chunks each: one on the bus while the other is
+// converted) and write the caller's array, page faults of a fresh array included, side by side: 5 ms.
+namespace {
+
+template <typename S, typename D>
+void convert(const void *src, void *dst, size_t n, int64_t shift)
+{
+    const S *s = static_cast<const S *>(src);
+    D *d = static_cast<D *>(dst);
+    for (size_t i = 0; i < n; i++) d[i] = (D)((int64_t)s[i] + shift);
+}
+
+typedef void (*ConvertFn)(const void *, void *, size_t, int64_t);
+
+// Symbols (1 or 2 bytes each on the device, complete on `st`) to `out`, of the type EOQ_B200_SYM_* names.
+eoq_error_t deliver(const uint8_t *dev, uint32_t elem, size_t n, void *out, int out_type, int64_t shift, cudaStream_t st)
+{
+    static const size_t width[7] = {1, 1, 2, 2, 4, 4, 8};
+    ConvertFn fn = nullptr;
+    switch (out_type) {
+        case EOQ_B200_SYM_I8: fn = elem == 1 ? convert<uint8_t, int8_t> : convert<uint16_t, int8_t>; break;
+        case EOQ_B200_SYM_U8: fn = elem == 1 ? convert<uint8_t, uint8_t> : convert<uint16_t, uint8_t>; break;
+        case EOQ_B200_SYM_I16: fn = elem == 1 ? convert<uint8_t, int16_t> : convert<uint16_t, int16_t>; break;
+        case EOQ_B200_SYM_U16: fn = elem == 1 ? convert<uint8_t, uint16_t> : convert<uint16_t, uint16_t>; break;
+        case EOQ_B200_SYM_I32: fn = elem == 1 ? convert<uint8_t, int32_t> : convert<uint16_t, int32_t>; break;
+        case EOQ_B200_SYM_I64: fn = elem == 1 ? convert<uint8_t, int64_t> : convert<uint16_t, int64_t>; break;
+        default: return EOQ_ERR_UNSUPPORTED;
+    }
+    PinnedBlock pinned;
+    if (pinned.acquire() != cudaSuccess) return EOQ_ERR_ALLOC;
+    int device = 0;
+    CU_TRY(cudaGetDevice(&device));
+    const size_t per = kPinnedChunk / elem, chunks = (n + per - 1) / per;
+    // a thread costs some tens of microseconds to start, a chunk of 256 Ki symbols about a hundred to convert to int64
+    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t threads = std::max<size_t>(1, std::min<size_t>({kPinnedThreads, hw, (chunks + 1) / 2}));
+    std::atomic<int> failed{0};
+    parallel_for(threads, [&](size_t t) {
+        cudaEvent_t done[2] = {nullptr, nullptr};
+        bool ok = cudaSetDevice(device) == cudaSuccess && cudaEventCreateWithFlags(&done[0], cudaEventDisableTiming) == cudaSuccess &&
+                  cudaEventCreateWithFlags(&done[1], cudaEventDisableTiming) == cudaSuccess;
+        auto request = [&](size_t c, int slot) {
+            const size_t lo = c * per, cnt = std::min(per, n - lo);
+            ok = ok && cudaMemcpyAsync(pinned.chunk(2 * t + slot), dev + lo * elem, cnt * elem, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+                 cudaEventRecord(done[slot], st) == cudaSuccess;
+        };
+        if (ok && t < chunks) request(t, 0);
+        int slot = 0;
+        for (size_t c = t; ok && c < chunks; c += threads, slot ^= 1) {
+            if (c + threads < chunks) request(c + threads, slot ^ 1);
+            ok = ok && cudaEventSynchronize(done[slot]) == cudaSuccess;
+            const size_t lo = c * per, cnt = std::min(per, n - lo);
+            if (ok) fn(pinned.chunk(2 * t + slot), static_cast<uint8_t *>(out) + lo * width[out_type], cnt, shift);
+        }
+        if (!ok) failed.store(1);
+        for (cudaEvent_t e : done) if (e) cudaEventDestroy(e);
+    }, threads);
+    if (failed.load()) { cudaStreamSynchronize(st); return EOQ_ERR_CUDA; }      // nothing may still be on its way into the staging memory
+    return EOQ_OK;
+}
+
+}  // namespace
+
+extern "C" eoq_error_t eoq_b200_decode_blocked_as(const uint32_t *freq, uint32_t alphabet, uint32_t precision_bits, const uint8_t *data,
+                                                  size_t data_len, const uint32_t *offsets, uint32_t num_blocks, uint32_t block_size,
+                                                  uint32_t num_symbols, void *out, int out_type, int64_t shift, void *stream)
+{
+    if (num_symbols == 0) return EOQ_OK;
+    if (!out) return EOQ_ERR_NULL_PTR;
+    if (out_type < EOQ_B200_SYM_I8 || out_type > EOQ_B200_SYM_I64 || out_type == EOQ_B200_SYM_U32) return EOQ_ERR_UNSUPPORTED;
+    V1Job job;
+    eoq_error_t rc = blocked_job(freq, alphabet, precision_bits, data, data_len, offsets, num_blocks, block_size, num_symbols,
+                                 alphabet <= 256 ? 1 : 2, job);
+    if (rc != EOQ_OK) return rc;
+    if (!have_device()) return EOQ_ERR_CUDA;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    V1Job *one = &job;
+    DeviceArena arena;
+    rc = decode_jobs(&one, 1, st, arena, false);
+    if (rc == EOQ_OK) rc = deliver(arena.base() + job.at_out, job.out_elem_bytes, num_symbols, out, out_type, shift, st);
+    if (rc != EOQ_OK) return rc;
+    CU_TRY(cudaStreamSynchronize(st));
     return EOQ_OK;
 }
 
@@ -667,6 +896,18 @@ extern "C" eoq_error_t eoq_b200_encode_blocked(const uint32_t *freq, uint32_t al
     for (uint32_t s = 0; s < alphabet; s++) { if (!freq[s]) return EOQ_ERR_INVALID_HEADER; sum += freq[s]; cdf[s + 1] = cdf[s] + freq[s]; }
     if (sum != (1ull << precision_bits)) return EOQ_ERR_INVALID_HEADER;
     for (uint32_t i = 0; i < num_symbols; i++) if (symbols[i] >= alphabet) return EOQ_ERR_CORRUPT_STREAM;
+    if (precision_bits <= 16) {
+        eoq_b200_wire_t *w = nullptr;
+        size_t total = 0;
+        eoq_error_t rc = eoq_b200_wire_encode(symbols, EOQ_B200_SYM_U32, num_symbols, 0, 0, freq, alphabet, precision_bits, block_size, &w, &total);
+        if (rc != EOQ_OK) return rc;
+        const bool fits = total <= *out_len;
+        eoq_b200_wire_take(w, fits ? out : nullptr, fits ? offsets : nullptr);
+        if (!fits) return EOQ_ERR_BUFFER_TOO_SMALL;
+        *out_len = total;
+        return EOQ_OK;
+    }
+    // states wider than 32 bits: one division per symbol
     const uint32_t nb = (uint32_t)(((uint64_t)num_symbols + block_size - 1) / block_size);
     // blocks are independent streams: ranges of blocks are encoded on the host's cores (one range, on the calling thread,
     // for small inputs), then laid out back to back in block order
@@ -703,16 +944,65 @@ extern "C" eoq_error_t eoq_b200_encode_blocked(const uint32_t *freq, uint32_t al
 
 // -- resident weights ---------------------------------------------------------
 
+// Status words of the resident weights: 64 bytes each of page-locked memory that the device can address, dealt out of
+// pages (a page-locked allocation per weight, and its release, took 1.5 ms each).  A page whose words have all come
+// back is given back unless it is the only one.
+class StatusWords {
+  public:
+    static cudaError_t take(uint32_t **host, uint32_t **dev)
+    {
+        std::lock_guard<std::mutex> lock(mu());
+        Page *page = nullptr;
+        for (Page &p : pages()) if (p.used != ~0ull) { page = &p; break; }
+        if (!page) {
+            Page fresh;
+            cudaError_t e = cudaHostAlloc(reinterpret_cast<void **>(&fresh.host), 64 * 64, cudaHostAllocPortable | cudaHostAllocMapped);
+            if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&fresh.dev), fresh.host, 0);
+            if (e != cudaSuccess) return e;
+            pages().push_back(fresh);
+            page = &pages().back();
+        }
+        int slot = 0;
+        while ((page->used >> slot) & 1) slot++;
+        page->used |= 1ull << slot;
+        *host = reinterpret_cast<uint32_t *>(page->host + 64 * slot);
+        *dev = reinterpret_cast<uint32_t *>(page->dev + 64 * slot);
+        std::memset(*host, 0, 64);
+        return cudaSuccess;
+    }
+    static void give(uint32_t *word)
+    {
+        if (!word) return;
+        std::lock_guard<std::mutex> lock(mu());
+        uint8_t *at = reinterpret_cast<uint8_t *>(word);
+        for (size_t i = 0; i < pages().size(); i++) {
+            Page &p = pages()[i];
+            if (at < p.host || at >= p.host + 64 * 64) continue;
+            p.used &= ~(1ull << ((at - p.host) / 64));
+            if (p.used == 0 && pages().size() > 1) { cudaFreeHost(p.host); pages().erase(pages().begin() + i); }
+            return;
+        }
+    }
+
+  private:
+    struct Page { uint8_t *host = nullptr, *dev = nullptr; uint64_t used = 0; };
+    static std::mutex &mu() { static std::mutex *m = new std::mutex(); return *m; }
+    static std::vector<Page> &pages() { static std::vector<Page> *v = new std::vector<Page>(); return *v; }
+};
+
 struct eoq_b200_weight {
     int device = 0;
     uint32_t N = 0, K = 0, Npad = 0, G = 0, bits = 0, p = 0, group = 0, kind = 0, alphabet = 0;
     uint32_t ntiles = 0, nseg = 0, nrb = 0;
     uint32_t stage_bytes = 0, max_ncols = 0;          // geometry of the pair kernel's staging buffers (see GemvArgs)
     uint32_t head_bytes = 0;                          // TiledWeights::head_bytes
-    DeviceBuf scales_t;                               // transposed copy of the scales for the pair kernel (INT4 x 3 only)
-    DeviceBuf pair_partials;                          // partial rows of the pair kernel, every word 0xFFFFFFFF between launches
+    // scales_t: transposed copy of the scales for the pair kernel (INT4 x 3 only); pair_partials: partial rows of the pair
+    // kernel, every word 0xFFFFFFFF between launches
     size_t pair_partial_bytes = 0;
-    DeviceBuf table, tiles, stream, scales, centroids, partials, counters, status, xbuf, ybuf, biasbuf;
+    DeviceBuf slab, stream;                           // everything but the stream in one allocation, the parts below point into it
+    DeviceView table, tiles, scales, scales_t, centroids, counters, pair_partials;
+    DeviceBuf partials;                               // the ring kernel's scratch
+    DeviceBuf xbuf, ybuf, biasbuf;                    // staging of the host-buffer calls, allocated by their first
     DeviceBuf gemm_x, gemm_partials, gemm_counters;   // scratch of the tensor-core path, allocated by its first call
     uint32_t gemm_rows = 0;                           // activation rows per pass that scratch was sized for
     // The status word the kernels set when a bounded wait expires lives in pinned host memory that the device writes
@@ -723,7 +1013,11 @@ struct eoq_b200_weight {
     {
         return status_dev;
     }
-    ~eoq_b200_weight() { if (status_host) cudaFreeHost(status_host); }
+    ~eoq_b200_weight()
+    {
+        slab.release();       // waits for the device: no launch can write the word below any more
+        StatusWords::give(status_host);
+    }
     size_t stream_bytes = 0, scale_bytes = 0, partial_bytes = 0;
     std::mutex mu;   // one call at a time may use the scratch of a weight
     std::mutex scratch_mu;   // guards the late allocation of `partials`
@@ -782,45 +1076,37 @@ eoq_error_t upload_weight(const TiledWeights &tw, const uint16_t *scales, const 
     // activation rows x 32 lanes of fp32 = 3 KB) go into the first, its share of a cooperative meeting into the second.
     // Tiles shorter than that (32-column tiles, low-entropy weights) get buffers of that size all the same.
     if (pairs_layout) w->stage_bytes = std::max(w->stage_bytes, 3072u);
-    if (w->table.alloc(tw.table.size() * 4) != cudaSuccess || w->tiles.alloc(tw.tiles.size() * sizeof(TileDesc)) != cudaSuccess ||
-        (!built && w->stream.alloc(tw.stream.size()) != cudaSuccess) || w->scales.alloc(w->scale_bytes) != cudaSuccess ||
-        (!pairs_layout && w->partials.alloc(w->partial_bytes) != cudaSuccess) || w->counters.alloc((size_t)tw.nrb * 4) != cudaSuccess ||
-        w->status.alloc(4) != cudaSuccess ||
-        w->xbuf.alloc((size_t)8 * tw.K * 4) != cudaSuccess || w->ybuf.alloc((size_t)8 * tw.N * 4) != cudaSuccess ||
-        w->biasbuf.alloc((size_t)tw.N * 4) != cudaSuccess)
+    // one allocation for all the small parts (ten of them, and their release, took 2 ms of a 7 ms load)
+    w->pair_partial_bytes = pairs_layout ? (size_t)pair_partial_slots(tw.nrb, tw.nseg) * tw.Npad * 4 * sizeof(float) : 0;
+    const uint32_t sg = tw.K / tw.group, triples = tw.Npad / 3;
+    size_t used = 0;
+    auto part = [&](size_t bytes) { const size_t at = used; used += (bytes + 255) & ~(size_t)255; return at; };
+    const size_t at_table = part(tw.table.size() * 4), at_tiles = part(tw.tiles.size() * sizeof(TileDesc)), at_scales = part(w->scale_bytes),
+                 at_scales_t = part(pairs_layout ? (size_t)sg * triples * 8 : 0), at_cent = part(32 * 4), at_counters = part((size_t)tw.nrb * 4),
+                 at_partials = part(w->pair_partial_bytes);
+    if (w->slab.alloc_pooled(used) != cudaSuccess || (!built && w->stream.alloc_pooled(tw.stream.size()) != cudaSuccess) ||
+        (!pairs_layout && w->partials.alloc(w->partial_bytes) != cudaSuccess))
         return EOQ_ERR_ALLOC;
+    uint8_t *base = w->slab.as<uint8_t>();
+    w->table.p = base + at_table; w->tiles.p = base + at_tiles; w->scales.p = base + at_scales; w->counters.p = base + at_counters;
+    if (built) w->stream.take(*built);
+    else CU_TRY(upload(w->stream.p, tw.stream.data(), tw.stream.size(), nullptr));
     if (centroids) {
-        if (w->centroids.alloc(32 * 4) != cudaSuccess) return EOQ_ERR_ALLOC;
-        CU_TRY(cudaMemcpy(w->centroids.p, centroids, 32 * 4, cudaMemcpyHostToDevice));
+        w->centroids.p = base + at_cent;
+        CU_TRY(cudaMemcpyAsync(w->centroids.p, centroids, 32 * 4, cudaMemcpyHostToDevice, nullptr));
     }
-    CU_TRY(cudaMemcpy(w->table.p, tw.table.data(), tw.table.size() * 4, cudaMemcpyHostToDevice));
-    CU_TRY(cudaMemcpy(w->tiles.p, tw.tiles.data(), tw.tiles.size() * sizeof(TileDesc), cudaMemcpyHostToDevice));
-    if (built) { w->stream.p = built->p; built->p = nullptr; }
-    else CU_TRY(cudaMemcpy(w->stream.p, tw.stream.data(), tw.stream.size(), cudaMemcpyHostToDevice));
-    CU_TRY(cudaMemcpy(w->scales.p, scales, w->scale_bytes, cudaMemcpyHostToDevice));
+    CU_TRY(cudaMemcpyAsync(w->table.p, tw.table.data(), tw.table.size() * 4, cudaMemcpyHostToDevice, nullptr));
+    CU_TRY(cudaMemcpyAsync(w->tiles.p, tw.tiles.data(), tw.tiles.size() * sizeof(TileDesc), cudaMemcpyHostToDevice, nullptr));
+    CU_TRY(upload(w->scales.p, scales, w->scale_bytes, nullptr));
     if (pairs_layout) {
-        w->pair_partial_bytes = (size_t)pair_partial_slots(tw.nrb, tw.nseg) * tw.Npad * 4 * sizeof(float);
-        if (w->pair_partials.alloc(w->pair_partial_bytes) != cudaSuccess) return EOQ_ERR_ALLOC;
-        CU_TRY(cudaMemset(w->pair_partials.p, 0xFF, w->pair_partial_bytes));
-        // [group][row triple] -> {s0 | s1 << 16, s2}, zero for rows past N: what a lane of the pair kernel needs for one
-        // run of columns, in one coalesced 8-byte load
-        const uint32_t sg = tw.K / tw.group, triples = tw.Npad / 3;
-        std::vector<uint32_t> t((size_t)sg * triples * 2, 0u);
-        for (uint32_t g = 0; g < sg; g++)
-            for (uint32_t i = 0; i < triples; i++) {
-                uint32_t v[3];
-                for (uint32_t j = 0; j < 3; j++) v[j] = 3 * i + j < tw.N ? scales[(size_t)(3 * i + j) * sg + g] : 0u;
-                t[((size_t)g * triples + i) * 2] = v[0] | (v[1] << 16);
-                t[((size_t)g * triples + i) * 2 + 1] = v[2];
-            }
-        if (w->scales_t.alloc(t.size() * 4) != cudaSuccess) return EOQ_ERR_ALLOC;
-        CU_TRY(cudaMemcpy(w->scales_t.p, t.data(), t.size() * 4, cudaMemcpyHostToDevice));
+        w->scales_t.p = base + at_scales_t;
+        w->pair_partials.p = base + at_partials;
+        CU_TRY(cudaMemsetAsync(w->pair_partials.p, 0xFF, w->pair_partial_bytes, nullptr));
+        if (launch_transpose_scales(w->scales.as<uint16_t>(), w->scales_t.as<uint2>(), tw.N, sg, triples, nullptr) != 0) return EOQ_ERR_CUDA;
     }
-    CU_TRY(cudaMemset(w->counters.p, 0, (size_t)tw.nrb * 4));
-    CU_TRY(cudaMemset(w->status.p, 0, 4));
-    CU_TRY(cudaMallocHost(reinterpret_cast<void **>(&w->status_host), 64));
-    std::memset(w->status_host, 0, 64);
-    CU_TRY(cudaHostGetDevicePointer(reinterpret_cast<void **>(&w->status_dev), w->status_host, 0));
+    CU_TRY(cudaMemsetAsync(w->counters.p, 0, (size_t)tw.nrb * 4, nullptr));
+    CU_TRY(StatusWords::take(&w->status_host, &w->status_dev));
+    CU_TRY(cudaStreamSynchronize(nullptr));            // what the weight holds is there for every stream
     *out = w.release();
     return EOQ_OK;
 }
@@ -921,7 +1207,7 @@ static eoq_error_t build_tiled_device(const uint8_t *d_sym, const eoq_b200_weigh
     }
     rc = tiled_layout(tw, stream_bytes);
     if (rc != EOQ_OK) return rc;
-    if (stream.alloc(stream_bytes) != cudaSuccess) return EOQ_ERR_ALLOC;
+    if (stream.alloc_pooled(stream_bytes) != cudaSuccess) return EOQ_ERR_ALLOC;
     CU_TRY(cudaMemsetAsync(stream.p, 0, stream_bytes, st));
     CU_TRY(cudaMemcpyAsync(d + at_tiles, tw.tiles.data(), ntiles * sizeof(TileDesc), cudaMemcpyHostToDevice, st));
     TileScatterArgs sa = {};
@@ -1380,6 +1666,11 @@ extern "C" eoq_error_t eoq_b200_gemv_host_async(eoq_b200_weight_t *w, const void
     if (drc != EOQ_OK) return drc;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     std::lock_guard<std::mutex> lock(w->mu);
+    if (!w->xbuf.p && (w->xbuf.alloc((size_t)8 * w->K * 4) != cudaSuccess || w->ybuf.alloc((size_t)8 * w->N * 4) != cudaSuccess ||
+                       w->biasbuf.alloc((size_t)w->N * 4) != cudaSuccess)) {
+        for (DeviceBuf *b : {&w->xbuf, &w->ybuf, &w->biasbuf}) if (b->p) { cudaFree(b->p); b->p = nullptr; }
+        return EOQ_ERR_ALLOC;
+    }
     CU_TRY(cudaMemcpyAsync(w->xbuf.p, x, (size_t)batch * w->K * esz[x_dtype], cudaMemcpyHostToDevice, st));
     if (bias_host) CU_TRY(cudaMemcpyAsync(w->biasbuf.p, bias_host, (size_t)w->N * 4, cudaMemcpyHostToDevice, st));
     // A pinned (page-locked) y is device-addressable: the kernel then stores its results straight into it and the

@@ -89,8 +89,9 @@ eoq_error_t normalize_reference(const uint32_t *raw, uint32_t alphabet, uint32_t
 void encode_block_v1(const uint32_t *freq, const uint32_t *cdf, uint32_t p,
                      const uint32_t *syms, uint32_t n, std::vector<uint8_t> &out);
 
-// fn(0) ... fn(n - 1) on the host's cores (at most 64 threads, joined before it returns).
-void parallel_for(size_t n, const std::function<void(size_t)> &fn);
+// fn(0) ... fn(n - 1) on the host's cores (at most `threads`, 0: as many as there are, up to 64; the caller's among them;
+// joined before it returns).
+void parallel_for(size_t n, const std::function<void(size_t)> &fn, size_t threads = 0);
 
 // The pieces of build_tiled that do not touch the symbols, shared with the device-side tile encoder: geometry
 // (padded rows, row blocks, column segments, tile descriptors without sizes), joint-symbol frequencies and decode table
@@ -272,5 +273,7 @@ int launch_tile_hist(const uint8_t *sym, uint32_t N, uint32_t K, uint32_t Npad, 
                      void *stream);
 int launch_tile_encode(const TileEncodeArgs &a, void *stream);
 int launch_tile_scatter(const TileScatterArgs &a, void *stream);
+// [N][groups] fp16 scales to [groups][triples] words {s0 | s1 << 16, s2} of three rows each, zero for rows past N
+int launch_transpose_scales(const uint16_t *scales, uint2 *out, uint32_t N, uint32_t groups, uint32_t triples, void *stream);
 
 }  // namespace eoq

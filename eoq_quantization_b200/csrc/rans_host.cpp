@@ -135,16 +135,15 @@ static eoq_error_t normalize_joint(const std::vector<uint64_t> &count, uint32_t 
     return EOQ_OK;
 }
 
-void parallel_for(size_t n, const std::function<void(size_t)> &fn)
+void parallel_for(size_t n, const std::function<void(size_t)> &fn, size_t threads)
 {
-    unsigned hw = std::thread::hardware_concurrency();
-    size_t nt = std::min<size_t>(hw ? hw : 4, std::max<size_t>(n, 1));
-    nt = std::min<size_t>(nt, 64);
-    if (nt <= 1) { for (size_t i = 0; i < n; i++) fn(i); return; }
+    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t nt = std::min<size_t>({threads ? threads : std::min<size_t>(hw, 64), n});
     std::atomic<size_t> next(0);
+    auto work = [&] { for (size_t i; (i = next.fetch_add(1)) < n;) fn(i); };
     std::vector<std::thread> pool;
-    for (size_t t = 0; t < nt; t++)
-        pool.emplace_back([&] { for (size_t i; (i = next.fetch_add(1)) < n;) fn(i); });
+    for (size_t t = 1; t < nt; t++) pool.emplace_back(work);
+    work();
     for (auto &t : pool) t.join();
 }
 

@@ -22,6 +22,9 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <cstring>
+#include <vector>
+
 #include "../../include/eoq_b200.h"
 
 namespace {
@@ -184,7 +187,147 @@ PyObject *polar_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
     GUARD_END
 }
 
+// -- codec ---------------------------------------------------------------------
+
+// A C-contiguous buffer for as long as it is in scope.
+struct Buffer {
+    Py_buffer v;
+    bool ok;
+    explicit Buffer(PyObject *o, bool writable = false) : ok(PyObject_GetBuffer(o, &v, writable ? PyBUF_CONTIG : PyBUF_CONTIG_RO) == 0) {}
+    Buffer(const Buffer &) = delete;
+    Buffer &operator=(const Buffer &) = delete;
+    ~Buffer() { if (ok) PyBuffer_Release(&v); }
+};
+
+PyObject *codec_error(eoq_error_t rc) { return PyLong_FromLong((long)rc); }      // the caller raises EOQError of it
+
+// count_symbols(array, type, shift, clamp, alphabet) -> ([counts], least, greatest) or an error code
+PyObject *count_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
+{
+    if (n != 5) { PyErr_SetString(PyExc_TypeError, "count_symbols takes 5 arguments"); return nullptr; }
+    GUARD_BEGIN
+    Buffer sym(a[0]);
+    if (!sym.ok) return nullptr;
+    const int type = (int)PyLong_AsLong(a[1]), clamp = (int)PyLong_AsLong(a[3]);
+    const int64_t shift = PyLong_AsLongLong(a[2]), alphabet = PyLong_AsLongLong(a[4]);
+    if (PyErr_Occurred()) return nullptr;
+    if (alphabet < 1 || alphabet > (1 << 20)) return codec_error(EOQ_ERR_UNSUPPORTED);
+    std::vector<uint64_t> counts((size_t)alphabet);
+    int64_t range[2];
+    eoq_error_t rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = eoq_b200_count_symbols(sym.v.buf, type, (size_t)(sym.v.len / sym.v.itemsize), shift, clamp, (uint32_t)alphabet, counts.data(), range);
+    Py_END_ALLOW_THREADS
+    if (rc != EOQ_OK) return codec_error(rc);
+    PyObject *list = PyList_New((Py_ssize_t)alphabet);
+    if (!list) return nullptr;
+    for (int64_t s = 0; s < alphabet; s++) PyList_SET_ITEM(list, s, PyLong_FromUnsignedLongLong(counts[(size_t)s]));
+    return Py_BuildValue("NLL", list, (long long)range[0], (long long)range[1]);
+    GUARD_END
+}
+
+// encode_symbols(array, type, shift, clamp, freq, precision, block_size, head, table): with head None (bytes, [offsets]), else the
+// container in one piece: head, u32 data size, table, u32 offsets, data; or an error code.
+PyObject *encode_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
+{
+    if (n != 9) { PyErr_SetString(PyExc_TypeError, "encode_symbols takes 9 arguments"); return nullptr; }
+    GUARD_BEGIN
+    Buffer sym(a[0]);
+    if (!sym.ok) return nullptr;
+    Buffer freq(a[4]);
+    if (!freq.ok) return nullptr;
+    const int type = (int)PyLong_AsLong(a[1]), clamp = (int)PyLong_AsLong(a[3]);
+    const int64_t shift = PyLong_AsLongLong(a[2]), p = PyLong_AsLongLong(a[5]), block = PyLong_AsLongLong(a[6]);
+    if (PyErr_Occurred()) return nullptr;
+    const int64_t count = sym.v.len / sym.v.itemsize, alphabet = freq.v.len / 4;
+    if (count < 1 || count > 0xFFFFFFFFll || block < 1 || block > 0xFFFFFFFFll || p < 1 || p > 16) return codec_error(EOQ_ERR_UNSUPPORTED);
+    eoq_b200_wire_t *w = nullptr;
+    size_t bytes = 0;
+    eoq_error_t rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = eoq_b200_wire_encode(sym.v.buf, type, (uint32_t)count, shift, clamp, static_cast<const uint32_t *>(freq.v.buf), (uint32_t)alphabet, (uint32_t)p,
+                              (uint32_t)block, &w, &bytes);
+    Py_END_ALLOW_THREADS
+    if (rc != EOQ_OK) return codec_error(rc);
+    const int64_t nb = (count + block - 1) / block;
+    if (a[7] == Py_None) {
+        PyObject *data = PyBytes_FromStringAndSize(nullptr, (Py_ssize_t)bytes);
+        PyObject *list = data ? PyList_New((Py_ssize_t)nb) : nullptr;
+        if (!list) { Py_XDECREF(data); eoq_b200_wire_take(w, nullptr, nullptr); return nullptr; }
+        std::vector<uint32_t> offs((size_t)nb);
+        uint8_t *to = reinterpret_cast<uint8_t *>(PyBytes_AS_STRING(data));
+        Py_BEGIN_ALLOW_THREADS
+        eoq_b200_wire_take(w, to, offs.data());
+        Py_END_ALLOW_THREADS
+        for (int64_t b = 0; b < nb; b++) PyList_SET_ITEM(list, b, PyLong_FromUnsignedLong(offs[(size_t)b]));
+        return Py_BuildValue("NN", data, list);
+    }
+    // container: head, data size, table, offsets, data
+    Buffer head(a[7]), table(a[8]);
+    if (!head.ok || !table.ok) { eoq_b200_wire_take(w, nullptr, nullptr); return nullptr; }
+    const size_t at_table = (size_t)head.v.len + 4, at_offs = at_table + (size_t)table.v.len, at_data = at_offs + 4 * (size_t)nb;
+    PyObject *whole = PyBytes_FromStringAndSize(nullptr, (Py_ssize_t)(at_data + bytes));
+    if (!whole) { eoq_b200_wire_take(w, nullptr, nullptr); return nullptr; }
+    uint8_t *to = reinterpret_cast<uint8_t *>(PyBytes_AS_STRING(whole));
+    const uint32_t size32 = (uint32_t)bytes;
+    std::memcpy(to, head.v.buf, (size_t)head.v.len);
+    std::memcpy(to + head.v.len, &size32, 4);
+    std::memcpy(to + at_table, table.v.buf, (size_t)table.v.len);
+    std::vector<uint32_t> offs((size_t)nb);
+    Py_BEGIN_ALLOW_THREADS
+    eoq_b200_wire_take(w, to + at_data, offs.data());
+    std::memcpy(to + at_offs, offs.data(), 4 * (size_t)nb);
+    Py_END_ALLOW_THREADS
+    return whole;
+    GUARD_END
+}
+
+// decode_symbols(freq, precision, data, offsets (list or u32 buffer), block_size, out, out_type, shift) -> None or an error code
+PyObject *decode_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
+{
+    if (n != 8) { PyErr_SetString(PyExc_TypeError, "decode_symbols takes 8 arguments"); return nullptr; }
+    GUARD_BEGIN
+    Buffer freq(a[0]);
+    if (!freq.ok) return nullptr;
+    Buffer data(a[2]);
+    if (!data.ok) return nullptr;
+    Buffer out(a[5], true);
+    if (!out.ok) return nullptr;
+    const int64_t p = PyLong_AsLongLong(a[1]), block = PyLong_AsLongLong(a[4]), shift = PyLong_AsLongLong(a[7]);
+    const int type = (int)PyLong_AsLong(a[6]);
+    if (PyErr_Occurred()) return nullptr;
+    std::vector<uint32_t> offs;
+    if (PyList_CheckExact(a[3])) {
+        const Py_ssize_t nb = PyList_GET_SIZE(a[3]);
+        offs.resize((size_t)nb);
+        for (Py_ssize_t b = 0; b < nb; b++) {
+            const int64_t v = PyLong_AsLongLong(PyList_GET_ITEM(a[3], b));
+            if (v == -1 && PyErr_Occurred()) return nullptr;
+            if (v < 0 || v > 0xFFFFFFFFll) { PyErr_SetString(PyExc_OverflowError, "block offset out of bounds for a 32-bit number"); return nullptr; }
+            offs[(size_t)b] = (uint32_t)v;
+        }
+    } else {
+        Buffer o(a[3]);
+        if (!o.ok) return nullptr;
+        offs.assign(static_cast<const uint32_t *>(o.v.buf), static_cast<const uint32_t *>(o.v.buf) + o.v.len / 4);
+    }
+    const int64_t count = out.v.len / out.v.itemsize;
+    if (count > 0xFFFFFFFFll || block < 1 || block > 0xFFFFFFFFll || p < 1 || p > 16) return codec_error(EOQ_ERR_UNSUPPORTED);
+    eoq_error_t rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = eoq_b200_decode_blocked_as(static_cast<const uint32_t *>(freq.v.buf), (uint32_t)(freq.v.len / 4), (uint32_t)p,
+                                    static_cast<const uint8_t *>(data.v.buf), (size_t)data.v.len, offs.data(), (uint32_t)offs.size(),
+                                    (uint32_t)block, (uint32_t)count, out.v.buf, type, shift, nullptr);
+    Py_END_ALLOW_THREADS
+    if (rc != EOQ_OK) return codec_error(rc);
+    Py_RETURN_NONE;
+    GUARD_END
+}
+
 PyMethodDef methods[] = {
+    {"count_symbols", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(count_symbols)), METH_FASTCALL, nullptr},
+    {"encode_symbols", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(encode_symbols)), METH_FASTCALL, nullptr},
+    {"decode_symbols", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(decode_symbols)), METH_FASTCALL, nullptr},
     {"weight_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(weight_linear)), METH_FASTCALL, nullptr},
     {"packed_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(packed_linear)), METH_FASTCALL, nullptr},
     {"polar_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(polar_linear)), METH_FASTCALL, nullptr},

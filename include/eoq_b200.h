@@ -205,12 +205,37 @@ eoq_error_t eoq_b200_decode_blocked(const uint32_t *freq, uint32_t alphabet, uin
                                     uint32_t num_blocks, uint32_t block_size, uint32_t num_symbols,
                                     void *out, int out_elem_bytes, int out_on_device, void *stream);
 
+/* The same with a host array of another integer type as the result: out[i] = (type)(symbol + shift), out_type one of
+ * EOQ_B200_SYM_* below (not U32). */
+eoq_error_t eoq_b200_decode_blocked_as(const uint32_t *freq, uint32_t alphabet, uint32_t precision_bits, const uint8_t *data,
+                                       size_t data_len, const uint32_t *offsets, uint32_t num_blocks, uint32_t block_size,
+                                       uint32_t num_symbols, void *out, int out_type, int64_t shift, void *stream);
+
 /* Host encoder behind core/rans_blocked.py:72-114 (wire-compatible with
  * core/rans.py:210-276).  Writes blocks back to back into `out` and their
  * offsets into `offsets`; *out_len in = capacity, out = bytes used. */
 eoq_error_t eoq_b200_encode_blocked(const uint32_t *freq, uint32_t alphabet, uint32_t precision_bits,
                                     const uint32_t *symbols, uint32_t num_symbols, uint32_t block_size,
                                     uint8_t *out, size_t *out_len, uint32_t *offsets);
+
+/* The same encoder on symbols of any integer type, without a copy of the array.  A symbol is value + shift.
+ * count_symbols: histogram over `alphabet` symbols; with `clamp` values outside go to the nearest end
+ * (core/rans_bitpacked.py:95), else they are left out and range[0..1] tells the least and greatest symbol seen.
+ * wire_encode: blocks of `block_size` (precision up to 16; a symbol out of range without `clamp`: CORRUPT_STREAM), *bytes in all;
+ * wire_take writes the blocks back to back and every block's offset, and frees the handle (also with null pointers). */
+#define EOQ_B200_SYM_I8 0
+#define EOQ_B200_SYM_U8 1
+#define EOQ_B200_SYM_I16 2
+#define EOQ_B200_SYM_U16 3
+#define EOQ_B200_SYM_I32 4
+#define EOQ_B200_SYM_U32 5
+#define EOQ_B200_SYM_I64 6
+typedef struct eoq_b200_wire eoq_b200_wire_t;
+eoq_error_t eoq_b200_count_symbols(const void *symbols, int elem, size_t n, int64_t shift, int clamp, uint32_t alphabet,
+                                   uint64_t *counts, int64_t *range);
+eoq_error_t eoq_b200_wire_encode(const void *symbols, int elem, uint32_t n, int64_t shift, int clamp, const uint32_t *freq,
+                                 uint32_t alphabet, uint32_t precision_bits, uint32_t block_size, eoq_b200_wire_t **out, size_t *bytes);
+void eoq_b200_wire_take(eoq_b200_wire_t *w, uint8_t *data, uint32_t *offsets);
 
 /* A weight matrix resident in HBM as entropy-coded tiles. */
 typedef struct eoq_b200_weight eoq_b200_weight_t;
