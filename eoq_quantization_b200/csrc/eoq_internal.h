@@ -235,6 +235,26 @@ void set_dequant_vec(int v);
 int launch_gemv_packed(const PackedGemvArgs &a, void *stream);
 int launch_dequant_packed(const uint8_t *packed, const uint16_t *scales, uint32_t K, uint32_t row_bytes, uint32_t bits,
                           uint32_t group, uint32_t row_lo, uint32_t row_hi, void *out, int out_dtype, void *stream);
+// Activations x quantised weights on the tensor cores (qmm.cu).  x: [M][K] of 16-bit values, or with split_x two fp16
+// planes [2][M][K] (nearest, then nearest to the remainder) times tok_scale[m] (or 1).  centroids: PolarLinear's byte codes.
+struct QmmCall {
+    const uint8_t *packed;
+    const uint16_t *scales;
+    const float *centroids, *tok_scale;
+    const void *bias;            // [N] fp32, or fp16 with bias_half
+    const void *x;
+    void *y;
+    uint32_t N, K, M, bits, group;
+    int bf16, split_x, y_dtype, bias_half, late;     // late: `packed` is written by the kernel before this one in the stream
+    uint32_t blocked_rows;       // not 0: 4-bit codes as [K / 16][blocked_rows] words of sixteen, as the decoder leaves them
+};
+bool qmm_takes(uint32_t K, uint32_t bits, uint32_t group, const void *packed, const void *x);
+int launch_qmm(const QmmCall &c, void *stream);
+bool qmm_preferred(const QmmCall &c, double copy_us);
+uint32_t qmm_status();
+bool split_rows_takes(uint32_t K, uint32_t block);
+int launch_split_rows(const void *x, int x_dtype, uint32_t K, uint32_t M, uint32_t block, void *planes, float *tok_scale, void *stream);
+void count_launch();
 int launch_gemm_tc(const uint32_t *table, const TileDesc *tiles, const uint8_t *stream, const uint2 *scales_t, const void *x,
                    void *xhalf, float *partials, uint32_t *counters, void *y, const float *bias, uint32_t *status, uint32_t N,
                    uint32_t K, uint32_t group, uint32_t p, uint32_t nseg, uint32_t nrb, uint32_t head_bytes, uint32_t M, int x_dtype, int y_dtype,

@@ -23,6 +23,8 @@ namespace eoq {
 static std::atomic<uint64_t> g_launches{0};
 uint64_t launch_counter() { return g_launches.load(); }
 
+void count_launch() { g_launches++; }
+
 int device_sm_count()
 {
     int dev = 0, sms = 0;

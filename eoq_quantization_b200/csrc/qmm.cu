@@ -210,3 +210,755 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16])
                  : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
                    "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]) :: "memory");
 }
+
+struct QmmArgs {
+    const uint16_t *scales;      // [N][K / group] fp16 (polar: norms)
+    const float *centroids;      // polar: `entries` of them
+    const void *bias;            // [N] fp32 (bias_half: fp16), or null
+    const float *tok_scale;      // [M] factor of every activation row, or null
+    void *y;                     // [M][N]
+    uint32_t N, K, M, T, group, sgroups, seg, units, split, planes, entries;
+    uint32_t nw, ns, a_base;     // stages of packed weights and of operands (A in TMEM, activations in shared memory); first A column
+    uint32_t at_x, at_bar;       // shared-memory offsets
+    int y_dtype, bias_half, late;   // late: the packed codes are the previous kernel's to write
+};
+
+template <int BITS, int KB>
+struct Unit {                    // what one weight copy brings: 128 rows of kBytes, in blocks of KB columns (a stage of operands)
+    static constexpr uint32_t kBytes = BITS == 2 ? 64u : 128u;
+    static constexpr uint32_t kCols = BITS == 2 || BITS == 4 || BITS == kBlocked4 ? 256u : 128u;
+    static constexpr uint32_t kBlocks = kCols / KB;
+    static constexpr uint32_t kStage = kRows * kBytes;
+    static constexpr int kWords = BITS == 4 || BITS == kBlocked4 ? 8 : BITS == 2 ? 4 : 16;       // words of one row and 64 columns
+};
+
+// Position in a ring of n stages and the parity of its current lap.
+struct Ring {
+    uint32_t at = 0, lap = 0;
+    __device__ __forceinline__ void next(uint32_t n) { if (++at == n) { at = 0; lap ^= 1u; } }
+};
+
+// barriers, in this order, eight bytes each
+enum { kWFull = 0, kWEmpty = 8, kFull = 16, kEmpty = 24, kDFull = 32, kDEmpty = 34, kSFull = 36, kSEmpty = 40, kTmemSlot = 44 };
+constexpr uint32_t kScaleRing = 4, kScaleGroups = 8, kScaleEntry = kScaleGroups * kRows * 2u;      // scales of 8 groups x 128 rows an entry
+
+// The scales of one weight row in the order of the groups, out of the ring that a warp of the CTA keeps filled.
+struct ScaleReader {
+    uint32_t full, empty, at, row, entry = 0;      // barrier addresses, ring address
+    Ring ring;
+    bool here = false;                             // this entry has been waited for
+    __device__ __forceinline__ uint16_t get(uint32_t g, uint32_t lane)      // g: group, counted from the CTA's first
+    {
+        while ((g >> 3) > entry) {
+            __syncwarp();
+            if (lane == 0) bar_arrive(empty + 8u * ring.at);
+            ring.next(kScaleRing);
+            entry++;
+            here = false;
+        }
+        if (!here) { bar_wait(full + 8u * ring.at, ring.lap); here = true; }
+        uint16_t v;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(at + ring.at * kScaleEntry + (g & 7u) * (kRows * 2u) + row * 2u));
+        return v;
+    }
+};
+
+template <int BITS, bool BF16, bool FOLD, int NP, int NF, int TC, int KB>
+__global__ void __launch_bounds__((4 * NP + 4 * NF + 4) * 32, 1)
+qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap)
+{
+    using U = Unit<BITS, KB>;
+    constexpr bool kPol = BITS == kPolar;
+    constexpr int kCode = kPol ? 8 : BITS == kBlocked4 ? 4 : BITS;
+    constexpr uint32_t kHalves = KB / 64;                         // 64-column parts of a block
+    constexpr uint32_t kACols = (kPol ? 64u : 32u) * kHalves;     // TMEM columns of a block (polar: high and low halves)
+    constexpr uint32_t kB16 = KB / 16;                            // products (K = 16) of a block
+    constexpr uint32_t kTmem = 512u;
+    extern __shared__ uint8_t raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(raw) + 1023u) & ~(uintptr_t)1023u);
+    const uint32_t base = saddr(smem), bars = base + a.at_bar;
+    auto bar = [&](uint32_t i) { return bars + 8u * i; };
+    const uint32_t scale_ring = bars + 512u;
+    uint32_t *table = reinterpret_cast<uint32_t *>(smem + a.at_bar + 512 + kScaleRing * kScaleEntry);      // polar: centroids as {high half, low half}
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;       // the same in all lanes, and known to be
+    const uint32_t rank = blockIdx.x % a.split, row0 = blockIdx.x / a.split * kRows, tok0 = blockIdx.y * a.T;
+    const uint32_t u0 = (uint32_t)((uint64_t)a.units * rank / a.split), u1 = (uint32_t)((uint64_t)a.units * (rank + 1) / a.split);
+    const uint32_t kb0 = u0 * U::kBlocks, nkb = min(u1 * U::kBlocks, (a.K + KB - 1) / KB) - kb0;
+    const uint32_t k16_0 = kb0 * kB16, k16_n = min((kb0 + nkb) * kB16, a.K / 16u), g16 = a.group / 16u;
+    const uint32_t grp0 = k16_0 / g16, ngroups = (k16_n - 1u) / g16 - grp0 + 1u;
+    // fold: an accumulator runs over `seg` columns, a group or an equal part of a long one (of 128 at most: the tensor cores
+    // round each addition towards zero, which 1024 columns of byte codes show: 2e-6 against 3e-7)
+    const uint32_t f16 = a.seg / 16u, seg0 = k16_0 / f16, nseg = (k16_n - 1u) / f16 - seg0 + 1u;
+    const uint32_t plane = a.T * 128u * kHalves, xstage = plane * a.planes;
+
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (threadIdx.x == 0) {
+        for (uint32_t i = 0; i < 8; i++) {
+            bar_init(bar(kWFull + i), 1); bar_init(bar(kWEmpty + i), 4 * U::kBlocks);
+            bar_init(bar(kFull + i), 5); bar_init(bar(kEmpty + i), 1);          // four producer warps and the activation copy
+        }
+        for (uint32_t i = 0; i < kScaleRing; i++) { bar_init(bar(kSFull + i), 1); bar_init(bar(kSEmpty + i), 4 * (FOLD ? NF : NP)); }
+        for (uint32_t i = 0; i < 2; i++) { bar_init(bar(kDFull + i), 1); bar_init(bar(kDEmpty + i), 4 * NF); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (kPol) {
+        for (uint32_t i = threadIdx.x; i < a.entries; i += blockDim.x) {
+            const float c = __ldg(a.centroids + i);
+            const __half hi = __float2half_rn(c), lo = __float2half_rn(c - __half2float(hi));
+            table[i] = __half_as_ushort(hi) | ((uint32_t)__half_as_ushort(lo) << 16);
+        }
+    }
+    __syncwarp();
+    if (warp == 4 * NP + 4 * NF) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(bar(kTmemSlot)), "n"(kTmem) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    // all 512 columns are this CTA's, so they start at column 0: addresses below are constants plus offsets
+    constexpr uint32_t tmem = 0;
+
+    if (warp < 4 * NP) {
+        // ---- producers: packed codes of one row, a block of columns at a time, to the A operand in tensor memory
+        const uint32_t set = warp >> 2, r = (warp & 3u) * 32u + lane;
+        const uint32_t lane_base = tmem + (((warp & 3u) * 32u) << 16) + a.a_base;
+        const uint32_t tab_addr = saddr(table), tab_mask = (a.entries - 1u) << 2;
+        // scaled: the groups of 32-column parts, counted along
+        ScaleReader sr{bar(kSFull), bar(kSEmpty), scale_ring, r};
+        uint32_t gi = 0, pos = 0;
+        if (!FOLD) {
+            const uint32_t c = (kb0 + set) * KB;
+            gi = c / a.group; pos = c - gi * a.group; gi -= grp0;
+        }
+        Ring wr, ar;
+        uint32_t unit = 0;
+        for (uint32_t j = 0; j < set; j++) ar.next(a.ns);
+        for (uint32_t i = set; i < nkb; i += NP) {
+            const uint32_t q = i % U::kBlocks, st = ar.at;
+            for (; unit < i / U::kBlocks; unit++) wr.next(a.nw);
+            const uint32_t ws = wr.at, row_at = base + ws * U::kStage + r * U::kBytes;
+            const uint32_t sw = BITS == 2 ? (r >> 1) & 3u : r & 7u;
+            bar_wait(bar(kWFull + ws), wr.lap);
+#pragma unroll
+            for (uint32_t part = 0; part < kHalves; part++) {
+                uint32_t w[U::kWords];
+                if (BITS == kBlocked4) {
+#pragma unroll
+                    for (uint32_t c = 0; c < U::kWords / 2; c++)
+                        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(w[2 * c]), "=r"(w[2 * c + 1])
+                                     : "r"(base + ws * U::kStage + ((q * kHalves + part) * 4u + c) * (kRows * 8u) + r * 8u));
+                }
+#pragma unroll
+                for (uint32_t c = 0; c < (BITS == kBlocked4 ? 0u : U::kWords / 4); c++) {
+                    const uint32_t at = row_at + ((((q * kHalves + part) * (U::kWords / 4) + c) ^ sw) << 4);
+                    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[4 * c]), "=r"(w[4 * c + 1]), "=r"(w[4 * c + 2]), "=r"(w[4 * c + 3]) : "r"(at));
+                }
+                uint32_t h[32], lo[kPol ? 32 : 1];
+                if (kPol) {
+#pragma unroll
+                    for (int c = 0; c < 16; c++) {
+                        uint32_t e[4];
+#pragma unroll
+                        for (int b = 0; b < 4; b++) {
+                            const uint32_t off = (b == 0 ? w[c % U::kWords] << 2 : w[c % U::kWords] >> (8 * b - 2)) & tab_mask;
+                            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(e[b]) : "r"(tab_addr + off));
+                        }
+#pragma unroll
+                        for (int b = 0; b < 2; b++) {
+                            h[2 * c + b] = __byte_perm(e[2 * b], e[2 * b + 1], 0x5410u);
+                            lo[kPol ? 2 * c + b : 0] = __byte_perm(e[2 * b], e[2 * b + 1], 0x7632u);
+                        }
+                    }
+                } else if (FOLD) {
+#pragma unroll
+                    for (int c = 0; c < U::kWords; c++) codes_exact<kCode, BF16>(w[c], h + c * (32 / U::kWords));
+                } else {
+                    const uint16_t s0 = sr.get(gi, lane);
+                    const bool other = pos + 32u >= a.group && (kb0 + i) * KB + part * 64u + 32u < a.K;
+                    const uint16_t s1 = other ? sr.get(gi + 1u, lane) : s0;
+                    for (pos += part + 1 == kHalves ? 64u + KB * (NP - 1) : 64u; pos >= a.group; pos -= a.group) gi++;
+#pragma unroll
+                    for (int c = 0; c < U::kWords; c++) codes_scaled<kCode, BF16>(w[c], h + c * (32 / U::kWords), c < U::kWords / 2 ? s0 : s1);
+                }
+                if (part == 0) {
+                    bar_wait(bar(kEmpty + st), ar.lap ^ 1u);
+                    fence_after();
+                }
+                __syncwarp();
+                tmem_st32(lane_base + st * kACols + part * 32u, h);
+                if constexpr (kPol) tmem_st32(lane_base + st * kACols + (kHalves + part) * 32u, lo);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            fence_before();
+            __syncwarp();
+            // every lane's codes are in its registers, converted and stored: only now may the copy engine have the stage
+            // (an arrival straight behind the shared-memory loads let it overwrite rows that were still on their way)
+            if (lane == 0) { bar_arrive(bar(kFull + st)); bar_arrive(bar(kWEmpty + ws)); }
+#pragma unroll
+            for (int j = 0; j < NP; j++) ar.next(a.ns);
+        }
+    } else if (warp < 4 * NP + 4 * NF) {
+        // ---- readers: accumulators to fp32 totals (fold) and totals to shared memory, [token][row]
+        const uint32_t set = (warp - 4 * NP) >> 2, r = (warp & 3u) * 32u + lane, cols = a.T / NF;
+        const uint32_t lane_base = tmem + (((warp & 3u) * 32u) << 16) + set * cols;
+        float *stage = reinterpret_cast<float *>(smem) + (size_t)set * cols * kRows + r;
+        if (FOLD) {
+            ScaleReader sr{bar(kSFull), bar(kSEmpty), scale_ring, r};
+            float tot[TC];
+#pragma unroll
+            for (int c = 0; c < TC; c++) tot[c] = 0.0f;
+            uint32_t g = 0, in_group = seg0 - grp0 * (g16 / f16);           // segments of group g that are behind
+            for (uint32_t s = 0; s < nseg; s++) {
+                const float sc = __half2float(__ushort_as_half(sr.get(g, lane)));
+                if (++in_group == g16 / f16) { in_group = 0; g++; }
+                bar_wait(bar(kDFull + (s & 1u)), (s >> 1) & 1u);
+                __syncwarp();
+                fence_after();
+#pragma unroll
+                for (int c = 0; c < TC; c += 32) {
+                    if ((uint32_t)c >= cols) break;
+                    uint32_t v[2][16];
+                    tmem_ld16(lane_base + (s & 1u) * a.T + c, v[0]);
+                    if (c + 16u < cols) tmem_ld16(lane_base + (s & 1u) * a.T + c + 16, v[1]);
+                    tmem_ld_wait(v[0]);
+                    tmem_ld_wait(v[1]);
+                    if (c + 32u >= cols) {              // the last read of this accumulator: the next segment may have it
+                        fence_before();
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(bar(kDEmpty + (s & 1u)));
+                    }
+#pragma unroll
+                    for (int j = 0; j < 16; j++) tot[c + j] = fmaf(sc, __uint_as_float(v[0][j]), tot[c + j]);
+                    if (c + 16u < cols) {
+#pragma unroll
+                        for (int j = 0; j < 16; j++) tot[c + 16 + j] = fmaf(sc, __uint_as_float(v[1][j]), tot[c + 16 + j]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < TC; c++)
+                if ((uint32_t)c < cols) stage[c * kRows] = tot[c];
+        } else {
+            bar_wait(bar(kDFull), 0u);
+            __syncwarp();
+            fence_after();
+            for (uint32_t c = 0; c < cols; c += 16) {
+                uint32_t v[16];
+                tmem_ld16(lane_base + c, v);
+                tmem_ld_wait(v);
+#pragma unroll
+                for (int j = 0; j < 16; j++) stage[(c + j) * kRows] = __uint_as_float(v[j]);
+            }
+            fence_before();
+        }
+    } else if (warp == 4 * NP + 4 * NF) {
+        // ---- products.  This warp's instructions are what a block costs when tokens are few: one barrier and one commit a
+        // block, and where segments are whole blocks, no tests between the products
+        const uint32_t idesc = (1u << 4) | (BF16 ? (1u << 7) | (1u << 10) : 0u) | ((a.T >> 3) << 17) | ((kRows >> 4) << 24);
+        const uint64_t desc0 = sw128_desc(base + a.at_x);
+        const bool whole = !FOLD || f16 % kB16 == 0;
+        const bool two = a.planes == 2;
+        const uint32_t half16 = (a.T * 128u) >> 4;                 // the second 64 columns of a plane, in descriptor units
+        uint32_t seg = 0, in_seg = k16_0 - seg0 * f16, acc = 0, d = tmem;
+        Ring ar;
+        for (uint32_t i = 0; i < nkb; i++) {
+            bar_wait(bar(kFull + ar.at), ar.lap);
+            fence_after();
+            const uint32_t at = tmem + a.a_base + ar.at * kACols, left = k16_n - (kb0 + i) * kB16;
+            const uint64_t desc = desc0 + ((ar.at * xstage) >> 4);
+            auto product = [&](uint32_t j) {
+                const uint64_t b = desc + (j / 4u) * half16 + (j & 3u) * 2u;
+                mma_ts(d, at + j * 8u, b, idesc, acc);
+                acc = 1;
+                if (two) mma_ts(d, at + j * 8u, b + (plane >> 4), idesc, 1u);
+                if (kPol) mma_ts(d, at + kHalves * 32u + j * 8u, b, idesc, 1u);
+            };
+            auto open = [&]() {
+                d = tmem + (seg & 1u) * a.T;
+                bar_wait(bar(kDEmpty + (seg & 1u)), ((seg >> 1) & 1u) ^ 1u);
+                fence_after();
+            };
+            auto close = [&]() {
+                mma_commit(bar(kDFull + (seg & 1u)));
+                seg++; in_seg = 0; acc = 0;
+            };
+            if (whole && left >= kB16) {
+                if (FOLD && acc == 0) open();
+#pragma unroll
+                for (uint32_t j = 0; j < kB16; j++) product(j);
+                in_seg += kB16;
+                if (FOLD && (in_seg == f16 || left == kB16)) close();
+            } else {
+                // segments are multiples of 32 columns: their ends fall between pairs of products
+#pragma unroll
+                for (uint32_t j = 0; j < kB16; j += 2) {
+                    if (j >= left) break;
+                    if (FOLD && acc == 0) open();
+                    product(j);
+                    product(j + 1);
+                    in_seg += 2;
+                    if (FOLD && (in_seg == f16 || j + 2 >= left)) close();
+                }
+            }
+            mma_commit(bar(kEmpty + ar.at));
+            ar.next(a.ns);
+        }
+        if (!FOLD) mma_commit(bar(kDFull));
+    } else if (warp == 4 * NP + 4 * NF + 1) {
+        // ---- weight copies: a resident weight depends on nothing that came before in the stream
+        const bool leader = elect();
+        if (a.late) asm volatile("griddepcontrol.wait;" ::: "memory");
+        Ring wr;
+        for (uint32_t u = u0; u < u1; u++) {
+            bar_wait(bar(kWEmpty + wr.at), wr.lap ^ 1u);
+            if (leader) {
+                bar_expect(bar(kWFull + wr.at), U::kStage);
+                if (BITS == kBlocked4) tma_2d(base + wr.at * U::kStage, &wmap, row0, u * (U::kCols / 16), bar(kWFull + wr.at));
+                else tma_2d(base + wr.at * U::kStage, &wmap, u * U::kBytes, row0, bar(kWFull + wr.at));
+            }
+            __syncwarp();
+            wr.next(a.nw);
+        }
+    } else if (warp == 4 * NP + 4 * NF + 2) {
+        // ---- activation copies
+        const bool leader = elect();
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        Ring xr;
+        for (uint32_t i = 0; i < nkb; i++) {
+            bar_wait(bar(kEmpty + xr.at), xr.lap ^ 1u);
+            if (leader) {
+                bar_expect(bar(kFull + xr.at), xstage);
+                for (uint32_t p = 0; p < a.planes; p++)
+#pragma unroll
+                    for (uint32_t q = 0; q < kHalves; q++)
+                        tma_2d(base + a.at_x + xr.at * xstage + p * plane + q * a.T * 128u, &xmap, (kb0 + i) * KB + q * 64u, p * a.M + tok0, bar(kFull + xr.at));
+            }
+            __syncwarp();
+            xr.next(a.ns);
+        }
+    } else {
+        // ---- scales: eight groups of 128 rows at a time, transposed on the way ([group][row])
+        Ring sr;
+        for (uint32_t g0 = 0; g0 < ngroups; g0 += kScaleGroups) {
+            uint16_t v[4][kScaleGroups];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; j++) {
+                const uint16_t *srow = a.scales + (size_t)min(row0 + lane + 32u * j, a.N - 1u) * a.sgroups;
+#pragma unroll
+                for (uint32_t g = 0; g < kScaleGroups; g++) v[j][g] = __ldg(srow + min(grp0 + g0 + g, a.sgroups - 1u));
+            }
+            bar_wait(bar(kSEmpty + sr.at), sr.lap ^ 1u);
+            const uint32_t to = scale_ring + sr.at * kScaleEntry + lane * 2u;
+#pragma unroll
+            for (uint32_t j = 0; j < 4; j++)
+#pragma unroll
+                for (uint32_t g = 0; g < kScaleGroups; g++)
+                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(to + g * (kRows * 2u) + j * 64u), "h"(v[j][g]) : "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(bar(kSFull + sr.at));
+            sr.next(kScaleRing);
+        }
+    }
+    __syncwarp();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __syncthreads();
+    if (warp == 4 * NP + 4 * NF) {
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kTmem) : "memory");
+    }
+    cg::cluster_group cluster = cg::this_cluster();
+    if (a.split > 1) cluster.sync();
+    // totals of all the cluster's CTAs, four rows of a token at a time, this CTA's share of them
+    const float *mine = reinterpret_cast<const float *>(smem);
+    const bool vec = (a.N & 3u) == 0;
+    for (uint32_t e = rank * blockDim.x + threadIdx.x; e < a.T * 32u; e += blockDim.x * a.split) {
+        const uint32_t t = e >> 5, r = (e & 31u) * 4u, m = tok0 + t, n = row0 + r;
+        if (m >= a.M || n >= a.N) continue;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (a.split == 1) {
+            v = *reinterpret_cast<const float4 *>(mine + t * kRows + r);
+        } else {
+            // all of them requested before the first is added: a load from another SM takes some seven hundred cycles
+            float4 o[8];
+#pragma unroll
+            for (uint32_t k = 0; k < 8; k++)
+                o[k] = k < a.split ? *reinterpret_cast<const float4 *>(cluster.map_shared_rank(mine, k) + t * kRows + r) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+            for (uint32_t k = 0; k < 8; k++) { v.x += o[k].x; v.y += o[k].y; v.z += o[k].z; v.w += o[k].w; }
+        }
+        float o[4] = {v.x, v.y, v.z, v.w};
+        const float ts = a.tok_scale ? __ldg(a.tok_scale + m) : 1.0f;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float b = !a.bias || n + j >= a.N ? 0.0f
+                          : a.bias_half ? __half2float(reinterpret_cast<const __half *>(a.bias)[n + j]) : reinterpret_cast<const float *>(a.bias)[n + j];
+            o[j] = o[j] * ts + b;
+        }
+        const size_t at = (size_t)m * a.N + n;
+        if (a.y_dtype == EOQ_B200_F32) {
+            float *y = reinterpret_cast<float *>(a.y) + at;
+            if (vec) *reinterpret_cast<float4 *>(y) = make_float4(o[0], o[1], o[2], o[3]);
+            else for (int j = 0; j < 4; j++) if (n + j < a.N) y[j] = o[j];
+        } else {
+            uint32_t p[2];
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                if (a.y_dtype == EOQ_B200_F16) { const __half2 q = __floats2half2_rn(o[2 * j], o[2 * j + 1]); p[j] = *reinterpret_cast<const uint32_t *>(&q); }
+                else p[j] = pack_bf16(o[2 * j], o[2 * j + 1]);
+            }
+            uint16_t *y = reinterpret_cast<uint16_t *>(a.y) + at;
+            if (vec) *reinterpret_cast<uint2 *>(y) = make_uint2(p[0], p[1]);
+            else for (int j = 0; j < 4; j++) if (n + j < a.N) y[j] = (uint16_t)(p[j >> 1] >> (16 * (j & 1)));
+        }
+    }
+    if (a.split > 1) cluster.sync();               // nobody leaves while its totals are being read
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------------
+// Activations as two fp16 planes (the nearest fp16, then the nearest to the remainder: 22 bits), rotated first where the
+// weight is PolarLinear's: every block of 32 V columns times the normalised Hadamard matrix of that order (Sylvester
+// construction, core/polar_quant.py:104-120) over sqrt(block), a fast Walsh-Hadamard transform inside a warp.  A row is
+// brought to a largest magnitude of 2^14 .. 2^15 by a power of two, which goes to tok_scale inverted: the planes then hold
+// any fp32 row, large or small, with the same relative precision.  One CTA per row, the row in shared memory between
+// finding the largest value and writing the planes.
+// ---------------------------------------------------------------------------
+template <int V>
+__global__ void __launch_bounds__(512) split_rows_kernel(const void *__restrict__ x, int x_dtype, uint32_t K, uint32_t M, __half *__restrict__ planes,
+                                                         float *__restrict__ tok_scale)
+{
+    extern __shared__ float row[];
+    __shared__ float part[16];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, nwarps = blockDim.x >> 5, m = blockIdx.x;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    auto load = [&](uint32_t k) -> float {
+        const size_t i = (size_t)m * K + k;
+        if (x_dtype == EOQ_B200_F32) return __ldg(reinterpret_cast<const float *>(x) + i);
+        const uint16_t b = __ldg(reinterpret_cast<const uint16_t *>(x) + i);
+        return x_dtype == EOQ_B200_F16 ? __half2float(__ushort_as_half(b)) : __uint_as_float((uint32_t)b << 16);
+    };
+    float most = 0.0f;
+    if (V == 0) {
+        for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) {
+            const float v = load(k);
+            row[k] = v;
+            most = fmaxf(most, fabsf(v));
+        }
+    } else {
+        constexpr int kV = V ? V : 1;
+        for (uint32_t b = warp * 32u * kV; b < K; b += nwarps * 32u * kV) {
+            float v[kV];
+#pragma unroll
+            for (int j = 0; j < kV; j++) v[j] = load(b + 32u * j + lane);
+#pragma unroll
+            for (int h = 1; h < kV; h <<= 1)
+#pragma unroll
+                for (int j = 0; j < kV; j++)
+                    if (!(j & h)) { const float p = v[j], q = v[j | h]; v[j] = p + q; v[j | h] = p - q; }
+#pragma unroll
+            for (uint32_t h = 1; h < 32; h <<= 1)
+#pragma unroll
+                for (int j = 0; j < kV; j++) {
+                    const float o = __shfl_xor_sync(0xffffffffu, v[j], h);
+                    v[j] = lane & h ? o - v[j] : v[j] + o;
+                }
+#pragma unroll
+            for (int j = 0; j < kV; j++) {
+                v[j] *= 1.0f / (32.0f * kV);
+                row[b + 32u * j + lane] = v[j];
+                most = fmaxf(most, fabsf(v[j]));
+            }
+        }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, d));
+    if (lane == 0) part[warp] = most;
+    __syncthreads();
+    most = 0.0f;
+    for (uint32_t w = 0; w < nwarps; w++) most = fmaxf(most, part[w]);
+    // 2^e with 2^14 <= most 2^e < 2^15, e within what a float holds; zero rows and rows with infinities stay as they are
+    int e = 0;
+    if (most > 0.0f && most < __int_as_float(0x7f800000)) e = min(120, 141 - (int)(__float_as_uint(most) >> 23));
+    const float up = __uint_as_float((uint32_t)(127 + e) << 23);
+    if (threadIdx.x == 0) tok_scale[m] = __uint_as_float((uint32_t)(127 - e) << 23);
+    for (uint32_t k = threadIdx.x * 2u; k < K; k += blockDim.x * 2u) {
+        const float a = row[k] * up, b = row[k + 1] * up;
+        const __half ha = __float2half_rn(a), hb = __float2half_rn(b);
+        const __half la = __float2half_rn(a - __half2float(ha)), lb = __float2half_rn(b - __half2float(hb));
+        *reinterpret_cast<__half2 *>(planes + (size_t)m * K + k) = __halves2half2(ha, hb);
+        *reinterpret_cast<__half2 *>(planes + (size_t)(M + m) * K + k) = __halves2half2(la, lb);
+    }
+}
+
+namespace {
+
+typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                             const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeFn encode_fn()
+{
+    static EncodeFn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
+        return reinterpret_cast<EncodeFn>(p);
+    }();
+    return fn;
+}
+
+bool map_2d(CUtensorMap &m, CUtensorMapDataType type, const void *p, uint64_t inner, uint64_t rows, uint64_t row_bytes, uint32_t box_inner,
+            uint32_t box_rows, CUtensorMapSwizzle sw)
+{
+    const cuuint64_t dims[2] = {inner, rows}, strides[1] = {row_bytes};
+    const cuuint32_t box[2] = {box_inner, box_rows}, step[2] = {1, 1};
+    EncodeFn fn = encode_fn();
+    return fn && fn(&m, type, 2, const_cast<void *>(p), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// CTAs of a kernel in clusters of `split` that fit on the device at once, asked once per kernel, size and shared memory.
+uint32_t resident_ctas(const void *kern, uint32_t threads, size_t smem, uint32_t split)
+{
+    struct Known { const void *k; size_t smem; uint32_t split; int dev; uint32_t n; };
+    static std::mutex mu;
+    static std::vector<Known> known;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    std::lock_guard<std::mutex> lock(mu);
+    for (const Known &k : known) if (k.k == kern && k.smem == smem && k.split == split && k.dev == dev) return k.n;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(split);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
+    known.push_back(Known{kern, smem, split, dev, (uint32_t)std::max(n, 0) * split});
+    return known.back().n;
+}
+
+struct Shape { uint32_t T, nw, ns, a_base; size_t smem; uint32_t at_x, at_bar; };
+
+// Stages and shared memory of a kernel variant for a token tile T.  A producer set has to come by every stage on every lap
+// (its parity waits look one lap back): operand stages in multiples of the sets, weight stages in multiples of the copies
+// that a set steps over.
+void place(Shape &s, uint32_t stage_w, uint32_t unit_blocks, uint32_t sets, uint32_t planes, uint32_t a_cols, uint32_t kb, bool fold)
+{
+    const size_t fixed = 512 + 1024 + 1024 + kScaleRing * kScaleEntry, room = 226u * 1024u - fixed;
+    const uint32_t xstage = s.T * 2u * kb * planes, step = std::max(1u, sets / unit_blocks);
+    s.a_base = fold ? 2 * s.T : s.T;
+    s.ns = std::min(8u, (512u - s.a_base) / a_cols) / sets * sets;
+    while (s.ns > sets && room < (size_t)s.ns * xstage + std::max(4u, step) * stage_w) s.ns -= sets;
+    s.nw = (uint32_t)std::min<size_t>(8, (room - (size_t)s.ns * xstage) / stage_w) / step * step;      // the rest of the room hides DRAM
+    s.at_x = s.nw * stage_w;
+    s.at_bar = std::max(s.at_x + s.ns * xstage, s.T * kRows * 4u);
+    s.smem = s.at_bar + fixed;
+}
+
+// How a call is cut: token tiles of at most `most` tokens (multiples of `step`) and the columns over the CTAs of a cluster.
+// The cut with the least rounds of resident CTAs x what a CTA takes: its blocks of 64 columns, each the longer of its
+// products (two cycles a token) and its producers' work, and some four thousand cycles to start, fill and store (half as
+// many more to meet in a cluster).  The constants are measured (1024 x 4096 to 11008 x 4096, 8 to 2048 tokens).
+struct Plan { uint32_t T, tok_tiles, split; double cycles; };
+struct PlanKey {
+    uint32_t rows, K, M, planes;
+    int dev;
+    bool operator==(const PlanKey &o) const { return rows == o.rows && K == o.K && M == o.M && planes == o.planes && dev == o.dev; }
+};
+
+// With `cycles`: what the call would take by the plan's own estimate, nothing launched.
+template <int BITS, bool BF16, bool FOLD, int NP, int NF, int TC, int KB>
+int run_variant(QmmArgs a, uint32_t most, uint32_t step, const void *packed, uint64_t row_bytes, const void *x, cudaStream_t st, double *cycles)
+{
+    using U = Unit<BITS, KB>;
+    auto kern = qmm_kernel<BITS, BF16, FOLD, NP, NF, TC, KB>;
+    constexpr uint32_t threads = (4 * NP + 4 * NF + 4) * 32, a_cols = (BITS == kPolar ? 64u : 32u) * (KB / 64);
+    const uint32_t rows = (a.N + kRows - 1) / kRows;
+    a.units = (a.K + U::kCols - 1) / U::kCols;
+    auto placed = [&](uint32_t T) {
+        Shape s = {};
+        s.T = T;
+        place(s, U::kStage, U::kBlocks, NP, a.planes, a_cols, KB, FOLD);
+        return s;
+    };
+    // the plans of the last shapes this kernel was called with (a model has a handful)
+    static std::mutex mu;
+    static PlanKey keys[32];
+    static Plan plans[32];
+    static uint32_t used = 0;
+    PlanKey key{rows, a.K, a.M, a.planes, 0};
+    if (cudaGetDevice(&key.dev) != cudaSuccess) return (int)cudaErrorInvalidDevice;
+    Plan plan = {};
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        for (uint32_t i = 0; i < std::min(used, 32u); i++) if (keys[i] == key) plan = plans[i];
+    }
+    if (!plan.T) {
+        const double producers = BITS == kPolar ? 700.0 : FOLD ? 450.0 : !BF16 ? 400.0 : BITS == 8 ? 600.0 : 660.0, products = BITS == kPolar ? 3.0 : a.planes;
+        double best = 1e30;
+        const uint32_t least = (a.M + most - 1) / most;
+        for (uint32_t n = least; n < least + 4; n++) {
+            const uint32_t T = ((a.M + n - 1) / n + step - 1) / step * step;
+            if (T > most || (n > least && (T >= plan.T || (a.M + T - 1) / T < n))) continue;
+            const Shape s = placed(T);
+            const double block = std::max(producers, 2.0 * T * products + 150.0);
+            for (uint32_t split = 1; split <= 8 && split <= a.units; split++) {
+                const uint32_t room = resident_ctas(reinterpret_cast<const void *>(kern), threads, s.smem, split);
+                if (room == 0) continue;
+                const double cost = (double)((rows * n * split + room - 1) / room) *
+                                    ((double)((a.units + split - 1) / split) * (U::kCols / 64) * block + 4000.0 + (split > 1 ? 2000.0 : 0.0));
+                // a cut into more token tiles repeats the producers' work: only for a clear gain
+                if (cost < best * (n > plan.tok_tiles && plan.T ? 0.95 : 0.999)) { best = cost; plan = Plan{T, n, split, cost}; }
+            }
+        }
+        if (!plan.T) return (int)cudaErrorLaunchOutOfResources;
+        std::lock_guard<std::mutex> lock(mu);
+        keys[used % 32] = key;
+        plans[used % 32] = plan;
+        used = used + 1 >= 64 ? 32 : used + 1;
+    }
+    if (cycles) { *cycles = plan.cycles; return 0; }
+    const Shape s = placed(plan.T);
+    a.T = s.T; a.nw = s.nw; a.ns = s.ns; a.a_base = s.a_base; a.at_x = s.at_x; a.at_bar = s.at_bar; a.split = plan.split;
+    CUtensorMap wmap, xmap;
+    const bool mapped = BITS == kBlocked4
+        ? map_2d(wmap, CU_TENSOR_MAP_DATA_TYPE_INT64, packed, row_bytes / 8, a.K / 16, row_bytes, kRows, U::kCols / 16, CU_TENSOR_MAP_SWIZZLE_NONE)
+        : map_2d(wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, packed, row_bytes, a.N, row_bytes, U::kBytes, kRows,
+                 BITS == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
+    if (!mapped ||
+        !map_2d(xmap, BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, a.K, (uint64_t)a.M * a.planes, (uint64_t)a.K * 2,
+                64, s.T, CU_TENSOR_MAP_SWIZZLE_128B))
+        return (int)cudaErrorInvalidValue;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(rows * a.split, plan.tok_tiles);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = s.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = a.split; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a, wmap, xmap);
+    count_launch();
+    return (int)(e != cudaSuccess ? e : cudaGetLastError());
+}
+
+template <int BITS, bool BF16>
+int run_fold(const QmmArgs &a, const void *packed, uint64_t row_bytes, const void *x, cudaStream_t st, double *cycles)
+{
+    // few tokens: long blocks (polar centroids take two operand planes, which leaves room for short ones), and as few
+    // warps as keep up: 4096 x 4096, 24 tokens takes 9.1 us with two producer sets and one reader set, 9.8 with four sets
+    constexpr int kLong = BITS == kPolar ? 64 : 128;
+    if (a.M <= 32) return run_variant<BITS, BF16, true, 2, 1, 32, kLong>(a, 32, 16, packed, row_bytes, x, st, cycles);
+    if (a.M <= 64) return run_variant<BITS, BF16, true, 2, 2, 32, kLong>(a, 64, 32, packed, row_bytes, x, st, cycles);
+    return run_variant<BITS, BF16, true, 2, 2, 64, 64>(a, 128, 32, packed, row_bytes, x, st, cycles);
+}
+
+template <int BITS, bool BF16>
+int run_scaled(const QmmArgs &a, const void *packed, uint64_t row_bytes, const void *x, cudaStream_t st, double *cycles)
+{
+    return run_variant<BITS, BF16, false, 4, 1, 32, 64>(a, 256, 16, packed, row_bytes, x, st, cycles);
+}
+
+int qmm(const QmmCall &c, void *stream, double *cycles)
+{
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    QmmArgs a = {};
+    a.scales = c.scales; a.centroids = c.centroids; a.bias = c.bias; a.tok_scale = c.tok_scale; a.y = c.y;
+    a.N = c.N; a.K = c.K; a.M = c.M; a.group = c.group; a.sgroups = c.K / c.group; a.y_dtype = c.y_dtype;
+    a.bias_half = c.bias_half;
+    a.late = c.late;
+    for (uint32_t parts = 1; a.seg == 0; parts++)              // the fewest equal parts of a group, of 32-column multiples, that are short enough
+        if (c.group % (32u * parts) == 0 && c.group / parts <= 128u) a.seg = c.group / parts;
+    a.planes = c.split_x ? 2u : 1u;
+    a.entries = c.centroids ? 1u << c.bits : 1u;
+    const bool bf = c.bf16 && !c.split_x;
+    const uint64_t row_bytes = c.blocked_rows ? (uint64_t)c.blocked_rows * 8 : c.centroids ? c.K : c.bits == 4 ? c.K / 2 : c.bits == 2 ? c.K / 4 : c.K;
+    if (c.centroids) return run_fold<kPolar, false>(a, c.packed, row_bytes, c.x, st, cycles);
+    const bool fold = c.split_x || c.M <= 128u;
+#define EOQ_QMM(B)                                                                                                                      \
+    (fold ? (bf ? run_fold<B, true>(a, c.packed, row_bytes, c.x, st, cycles) : run_fold<B, false>(a, c.packed, row_bytes, c.x, st, cycles)) \
+          : (bf ? run_scaled<B, true>(a, c.packed, row_bytes, c.x, st, cycles) : run_scaled<B, false>(a, c.packed, row_bytes, c.x, st, cycles)))
+    if (c.blocked_rows) return EOQ_QMM(kBlocked4);
+    if (c.bits == 4) return EOQ_QMM(4);
+    if (c.bits == 2) return EOQ_QMM(2);
+    return EOQ_QMM(8);
+#undef EOQ_QMM
+}
+
+}  // namespace
+
+// Whether the kernels above take a packed weight of this shape: whole groups per row, copies aligned.
+bool qmm_takes(uint32_t K, uint32_t bits, uint32_t group, const void *packed, const void *x)
+{
+    const uint32_t per16 = bits == 4 ? 32u : bits == 2 ? 64u : 16u;
+    return K % per16 == 0 && group % 32u == 0 && K % group == 0 && ((reinterpret_cast<uintptr_t>(packed) | reinterpret_cast<uintptr_t>(x)) & 15u) == 0;
+}
+
+int launch_qmm(const QmmCall &c, void *stream) { return qmm(c, stream, nullptr); }
+
+// Whether the call is to be preferred to a dequantised copy of the weight and a library GEMM, given the microseconds that
+// the copy takes longer than what this kernel reads takes to make.  fp32 activations: always (the library multiplies them
+// on the CUDA cores: 13 x slower at 512 rows).  16-bit ones: up to 32 rows, where rows of y are not 16-byte multiples (the
+// library's kernels for those are three to ten times slower), or where the plan's estimate, at the 1.5 cycles a nanosecond
+// that long products run at, is not above the GEMM's (1.45 PFLOP/s, 8 us at least).  From packed codes, fp16, 777 rows:
+// 4096 x 11008 62 against 77 us, 11008 x 4096 71 against 71; 2048 rows: 141 / 142 and 153 / 156.
+bool qmm_preferred(const QmmCall &c, double copy_us)
+{
+    if (c.split_x || c.M <= 32u || c.N % 8u) return true;
+    double cycles = 0;
+    if (qmm(c, nullptr, &cycles) != 0) return false;
+    return cycles / 1500.0 <= std::max(8.0, 2.0 * c.M * (double)c.N * c.K / 1.45e9) + copy_us + 4.0;
+}
+
+bool split_rows_takes(uint32_t K, uint32_t block) { return K % 16u == 0 && K <= 48u * 1024u && (block == 1 || block == 64 || block == 128 || block == 256); }
+
+// x [M][K] to two fp16 planes [2][M][K] and M factors; block 1: no rotation.
+int launch_split_rows(const void *x, int x_dtype, uint32_t K, uint32_t M, uint32_t block, void *planes, float *tok_scale, void *stream)
+{
+    auto kern = block == 1 ? split_rows_kernel<0> : block == 64 ? split_rows_kernel<2> : block == 128 ? split_rows_kernel<4> : split_rows_kernel<8>;
+    static std::atomic<uint64_t> asked{0};                  // kernels whose shared-memory limit has been raised, per device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    const uint64_t mark = dev < 16 ? 1ull << (dev * 4 + (block == 1 ? 0 : block == 64 ? 1 : block == 128 ? 2 : 3)) : 0u;
+    if (!mark || !(asked.load() & mark)) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024 * 4);
+        if (e != cudaSuccess) return (int)e;
+        asked.fetch_or(mark);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(M);
+    cfg.blockDim = dim3(512);
+    cfg.dynamicSmemBytes = (size_t)K * 4;
+    cfg.stream = reinterpret_cast<cudaStream_t>(stream);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kern, x, x_dtype, K, M, reinterpret_cast<__half *>(planes), tok_scale);
+    count_launch();
+    return (int)(e != cudaSuccess ? e : cudaGetLastError());
+}
+
+uint32_t qmm_status()
+{
+    uint32_t v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_qmm_status, 4) != cudaSuccess) return ~0u;
+    if (v && cudaMemcpyToSymbol(g_qmm_status, &zero, 4) != cudaSuccess) return ~0u;
+    return v;
+}
+
+}  // namespace eoq
