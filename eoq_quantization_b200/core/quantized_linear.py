@@ -1,9 +1,9 @@
 """``QuantizedLinear`` with the interface of the reference's
 ``core/quantized_linear.py``.  Buffers, packing and ``from_float`` are the
-reference's; ``forward`` runs on the GPU: for up to 8 activation rows the
-weights are kept entropy-coded in HBM and consumed by the fused
-decode+dequantise+GEMV kernel, otherwise they are dequantised by the library
-and multiplied with a library GEMM."""
+reference's; ``forward`` multiplies straight from the packed codes on the tensor
+cores for any number of rows (or from a dequantised copy where that and a library
+GEMM are quicker); shapes those kernels do not take go through an entropy-coded
+copy (few rows) or a dequantised one."""
 from __future__ import annotations
 
 from typing import Optional
@@ -13,7 +13,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _lib
-from ..fused import GEMM_MAX_ROWS, EOQWeight, dequant_packed, fused_rows, gemv_packed, PACKED_TENSOR_ROWS, packed_gemv_rows, require_cuda
+from ..fused import GEMM_MAX_ROWS, EOQWeight, dequant_packed, fused_rows, require_cuda
 
 
 class QuantizedLinear(nn.Module):
@@ -130,23 +130,13 @@ class QuantizedLinear(nn.Module):
         """x of shape (..., in_features), any float dtype -> (..., out_features) in x.dtype."""
         buffers = self._buffers                 # not through nn.Module.__getattr__, which costs as much as the call
         bias = buffers["bias_param"] if "bias_param" in buffers else self.bias_param
-        most = packed_gemv_rows(self.in_features, self.bits, self.block_size)
-        if most == PACKED_TENSOR_ROWS or not self._fusable():
-            y = _lib.native().packed_linear(buffers["packed_weight"], buffers["scales"], self.out_features, self.in_features, self.bits,
-                                            self.block_size, most if most == PACKED_TENSOR_ROWS else 0, x, bias)
-            if y is not None:
-                return y
+        y = _lib.native().packed_linear(buffers["packed_weight"], buffers["scales"], self.out_features, self.in_features, self.bits,
+                                        self.block_size, x, bias)
+        if y is not None:
+            return y
         require_cuda(x, "QuantizedLinear.forward")
         require_cuda(self.packed_weight, "QuantizedLinear.forward")
         rows = x.numel() // max(self.in_features, 1)
-        if x.dtype in (torch.float16, torch.bfloat16, torch.float32) and \
-                1 <= rows <= PACKED_TENSOR_ROWS == packed_gemv_rows(self.in_features, self.bits, self.block_size, x.dtype):
-            # up to 32 rows: one pass over the packed codes this module keeps resident, codes to exact 16-bit floats in
-            # registers and warp-level tensor-core products (fp32 activations as two fp16 halves each); the
-            # entropy-coded form of the same weight (`eoq_weight()`) trades that speed for 7-15 % less memory and is
-            # what `EOQLinear` holds.  Other group sizes take the routes below.
-            return gemv_packed(self.packed_weight, self.scales, self.out_features, self.in_features, self.bits, self.block_size,
-                               x, self.bias_param)
         if self._fusable() and rows >= 1 and x.dtype in (torch.float16, torch.bfloat16, torch.float32):
             # up to fused_rows (4 rows of 16-bit activations, 8 of fp32): fused decode + GEMV, fp32 accumulate; beyond
             # that one dequantisation amortises over enough rows for a library GEMM to win (the fused tensor-core

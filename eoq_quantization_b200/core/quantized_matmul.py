@@ -10,6 +10,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from .. import _lib
 from ..fused import GEMM_MAX_ROWS, EOQWeight, dequant_packed, fused_rows, gemv_packed, PACKED_TENSOR_ROWS, packed_gemv_rows, require_cuda
 
 _SUPPORTED_BITS = (2, 4, 8)
@@ -132,6 +133,12 @@ class QuantizedLinearFast(nn.Module):
         return self._eoq
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        if self.strategy == "auto":
+            buffers = self._buffers
+            y = _lib.native().packed_linear(buffers["packed_weight"], buffers["scales"], self.out_features, self.in_features, self.bits,
+                                            self.block_size, x, buffers["bias_param"] if "bias_param" in buffers else self.bias_param)
+            if y is not None:                   # straight from the packed codes, see QuantizedLinear.forward
+                return y
         require_cuda(x, "QuantizedLinearFast.forward")
         rows = x.numel() // max(self.in_features, 1)
         if self.strategy == "auto" and x.dtype in (torch.float16, torch.bfloat16, torch.float32) and \

@@ -1732,6 +1732,16 @@ extern "C" eoq_error_t eoq_b200_dequant_packed(const uint8_t *d_packed, const ui
     return EOQ_OK;
 }
 
+static QmmCall packed_call(const uint8_t *d_packed, const uint16_t *d_scales_fp16, uint32_t rows, uint32_t cols, uint32_t bits, uint32_t group,
+                           const void *x, int x_dtype, uint32_t batch, void *d_scratch, void *y, int y_dtype, const float *bias)
+{
+    QmmCall c = {};
+    c.packed = d_packed; c.scales = d_scales_fp16; c.bias = bias; c.x = x; c.y = y; c.N = rows; c.K = cols; c.M = batch; c.bits = bits;
+    c.group = group; c.bf16 = x_dtype == EOQ_B200_BF16; c.y_dtype = y_dtype;
+    if (x_dtype == EOQ_B200_F32) { c.split_x = 1; c.x = d_scratch; }
+    return c;
+}
+
 extern "C" eoq_error_t eoq_b200_gemv_packed(const uint8_t *d_packed, const uint16_t *d_scales_fp16, uint32_t rows, uint32_t cols,
                                             uint32_t bits, uint32_t group, const void *x, int x_dtype, uint32_t batch, void *d_scratch,
                                             void *y, int y_dtype, const float *bias, void *stream)
@@ -1744,25 +1754,88 @@ extern "C" eoq_error_t eoq_b200_gemv_packed(const uint8_t *d_packed, const uint1
     // the dequantise kernel
     const uint32_t per16 = bits == 4 ? 32u : bits == 2 ? 64u : 16u;
     if (cols % per16 || group % 8u || cols % group || (reinterpret_cast<uintptr_t>(d_packed) & 15u)) return EOQ_ERR_UNSUPPORTED;
-    PackedGemvArgs a = {};
-    a.packed = d_packed; a.scales = d_scales_fp16; a.x = x; a.y = y; a.bias = bias;
-    a.N = rows; a.K = cols; a.group = group; a.batch = batch; a.bits = bits; a.x_dtype = x_dtype; a.y_dtype = y_dtype;
-    // row stride of QuantizedLinear.packed_weight (core/quantized_linear.py:49-66)
-    a.row_bytes = bits == 4 ? cols / 2 : bits == 2 ? cols / 4 : cols;
-    // fp32 activations reach the tensor cores as two fp16 halves, written into the caller's scratch by one small launch
-    const bool split = x_dtype == EOQ_B200_F32 && d_scratch && (reinterpret_cast<uintptr_t>(d_scratch) & 15u) == 0 &&
-                       cols % 128u == 0 && group % 128u == 0;
-    if (split) a.xsplit = static_cast<const uint16_t *>(d_scratch);
-    if (batch > gemv_packed_rows(a)) return EOQ_ERR_UNSUPPORTED;
+    const bool f32 = x_dtype == EOQ_B200_F32;
+    // rows of the tensor-core forms: 32 where a group is whole 128-column spans, 8 otherwise
+    const bool wide = cols % 128u == 0 && group % 128u == 0 &&
+                      (f32 ? d_scratch && (reinterpret_cast<uintptr_t>(d_scratch) & 15u) == 0 : (reinterpret_cast<uintptr_t>(x) & 15u) == 0);
+    if (batch > (wide ? 32u : 8u)) return EOQ_ERR_UNSUPPORTED;
     if (!have_device()) return EOQ_ERR_CUDA;
-    if (split) {
-        int e = launch_polar_rotate(x, x_dtype, cols, 0, batch, nullptr, static_cast<uint16_t *>(d_scratch), stream);      // block of 1: no rotation, only the split
-        if (e != 0) { std::fprintf(stderr, "eoq_b200_gemv_packed: launch failed: %s\n", cudaGetErrorString((cudaError_t)e)); return EOQ_ERR_CUDA; }
+    int e = 0;
+    if (wide && (f32 || batch > 8)) {
+        // fp32 activations reach the tensor cores as two fp16 halves, written into the caller's scratch by one small launch
+        if (f32) e = launch_polar_rotate(x, x_dtype, cols, 0, batch, nullptr, static_cast<uint16_t *>(d_scratch), stream);      // block of 1: no rotation, only the split
+        if (e == 0) e = launch_qmm(packed_call(d_packed, d_scales_fp16, rows, cols, bits, group, x, x_dtype, batch, d_scratch, y, y_dtype, bias), stream);
+    } else {
+        PackedGemvArgs a = {};
+        a.packed = d_packed; a.scales = d_scales_fp16; a.x = x; a.y = y; a.bias = bias;
+        a.N = rows; a.K = cols; a.group = group; a.batch = batch; a.bits = bits; a.x_dtype = x_dtype; a.y_dtype = y_dtype;
+        // row stride of QuantizedLinear.packed_weight (core/quantized_linear.py:49-66)
+        a.row_bytes = bits == 4 ? cols / 2 : bits == 2 ? cols / 4 : cols;
+        e = launch_gemv_packed(a, stream);
     }
-    int e = launch_gemv_packed(a, stream);
     if (e != 0) { std::fprintf(stderr, "eoq_b200_gemv_packed: launch failed: %s\n", cudaGetErrorString((cudaError_t)e)); return EOQ_ERR_CUDA; }
     return EOQ_OK;
 }
+
+extern "C" eoq_error_t eoq_b200_linear_packed(const uint8_t *d_packed, const uint16_t *d_scales_fp16, uint32_t rows, uint32_t cols,
+                                              uint32_t bits, uint32_t group, const void *x, int x_dtype, uint32_t batch, void *d_scratch,
+                                              void *y, int y_dtype, const float *bias, void *stream)
+{
+    if (!d_packed || !d_scales_fp16 || !x || !y) return EOQ_ERR_NULL_PTR;
+    if (batch == 0 || rows == 0) return EOQ_OK;
+    if (x_dtype < 0 || x_dtype > 2 || y_dtype < 0 || y_dtype > 2) return EOQ_ERR_UNSUPPORTED;
+    if (bits < 2 || bits > 8 || group == 0 || cols == 0) return EOQ_ERR_INVALID_HEADER;
+    const bool split = x_dtype == EOQ_B200_F32;
+    if (split && !d_scratch) return EOQ_ERR_NULL_PTR;
+    if (!qmm_takes(cols, bits, group, d_packed, split ? d_scratch : x) || (split && !split_rows_takes(cols, 1))) return EOQ_ERR_UNSUPPORTED;
+    if (!have_device()) return EOQ_ERR_CUDA;
+    QmmCall c = packed_call(d_packed, d_scales_fp16, rows, cols, bits, group, x, x_dtype, batch, d_scratch, y, y_dtype, bias);
+    int e = 0;
+    if (split) {
+        float *factors = reinterpret_cast<float *>(static_cast<uint8_t *>(d_scratch) + (size_t)batch * cols * 4);
+        c.tok_scale = factors;
+        e = launch_split_rows(x, x_dtype, cols, batch, 1, d_scratch, factors, stream);
+    }
+    if (e == 0) e = launch_qmm(c, stream);
+    if (e != 0) { std::fprintf(stderr, "eoq_b200_linear_packed: launch failed: %s\n", cudaGetErrorString((cudaError_t)e)); return EOQ_ERR_CUDA; }
+    return EOQ_OK;
+}
+
+// For the torch-facing front (not in the public header): whether eoq_b200_linear_packed takes the call and is to be
+// preferred to a dequantised copy (2 T weights/s) and a library GEMM.
+extern "C" int eoq_b200_linear_packed_preferred(const uint8_t *d_packed, uint32_t rows, uint32_t cols, uint32_t bits, uint32_t group,
+                                                const void *x, int x_dtype, uint32_t batch)
+{
+    const bool split = x_dtype == EOQ_B200_F32;
+    if (!qmm_takes(cols, bits, group, d_packed, x) || (split && !split_rows_takes(cols, 1))) return 0;
+    return qmm_preferred(packed_call(d_packed, nullptr, rows, cols, bits, group, x, x_dtype, batch, nullptr, nullptr, x_dtype, nullptr),
+                         (double)rows * cols / 2.05e6) ? 1 : 0;
+}
+
+extern "C" eoq_error_t eoq_b200_linear_polar_codes(const uint8_t *d_codes, const uint16_t *d_norms_fp16, const float *d_centroids,
+                                                   uint32_t rows, uint32_t cols, uint32_t bits, uint32_t block, const void *x, int x_dtype,
+                                                   uint32_t batch, void *d_scratch, void *y, int y_dtype, const void *bias, int bias_dtype,
+                                                   void *stream)
+{
+    if (!d_codes || !d_norms_fp16 || !d_centroids || !x || !y || !d_scratch) return EOQ_ERR_NULL_PTR;
+    if (bias && bias_dtype != EOQ_B200_F32 && bias_dtype != EOQ_B200_F16) return EOQ_ERR_UNSUPPORTED;
+    if (batch == 0 || rows == 0) return EOQ_OK;
+    if (x_dtype < 0 || x_dtype > 2 || y_dtype < 0 || y_dtype > 2) return EOQ_ERR_UNSUPPORTED;
+    if (bits < 1 || bits > 8 || block == 0 || cols == 0) return EOQ_ERR_INVALID_HEADER;
+    if (block < 64 || !qmm_takes(cols, 8, block, d_codes, d_scratch) || !split_rows_takes(cols, block)) return EOQ_ERR_UNSUPPORTED;
+    if (!have_device()) return EOQ_ERR_CUDA;
+    QmmCall c = {};
+    float *factors = reinterpret_cast<float *>(static_cast<uint8_t *>(d_scratch) + (size_t)batch * cols * 4);
+    c.packed = d_codes; c.scales = d_norms_fp16; c.centroids = d_centroids; c.bias = bias; c.x = d_scratch; c.tok_scale = factors; c.y = y;
+    c.bias_half = bias_dtype == EOQ_B200_F16;
+    c.N = rows; c.K = cols; c.M = batch; c.bits = bits; c.group = block; c.split_x = 1; c.y_dtype = y_dtype;
+    int e = launch_split_rows(x, x_dtype, cols, batch, block, d_scratch, factors, stream);
+    if (e == 0) e = launch_qmm(c, stream);
+    if (e != 0) { std::fprintf(stderr, "eoq_b200_linear_polar_codes: launch failed: %s\n", cudaGetErrorString((cudaError_t)e)); return EOQ_ERR_CUDA; }
+    return EOQ_OK;
+}
+
+extern "C" uint32_t eoq_b200_linear_status(void) { return qmm_status(); }
 
 extern "C" eoq_error_t eoq_b200_gemv_polar_codes(const uint8_t *d_codes, const uint16_t *d_norms_fp16, const float *d_centroids,
                                                  uint32_t rows, uint32_t cols, uint32_t bits, uint32_t block, const void *x, int x_dtype,
@@ -1781,15 +1854,22 @@ extern "C" eoq_error_t eoq_b200_gemv_polar_codes(const uint8_t *d_codes, const u
         ((reinterpret_cast<uintptr_t>(d_codes) | reinterpret_cast<uintptr_t>(d_scratch)) & 15u))
         return EOQ_ERR_UNSUPPORTED;
     if (!have_device()) return EOQ_ERR_CUDA;
-    PolarCodesArgs a = {};
-    a.codes = d_codes; a.norms = d_norms_fp16; a.centroids = d_centroids; a.y = y; a.bias = bias;
-    if (split) a.xsplit = static_cast<const uint16_t *>(d_scratch);
-    else a.xrot = static_cast<const float *>(d_scratch);
-    a.N = rows; a.K = cols; a.batch = batch; a.entries = 1u << bits; a.y_dtype = y_dtype;
-    for (a.block_shift = 4; (1u << a.block_shift) < block; a.block_shift++) {}
-    int e = launch_polar_rotate(x, x_dtype, cols, a.block_shift, batch, split ? nullptr : static_cast<float *>(d_scratch),
+    uint32_t shift = 4;
+    while ((1u << shift) < block) shift++;
+    int e = launch_polar_rotate(x, x_dtype, cols, shift, batch, split ? nullptr : static_cast<float *>(d_scratch),
                                 split ? static_cast<uint16_t *>(d_scratch) : nullptr, stream);
-    if (e == 0) e = launch_gemv_polar_codes(a, stream);
+    if (e == 0 && split) {
+        QmmCall c = {};
+        c.packed = d_codes; c.scales = d_norms_fp16; c.centroids = d_centroids; c.bias = bias; c.x = d_scratch; c.y = y;
+        c.N = rows; c.K = cols; c.M = batch; c.bits = bits; c.group = block; c.split_x = 1; c.y_dtype = y_dtype;
+        e = launch_qmm(c, stream);
+    } else if (e == 0) {
+        PolarCodesArgs a = {};
+        a.codes = d_codes; a.norms = d_norms_fp16; a.centroids = d_centroids; a.y = y; a.bias = bias;
+        a.xrot = static_cast<const float *>(d_scratch);
+        a.N = rows; a.K = cols; a.batch = batch; a.entries = 1u << bits; a.y_dtype = y_dtype; a.block_shift = shift;
+        e = launch_gemv_polar_codes(a, stream);
+    }
     if (e != 0) { std::fprintf(stderr, "eoq_b200_gemv_polar_codes: launch failed: %s\n", cudaGetErrorString((cudaError_t)e)); return EOQ_ERR_CUDA; }
     return EOQ_OK;
 }

@@ -210,7 +210,6 @@ struct PackedGemvArgs {
     const uint8_t *packed;      // [N][row_bytes]
     const uint16_t *scales;     // fp16 bits, [N][K / group]
     const void *x;              // [batch][K]
-    const uint16_t *xsplit;     // fp32 activations on the tensor cores: fp16 bits [2][batch][K], the nearest fp16 and the nearest to the remainder
     void *y;                    // [batch][N]
     const float *bias;          // [N] or null
     uint32_t N, K, group, row_bytes, batch, bits;
@@ -221,7 +220,6 @@ struct PolarCodesArgs {
     const uint16_t *norms;      // fp16 bits, [N][K / block]
     const float *centroids;     // [entries]
     const float *xrot;          // [batch][K]: activations rotated per block and divided by sqrt(block)
-    const uint16_t *xsplit;     // or (tensor-core form) fp16 bits [2][batch][K]: the fp16 nearest to each rotated activation, then the remainder
     void *y;                    // [batch][N]
     const float *bias;          // [N] or null
     uint32_t N, K, block_shift, batch, entries;
@@ -229,7 +227,6 @@ struct PolarCodesArgs {
 };
 int launch_gemv_polar_codes(const PolarCodesArgs &a, void *stream);
 int launch_polar_rotate(const void *x, int x_dtype, uint32_t K, uint32_t block_shift, uint32_t batch, float *out32, uint16_t *out_split, void *stream);
-uint32_t gemv_packed_rows(const PackedGemvArgs &a);
 void set_packed_warps(int v);
 void set_dequant_vec(int v);
 int launch_gemv_packed(const PackedGemvArgs &a, void *stream);

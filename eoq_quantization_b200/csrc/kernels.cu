@@ -3136,14 +3136,13 @@ __device__ __forceinline__ void unpack_span(const uint32_t (&w)[BITS], uint32_t 
 // rotation).  Lanes whose activation row does not exist read zeros from a constant block instead of branching.
 __device__ const uint4 kZeroBlock[4] = {};
 
-template <int BITS, bool BF16, int NB, bool SPLIT = false>
-__global__ void __launch_bounds__(BITS == 8 ? 256 : 512, NB > 1 || SPLIT ? 1 : BITS == 8 ? 3 : 2) gemv_packed_mma_kernel(const PackedGemvArgs a)
+template <int BITS, bool BF16>
+__global__ void __launch_bounds__(BITS == 8 ? 256 : 512, BITS == 8 ? 3 : 2) gemv_packed_mma_kernel(const PackedGemvArgs a)
 {
     static_assert(BITS == 2 || BITS == 4 || BITS == 8, "two or four bits packed, or one code per byte");
-    static_assert(!(SPLIT && BF16), "the two halves of an fp32 activation are fp16");
     constexpr int kRows = 2;                                       // a lane's weight rows: g and g + 8 of the tile
     constexpr int kDepth = 2;                                      // register sets of weights: kDepth - 1 spans requested ahead
-    __shared__ float red[kMmaMaxWarps][NB][16][8];
+    __shared__ float red[kMmaMaxWarps][16][8];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5, g = lane >> 2, t = lane & 3u;
     const uint32_t row0 = blockIdx.x * 16u;
     const uint32_t sgroups = a.K / a.group, nspans = a.K >> 7, gspans = a.group >> 7;
@@ -3155,20 +3154,11 @@ __global__ void __launch_bounds__(BITS == 8 ? 256 : 512, NB > 1 || SPLIT ? 1 : B
         pw[r] = a.packed + (size_t)row * a.row_bytes + t * (4u * BITS);
         ps[r] = a.scales + (size_t)row * sgroups;
     }
-    // a lane's 64 bytes of activation row 8n + g per span, or the zero block with no stride where that row does not exist
-    const uint16_t *xr[NB];
-    uint32_t xstep[NB];
-#pragma unroll
-    for (int n = 0; n < NB; n++) {
-        const bool has = 8u * n + g < a.batch;
-        xr[n] = has ? (SPLIT ? a.xsplit : reinterpret_cast<const uint16_t *>(a.x)) + (size_t)(8u * n + g) * a.K + t * 32u : reinterpret_cast<const uint16_t *>(kZeroBlock);
-        xstep[n] = has ? 128u : 0u;
-    }
-    float tot[NB][4];
-#pragma unroll
-    for (int n = 0; n < NB; n++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) tot[n][i] = 0.0f;
+    // a lane's 64 bytes of activation row g per span, or the zero block with no stride where that row does not exist
+    const bool has = g < a.batch;
+    const uint16_t *xr = has ? reinterpret_cast<const uint16_t *>(a.x) + (size_t)g * a.K + t * 32u : reinterpret_cast<const uint16_t *>(kZeroBlock);
+    const uint32_t xstep = has ? 128u : 0u;
+    float tot[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 
     auto load_span = [&](uint32_t s, uint32_t (&w)[kRows][BITS], uint16_t (&sc)[kRows]) {
         if (s >= nspans) return;
@@ -3213,35 +3203,20 @@ __global__ void __launch_bounds__(BITS == 8 ? 256 : 512, NB > 1 || SPLIT ? 1 : B
                 }
             }
         };
+        uint32_t xp[16];
+        float c[4], d[4];
+        load_xp(xr + s * xstep, xp);
+        // two accumulators: consecutive instructions do not wait for one another
+        mma_m16n8k16_first<BF16>(c, h0[0], h1[0], h0[1], h1[1], xp[0], xp[1]);
+        mma_m16n8k16_first<BF16>(d, h0[2], h1[2], h0[3], h1[3], xp[2], xp[3]);
 #pragma unroll
-        for (int n = 0; n < NB; n++) {
-            uint32_t xp[16];
-            float c[4], d[4];
-            load_xp(xr[n] + s * xstep[n], xp);
-            if (!SPLIT) {
-                // two accumulators: consecutive instructions do not wait for one another
-                mma_m16n8k16_first<BF16>(c, h0[0], h1[0], h0[1], h1[1], xp[0], xp[1]);
-                mma_m16n8k16_first<BF16>(d, h0[2], h1[2], h0[3], h1[3], xp[2], xp[3]);
-#pragma unroll
-                for (int m = 2; m < 8; m += 2) {
-                    mma_m16n8k16<BF16>(c, h0[2 * m], h1[2 * m], h0[2 * m + 1], h1[2 * m + 1], xp[2 * m], xp[2 * m + 1]);
-                    mma_m16n8k16<BF16>(d, h0[2 * m + 2], h1[2 * m + 2], h0[2 * m + 3], h1[2 * m + 3], xp[2 * m + 2], xp[2 * m + 3]);
-                }
-            } else {
-                // fp32 activations as two fp16 halves (the nearest fp16, then the nearest to the remainder): the codes are
-                // exact, so code * hi + code * lo is the fp32 product to about 2^-22; one accumulator per half
-                mma_m16n8k16_first<false>(c, h0[0], h1[0], h0[1], h1[1], xp[0], xp[1]);
-#pragma unroll
-                for (int m = 1; m < 8; m++) mma_m16n8k16<false>(c, h0[2 * m], h1[2 * m], h0[2 * m + 1], h1[2 * m + 1], xp[2 * m], xp[2 * m + 1]);
-                load_xp(xr[n] + (xstep[n] ? (size_t)a.batch * a.K : 0u) + s * xstep[n], xp);
-                mma_m16n8k16_first<false>(d, h0[0], h1[0], h0[1], h1[1], xp[0], xp[1]);
-#pragma unroll
-                for (int m = 1; m < 8; m++) mma_m16n8k16<false>(d, h0[2 * m], h1[2 * m], h0[2 * m + 1], h1[2 * m + 1], xp[2 * m], xp[2 * m + 1]);
-            }
-            const float fa = half_bits_to_float(sc[0]), fb = half_bits_to_float(sc[1]);
-            tot[n][0] = fmaf(fa, c[0] + d[0], tot[n][0]); tot[n][1] = fmaf(fa, c[1] + d[1], tot[n][1]);
-            tot[n][2] = fmaf(fb, c[2] + d[2], tot[n][2]); tot[n][3] = fmaf(fb, c[3] + d[3], tot[n][3]);
+        for (int m = 2; m < 8; m += 2) {
+            mma_m16n8k16<BF16>(c, h0[2 * m], h1[2 * m], h0[2 * m + 1], h1[2 * m + 1], xp[2 * m], xp[2 * m + 1]);
+            mma_m16n8k16<BF16>(d, h0[2 * m + 2], h1[2 * m + 2], h0[2 * m + 3], h1[2 * m + 3], xp[2 * m + 2], xp[2 * m + 3]);
         }
+        const float fa = half_bits_to_float(sc[0]), fb = half_bits_to_float(sc[1]);
+        tot[0] = fmaf(fa, c[0] + d[0], tot[0]); tot[1] = fmaf(fa, c[1] + d[1], tot[1]);
+        tot[2] = fmaf(fb, c[2] + d[2], tot[2]); tot[3] = fmaf(fb, c[3] + d[3], tot[3]);
     };
 
     // The weights and scales do not depend on the kernel before this one in the stream, the activations may: the
@@ -3261,16 +3236,13 @@ __global__ void __launch_bounds__(BITS == 8 ? 256 : 512, NB > 1 || SPLIT ? 1 : B
             compute_span(sd, wbuf[d], sbuf[d]);
         }
     }
-#pragma unroll
-    for (int n = 0; n < NB; n++) {
-        red[warp][n][g][2 * t] = tot[n][0]; red[warp][n][g][2 * t + 1] = tot[n][1];
-        red[warp][n][g + 8][2 * t] = tot[n][2]; red[warp][n][g + 8][2 * t + 1] = tot[n][3];
-    }
+    red[warp][g][2 * t] = tot[0]; red[warp][g][2 * t + 1] = tot[1];
+    red[warp][g + 8][2 * t] = tot[2]; red[warp][g + 8][2 * t + 1] = tot[3];
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < NB * 128u; i += blockDim.x) {
-        const uint32_t n = i >> 7, r = (i >> 3) & 15u, b = 8u * n + (i & 7u), row = row0 + r;
+    for (uint32_t i = threadIdx.x; i < 128u; i += blockDim.x) {
+        const uint32_t r = (i >> 3) & 15u, b = i & 7u, row = row0 + r;
         float v = 0.0f;
-        for (uint32_t w = 0; w < nwarps; w++) v += red[w][n][r][i & 7u];
+        for (uint32_t w = 0; w < nwarps; w++) v += red[w][r][b];
         if (row < a.N && b < a.batch) store_y(a.y, (size_t)b * a.N + row, v + (a.bias ? __ldg(a.bias + row) : 0.0f), a.y_dtype);
     }
 }
@@ -3278,8 +3250,8 @@ __global__ void __launch_bounds__(BITS == 8 ? 256 : 512, NB > 1 || SPLIT ? 1 : B
 // bits: 2 and 4 as packed by QuantizedLinear (low bits first, code + qmax), anything else one signed code per byte.
 // K a multiple of the group and of the columns in sixteen bytes (32 nibbles, 64 two-bit codes, 16 bytes), the group a
 // multiple of 8, packed rows 16-byte aligned: checked by the caller.
-// Activation rows one launch takes: 32 on the tensor-core form (16-bit activations, 16-byte aligned, or fp32 ones with a
-// split copy, against scale groups of whole 128-column spans), 8 otherwise.
+// Up to eight activation rows; the tensor-core form for 16-bit ones, 16-byte aligned, against scale groups of whole
+// 128-column spans.
 static std::atomic<int> g_packed_warps{0};              // 0 = by shape; "packed_warps" in eoq_b200_tune
 void set_packed_warps(int v) { g_packed_warps.store(v >= 1 && v <= 16 ? v : 0); }
 
@@ -3288,12 +3260,12 @@ void set_packed_warps(int v) { g_packed_warps.store(v >= 1 && v <= 16 ? v : 0); 
 // grid is resident at once (given the registers the compiler gave this instantiation) and every warp still has two
 // spans; when no choice fits, the one with the most resident warps per SM.
 template <typename Kern, typename Args>
-static cudaError_t launch_packed_mma(Kern kern, uint32_t fixed_warps, uint32_t tiles, uint32_t nspans, cudaStream_t st, const Args &a, size_t smem = 0)
+static cudaError_t launch_packed_mma(Kern kern, uint32_t fixed_warps, uint32_t tiles, uint32_t nspans, cudaStream_t st, const Args &a)
 {
     // byte codes and more than eight activation rows (more registers, longer spans of work per warp): 8 warps measured best
     if (fixed_warps) {
         const uint32_t w = g_packed_warps.load() ? std::min((uint32_t)g_packed_warps.load(), fixed_warps) : nspans >= 16u ? fixed_warps : 4u;
-        return launch_with_pdl(kern, dim3(tiles), dim3(w * 32u), smem, st, a);
+        return launch_with_pdl(kern, dim3(tiles), dim3(w * 32u), 0, st, a);
     }
     const uint32_t max_warps = 16;
     // registers per kernel, asked once (kernels of one signature share this function: the key is the kernel, not its type)
@@ -3324,45 +3296,19 @@ static cudaError_t launch_packed_mma(Kern kern, uint32_t fixed_warps, uint32_t t
     }
     if (!warps) warps = fallback;
     if (g_packed_warps.load()) warps = std::min((uint32_t)g_packed_warps.load(), max_warps);
-    return launch_with_pdl(kern, dim3(tiles), dim3(warps * 32u), smem, st, a);
-}
-
-uint32_t gemv_packed_rows(const PackedGemvArgs &a)
-{
-    const bool tensor = a.K % 128u == 0 && a.group % 128u == 0 &&
-                        (a.x_dtype == EOQ_B200_F32 ? a.xsplit != nullptr : (reinterpret_cast<uintptr_t>(a.x) & 15u) == 0);
-    return tensor ? 32u : 8u;
+    return launch_with_pdl(kern, dim3(tiles), dim3(warps * 32u), 0, st, a);
 }
 
 int launch_gemv_packed(const PackedGemvArgs &a, void *stream)
 {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (gemv_packed_rows(a) > 8u) {
+    if (a.batch <= 8 && a.x_dtype != EOQ_B200_F32 && a.K % 128u == 0 && a.group % 128u == 0 && (reinterpret_cast<uintptr_t>(a.x) & 15u) == 0) {
         const uint32_t tiles = (a.N + 15u) / 16u, nspans = a.K >> 7;
-        cudaError_t e = cudaSuccess;
-#define EOQ_LAUNCH_MMA(B, H)                                                                                             \
-    do {                                                                                                                 \
-        if (a.batch <= 8) e = launch_packed_mma(gemv_packed_mma_kernel<B, H, 1>, B == 8 ? 8u : 0u, tiles, nspans, st, a);  \
-        else if (a.batch <= 16) e = launch_packed_mma(gemv_packed_mma_kernel<B, H, 2>, 8u, tiles, nspans, st, a);        \
-        else e = launch_packed_mma(gemv_packed_mma_kernel<B, H, 4>, 8u, tiles, nspans, st, a);                           \
-    } while (0)
         const bool bf = a.x_dtype == EOQ_B200_BF16;
-        if (a.x_dtype == EOQ_B200_F32) {
-#define EOQ_LAUNCH_SPLIT(B)                                                                                              \
-    do {                                                                                                                 \
-        if (a.batch <= 8) e = launch_packed_mma(gemv_packed_mma_kernel<B, false, 1, true>, 8u, tiles, nspans, st, a);    \
-        else if (a.batch <= 16) e = launch_packed_mma(gemv_packed_mma_kernel<B, false, 2, true>, 8u, tiles, nspans, st, a); \
-        else e = launch_packed_mma(gemv_packed_mma_kernel<B, false, 4, true>, 8u, tiles, nspans, st, a);                 \
-    } while (0)
-            if (a.bits == 4) EOQ_LAUNCH_SPLIT(4);
-            else if (a.bits == 2) EOQ_LAUNCH_SPLIT(2);
-            else EOQ_LAUNCH_SPLIT(8);
-#undef EOQ_LAUNCH_SPLIT
-        } else
-        if (a.bits == 4) { if (bf) EOQ_LAUNCH_MMA(4, true); else EOQ_LAUNCH_MMA(4, false); }
-        else if (a.bits == 2) { if (bf) EOQ_LAUNCH_MMA(2, true); else EOQ_LAUNCH_MMA(2, false); }
-        else { if (bf) EOQ_LAUNCH_MMA(8, true); else EOQ_LAUNCH_MMA(8, false); }
-#undef EOQ_LAUNCH_MMA
+        cudaError_t e;
+        if (a.bits == 4) e = bf ? launch_packed_mma(gemv_packed_mma_kernel<4, true>, 0u, tiles, nspans, st, a) : launch_packed_mma(gemv_packed_mma_kernel<4, false>, 0u, tiles, nspans, st, a);
+        else if (a.bits == 2) e = bf ? launch_packed_mma(gemv_packed_mma_kernel<2, true>, 0u, tiles, nspans, st, a) : launch_packed_mma(gemv_packed_mma_kernel<2, false>, 0u, tiles, nspans, st, a);
+        else e = bf ? launch_packed_mma(gemv_packed_mma_kernel<8, true>, 8u, tiles, nspans, st, a) : launch_packed_mma(gemv_packed_mma_kernel<8, false>, 8u, tiles, nspans, st, a);
         g_launches++;
         return (int)e;
     }
@@ -3526,150 +3472,12 @@ __global__ void __launch_bounds__(256) gemv_polar_codes_kernel(const PolarCodesA
         }
 }
 
-// The same product on the warp-level tensor cores, for blocks of 64 columns and more.  The operands of
-// mma.sync.m16n8k16 are fp16, a centroid and a rotated activation are fp32: each is split into the fp16 nearest to it
-// and the fp16 nearest to the remainder (c = c_hi + c_lo to about 2^-22), and the product is taken as
-// c_hi x_hi + (c_hi x_lo + c_lo x_hi), three instructions per sixteen columns with fp32 accumulation; the term left
-// out is 2^-22 of the result.  The centroid table holds both halves of an entry in one 32-bit word, once per lane
-// (conflict-free, as above); two look-ups and two byte permutes give the pair registers {hi_a, hi_b}, {lo_a, lo_b} of
-// two adjacent columns, which is the order the activations are stored in, so they need no permutation.  Lane (g, t)
-// takes sixteen codes of rows g and g + 8 per 64-column span (one 16-byte load each, the next span's requested
-// before this one's are consumed) and the same sixteen columns of activation row g from the caller's split copy
-// (xsplit: [hi | lo][batch][K] fp16).  A CTA is a 16-row tile; its warps share the spans and meet in shared memory.
-template <int NB>
-__global__ void __launch_bounds__(512) gemv_polar_mma_kernel(const PolarCodesArgs a)
-{
-    extern __shared__ uint32_t polar_lut2[];                     // [entries][32 lanes]: lo << 16 | hi
-    __shared__ float red[kMmaMaxWarps][NB][16][8];
-    for (uint32_t i = threadIdx.x; i < a.entries * 32u; i += blockDim.x) {
-        const float c = __ldg(a.centroids + (i >> 5));
-        const __half hi = __float2half_rn(c), lo = __float2half_rn(c - __half2float(hi));
-        polar_lut2[i] = (uint32_t)__half_as_ushort(hi) | ((uint32_t)__half_as_ushort(lo) << 16);
-    }
-    __syncthreads();
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5, g = lane >> 2, t = lane & 3u;
-    const uint32_t row0 = blockIdx.x * 16u, nspans = a.K >> 6, blocks_per_row = a.K >> a.block_shift;
-    const uint32_t lut_lane = (uint32_t)__cvta_generic_to_shared(polar_lut2) + lane * 4u, emask = (a.entries - 1u) << 7;
-    const uint8_t *pw[2];
-    const uint16_t *pn[2];
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-        const uint32_t row = min(row0 + r * 8u + g, a.N - 1u);
-        pw[r] = a.codes + (size_t)row * a.K + t * 16u;
-        pn[r] = a.norms + (size_t)row * blocks_per_row;
-    }
-    // activation rows 8n + g: their hi and lo halves, or the zero block with no stride where a row does not exist
-    const uint16_t *xh[NB], *xl[NB];
-    uint32_t xstep[NB];
-    float tot[NB][4];
-#pragma unroll
-    for (int n = 0; n < NB; n++) {
-        const bool has = 8u * n + g < a.batch;
-        xh[n] = has ? a.xsplit + (size_t)(8u * n + g) * a.K + t * 16u : reinterpret_cast<const uint16_t *>(kZeroBlock);
-        xl[n] = has ? xh[n] + (size_t)a.batch * a.K : xh[n];
-        xstep[n] = has ? 64u : 0u;
-#pragma unroll
-        for (int i = 0; i < 4; i++) tot[n][i] = 0.0f;
-    }
-
-    auto load_span = [&](uint32_t s, uint32_t (&w)[2][4], uint16_t (&nr)[2]) {
-        if (s >= nspans) return;
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(pw[r] + s * 64u));
-            w[r][0] = v.x; w[r][1] = v.y; w[r][2] = v.z; w[r][3] = v.w;
-            nr[r] = __ldg(pn[r] + ((s << 6) >> a.block_shift));
-        }
-    };
-    auto compute_span = [&](uint32_t s, const uint32_t (&w)[2][4], const uint16_t (&nr)[2]) {
-        uint32_t hi[2][8], lo[2][8];                              // [row g, row g + 8][pair]: columns 2 pair, 2 pair + 1 of the lane's sixteen
-#pragma unroll
-        for (int r = 0; r < 2; r++)
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-#pragma unroll
-                for (int p = 0; p < 2; p++) {
-                    const uint32_t wj = w[r][j];
-                    const uint32_t oa = (p == 0 ? wj << 7 : wj >> 9) & emask, ob = (p == 0 ? wj >> 1 : wj >> 17) & emask;      // 128 * code
-                    uint32_t ea, eb;
-                    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(ea) : "r"(lut_lane + oa));
-                    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(eb) : "r"(lut_lane + ob));
-                    hi[r][2 * j + p] = __byte_perm(ea, eb, 0x5410u);
-                    lo[r][2 * j + p] = __byte_perm(ea, eb, 0x7632u);
-                }
-        const float fa = half_bits_to_float(nr[0]), fb = half_bits_to_float(nr[1]);
-#pragma unroll
-        for (int n = 0; n < NB; n++) {
-            uint32_t xq[2][8];                                    // [hi, lo][pair of adjacent columns]
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const uint4 vh = __ldg(reinterpret_cast<const uint4 *>(xh[n] + s * xstep[n]) + h), vl = __ldg(reinterpret_cast<const uint4 *>(xl[n] + s * xstep[n]) + h);
-                xq[0][4 * h] = vh.x; xq[0][4 * h + 1] = vh.y; xq[0][4 * h + 2] = vh.z; xq[0][4 * h + 3] = vh.w;
-                xq[1][4 * h] = vl.x; xq[1][4 * h + 1] = vl.y; xq[1][4 * h + 2] = vl.z; xq[1][4 * h + 3] = vl.w;
-            }
-            float c[4], d[4];
-            mma_m16n8k16_first<false>(c, hi[0][0], hi[1][0], hi[0][1], hi[1][1], xq[0][0], xq[0][1]);
-            mma_m16n8k16_first<false>(d, hi[0][0], hi[1][0], hi[0][1], hi[1][1], xq[1][0], xq[1][1]);
-            mma_m16n8k16<false>(d, lo[0][0], lo[1][0], lo[0][1], lo[1][1], xq[0][0], xq[0][1]);
-#pragma unroll
-            for (int m = 1; m < 4; m++) {
-                mma_m16n8k16<false>(c, hi[0][2 * m], hi[1][2 * m], hi[0][2 * m + 1], hi[1][2 * m + 1], xq[0][2 * m], xq[0][2 * m + 1]);
-                mma_m16n8k16<false>(d, hi[0][2 * m], hi[1][2 * m], hi[0][2 * m + 1], hi[1][2 * m + 1], xq[1][2 * m], xq[1][2 * m + 1]);
-                mma_m16n8k16<false>(d, lo[0][2 * m], lo[1][2 * m], lo[0][2 * m + 1], lo[1][2 * m + 1], xq[0][2 * m], xq[0][2 * m + 1]);
-            }
-            tot[n][0] = fmaf(fa, c[0] + d[0], tot[n][0]); tot[n][1] = fmaf(fa, c[1] + d[1], tot[n][1]);
-            tot[n][2] = fmaf(fb, c[2] + d[2], tot[n][2]); tot[n][3] = fmaf(fb, c[3] + d[3], tot[n][3]);
-        }
-    };
-
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    uint32_t wbuf[2][2][4];
-    uint16_t nbuf[2][2];
-    load_span(warp, wbuf[0], nbuf[0]);
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (uint32_t s = warp; s < nspans; s += 2u * nwarps) {
-#pragma unroll
-        for (int dd = 0; dd < 2; dd++) {
-            const uint32_t sd = s + dd * nwarps;
-            if (sd >= nspans) break;
-            load_span(sd + nwarps, wbuf[dd ^ 1], nbuf[dd ^ 1]);
-            compute_span(sd, wbuf[dd], nbuf[dd]);
-        }
-    }
-#pragma unroll
-    for (int n = 0; n < NB; n++) {
-        red[warp][n][g][2 * t] = tot[n][0]; red[warp][n][g][2 * t + 1] = tot[n][1];
-        red[warp][n][g + 8][2 * t] = tot[n][2]; red[warp][n][g + 8][2 * t + 1] = tot[n][3];
-    }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < NB * 128u; i += blockDim.x) {
-        const uint32_t n = i >> 7, r = (i >> 3) & 15u, b = 8u * n + (i & 7u), row = row0 + r;
-        float v = 0.0f;
-        for (uint32_t w = 0; w < nwarps; w++) v += red[w][n][r][i & 7u];
-        if (row < a.N && b < a.batch) store_y(a.y, (size_t)b * a.N + row, v + (a.bias ? __ldg(a.bias + row) : 0.0f), a.y_dtype);
-    }
-}
-
 // K a multiple of 16 and of the block, the block a power of two >= 16, entries a power of two <= 256, codes and the
-// activations 16-byte aligned, batch <= 8: checked by the caller.  With a split copy of the activations (xsplit) and
-// blocks of 64 columns or more: the tensor-core form, batch <= 32.
+// activations 16-byte aligned, batch <= 8: checked by the caller.
 int launch_gemv_polar_codes(const PolarCodesArgs &a, void *stream)
 {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const size_t smem = (size_t)a.entries * 128u;                   // the table, once per lane
-    if (a.xsplit) {
-        const uint32_t tiles = (a.N + 15u) / 16u, nspans = a.K >> 6;
-        cudaError_t e = cudaSuccess;
-        if (a.batch <= 8) e = launch_packed_mma(gemv_polar_mma_kernel<1>, 0u, tiles, nspans, st, a, smem);
-        else if (a.batch <= 16) e = launch_packed_mma(gemv_polar_mma_kernel<2>, 0u, tiles, nspans, st, a, smem);
-        else {
-            // 32 KB of meeting space beside a table of up to 32 KB: past the 48 KB a kernel gets without asking
-            if (smem > 16u * 1024u) e = cudaFuncSetAttribute(gemv_polar_mma_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e == cudaSuccess) e = launch_packed_mma(gemv_polar_mma_kernel<4>, 0u, tiles, nspans, st, a, smem);
-        }
-        g_launches++;
-        return (int)e;
-    }
     const uint32_t warps = 8, grid = (a.N + warps * 2u - 1u) / (warps * 2u);
     if (a.batch > 8) return (int)cudaErrorInvalidValue;
     if (a.batch <= 1) gemv_polar_codes_kernel<1><<<grid, warps * 32, smem, st>>>(a);

@@ -27,9 +27,16 @@
 
 #include "../../include/eoq_b200.h"
 
+extern "C" int eoq_b200_linear_packed_preferred(const uint8_t *d_packed, uint32_t rows, uint32_t cols, uint32_t bits, uint32_t group,
+                                                const void *x, int x_dtype, uint32_t batch);
+
 namespace {
 
 using at::Tensor;
+
+// A single row against a large PolarLinear is the CUDA-core kernel's: 14336 x 4096 34.0 against 37.5 us; 4096 x 4096 16.1
+// against 13.9, two rows of the former 79 against 37.7.
+constexpr int64_t kPolarSingleRowWeights = 32 << 20;
 
 int dtype_code(at::ScalarType t)
 {
@@ -125,65 +132,88 @@ PyObject *weight_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
     GUARD_END
 }
 
-// packed_linear(packed, scales, N, K, bits, group, rows, x, bias): QuantizedLinear.forward.  Up to `rows` rows straight
-// from the packed codes, more by one dequantisation and a library GEMM.
+// packed_linear(packed, scales, N, K, bits, group, x, bias): QuantizedLinear.forward.  Up to eight rows of 16-bit
+// activations against groups of whole 128-column spans by the warp-level tensor-core GEMV, otherwise by the tcgen05 kernel
+// where it takes the shape and is the quicker one, else by a dequantised copy and a library GEMM.
 PyObject *packed_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
-    if (n != 9) { PyErr_SetString(PyExc_TypeError, "packed_linear takes 9 arguments"); return nullptr; }
+    if (n != 8) { PyErr_SetString(PyExc_TypeError, "packed_linear takes 8 arguments"); return nullptr; }
     GUARD_BEGIN
-    const Tensor *pk = tensor_of(a[0]), *sc = tensor_of(a[1]), *x = tensor_of(a[7]);
-    const int64_t N = PyLong_AsLongLong(a[2]), K = PyLong_AsLongLong(a[3]), bits = PyLong_AsLongLong(a[4]),
-                  group = PyLong_AsLongLong(a[5]), most = PyLong_AsLongLong(a[6]);
+    const Tensor *pk = tensor_of(a[0]), *sc = tensor_of(a[1]), *x = tensor_of(a[6]);
+    const int64_t N = PyLong_AsLongLong(a[2]), K = PyLong_AsLongLong(a[3]), bits = PyLong_AsLongLong(a[4]), group = PyLong_AsLongLong(a[5]);
     int code;
     int64_t rows;
     const float *b;
-    if (!x || !pk || !activations(*x, K, code, rows) || !bias_ptr(a[8], *x, N, b) || group <= 0) Py_RETURN_NONE;
+    if (!x || !pk || !activations(*x, K, code, rows) || !bias_ptr(a[7], *x, N, b) || group <= 0) Py_RETURN_NONE;
     const at::ScalarType pt = bits == 4 || bits == 2 ? at::kByte : at::kChar;
     const int64_t row_bytes = bits == 4 ? (K + 1) / 2 : bits == 2 ? (K + 3) / 4 : K;
     if (!resident(pk, *x, pt) || !resident(sc, *x, at::kHalf) || pk->numel() != N * row_bytes || sc->numel() < (N * K + group - 1) / group)
         Py_RETURN_NONE;
+    // two-bit codes in groups below 128 columns against a few fp32 rows stay with the entropy-coded GEMV
+    if (bits == 2 && code == EOQ_B200_F32 && rows <= 8 && group % 128 && group % 16 == 0 && K % group == 0) Py_RETURN_NONE;
     void *st = stream_of(*x);
     const uint8_t *codes = static_cast<const uint8_t *>(pk->data_ptr());
     const uint16_t *scales = static_cast<const uint16_t *>(sc->data_ptr());
-    if (rows <= most) {
-        Tensor y = result(*x, N, x->scalar_type()), scratch;
-        // fp32 activations on the tensor cores: room for their two fp16 halves
-        if (code == EOQ_B200_F32) scratch = at::detail::empty_cuda({rows, K}, at::kFloat, x->device(), std::nullopt);
+    const bool f32 = code == EOQ_B200_F32, aligned = (reinterpret_cast<uintptr_t>(codes) & 15u) == 0;
+    if (rows <= 8 && !f32 && aligned && K % 128 == 0 && group % 128 == 0 && K % group == 0) {
+        Tensor y = result(*x, N, x->scalar_type());
         return done(eoq_b200_gemv_packed(codes, scales, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)group, x->data_ptr(), code,
-                                         (uint32_t)rows, scratch.defined() ? scratch.data_ptr() : nullptr, y.data_ptr(), code, b, st),
+                                         (uint32_t)rows, nullptr, y.data_ptr(), code, b, st),
                     std::move(y));
     }
+    if (eoq_b200_linear_packed_preferred(codes, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)group, x->data_ptr(), code, (uint32_t)rows)) {
+        Tensor y = result(*x, N, x->scalar_type()), scratch;
+        // fp32 activations: room for their two fp16 halves and a factor per row
+        if (f32) scratch = at::detail::empty_cuda({rows, K + 1}, at::kFloat, x->device(), std::nullopt);
+        return done(eoq_b200_linear_packed(codes, scales, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)group, x->data_ptr(), code,
+                                           (uint32_t)rows, f32 ? scratch.data_ptr() : nullptr, y.data_ptr(), code, b, st),
+                    std::move(y));
+    }
+    if (rows <= 8) Py_RETURN_NONE;           // shapes none of these kernels takes: the entropy-coded form may
     Tensor dense = at::detail::empty_cuda({N, K}, x->scalar_type(), x->device(), std::nullopt);
     if (eoq_b200_dequant_packed(codes, scales, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)group, 0, (uint32_t)N, dense.data_ptr(),
                                 code, st) != EOQ_OK)
         Py_RETURN_NONE;
     at::AutoDispatchBelowADInplaceOrView guard;
     std::optional<Tensor> bias;
-    if (b) bias = THPVariable_Unpack(a[8]).to(x->scalar_type());
+    if (b) bias = THPVariable_Unpack(a[7]).to(x->scalar_type());
     return THPVariable_Wrap(at::linear(*x, dense, bias));
     GUARD_END
 }
 
-// polar_linear(codes, norms, centroids, N, K, bits, block, x): the product of PolarLinear.forward as fp16, without bias,
-// up to 32 rows (8 for blocks below 64 columns) straight from the byte codes.
+// polar_linear(codes, norms, centroids, N, K, bits, block, x, bias): PolarLinear.forward, fp16 results, from the byte codes.
+// One row on the CUDA cores; more, and blocks of 64, 128 or 256 columns, by the tcgen05 kernel.
 PyObject *polar_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
-    if (n != 8) { PyErr_SetString(PyExc_TypeError, "polar_linear takes 8 arguments"); return nullptr; }
+    if (n != 9) { PyErr_SetString(PyExc_TypeError, "polar_linear takes 9 arguments"); return nullptr; }
     GUARD_BEGIN
     const Tensor *cd = tensor_of(a[0]), *nr = tensor_of(a[1]), *ct = tensor_of(a[2]), *x = tensor_of(a[7]);
     const int64_t N = PyLong_AsLongLong(a[3]), K = PyLong_AsLongLong(a[4]), bits = PyLong_AsLongLong(a[5]), block = PyLong_AsLongLong(a[6]);
     int code;
     int64_t rows;
     if (!x || !activations(*x, K, code, rows) || block < 16 || (block & (block - 1)) || K % block || bits < 1 || bits > 8) Py_RETURN_NONE;
-    if (rows > (block >= 64 ? 32 : 8) || !resident(cd, *x, at::kChar) || !resident(nr, *x, at::kHalf) || !resident(ct, *x, at::kFloat) ||
-        cd->numel() < N * K || nr->numel() < N * K / block || ct->numel() < (1 << bits))
+    if (!resident(cd, *x, at::kChar) || !resident(nr, *x, at::kHalf) || !resident(ct, *x, at::kFloat) || cd->numel() < N * K ||
+        nr->numel() < N * K / block || ct->numel() < (1 << bits))
         Py_RETURN_NONE;
-    Tensor y = result(*x, N, at::kHalf), scratch = at::detail::empty_cuda({rows, K}, at::kFloat, x->device(), std::nullopt);
-    return done(eoq_b200_gemv_polar_codes(static_cast<const uint8_t *>(cd->data_ptr()), static_cast<const uint16_t *>(nr->data_ptr()),
-                                          static_cast<const float *>(ct->data_ptr()), (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)block,
-                                          x->data_ptr(), code, (uint32_t)rows, scratch.data_ptr(), y.data_ptr(), EOQ_B200_F16, nullptr, -1,
-                                          stream_of(*x)),
-                std::move(y));
+    const Tensor *bias = a[8] == Py_None ? nullptr : tensor_of(a[8]);
+    if (a[8] != Py_None && (!resident(bias, *x, at::kHalf) || bias->numel() != N)) Py_RETURN_NONE;
+    const uint8_t *codes = static_cast<const uint8_t *>(cd->data_ptr());
+    const uint16_t *norms = static_cast<const uint16_t *>(nr->data_ptr());
+    const float *cent = static_cast<const float *>(ct->data_ptr());
+    Tensor y = result(*x, N, at::kHalf), scratch = at::detail::empty_cuda({rows, K + 1}, at::kFloat, x->device(), std::nullopt);
+    if (rows > 1 || N * K < kPolarSingleRowWeights) {
+        eoq_error_t rc = eoq_b200_linear_polar_codes(codes, norms, cent, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)block, x->data_ptr(), code,
+                                                     (uint32_t)rows, scratch.data_ptr(), y.data_ptr(), EOQ_B200_F16,
+                                                     bias ? bias->data_ptr() : nullptr, EOQ_B200_F16, stream_of(*x));
+        if (rc == EOQ_OK) return THPVariable_Wrap(std::move(y));
+    }
+    if (rows > (block >= 64 ? 32 : 8)) Py_RETURN_NONE;
+    if (eoq_b200_gemv_polar_codes(codes, norms, cent, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)block, x->data_ptr(), code, (uint32_t)rows,
+                                  scratch.data_ptr(), y.data_ptr(), EOQ_B200_F16, nullptr, -1, stream_of(*x)) != EOQ_OK)
+        Py_RETURN_NONE;
+    at::AutoDispatchBelowADInplaceOrView guard;
+    if (bias) y.add_(*bias);
+    return THPVariable_Wrap(std::move(y));
     GUARD_END
 }
 

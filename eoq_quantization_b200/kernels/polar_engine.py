@@ -109,10 +109,9 @@ class PolarLinear(nn.Module):
         buffers = self._buffers                 # not through nn.Module.__getattr__, which costs as much as the call
         if not self.entropy_coded and buffers["awq_scales"] is None:
             y = _lib.native().polar_linear(buffers["codes"], buffers["norms"], buffers["centroids"], self.out_features, self.in_features,
-                                           self.bits, self.block_size, x)
+                                           self.bits, self.block_size, x, buffers["bias"] if "bias" in buffers else self.bias)
             if y is not None:
-                bias = buffers["bias"] if "bias" in buffers else self.bias
-                return y + bias if bias is not None else y
+                return y
         require_cuda(x, "PolarLinear.forward")
         require_cuda(self.codes, "PolarLinear.forward")
         x2 = x.reshape(-1, self.in_features)

@@ -475,6 +475,28 @@ eoq_error_t eoq_b200_gemv_packed(const uint8_t *d_packed, const uint16_t *d_scal
                                  uint32_t bits, uint32_t group, const void *x, int x_dtype, uint32_t batch, void *d_scratch,
                                  void *y, int y_dtype, const float *bias, void *stream);
 
+/* y = x @ W.T (+ bias) from the same packed form for any number of activation rows, on the fifth-generation tensor cores:
+ * dequantised tiles exist in tensor memory only.  Up to 128 rows (any number of fp32 ones) the codes are multiplied exactly
+ * and the scales applied in fp32; beyond, code x scale is rounded to x's 16-bit type first, as dequantise-then-matmul does.
+ * Takes whole scale groups per row, groups that are multiples of 32, rows of codes that are multiples of 16 bytes, and
+ * 16-byte aligned pointers (EOQ_ERR_UNSUPPORTED otherwise, nothing launched).  d_scratch: batch * (cols + 1) * 4 bytes,
+ * 16-byte aligned, for fp32 x (its two fp16 halves and row factors); unused, may be NULL, for 16-bit x.  Device pointers;
+ * asynchronous. */
+eoq_error_t eoq_b200_linear_packed(const uint8_t *d_packed, const uint16_t *d_scales_fp16, uint32_t rows, uint32_t cols,
+                                   uint32_t bits, uint32_t group, const void *x, int x_dtype, uint32_t batch, void *d_scratch,
+                                   void *y, int y_dtype, const float *bias, void *stream);
+
+/* The same from PolarLinear's byte codes (see eoq_b200_gemv_polar_codes), any number of activation rows, blocks of 64, 128
+ * or 256 columns; rotated activations and centroids as two fp16 halves each.  bias: NULL, fp32 or fp16.  d_scratch:
+ * batch * (cols + 1) * 4 bytes. */
+eoq_error_t eoq_b200_linear_polar_codes(const uint8_t *d_codes, const uint16_t *d_norms_fp16, const float *d_centroids,
+                                        uint32_t rows, uint32_t cols, uint32_t bits, uint32_t block, const void *x, int x_dtype,
+                                        uint32_t batch, void *d_scratch, void *y, int y_dtype, const void *bias, int bias_dtype,
+                                        void *stream);
+
+/* 0, or nonzero if a bounded wait of one of these kernels has run out on the current device since the last call (synchronises). */
+uint32_t eoq_b200_linear_status(void);
+
 /* y = x @ W.T (+ bias) straight from PolarLinear's in-memory form (kernels/polar_engine.py:144-360: one centroid index
  * per byte, one fp16 norm per block of each row, 2^bits fp32 centroids), for up to 8 activation rows on the CUDA cores
  * and 32 on the tensor cores.  Two launches:

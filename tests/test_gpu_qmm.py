@@ -1,0 +1,91 @@
+"""``eoq_b200_linear_packed`` / ``eoq_b200_linear_polar_codes``: activations times weights that stay quantised, on tcgen05 tensor
+cores, against the dequantised product in fp64 at the edges of its tiles: weight rows around 128, tokens around the token
+tiles of every variant, column counts that end inside a block or a weight copy, groups of half a block to several."""
+import numpy as np
+import pytest
+import torch
+
+from eoq_quantization_b200 import _lib as L
+from eoq_quantization_b200.core.polar_quant import hadamard_matrix
+from eoq_quantization_b200.core.quantized_linear import QuantizedLinear
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+CODE = {torch.float16: L.F16, torch.bfloat16: L.BF16, torch.float32: L.F32}
+
+
+def _pack(c, bits):
+    if bits == 8:
+        return c.to(torch.int8).contiguous()
+    u = (c + (1 << (bits - 1)) - 1).to(torch.uint8)
+    per = 8 // bits
+    return sum(u[:, i::per] << (bits * i) for i in range(per)).to(torch.uint8).contiguous()
+
+
+def _stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+@pytest.mark.parametrize("bits", [2, 4, 8])
+@pytest.mark.parametrize("n,k,group", [(1, 128, 32), (127, 192, 64), (300, 1344, 96), (129, 4096, 256), (1000, 2816, 128), (2500, 1024, 1024)])
+def test_packed_product(bits, n, k, group):
+    g = torch.Generator(device="cuda").manual_seed(bits + n)
+    qmax = (1 << (bits - 1)) - 1
+    c = torch.randint(-qmax, qmax + 1, (n, k), generator=g, device="cuda")
+    s = (torch.rand(n, k // group, generator=g, device="cuda") * 0.01 + 1e-3).half()
+    dense = (c.double().view(n, -1, group) * s.double()[:, :, None]).view(n, k) if k % group == 0 else None
+    packed, bias = _pack(c, bits), torch.randn(n, generator=g, device="cuda")
+    for dt in CODE:
+        for m in (1, 16, 17, 32, 33, 64, 65, 128, 129, 257, 600):
+            x = torch.randn(m, k, generator=g, device="cuda").to(dt)
+            y = torch.empty(m, n, dtype=torch.float32, device="cuda")
+            scratch = torch.empty(m * (k + 1), device="cuda")
+            rc = L.lib().eoq_b200_linear_packed(packed.data_ptr(), s.data_ptr(), n, k, bits, group, x.data_ptr(), CODE[dt], m, scratch.data_ptr(),
+                                                y.data_ptr(), L.F32, bias.data_ptr(), _stream())
+            if k % (64 if bits == 2 else 32 if bits == 4 else 16):
+                assert rc == L.EOQ_ERR_UNSUPPORTED
+                continue
+            assert rc == L.EOQ_OK
+            want = x.double() @ dense.T + bias.double()
+            # exact codes and fp32 scales, or (more than 128 rows of 16-bit activations) one rounding of code x scale
+            tol = 2e-6 if m <= 128 or dt == torch.float32 else 4e-4 if dt == torch.float16 else 3e-3
+            assert O.rel_l2(y.cpu().numpy(), want.cpu().numpy()) < tol, (dt, m)
+    assert L.lib().eoq_b200_linear_status() == 0
+
+
+@pytest.mark.parametrize("bits,block", [(3, 64), (5, 64), (8, 128), (4, 256)])
+@pytest.mark.parametrize("n,k", [(1, 256), (130, 1280), (700, 4096)])
+def test_polar_product(bits, block, n, k):
+    g = torch.Generator(device="cuda").manual_seed(bits + n)
+    codes = torch.randint(0, 1 << bits, (n, k), generator=g, device="cuda").to(torch.uint8)
+    norms = (torch.rand(n * k // block, generator=g, device="cuda") * 2 + 0.1).half()
+    cent = torch.sort(torch.randn(1 << bits, generator=g, device="cuda"))[0]
+    H = hadamard_matrix(block).cuda().double()
+    dense = ((cent.double()[codes.long()].view(-1, block) / block ** 0.5) @ H * norms.double()[:, None]).view(n, k)
+    bias = torch.randn(n, generator=g, device="cuda").half()
+    for dt in CODE:
+        for m, size in ((1, 1.0), (16, 1e-5), (33, 1.0), (128, 1e5), (200, 1.0)):          # rows of any magnitude
+            x = (torch.randn(m, k, generator=g, device="cuda") * (size if dt != torch.float16 else 1.0)).to(dt)
+            y = torch.empty(m, n, dtype=torch.float32, device="cuda")
+            scratch = torch.empty(m * (k + 1), device="cuda")
+            assert L.lib().eoq_b200_linear_polar_codes(codes.data_ptr(), norms.data_ptr(), cent.data_ptr(), n, k, bits, block, x.data_ptr(), CODE[dt], m,
+                                                       scratch.data_ptr(), y.data_ptr(), L.F32, bias.data_ptr(), L.F16, _stream()) == L.EOQ_OK
+            want = x.double() @ dense.T + bias.double()
+            assert O.rel_l2(y.cpu().numpy(), want.cpu().numpy()) < 2e-6, (dt, m)
+    assert L.lib().eoq_b200_linear_status() == 0
+
+
+def test_modules_fall_back_outside_the_native_route():
+    """Gradients through x, activations that are not contiguous or not aligned, no rows: the Python path, same results."""
+    torch.manual_seed(1)
+    ql = QuantizedLinear.from_float(torch.nn.Linear(256, 96), bits=4, block_size=64).cuda()
+    w = ql._dequantize_weight()
+    x = torch.randn(40, 256, device="cuda")
+    want = torch.nn.functional.linear(x, w, ql.bias_param)
+    for arg in (x, torch.randn(256, 40, device="cuda").copy_(x.T).T, torch.cat([x.flatten(), x.flatten()[:1]])[1:].view(40, 256)):
+        ref = want if arg is x or arg.shape == x.shape and torch.equal(arg, x) else torch.nn.functional.linear(arg, w, ql.bias_param)
+        assert O.rel_l2(ql(arg).cpu().numpy(), ref.cpu().numpy()) < 1e-5
+    assert ql(x[:0]).shape == (0, 96)
+    xg = x.clone().requires_grad_()
+    ql(xg).sum().backward()
+    assert O.rel_l2(xg.grad.cpu().numpy(), w.sum(0).expand(40, -1).cpu().numpy()) < 1e-5
