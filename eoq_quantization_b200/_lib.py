@@ -46,11 +46,11 @@ EXPORTS = [
     "eoq_b200_gather_create", "eoq_b200_gather_connect", "eoq_b200_gather_destroy", "eoq_b200_gather_buffer",
     "eoq_b200_gather_status", "eoq_b200_gather_set_timeout_ms", "eoq_b200_gather_wait", "eoq_b200_gemv_gather", "eoq_b200_gemv_static_scratch", "eoq_b200_gemv_host", "eoq_b200_gemv_host_async", "eoq_b200_weight_decode",
     "eoq_b200_dequant_packed", "eoq_b200_gemv_packed", "eoq_b200_gemv_polar_codes",
-    "eoq_b200_linear_packed", "eoq_b200_linear_polar_codes",
+    "eoq_b200_linear_packed", "eoq_b200_linear_polar_codes", "eoq_b200_weight_linear", "eoq_b200_weight_linear_scratch",
     "eoq_b200_linear_status", "eoq_b200_weight_status",
 ]
 #: exported for this project's benchmarks and tests only (declared in csrc/eoq_internal.h, not in the public header)
-INTERNAL_EXPORTS = ["eoq_b200_linear_packed_preferred", "eoq_b200_tune", "eoq_b200_launch_count", "eoq_b200_weight_read"]
+INTERNAL_EXPORTS = ["eoq_b200_linear_packed_preferred", "eoq_b200_weight_linear_preferred", "eoq_b200_tune", "eoq_b200_launch_count", "eoq_b200_weight_read"]
 
 
 class EOQError(RuntimeError):
@@ -180,6 +180,8 @@ def lib() -> C.CDLL:
         "eoq_b200_gemv_polar_codes": (C.c_int, [vp, vp, vp, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, vp, C.c_int, C.c_uint32, vp, vp, C.c_int, vp, C.c_int, vp]),
         "eoq_b200_linear_packed": (C.c_int, [vp, vp, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, vp, C.c_int, C.c_uint32, vp, vp, C.c_int, vp, vp]),
         "eoq_b200_linear_polar_codes": (C.c_int, [vp, vp, vp, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, vp, C.c_int, C.c_uint32, vp, vp, C.c_int, vp, C.c_int, vp]),
+        "eoq_b200_weight_linear": (C.c_int, [vp, vp, C.c_int, C.c_uint32, vp, vp, C.c_int, vp, vp]),
+        "eoq_b200_weight_linear_scratch": (C.c_size_t, [vp, C.c_uint32, C.c_int]),
         "eoq_b200_linear_status": (C.c_uint32, []),
         "eoq_b200_weight_status": (C.c_int, [vp, vp]),
         "eoq_b200_tune": (C.c_int, [C.c_char_p, C.c_int]),

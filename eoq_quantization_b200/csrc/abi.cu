@@ -1694,7 +1694,7 @@ extern "C" eoq_error_t eoq_b200_gemv_host(eoq_b200_weight_t *w, const void *x, i
     return eoq_b200_weight_status(w, stream);       // reads the status word and synchronises the stream
 }
 
-extern "C" eoq_error_t eoq_b200_weight_decode(eoq_b200_weight_t *w, uint8_t *d_sym, int packed, void *d_dequant, int out_dtype, void *stream)
+static eoq_error_t weight_decode(eoq_b200_weight_t *w, uint8_t *d_sym, int packed, void *d_dequant, int out_dtype, int early, void *stream)
 {
     if (!w) return EOQ_ERR_NULL_PTR;
     if (!d_sym && !d_dequant) return EOQ_OK;
@@ -1709,11 +1709,16 @@ extern "C" eoq_error_t eoq_b200_weight_decode(eoq_b200_weight_t *w, uint8_t *d_s
     a.scales = w->scales.as<uint16_t>(); a.centroids = w->centroids.as<float>();
     a.status = w->status_word();
     a.out_sym = d_sym; a.out_deq = d_dequant; a.N = w->N; a.K = w->K; a.group = w->group; a.p = w->p; a.ntiles = w->ntiles;
-    a.packed = packed; a.out_dtype = out_dtype;
+    a.packed = packed; a.out_dtype = out_dtype; a.early = early;
     a.scales_t = w->scales_t.as<uint2>(); a.nseg = w->nseg; a.nrb = w->nrb; a.Npad = w->Npad; a.stage_bytes = w->stage_bytes;
     int e = launch_decode_tiles(a, w->G, w->bits, w->kind, stream);
     if (e != 0) { std::fprintf(stderr, "eoq_b200_weight_decode: launch failed: %s\n", cudaGetErrorString((cudaError_t)e)); return EOQ_ERR_CUDA; }
     return EOQ_OK;
+}
+
+extern "C" eoq_error_t eoq_b200_weight_decode(eoq_b200_weight_t *w, uint8_t *d_sym, int packed, void *d_dequant, int out_dtype, void *stream)
+{
+    return weight_decode(w, d_sym, packed != 0, d_dequant, out_dtype, 0, stream);
 }
 
 extern "C" eoq_error_t eoq_b200_dequant_packed(const uint8_t *d_packed, const uint16_t *d_scales_fp16, uint32_t rows, uint32_t cols,
@@ -1833,6 +1838,59 @@ extern "C" eoq_error_t eoq_b200_linear_polar_codes(const uint8_t *d_codes, const
     if (e == 0) e = launch_qmm(c, stream);
     if (e != 0) { std::fprintf(stderr, "eoq_b200_linear_polar_codes: launch failed: %s\n", cudaGetErrorString((cudaError_t)e)); return EOQ_ERR_CUDA; }
     return EOQ_OK;
+}
+
+// Bytes of scratch eoq_b200_weight_linear needs in front of the activations' part: the weight's codes, two per byte.
+static size_t weight_codes_bytes(const eoq_b200_weight_t *w) { return ((size_t)w->Npad * w->K / 2 + 255) & ~(size_t)255; }
+
+// Layouts that eoq_b200_weight_linear takes: the pair layout (4-bit codes, three per step; tiles that the pair decoder
+// stages whole), groups the product kernel takes.
+static bool weight_linear_takes(const eoq_b200_weight_t *w, const void *x, int x_dtype)
+{
+    return w->kind == EOQ_B200_KIND_INT4_ABSMAX && w->bits == 4 && w->G == 3 && w->scales_t.p && w->stage_bytes <= 6144u && w->p <= 13u &&
+           qmm_takes(w->K, 4, w->group, nullptr, x) && (x_dtype != EOQ_B200_F32 || split_rows_takes(w->K, 1));
+}
+
+extern "C" size_t eoq_b200_weight_linear_scratch(const eoq_b200_weight_t *w, uint32_t batch, int x_dtype)
+{
+    return w ? weight_codes_bytes(w) + (x_dtype == EOQ_B200_F32 ? (size_t)batch * (w->K + 1u) * 4u : 0u) : 0u;
+}
+
+extern "C" eoq_error_t eoq_b200_weight_linear(eoq_b200_weight_t *w, const void *x, int x_dtype, uint32_t batch, void *d_scratch, void *y,
+                                              int y_dtype, const float *bias, void *stream)
+{
+    if (!w || !x || !y || !d_scratch) return EOQ_ERR_NULL_PTR;
+    if (batch == 0) return EOQ_OK;
+    if (x_dtype < 0 || x_dtype > 2 || y_dtype < 0 || y_dtype > 2) return EOQ_ERR_UNSUPPORTED;
+    if (!weight_linear_takes(w, x, x_dtype) || (reinterpret_cast<uintptr_t>(d_scratch) & 15u)) return EOQ_ERR_UNSUPPORTED;
+    eoq_error_t rc = check_device(w, "eoq_b200_weight_linear");
+    if (rc != EOQ_OK) return rc;
+    uint8_t *codes = static_cast<uint8_t *>(d_scratch), *halves = codes + weight_codes_bytes(w);
+    // the activations' halves first: the codes' kernel then is the one that the product follows directly and waits for
+    int e = 0;
+    float *factors = reinterpret_cast<float *>(halves + (size_t)batch * w->K * 4);
+    if (x_dtype == EOQ_B200_F32) e = launch_split_rows(x, x_dtype, w->K, batch, 1, halves, factors, stream);
+    if (e == 0) {
+        rc = weight_decode(w, codes, 2, nullptr, 0, 1, stream);
+        if (rc != EOQ_OK) return rc;
+        QmmCall c = packed_call(codes, w->scales.as<uint16_t>(), w->N, w->K, 4, w->group, x, x_dtype, batch, halves, y, y_dtype, bias);
+        if (x_dtype == EOQ_B200_F32) c.tok_scale = factors;
+        c.late = 1;
+        c.blocked_rows = w->Npad;
+        e = launch_qmm(c, stream);
+    }
+    if (e != 0) { std::fprintf(stderr, "eoq_b200_weight_linear: launch failed: %s\n", cudaGetErrorString((cudaError_t)e)); return EOQ_ERR_CUDA; }
+    return EOQ_OK;
+}
+
+// For the torch-facing front (not in the public header): whether eoq_b200_weight_linear takes the call and is to be
+// preferred to a dense decode and a library GEMM (both decode; neither copy is the longer one to speak of).
+extern "C" int eoq_b200_weight_linear_preferred(const eoq_b200_weight_t *w, const void *x, int x_dtype, uint32_t batch)
+{
+    if (!w || !weight_linear_takes(w, x, x_dtype)) return 0;
+    QmmCall c = packed_call(nullptr, nullptr, w->N, w->K, 4, w->group, x, x_dtype, batch, nullptr, nullptr, x_dtype, nullptr);
+    c.blocked_rows = w->Npad;
+    return qmm_preferred(c, 0.0) ? 1 : 0;
 }
 
 extern "C" uint32_t eoq_b200_linear_status(void) { return qmm_status(); }

@@ -160,11 +160,12 @@ struct DecodeArgs {
     const uint16_t *scales;
     const float    *centroids;  // unused for INT4
     uint32_t       *status;
-    uint8_t        *out_sym;    // packed nibbles [N, K/2] or bytes [N, K], or null
+    uint8_t        *out_sym;    // bytes [N, K] (packed = 0), nibbles [N, K/2] (1) or [K/16][Npad] words of sixteen nibbles (2), or null
     void           *out_deq;    // [N, K] or null
     uint32_t N, K, group, p, ntiles;
     uint32_t head_bytes;
     int packed, out_dtype;
+    int early = 0;              // packed codes: the next kernel in the stream may start (it waits before it reads them)
     // the pair layout's extras (4-bit weights, three codes per step): set, they let the dequantised matrix come from
     // the two-tiles-per-warp kernel
     const uint2 *scales_t = nullptr;      // [K / group][Npad / 3] {s0 | s1 << 16, s2}

@@ -1394,15 +1394,31 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_pairs_kernel(const GemvArgs a
         __syncthreads();
 
         if (leader) {
+            // several warps' sums are loaded before the first is added (still in warp order): one at a time the sixteen
+            // cost 2000 cycles of shared-memory latency
             const uint32_t run = min(cs - warp, a.nseg - seg);
-            for (uint32_t w = 1; w < run; w++) {
-                const float *red = reinterpret_cast<const float *>(mine + (size_t)w * region);
+            constexpr uint32_t kU = BT == 1 ? 5 : BT == 2 ? 3 : 1;
+            for (uint32_t w0 = 1; w0 < run; w0 += kU) {
+                float part[kU][2][G][BT];
 #pragma unroll
-                for (int k = 0; k < 2; k++)
+                for (uint32_t u = 0; u < kU; u++) {
+                    const float *red = reinterpret_cast<const float *>(mine + (size_t)min(w0 + u, run - 1u) * region);
 #pragma unroll
-                    for (int j = 0; j < G; j++)
+                    for (int k = 0; k < 2; k++)
 #pragma unroll
-                        for (int b = 0; b < BT; b++) y[k][j][b] += red[((k * G + j) * BT + b) * 32 + lane];
+                        for (int j = 0; j < G; j++)
+#pragma unroll
+                            for (int b = 0; b < BT; b++) part[u][k][j][b] = red[((k * G + j) * BT + b) * 32 + lane];
+                }
+#pragma unroll
+                for (uint32_t u = 0; u < kU; u++)
+                    if (w0 + u < run)
+#pragma unroll
+                        for (int k = 0; k < 2; k++)
+#pragma unroll
+                            for (int j = 0; j < G; j++)
+#pragma unroll
+                                for (int b = 0; b < BT; b++) y[k][j][b] += part[u][k][j][b];
             }
             // runs of this row-block pair are numbered by the chunk they fall in
             const uint32_t slot = t - chunk_of(first_q);
@@ -1971,17 +1987,25 @@ __device__ __forceinline__ void stg_256(void *p, uint32_t a0, uint32_t a1, uint3
                  : "memory");
 }
 
+// "OUT" beside the three float types: the codes themselves, two per byte.  kOutPacked: row by row as QuantizedLinear packs
+// them.  kOutBlocked: [K / 16][Npad] words of eight bytes (sixteen columns of a row), which the tcgen05 product reads as
+// readily and which a warp stores as one contiguous stretch: row by row its 32 lanes write eight bytes to 96 different
+// lines, and the L1's store path bounds the kernel (11008 x 4096: 29.7 us).
+constexpr int kOutPacked = 4, kOutBlocked = 5;
+
 template <int OUT>
 __global__ void __launch_bounds__(512, 1) dequant_pairs_kernel(const DecodeArgs a)
 {
     constexpr int G = 3, kWarps = 16;
     constexpr uint32_t kChunk = 1024, kMaxChunks = 8;
+    constexpr bool kPack = OUT == kOutPacked || OUT == kOutBlocked;
     using F = Fmt<G, 4>;
     using F0 = Int4Field<F::field_bit(0)>;
     using F1 = Int4Field<F::field_bit(1)>;
     using F2 = Int4Field<F::field_bit(2)>;
     extern __shared__ __align__(128) uint8_t dq_smem[];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    if (kPack && a.early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t tab_bytes = 4u << a.p;
     const uint32_t tab_addr = smem_addr(dq_smem), tab_bar = tab_addr + tab_bytes;
     const uint32_t region = 2u * a.stage_bytes + 128u;
@@ -2044,7 +2068,7 @@ __global__ void __launch_bounds__(512, 1) dequant_pairs_kernel(const DecodeArgs 
         uint2 sc_next[2];
         float sc[2][G];
 #pragma unroll
-        for (int k = 0; k < 2; k++) sc_next[k] = ldg_u32x2_pinned(sc_ptr[k] + (size_t)(col0 / a.group) * sc_stride);
+        for (int k = 0; k < 2; k++) if (!kPack) sc_next[k] = ldg_u32x2_pinned(sc_ptr[k] + (size_t)(col0 / a.group) * sc_stride);
         PairChain ch[2];
 #pragma unroll
         for (int k = 0; k < 2; k++) {
@@ -2054,8 +2078,9 @@ __global__ void __launch_bounds__(512, 1) dequant_pairs_kernel(const DecodeArgs 
             ch[k].w = lds_u16(ch[k].addr);
         }
         const uint32_t cend = col0 + ncols;
+        if (kPack && uses == 0) asm volatile("griddepcontrol.wait;" ::: "memory");      // the buffer may be the kernel before's to read
         for (uint32_t c = col0; c < cend; c += 16) {
-            if (c == col0 || c % a.group == 0) {
+            if (!kPack && (c == col0 || c % a.group == 0)) {
                 // a new scale group: take the scales requested a group ago, request the next
 #pragma unroll
                 for (int k = 0; k < 2; k++) {
@@ -2073,6 +2098,11 @@ __global__ void __launch_bounds__(512, 1) dequant_pairs_kernel(const DecodeArgs 
 #pragma unroll
             for (int half = 0; half < 2; half++) {
                 float v[2][G][8];
+                uint32_t word[2][G];                                 // kPack: eight codes
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+#pragma unroll
+                    for (int j = 0; j < G; j++) word[k][j] = 0u;
 #pragma unroll
                 for (int s = 0; s < 8; s++) {
                     uint32_t u[2][3];
@@ -2080,6 +2110,14 @@ __global__ void __launch_bounds__(512, 1) dequant_pairs_kernel(const DecodeArgs 
                     rans_step_int4<F0::kMask, F1::kMask, F2::kMask>(tab_addr, ch[1].x, mask, p, F::kBiasMask, magic0, magic1, magic2, u[1][0], u[1][1], u[1][2]);
 #pragma unroll
                     for (int k = 0; k < 2; k++) {
+                        if (kPack) {
+#pragma unroll
+                            for (int j = 0; j < G; j++) {
+                                const int bit = F::field_bit(j), to = 4 * s;
+                                word[k][j] |= (to >= bit ? u[k][j] << (to - bit) : u[k][j] >> (bit - to)) & (15u << to);
+                            }
+                            continue;
+                        }
                         v[k][0][s] = (__uint_as_float(u[k][0]) - F0::kOffset) * sc[k][0];
                         v[k][1][s] = (__uint_as_float(u[k][1]) - F1::kOffset) * sc[k][1];
                         v[k][2][s] = (__uint_as_float(u[k][2]) - F2::kOffset) * sc[k][2];
@@ -2100,7 +2138,13 @@ __global__ void __launch_bounds__(512, 1) dequant_pairs_kernel(const DecodeArgs 
 #pragma unroll
                     for (int j = 0; j < G; j++) {
                         const uint32_t r = row[k] + j;
-                        if (OUT == EOQ_B200_F32) {
+                        if (kPack) {
+                            if (half == 0) held[k][j][0] = word[k][j];
+                            else if (OUT == kOutBlocked)
+                                reinterpret_cast<uint2 *>(a.out_sym)[(size_t)(c / 16u) * a.Npad + r] = make_uint2(held[k][j][0], word[k][j]);
+                            else if (r < a.N)
+                                *reinterpret_cast<uint2 *>(a.out_sym + ((size_t)r * a.K + c) / 2u) = make_uint2(held[k][j][0], word[k][j]);
+                        } else if (OUT == EOQ_B200_F32) {
                             if (r < a.N)
                                 stg_256(reinterpret_cast<float *>(a.out_deq) + (size_t)r * a.K + c + half * 8,
                                         __float_as_uint(v[k][j][0]), __float_as_uint(v[k][j][1]), __float_as_uint(v[k][j][2]), __float_as_uint(v[k][j][3]),
@@ -2133,10 +2177,12 @@ __global__ void __launch_bounds__(512, 1) dequant_pairs_kernel(const DecodeArgs 
     }
 }
 
-// Whether the pair form serves this call: the dequantised matrix alone, of a weight laid out for the pair kernel.
+// Whether the pair form serves this call: the dequantised matrix alone, or the packed codes alone, of a weight laid out for
+// the pair kernel.
 static bool dequant_takes_pairs(const DecodeArgs &a, uint32_t G, uint32_t bits, uint32_t kind)
 {
-    if (!(kind == EOQ_B200_KIND_INT4_ABSMAX && bits == 4 && G == 3) || !a.out_deq || a.out_sym || !a.scales_t || a.stage_bytes == 0) return false;
+    if (!(kind == EOQ_B200_KIND_INT4_ABSMAX && bits == 4 && G == 3) || !a.scales_t || a.stage_bytes == 0) return false;
+    if (a.out_deq ? a.out_sym != nullptr : !(a.out_sym && a.packed && (reinterpret_cast<uintptr_t>(a.out_sym) & 7u) == 0)) return false;
     if (a.group % 16u != 0 || a.K % 16u != 0) return false;
     const size_t smem = ((size_t)4 << a.p) + 128 + (size_t)16 * (2u * a.stage_bytes + 128u);
     return smem <= 227 * 1024 && (size_t)8 * 1024 >= a.stage_bytes;
@@ -2147,13 +2193,23 @@ static int launch_dequant_pairs(const DecodeArgs &a, cudaStream_t st)
     const size_t smem = ((size_t)4 << a.p) + 128 + (size_t)16 * (2u * a.stage_bytes + 128u);
     const uint32_t npairs = ((a.nrb + 1u) / 2u) * a.nseg;
     const uint32_t grid = max(1u, min((uint32_t)device_sm_count(), npairs));
-    cudaError_t e = cudaSuccess;
-#define EOQ_LAUNCH_DQ(O)                                                                                          \
-    do {                                                                                                          \
-        e = cudaFuncSetAttribute(dequant_pairs_kernel<O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        if (e == cudaSuccess) dequant_pairs_kernel<O><<<grid, 512, smem, st>>>(a);                                \
+    static std::atomic<uint64_t> asked{0};                  // kernels whose shared-memory limit has been raised, per device and output
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+#define EOQ_LAUNCH_DQ(O)                                                                                                          \
+    do {                                                                                                                          \
+        const uint64_t mark = dev < 8 ? 1ull << (dev * 8 + O) : 0u;                                                              \
+        if (!mark || !(asked.load() & mark)) {                                                                                    \
+            e = cudaFuncSetAttribute(dequant_pairs_kernel<O>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);            \
+            if (e == cudaSuccess) asked.fetch_or(mark);                                                                           \
+        }                                                                                                                         \
+        if (e == cudaSuccess && O >= kOutPacked) e = launch_with_pdl(dequant_pairs_kernel<O>, dim3(grid), dim3(512), smem, st, a); \
+        else if (e == cudaSuccess) dequant_pairs_kernel<O><<<grid, 512, smem, st>>>(a);                                           \
     } while (0)
-    if (a.out_dtype == EOQ_B200_F16) EOQ_LAUNCH_DQ(EOQ_B200_F16);
+    if (!a.out_deq && a.packed == 2) EOQ_LAUNCH_DQ(kOutBlocked);
+    else if (!a.out_deq) EOQ_LAUNCH_DQ(kOutPacked);
+    else if (a.out_dtype == EOQ_B200_F16) EOQ_LAUNCH_DQ(EOQ_B200_F16);
     else if (a.out_dtype == EOQ_B200_BF16) EOQ_LAUNCH_DQ(EOQ_B200_BF16);
     else EOQ_LAUNCH_DQ(EOQ_B200_F32);
 #undef EOQ_LAUNCH_DQ

@@ -29,6 +29,7 @@
 
 extern "C" int eoq_b200_linear_packed_preferred(const uint8_t *d_packed, uint32_t rows, uint32_t cols, uint32_t bits, uint32_t group,
                                                 const void *x, int x_dtype, uint32_t batch);
+extern "C" int eoq_b200_weight_linear_preferred(const eoq_b200_weight_t *w, const void *x, int x_dtype, uint32_t batch);
 
 namespace {
 
@@ -37,6 +38,12 @@ using at::Tensor;
 // A single row against a large PolarLinear is the CUDA-core kernel's: 14336 x 4096 34.0 against 37.5 us; 4096 x 4096 16.1
 // against 13.9, two rows of the former 79 against 37.7.
 constexpr int64_t kPolarSingleRowWeights = 32 << 20;
+
+// Two, and three or four, rows against an entropy-coded weight: the fused GEMV above these many weights, below them the
+// decode and the tcgen05 product, whose time is the decoder's and hardly depends on the rows.  Device time, GEMV / product,
+// fp16: two rows 1001 x 2048 11.2 / 8.6 us, 2048 x 2048 11.0 / 9.7, 4096 x 4096 14.9 / 17.1; four rows 1001 x 2048
+// 24.1 / 8.7, 4096 x 4096 24.1 / 17.2, 11008 x 4096 31.0 / 37.4.  One row: 2048 x 2048 8.3 / 9.6, always the GEMV.
+constexpr int64_t kTwoRowWeights = 7 << 20, kFourRowWeights = 28 << 20;
 
 int dtype_code(at::ScalarType t)
 {
@@ -104,8 +111,10 @@ PyObject *done(eoq_error_t rc, Tensor &&y)
         return nullptr;                                                  \
     }
 
-// weight_linear(handle, device, N, K, rows16, rows32, x, bias): EOQWeight.linear.  Up to rows16 (rows32 for fp32) rows by
-// the fused decode + GEMV, more by one decode to a dense matrix and a library GEMM.
+// weight_linear(handle, device, N, K, rows16, rows32, x, bias): EOQWeight.linear.  One row, a few against a
+// large weight, and up to rows16 (rows32 for fp32) against layouts without a product kernel, by the fused decode + GEMV; more
+// by decoding the codes for the tcgen05 product kernel where it takes the layout and is the quicker, else by one decode to a
+// dense matrix and a library GEMM.
 PyObject *weight_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     if (n != 8) { PyErr_SetString(PyExc_TypeError, "weight_linear takes 8 arguments"); return nullptr; }
@@ -118,10 +127,18 @@ PyObject *weight_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
     if (!x || !activations(*x, K, code, rows) || x->get_device() != dev || !bias_ptr(a[7], *x, N, b)) Py_RETURN_NONE;
     eoq_b200_weight_t *w = static_cast<eoq_b200_weight_t *>(PyLong_AsVoidPtr(a[0]));
     void *st = stream_of(*x);
-    if (rows <= PyLong_AsLongLong(a[code == EOQ_B200_F32 ? 5 : 4])) {
+    const bool product = rows > 1 && eoq_b200_weight_linear_preferred(w, x->data_ptr(), code, (uint32_t)rows);
+    const bool few = product ? rows <= 4 && N * K > (rows == 2 ? kTwoRowWeights : kFourRowWeights)
+                             : rows <= PyLong_AsLongLong(a[code == EOQ_B200_F32 ? 5 : 4]);
+    if (few) {
         if (rows > 8) Py_RETURN_NONE;
         Tensor y = result(*x, N, x->scalar_type());
         return done(eoq_b200_gemv(w, x->data_ptr(), code, (uint32_t)rows, y.data_ptr(), code, b, st), std::move(y));
+    }
+    if (product) {
+        Tensor y = result(*x, N, x->scalar_type());
+        Tensor scratch = at::detail::empty_cuda({(int64_t)eoq_b200_weight_linear_scratch(w, (uint32_t)rows, code)}, at::kByte, x->device(), std::nullopt);
+        return done(eoq_b200_weight_linear(w, x->data_ptr(), code, (uint32_t)rows, scratch.data_ptr(), y.data_ptr(), code, b, st), std::move(y));
     }
     Tensor dense = at::detail::empty_cuda({N, K}, x->scalar_type(), x->device(), std::nullopt);
     if (eoq_b200_weight_decode(w, nullptr, 0, dense.data_ptr(), code, st) != EOQ_OK) Py_RETURN_NONE;

@@ -494,6 +494,14 @@ eoq_error_t eoq_b200_linear_polar_codes(const uint8_t *d_codes, const uint16_t *
                                         uint32_t batch, void *d_scratch, void *y, int y_dtype, const void *bias, int bias_dtype,
                                         void *stream);
 
+/* y = x @ W.T (+ bias) from a resident entropy-coded 4-bit weight for any number of activation rows: its codes are decoded,
+ * two per byte, into d_scratch (they stay in the L2 for matrices of this kind's usual sizes) and multiplied as
+ * eoq_b200_linear_packed does.  d_scratch: eoq_b200_weight_linear_scratch() bytes, 16-byte aligned.  The default layout
+ * (three codes per step), groups that are multiples of 32 and columns of 32 (EOQ_ERR_UNSUPPORTED otherwise). */
+size_t eoq_b200_weight_linear_scratch(const eoq_b200_weight_t *w, uint32_t batch, int x_dtype);
+eoq_error_t eoq_b200_weight_linear(eoq_b200_weight_t *w, const void *x, int x_dtype, uint32_t batch, void *d_scratch, void *y,
+                                   int y_dtype, const float *bias, void *stream);
+
 /* 0, or nonzero if a bounded wait of one of these kernels has run out on the current device since the last call (synchronises). */
 uint32_t eoq_b200_linear_status(void);
 

@@ -75,6 +75,28 @@ def test_polar_product(bits, block, n, k):
     assert L.lib().eoq_b200_linear_status() == 0
 
 
+@pytest.mark.parametrize("n,k,group", [(96, 128, 32), (97, 256, 64), (1000, 1024, 128), (2305, 640, 128), (5000, 4096, 128)])
+def test_entropy_coded_product(n, k, group):
+    """EOQWeight.linear beyond the fused GEMV's rows: codes decoded two per byte, then the same product; the packed codes
+    themselves against the symbols, odd numbers of row blocks and rows past the matrix among them."""
+    from eoq_quantization_b200.fused import EOQWeight
+    rng = np.random.default_rng(n)
+    codes, scales = O.quantize_absmax((rng.standard_normal((n, k)) * 0.02).astype(np.float32), 4, group)
+    s16 = scales.astype(np.float16)
+    w = EOQWeight.from_symbols((codes + 7).astype(np.uint8), s16, group=group)
+    assert np.array_equal(w.decode_symbols(packed=True).cpu().numpy(), O.pack_int4_rows(codes))
+    dense = torch.from_numpy((codes.reshape(-1, group).astype(np.float64) * s16.astype(np.float64)[:, None]).reshape(n, k)).cuda()
+    bias = torch.randn(n, device="cuda")
+    for dt in CODE:
+        for m in (1, 2, 3, 5, 8, 9, 40, 130, 300):
+            x = torch.randn(m, k, device="cuda").to(dt)
+            want = x.double() @ dense.T + bias.double()
+            tol = 1e-5 if dt == torch.float32 else 1e-3 if dt == torch.float16 else 6e-3
+            for _ in range(2):
+                assert O.rel_l2(w.linear(x, bias).double().cpu().numpy(), want.cpu().numpy()) < tol, (dt, m)
+    assert w.status() == 0 and L.lib().eoq_b200_linear_status() == 0
+
+
 def test_modules_fall_back_outside_the_native_route():
     """Gradients through x, activations that are not contiguous or not aligned, no rows: the Python path, same results."""
     torch.manual_seed(1)
