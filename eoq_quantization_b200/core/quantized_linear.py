@@ -112,10 +112,11 @@ class QuantizedLinear(nn.Module):
     def eoq_weight(self) -> EOQWeight:
         """The entropy-coded resident form of this layer's weight (built on first use, rebuilt if
         the buffers are replaced)."""
-        key = (self.packed_weight.data_ptr(), self.scales.data_ptr(), self.packed_weight._version, self.scales._version)
+        packed, scales = self._buffers["packed_weight"], self._buffers["scales"]
+        key = (packed.data_ptr(), scales.data_ptr(), packed._version, scales._version)
         if self._eoq is None or self._eoq_key != key:
-            with torch.cuda.device(self.packed_weight.device):
-                self._eoq = EOQWeight.from_packed(self.packed_weight, self.scales, self.in_features, self.bits, group=self.block_size)
+            with torch.cuda.device(packed.device):
+                self._eoq = EOQWeight.from_packed(packed, scales, self.in_features, self.bits, group=self.block_size)
             self._eoq_key = key
         return self._eoq
 
@@ -142,7 +143,7 @@ class QuantizedLinear(nn.Module):
             # that one dequantisation amortises over enough rows for a library GEMM to win (the fused tensor-core
             # kernel would take 9..GEMM_MAX_ROWS rows of 16-bit activations if that constant were raised)
             if rows <= fused_rows(x.dtype):
-                return self.eoq_weight().gemv(x, self.bias_param)
+                return self.eoq_weight().linear(x, bias)
             if 8 < rows <= GEMM_MAX_ROWS and x.dtype != torch.float32 and self.bits == 4:          # the tensor-core kernel is built for the 4-bit layout
                 return self.eoq_weight().gemm(x, self.bias_param)
         weight = dequant_packed(self.packed_weight, self.scales, self.out_features, self.in_features, self.bits,
