@@ -1807,14 +1807,14 @@ extern "C" eoq_error_t eoq_b200_linear_packed(const uint8_t *d_packed, const uin
 }
 
 // For the torch-facing front (not in the public header): whether eoq_b200_linear_packed takes the call and is to be
-// preferred to a dequantised copy (2 T weights/s) and a library GEMM.
+// preferred to a dequantised copy (1.2 T weights/s, and two launches: no call takes less than 5.5 us) and a library GEMM.
 extern "C" int eoq_b200_linear_packed_preferred(const uint8_t *d_packed, uint32_t rows, uint32_t cols, uint32_t bits, uint32_t group,
                                                 const void *x, int x_dtype, uint32_t batch)
 {
     const bool split = x_dtype == EOQ_B200_F32;
     if (!qmm_takes(cols, bits, group, d_packed, x) || (split && !split_rows_takes(cols, 1))) return 0;
     return qmm_preferred(packed_call(d_packed, nullptr, rows, cols, bits, group, x, x_dtype, batch, nullptr, nullptr, x_dtype, nullptr),
-                         (double)rows * cols / 2.05e6) ? 1 : 0;
+                         (double)rows * cols / 1.2e6, 5.5) ? 1 : 0;
 }
 
 extern "C" eoq_error_t eoq_b200_linear_polar_codes(const uint8_t *d_codes, const uint16_t *d_norms_fp16, const float *d_centroids,
@@ -1884,13 +1884,14 @@ extern "C" eoq_error_t eoq_b200_weight_linear(eoq_b200_weight_t *w, const void *
 }
 
 // For the torch-facing front (not in the public header): whether eoq_b200_weight_linear takes the call and is to be
-// preferred to a dense decode and a library GEMM (both decode; neither copy is the longer one to speak of).
+// preferred to a dense decode and a library GEMM.  Both decode; the dense result takes longer to store and to read back
+// (11008 x 4096: 30 us), the product 1 us longer to start.
 extern "C" int eoq_b200_weight_linear_preferred(const eoq_b200_weight_t *w, const void *x, int x_dtype, uint32_t batch)
 {
     if (!w || !weight_linear_takes(w, x, x_dtype)) return 0;
     QmmCall c = packed_call(nullptr, nullptr, w->N, w->K, 4, w->group, x, x_dtype, batch, nullptr, nullptr, x_dtype, nullptr);
     c.blocked_rows = w->Npad;
-    return qmm_preferred(c, 0.0) ? 1 : 0;
+    return qmm_preferred(c, (double)w->N * w->K / 1.5e6 - 1.0, 0.0) ? 1 : 0;
 }
 
 extern "C" uint32_t eoq_b200_linear_status(void) { return qmm_status(); }

@@ -248,7 +248,7 @@ struct QmmCall {
 };
 bool qmm_takes(uint32_t K, uint32_t bits, uint32_t group, const void *packed, const void *x);
 int launch_qmm(const QmmCall &c, void *stream);
-bool qmm_preferred(const QmmCall &c, double copy_us);
+bool qmm_preferred(const QmmCall &c, double copy_us, double least_us);
 uint32_t qmm_status();
 bool split_rows_takes(uint32_t K, uint32_t block);
 int launch_split_rows(const void *x, int x_dtype, uint32_t K, uint32_t M, uint32_t block, void *planes, float *tok_scale, void *stream);

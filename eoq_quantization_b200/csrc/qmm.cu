@@ -909,17 +909,22 @@ bool qmm_takes(uint32_t K, uint32_t bits, uint32_t group, const void *packed, co
 int launch_qmm(const QmmCall &c, void *stream) { return qmm(c, stream, nullptr); }
 
 // Whether the call is to be preferred to a dequantised copy of the weight and a library GEMM, given the microseconds that
-// the copy takes longer than what this kernel reads takes to make.  fp32 activations: always (the library multiplies them
-// on the CUDA cores: 13 x slower at 512 rows).  16-bit ones: up to 32 rows, where rows of y are not 16-byte multiples (the
-// library's kernels for those are three to ten times slower), or where the plan's estimate, at the 1.5 cycles a nanosecond
-// that long products run at, is not above the GEMM's (1.45 PFLOP/s, 8 us at least).  From packed codes, fp16, 777 rows:
-// 4096 x 11008 62 against 77 us, 11008 x 4096 71 against 71; 2048 rows: 141 / 142 and 153 / 156.
-bool qmm_preferred(const QmmCall &c, double copy_us)
+// the copy takes longer than what this kernel reads takes to make, and `least_us`, which the two launches of that route take
+// at any size.  fp32 activations: always (the library multiplies them on the CUDA cores: 13 x slower at 512 rows).  16-bit
+// ones: up to 32 rows, or where the plan's estimate, at the 1.5 cycles a nanosecond that long products run at (with a tenth
+// more where scales are applied before the product, and another for bf16, whose codes take a rounding more), is not above the
+// GEMM's (1.45 PFLOP/s, 7 us at least; where rows of y are not 16-byte multiples, cutting them out of padded ones besides)
+// less 4 us.  Fitted over thirteen shapes from 512 x 512 to 28672 x 8192, 40 to 2048 rows, fp16 and bf16, both ways timed:
+// the choice costs 0.8 % (from decoded codes) and 1.1 % (from packed ones) of device time on the mean against the better of
+// the two.
+bool qmm_preferred(const QmmCall &c, double copy_us, double least_us)
 {
-    if (c.split_x || c.M <= 32u || c.N % 8u) return true;
+    if (c.split_x || c.M <= 32u) return true;
+    if (c.N % 8u) copy_us += 4.0 + (double)c.M * c.N / 1e6;
     double cycles = 0;
     if (qmm(c, nullptr, &cycles) != 0) return false;
-    return cycles / 1500.0 <= std::max(8.0, 2.0 * c.M * (double)c.N * c.K / 1.45e9) + copy_us + 4.0;
+    if (c.M > 128u) cycles *= c.bf16 ? 1.21 : 1.1;
+    return cycles / 1500.0 <= std::max(least_us, std::max(7.0, 2.0 * c.M * (double)c.N * c.K / 1.45e9) + copy_us - 4.0);
 }
 
 bool split_rows_takes(uint32_t K, uint32_t block) { return K % 16u == 0 && K <= 48u * 1024u && (block == 1 || block == 64 || block == 128 || block == 256); }

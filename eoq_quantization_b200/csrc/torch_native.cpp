@@ -15,6 +15,7 @@
 #include <ATen/autocast_mode.h>
 #include <ATen/core/LegacyTypeDispatch.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <ATen/ops/constant_pad_nd.h>
 #include <ATen/ops/linear.h>
 #include <c10/core/GradMode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
@@ -104,6 +105,26 @@ PyObject *done(eoq_error_t rc, Tensor &&y)
     return THPVariable_Wrap(std::move(y));
 }
 
+// x @ W.T (+ bias) by the library, W written by `fill` into a dense matrix of x's type.  Where rows of a 16-bit y would not
+// be 16-byte multiples the matrix gets rows for them to be (whatever those hold ends in columns that are cut off): the
+// library's kernels for other widths are three to nine times slower.  fp16, as it is / padded and cut: 4595 x 2056, 26 rows
+// 25.5 / 11.5 us, 2048 rows 290 / 46; 1043 x 8888, 64 rows 67.6 / 18.8; 11007 x 4104, one row 36.7 / 19.5.  Not below 2048
+// columns of y and 33 rows (1573 x 1336, 8 rows 9.1 / 10.2), nor for fp32 (55 / 60).
+template <class Fill>
+PyObject *dense_linear(const Tensor &x, int64_t N, int64_t K, int64_t rows, PyObject *bias, Fill &&fill)
+{
+    const bool pad = x.scalar_type() != at::kFloat && N % 8 && K % 8 == 0 && (rows > 32 || N >= 2048);
+    const int64_t wide = pad ? (N + 7) & ~(int64_t)7 : N;
+    Tensor dense = at::detail::empty_cuda({wide, K}, x.scalar_type(), x.device(), std::nullopt);
+    if (fill(dense.data_ptr()) != EOQ_OK) Py_RETURN_NONE;
+    at::AutoDispatchBelowADInplaceOrView guard;
+    std::optional<Tensor> b;
+    if (bias != Py_None) b = THPVariable_Unpack(bias).to(x.scalar_type());
+    if (!pad) return THPVariable_Wrap(at::linear(x, dense, b));
+    if (b) b = at::constant_pad_nd(*b, {0, wide - N});
+    return THPVariable_Wrap(at::linear(x, dense, b).narrow(-1, 0, N).contiguous());
+}
+
 #define GUARD_BEGIN try {
 #define GUARD_END                                                        \
     } catch (const std::exception &e) {                                  \
@@ -140,12 +161,7 @@ PyObject *weight_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
         Tensor scratch = at::detail::empty_cuda({(int64_t)eoq_b200_weight_linear_scratch(w, (uint32_t)rows, code)}, at::kByte, x->device(), std::nullopt);
         return done(eoq_b200_weight_linear(w, x->data_ptr(), code, (uint32_t)rows, scratch.data_ptr(), y.data_ptr(), code, b, st), std::move(y));
     }
-    Tensor dense = at::detail::empty_cuda({N, K}, x->scalar_type(), x->device(), std::nullopt);
-    if (eoq_b200_weight_decode(w, nullptr, 0, dense.data_ptr(), code, st) != EOQ_OK) Py_RETURN_NONE;
-    at::AutoDispatchBelowADInplaceOrView guard;
-    std::optional<Tensor> bias;
-    if (b) bias = THPVariable_Unpack(a[7]).to(x->scalar_type());
-    return THPVariable_Wrap(at::linear(*x, dense, bias));
+    return dense_linear(*x, N, K, rows, a[7], [&](void *dense) { return eoq_b200_weight_decode(w, nullptr, 0, dense, code, st); });
     GUARD_END
 }
 
@@ -186,15 +202,11 @@ PyObject *packed_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
                                            (uint32_t)rows, f32 ? scratch.data_ptr() : nullptr, y.data_ptr(), code, b, st),
                     std::move(y));
     }
-    if (rows <= 8) Py_RETURN_NONE;           // shapes none of these kernels takes: the entropy-coded form may
-    Tensor dense = at::detail::empty_cuda({N, K}, x->scalar_type(), x->device(), std::nullopt);
-    if (eoq_b200_dequant_packed(codes, scales, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)group, 0, (uint32_t)N, dense.data_ptr(),
-                                code, st) != EOQ_OK)
-        Py_RETURN_NONE;
-    at::AutoDispatchBelowADInplaceOrView guard;
-    std::optional<Tensor> bias;
-    if (b) bias = THPVariable_Unpack(a[7]).to(x->scalar_type());
-    return THPVariable_Wrap(at::linear(*x, dense, bias));
+    // a few rows against whole groups per row: the entropy-coded form may take them
+    if (rows <= 8 && K % 16 == 0 && group % 16 == 0 && K % group == 0) Py_RETURN_NONE;
+    return dense_linear(*x, N, K, rows, a[7], [&](void *dense) {
+        return eoq_b200_dequant_packed(codes, scales, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)group, 0, (uint32_t)N, dense, code, st);
+    });
     GUARD_END
 }
 

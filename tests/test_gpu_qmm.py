@@ -111,3 +111,18 @@ def test_modules_fall_back_outside_the_native_route():
     xg = x.clone().requires_grad_()
     ql(xg).sum().backward()
     assert O.rel_l2(xg.grad.cpu().numpy(), w.sum(0).expand(40, -1).cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("n,k", [(2047, 136), (2049, 264), (41, 136), (2048, 136)])
+def test_rows_that_end_inside_a_scale_group(n, k):
+    """A dequantised copy with rows added until y's rows are 16-byte multiples: around the sizes where that starts."""
+    torch.manual_seed(n)
+    for bits in (2, 4, 8):
+        ql = QuantizedLinear.from_float(torch.nn.Linear(k, n), bits=bits, block_size=128).cuda()
+        w, b = ql._dequantize_weight().double(), ql.bias_param.double()
+        for dt, tol in ((torch.float16, 1e-3), (torch.bfloat16, 8e-3), (torch.float32, 1e-5)):
+            for m in (1, 8, 32, 33):
+                x = torch.randn(2, m, k, device="cuda").to(dt) if m > 8 else torch.randn(m, k, device="cuda").to(dt)
+                y = ql(x)
+                assert y.dtype == dt and y.shape == (*x.shape[:-1], n) and y.is_contiguous()
+                assert O.rel_l2(y.double().cpu().numpy(), (x.double() @ w.T + b).cpu().numpy()) < tol, (bits, dt, m)
