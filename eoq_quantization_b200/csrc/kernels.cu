@@ -3311,19 +3311,18 @@ __global__ void __launch_bounds__(BITS == 8 ? 256 : 512, BITS == 8 ? 3 : 2) gemv
 static std::atomic<int> g_packed_warps{0};              // 0 = by shape; "packed_warps" in eoq_b200_tune
 void set_packed_warps(int v) { g_packed_warps.store(v >= 1 && v <= 16 ? v : 0); }
 
-// Warps per CTA of the tensor-core form (they share a tile's spans).  The CTAs are short, so a grid that needs a second,
-// partly filled round of CTAs loses that fraction of the machine: take the most warps per CTA with which the whole
-// grid is resident at once (given the registers the compiler gave this instantiation) and every warp still has two
-// spans; when no choice fits, the one with the most resident warps per SM.
+// Warps per CTA of the tensor-core form (they share a tile's spans).  With programmatic launch a CTA goes wherever there is
+// room while the kernel before it drains, so an SM with room for s CTAs may get s tiles although the mean is below one
+// (2048 x 2048, 16 spans, 128 tiles: 3.7 us with four 8-warp CTAs to an SM, 2.2 with two of 16; 4096 x 1024, 8 spans, 256
+// tiles: 3.8 with 4 warps, 1.96 with 12, four of them idle), and a grid that needs a second, partly filled round loses that
+// fraction of the machine.  So: the most warps, i.e. the fewest CTAs to an SM, with which the whole grid is resident (given
+// the registers the compiler gave this instantiation).  Where none is, 8 warps: rounds of eight short tiles on every SM
+// take longer than four at a time in two (14336 x 4096: 14.7 us with 4 warps, 12.0 with 8; 28672 x 4096: 25.6 with 16,
+// 21.0 with 8).  Byte codes at 7168 to 9216 x 4096: 11.3 to 12.9 us with 8 warps, 8.6 to 9.1 with 6 (and
+// 10240 x 4096 13.0 with 8, 17.2 with 5, 12.5 with 4).
 template <typename Kern, typename Args>
-static cudaError_t launch_packed_mma(Kern kern, uint32_t fixed_warps, uint32_t tiles, uint32_t nspans, cudaStream_t st, const Args &a)
+static cudaError_t launch_packed_mma(Kern kern, uint32_t max_warps, uint32_t tiles, uint32_t nspans, cudaStream_t st, const Args &a)
 {
-    // byte codes and more than eight activation rows (more registers, longer spans of work per warp): 8 warps measured best
-    if (fixed_warps) {
-        const uint32_t w = g_packed_warps.load() ? std::min((uint32_t)g_packed_warps.load(), fixed_warps) : nspans >= 16u ? fixed_warps : 4u;
-        return launch_with_pdl(kern, dim3(tiles), dim3(w * 32u), 0, st, a);
-    }
-    const uint32_t max_warps = 16;
     // registers per kernel, asked once (kernels of one signature share this function: the key is the kernel, not its type)
     static std::mutex mu;
     static std::vector<std::pair<const void *, int>> known;
@@ -3342,15 +3341,14 @@ static cudaError_t launch_packed_mma(Kern kern, uint32_t fixed_warps, uint32_t t
     }
     const uint32_t per_thread = ((uint32_t)regs + 7u) & ~7u, sms = (uint32_t)device_sm_count();
     static const uint32_t kChoices[] = {16, 12, 10, 8, 6, 5, 4};
-    uint32_t warps = 0, best_resident = 0, fallback = 4;
+    const uint32_t useful = std::max(4u, tiles > sms ? nspans + nspans / 2u : nspans);     // idle warps only where they keep CTAs apart
+    uint32_t warps = 0;
     for (uint32_t w : kChoices) {
-        if (w > max_warps || (2u * w > nspans && w > 4u)) continue;
+        if (w > max_warps || w > useful || (w == (max_warps == 16u ? 4u : 5u) && nspans > 4u)) continue;
         const uint32_t ctas = std::min(64u / w, 65536u / (per_thread * 32u * w));
-        if (ctas == 0) continue;
         if (!warps && tiles <= sms * ctas) warps = w;
-        if (w * ctas > best_resident) { best_resident = w * ctas; fallback = w; }
     }
-    if (!warps) warps = fallback;
+    if (!warps) warps = std::min(8u, useful);
     if (g_packed_warps.load()) warps = std::min((uint32_t)g_packed_warps.load(), max_warps);
     return launch_with_pdl(kern, dim3(tiles), dim3(warps * 32u), 0, st, a);
 }
@@ -3362,8 +3360,8 @@ int launch_gemv_packed(const PackedGemvArgs &a, void *stream)
         const uint32_t tiles = (a.N + 15u) / 16u, nspans = a.K >> 7;
         const bool bf = a.x_dtype == EOQ_B200_BF16;
         cudaError_t e;
-        if (a.bits == 4) e = bf ? launch_packed_mma(gemv_packed_mma_kernel<4, true>, 0u, tiles, nspans, st, a) : launch_packed_mma(gemv_packed_mma_kernel<4, false>, 0u, tiles, nspans, st, a);
-        else if (a.bits == 2) e = bf ? launch_packed_mma(gemv_packed_mma_kernel<2, true>, 0u, tiles, nspans, st, a) : launch_packed_mma(gemv_packed_mma_kernel<2, false>, 0u, tiles, nspans, st, a);
+        if (a.bits == 4) e = bf ? launch_packed_mma(gemv_packed_mma_kernel<4, true>, 16u, tiles, nspans, st, a) : launch_packed_mma(gemv_packed_mma_kernel<4, false>, 16u, tiles, nspans, st, a);
+        else if (a.bits == 2) e = bf ? launch_packed_mma(gemv_packed_mma_kernel<2, true>, 16u, tiles, nspans, st, a) : launch_packed_mma(gemv_packed_mma_kernel<2, false>, 16u, tiles, nspans, st, a);
         else e = bf ? launch_packed_mma(gemv_packed_mma_kernel<8, true>, 8u, tiles, nspans, st, a) : launch_packed_mma(gemv_packed_mma_kernel<8, false>, 8u, tiles, nspans, st, a);
         g_launches++;
         return (int)e;
