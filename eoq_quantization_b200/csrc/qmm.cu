@@ -279,7 +279,8 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
     const uint32_t base = saddr(smem), bars = base + a.at_bar;
     auto bar = [&](uint32_t i) { return bars + 8u * i; };
     const uint32_t scale_ring = bars + 512u;
-    uint32_t *table = reinterpret_cast<uint32_t *>(smem + a.at_bar + 512 + kScaleRing * kScaleEntry);      // polar: centroids as {high half, low half}
+    uint32_t *table = reinterpret_cast<uint32_t *>(smem + a.at_bar + 512 + kScaleRing * kScaleEntry);      // polar: centroids, as {high half, low half} (fold) or fp32
+    uint32_t *largest = table + 256;              // polar, scaled: the largest norm of each row (bits of a float), then the largest centroid
     const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;       // the same in all lanes, and known to be
     const uint32_t rank = blockIdx.x % a.split, row0 = blockIdx.x / a.split * kRows, tok0 = blockIdx.y * a.T;
     const uint32_t u0 = (uint32_t)((uint64_t)a.units * rank / a.split), u1 = (uint32_t)((uint64_t)a.units * (rank + 1) / a.split);
@@ -302,11 +303,12 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (kPol) {
-        for (uint32_t i = threadIdx.x; i < a.entries; i += blockDim.x) {
-            const float c = __ldg(a.centroids + i);
+        for (uint32_t i = threadIdx.x; i < 256u; i += blockDim.x) {
+            const float c = __ldg(a.centroids + (i & (a.entries - 1u)));
             const __half hi = __float2half_rn(c), lo = __float2half_rn(c - __half2float(hi));
-            table[i] = __half_as_ushort(hi) | ((uint32_t)__half_as_ushort(lo) << 16);
+            table[i] = FOLD ? __half_as_ushort(hi) | ((uint32_t)__half_as_ushort(lo) << 16) : __float_as_uint(c);
         }
+        if (!FOLD) for (uint32_t i = threadIdx.x; i < kRows + 1u; i += blockDim.x) largest[i] = 0u;
     }
     __syncwarp();
     if (warp == 4 * NP + 4 * NF) {
@@ -319,11 +321,36 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
     // all 512 columns are this CTA's, so they start at column 0: addresses below are constants plus offsets
     constexpr uint32_t tmem = 0;
 
+    // polar, scaled: what a row's values are multiplied by, a power of two that brings the largest of centroid x norm to
+    // 2^14 .. 2^15, so that their two fp16 halves hold 22 bits of it and nothing of it is below what fp16 holds
+    float up = 1.0f, down = 1.0f;
+    if (kPol && !FOLD && warp < 4 * NP + 4 * NF) {
+        const uint32_t r = (warp & 3u) * 32u + lane;
+        if (warp < 4 * NP) {
+            const uint16_t *norms = a.scales + (size_t)min(row0 + r, a.N - 1u) * a.sgroups + grp0;
+            float most = 0.0f;
+#pragma unroll 16
+            for (uint32_t g = warp >> 2; g < ngroups; g += NP) most = fmaxf(most, fabsf(__half2float(__ushort_as_half(__ldg(norms + g)))));
+            atomicMax(largest + r, __float_as_uint(most));
+            if (threadIdx.x < 256u) atomicMax(largest + kRows, table[threadIdx.x] & 0x7fffffffu);
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"((4 * NP + 4 * NF) * 32) : "memory");
+        const float most = __uint_as_float(largest[r]) * __uint_as_float(largest[kRows]);
+        int e = 0;
+        if (most > 0.0f && most < __int_as_float(0x7f800000)) e = min(120, 141 - (int)(__float_as_uint(most) >> 23));
+        up = __uint_as_float((uint32_t)(127 + e) << 23);
+        down = __uint_as_float((uint32_t)(127 - e) << 23);
+    }
+
     if (warp < 4 * NP) {
         // ---- producers: packed codes of one row, a block of columns at a time, to the A operand in tensor memory
         const uint32_t set = warp >> 2, r = (warp & 3u) * 32u + lane;
         const uint32_t lane_base = tmem + (((warp & 3u) * 32u) << 16) + a.a_base;
-        const uint32_t tab_addr = saddr(table), tab_mask = (a.entries - 1u) << 2;
+        // a code to its table entry by one byte permute and one multiply-add (of the pipe that is free; a shift and a mask are
+        // two instructions of the half-rate one, which bounds the conversion); the table repeats up to 256 entries
+        const uint32_t tab_addr = saddr(table);
+        uint32_t four;
+        asm volatile("mov.b32 %0, 4;" : "=r"(four));
         // scaled: the groups of 32-column parts, counted along
         ScaleReader sr{bar(kSFull), bar(kSEmpty), scale_ring, r};
         uint32_t gi = 0, pos = 0;
@@ -355,14 +382,36 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
                     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[4 * c]), "=r"(w[4 * c + 1]), "=r"(w[4 * c + 2]), "=r"(w[4 * c + 3]) : "r"(at));
                 }
                 uint32_t h[32], lo[kPol ? 32 : 1];
-                if (kPol) {
+                if (kPol && !FOLD) {
+                    const float sc = __half2float(__ushort_as_half(sr.get(gi, lane))) * up;
+                    for (pos += part + 1 == kHalves ? 64u + KB * (NP - 1) : 64u; pos >= a.group; pos -= a.group) gi++;
+#pragma unroll
+                    for (int c = 0; c < 16; c++) {
+                        float e[4];
+#pragma unroll
+                        for (int b = 0; b < 4; b++) {
+                            uint32_t off;
+                            asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(off) : "r"(__byte_perm(w[c % U::kWords], 0u, 0x4440u + b)), "r"(four), "r"(tab_addr));
+                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(e[b]) : "r"(off));
+                        }
+#pragma unroll
+                        for (int b = 0; b < 2; b++) {
+                            const __half2 hi = __floats2half2_rn(e[2 * b] * sc, e[2 * b + 1] * sc);
+                            const float2 back = __half22float2(hi);
+                            const __half2 rest = __floats2half2_rn(fmaf(e[2 * b], sc, -back.x), fmaf(e[2 * b + 1], sc, -back.y));
+                            h[2 * c + b] = *reinterpret_cast<const uint32_t *>(&hi);
+                            lo[kPol ? 2 * c + b : 0] = *reinterpret_cast<const uint32_t *>(&rest);
+                        }
+                    }
+                } else if (kPol) {
 #pragma unroll
                     for (int c = 0; c < 16; c++) {
                         uint32_t e[4];
 #pragma unroll
                         for (int b = 0; b < 4; b++) {
-                            const uint32_t off = (b == 0 ? w[c % U::kWords] << 2 : w[c % U::kWords] >> (8 * b - 2)) & tab_mask;
-                            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(e[b]) : "r"(tab_addr + off));
+                            uint32_t off;
+                            asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(off) : "r"(__byte_perm(w[c % U::kWords], 0u, 0x4440u + b)), "r"(four), "r"(tab_addr));
+                            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(e[b]) : "r"(off));
                         }
 #pragma unroll
                         for (int b = 0; b < 2; b++) {
@@ -448,7 +497,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
                 tmem_ld16(lane_base + c, v);
                 tmem_ld_wait(v);
 #pragma unroll
-                for (int j = 0; j < 16; j++) stage[(c + j) * kRows] = __uint_as_float(v[j]);
+                for (int j = 0; j < 16; j++) stage[(c + j) * kRows] = kPol ? __uint_as_float(v[j]) * down : __uint_as_float(v[j]);
             }
             fence_before();
         }
@@ -752,7 +801,7 @@ struct Shape { uint32_t T, nw, ns, a_base; size_t smem; uint32_t at_x, at_bar; }
 // that a set steps over.
 void place(Shape &s, uint32_t stage_w, uint32_t unit_blocks, uint32_t sets, uint32_t planes, uint32_t a_cols, uint32_t kb, bool fold)
 {
-    const size_t fixed = 512 + 1024 + 1024 + kScaleRing * kScaleEntry, room = 226u * 1024u - fixed;
+    const size_t fixed = 512 + 1024 + 1024 + (kRows + 4) * 4 + kScaleRing * kScaleEntry, room = 226u * 1024u - fixed;
     const uint32_t xstage = s.T * 2u * kb * planes, step = std::max(1u, sets / unit_blocks);
     s.a_base = fold ? 2 * s.T : s.T;
     s.ns = std::min(8u, (512u - s.a_base) / a_cols) / sets * sets;
@@ -802,7 +851,8 @@ int run_variant(QmmArgs a, uint32_t most, uint32_t step, const void *packed, uin
         for (uint32_t i = 0; i < std::min(used, 32u); i++) if (keys[i] == key) plan = plans[i];
     }
     if (!plan.T) {
-        const double producers = BITS == kPolar ? 700.0 : FOLD ? 450.0 : !BF16 ? 400.0 : BITS == 8 ? 600.0 : 660.0, products = BITS == kPolar ? 3.0 : a.planes;
+        const double producers = BITS == kPolar ? FOLD ? 700.0 : 1100.0 : FOLD ? 450.0 : !BF16 ? 400.0 : BITS == 8 ? 600.0 : 660.0, products = BITS == kPolar ? 3.0 : a.planes;
+        const double fixed = BITS == kPolar && !FOLD ? 8000.0 : 4000.0;       // (a row's norms are read first, and tiles are large)
         double best = 1e30;
         const uint32_t least = (a.M + most - 1) / most;
         for (uint32_t n = least; n < least + 4; n++) {
@@ -814,7 +864,7 @@ int run_variant(QmmArgs a, uint32_t most, uint32_t step, const void *packed, uin
                 const uint32_t room = resident_ctas(reinterpret_cast<const void *>(kern), threads, s.smem, split);
                 if (room == 0) continue;
                 const double cost = (double)((rows * n * split + room - 1) / room) *
-                                    ((double)((a.units + split - 1) / split) * (U::kCols / 64) * block + 4000.0 + (split > 1 ? 2000.0 : 0.0));
+                                    ((double)((a.units + split - 1) / split) * (U::kCols / 64) * block + fixed * (split > 1 ? 1.5 : 1.0));
                 // a cut into more token tiles repeats the producers' work: only for a clear gain
                 if (cost < best * (n > plan.tok_tiles && plan.T ? 0.95 : 0.999)) { best = cost; plan = Plan{T, n, split, cost}; }
             }
@@ -871,6 +921,13 @@ int run_scaled(const QmmArgs &a, const void *packed, uint64_t row_bytes, const v
     return run_variant<BITS, BF16, false, 4, 1, 32, 64>(a, 256, 16, packed, row_bytes, x, st, cycles);
 }
 
+// Byte codes: up to this many tokens the centroids are multiplied and each block's sum scaled in fp32 (every 64 columns a
+// reader's pass over the accumulator, 128 tokens at most); beyond, centroid x norm goes in as two fp16 halves, a row at a
+// time brought to their range, and a CTA takes 256 tokens: a block costs 1100 cycles whatever the tokens up to some 160, so
+// fewer, larger tiles pay.  14336 x 4096, 64 columns a block, 128 tokens 55 us / 52, 256 tokens 100 / 82.  Both leave 22
+// bits of each factor.
+constexpr uint32_t kPolarFold = 112;
+
 int qmm(const QmmCall &c, void *stream, double *cycles)
 {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -885,6 +942,7 @@ int qmm(const QmmCall &c, void *stream, double *cycles)
     a.entries = c.centroids ? 1u << c.bits : 1u;
     const bool bf = c.bf16 && !c.split_x;
     const uint64_t row_bytes = c.blocked_rows ? (uint64_t)c.blocked_rows * 8 : c.centroids ? c.K : c.bits == 4 ? c.K / 2 : c.bits == 2 ? c.K / 4 : c.K;
+    if (c.centroids && c.M > kPolarFold) return run_variant<kPolar, false, false, 2, 1, 32, 64>(a, 256, 16, c.packed, row_bytes, c.x, st, cycles);
     if (c.centroids) return run_fold<kPolar, false>(a, c.packed, row_bytes, c.x, st, cycles);
     const bool fold = c.split_x || c.M <= 128u;
 #define EOQ_QMM(B)                                                                                                                      \

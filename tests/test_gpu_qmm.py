@@ -126,3 +126,25 @@ def test_rows_that_end_inside_a_scale_group(n, k):
                 y = ql(x)
                 assert y.dtype == dt and y.shape == (*x.shape[:-1], n) and y.is_contiguous()
                 assert O.rel_l2(y.double().cpu().numpy(), (x.double() @ w.T + b).cpu().numpy()) < tol, (bits, dt, m)
+
+
+@pytest.mark.parametrize("bits,block,n,k", [(5, 64, 130, 192), (8, 256, 77, 512), (3, 64, 300, 4160), (1, 128, 129, 384)])
+def test_polar_product_many_rows(bits, block, n, k):
+    """Centroid x norm as two halves: norms of one row four decades apart, rows all zero, token tiles around their sizes."""
+    g = torch.Generator(device="cuda").manual_seed(bits + n)
+    codes = torch.randint(0, 1 << bits, (n, k), generator=g, device="cuda").to(torch.uint8)
+    norms = (10 ** (torch.rand(n, k // block, generator=g, device="cuda") * 4 - 3)).half()
+    norms[n // 2] = 0
+    cent = torch.sort(torch.randn(1 << bits, generator=g, device="cuda"))[0]
+    H = hadamard_matrix(block).cuda().double()
+    dense = ((cent.double()[codes.long()].view(-1, block) / block ** 0.5) @ H * norms.double().view(-1, 1)).view(n, k)
+    for m in (112, 113, 255, 256, 257, 520):
+        x = torch.randn(m, k, generator=g, device="cuda")
+        y = torch.empty(m, n, device="cuda")
+        scratch = torch.empty(m * (k + 1), device="cuda")
+        assert L.lib().eoq_b200_linear_polar_codes(codes.data_ptr(), norms.data_ptr(), cent.data_ptr(), n, k, bits, block, x.data_ptr(), L.F32, m,
+                                                   scratch.data_ptr(), y.data_ptr(), L.F32, None, L.F32, _stream()) == L.EOQ_OK
+        want = x.double() @ dense.T
+        err = (y.double() - want).norm(dim=0) / want.norm(dim=0).clamp_min(1e-30)          # each row of the weight by itself
+        assert err.max().item() < 3e-6, m
+    assert L.lib().eoq_b200_linear_status() == 0
