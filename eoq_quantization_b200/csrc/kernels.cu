@@ -1394,31 +1394,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_pairs_kernel(const GemvArgs a
         __syncthreads();
 
         if (leader) {
-            // several warps' sums are loaded before the first is added (still in warp order): one at a time the sixteen
-            // cost 2000 cycles of shared-memory latency
             const uint32_t run = min(cs - warp, a.nseg - seg);
-            constexpr uint32_t kU = BT == 1 ? 5 : BT == 2 ? 3 : 1;
-            for (uint32_t w0 = 1; w0 < run; w0 += kU) {
-                float part[kU][2][G][BT];
+            for (uint32_t w = 1; w < run; w++) {
+                const float *red = reinterpret_cast<const float *>(mine + (size_t)w * region);
 #pragma unroll
-                for (uint32_t u = 0; u < kU; u++) {
-                    const float *red = reinterpret_cast<const float *>(mine + (size_t)min(w0 + u, run - 1u) * region);
+                for (int k = 0; k < 2; k++)
 #pragma unroll
-                    for (int k = 0; k < 2; k++)
+                    for (int j = 0; j < G; j++)
 #pragma unroll
-                        for (int j = 0; j < G; j++)
-#pragma unroll
-                            for (int b = 0; b < BT; b++) part[u][k][j][b] = red[((k * G + j) * BT + b) * 32 + lane];
-                }
-#pragma unroll
-                for (uint32_t u = 0; u < kU; u++)
-                    if (w0 + u < run)
-#pragma unroll
-                        for (int k = 0; k < 2; k++)
-#pragma unroll
-                            for (int j = 0; j < G; j++)
-#pragma unroll
-                                for (int b = 0; b < BT; b++) y[k][j][b] += part[u][k][j][b];
+                        for (int b = 0; b < BT; b++) y[k][j][b] += red[((k * G + j) * BT + b) * 32 + lane];
             }
             // runs of this row-block pair are numbered by the chunk they fall in
             const uint32_t slot = t - chunk_of(first_q);
