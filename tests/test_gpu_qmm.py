@@ -148,3 +148,20 @@ def test_polar_product_many_rows(bits, block, n, k):
         err = (y.double() - want).norm(dim=0) / want.norm(dim=0).clamp_min(1e-30)          # each row of the weight by itself
         assert err.max().item() < 3e-6, m
     assert L.lib().eoq_b200_linear_status() == 0
+
+
+@pytest.mark.parametrize("n,k", [(2400, 384), (2369, 1024), (9488, 640), (14224, 128), (16400, 256)])
+def test_packed_gemv_warp_counts(n, k):
+    """Few rows by the warp-level kernel where its CTAs have idle warps, an odd number of warps, or need a second round."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    for bits in (2, 4, 8):
+        qmax = (1 << (bits - 1)) - 1
+        c = torch.randint(-qmax, qmax + 1, (n, k), generator=g, device="cuda")
+        s = (torch.rand(n, k // 128, generator=g, device="cuda") * 0.01 + 1e-3).half()
+        dense, packed = (c.double().view(n, -1, 128) * s.double()[:, :, None]).view(n, k), _pack(c, bits)
+        for m in (1, 8):
+            x = torch.randn(m, k, generator=g, device="cuda").half()
+            y = torch.empty(m, n, device="cuda")
+            assert L.lib().eoq_b200_gemv_packed(packed.data_ptr(), s.data_ptr(), n, k, bits, 128, x.data_ptr(), L.F16, m, None, y.data_ptr(), L.F32,
+                                                None, _stream()) == L.EOQ_OK
+            assert O.rel_l2(y.cpu().numpy(), (x.double() @ dense.T).cpu().numpy()) < 2e-6, (bits, m)
