@@ -1001,8 +1001,8 @@ struct eoq_b200_weight {
     size_t pair_partial_bytes = 0;
     DeviceBuf slab, stream;                           // everything but the stream in one allocation, the parts below point into it
     DeviceView table, tiles, scales, scales_t, centroids, counters, pair_partials;
+    DeviceView xbuf, ybuf, biasbuf;                   // staging of the host-buffer calls: eight rows of fp32 each, one bias
     DeviceBuf partials;                               // the ring kernel's scratch
-    DeviceBuf xbuf, ybuf, biasbuf;                    // staging of the host-buffer calls, allocated by their first
     DeviceBuf gemm_x, gemm_partials, gemm_counters;   // scratch of the tensor-core path, allocated by its first call
     uint32_t gemm_rows = 0;                           // activation rows per pass that scratch was sized for
     // The status word the kernels set when a bounded wait expires lives in pinned host memory that the device writes
@@ -1083,12 +1083,14 @@ eoq_error_t upload_weight(const TiledWeights &tw, const uint16_t *scales, const 
     auto part = [&](size_t bytes) { const size_t at = used; used += (bytes + 255) & ~(size_t)255; return at; };
     const size_t at_table = part(tw.table.size() * 4), at_tiles = part(tw.tiles.size() * sizeof(TileDesc)), at_scales = part(w->scale_bytes),
                  at_scales_t = part(pairs_layout ? (size_t)sg * triples * 8 : 0), at_cent = part(32 * 4), at_counters = part((size_t)tw.nrb * 4),
-                 at_partials = part(w->pair_partial_bytes);
+                 at_partials = part(w->pair_partial_bytes), at_x = part((size_t)8 * tw.K * 4), at_y = part((size_t)8 * tw.N * 4),
+                 at_bias = part((size_t)tw.N * 4);
     if (w->slab.alloc_pooled(used) != cudaSuccess || (!built && w->stream.alloc_pooled(tw.stream.size()) != cudaSuccess) ||
         (!pairs_layout && w->partials.alloc(w->partial_bytes) != cudaSuccess))
         return EOQ_ERR_ALLOC;
     uint8_t *base = w->slab.as<uint8_t>();
     w->table.p = base + at_table; w->tiles.p = base + at_tiles; w->scales.p = base + at_scales; w->counters.p = base + at_counters;
+    w->xbuf.p = base + at_x; w->ybuf.p = base + at_y; w->biasbuf.p = base + at_bias;
     if (built) w->stream.take(*built);
     else CU_TRY(upload(w->stream.p, tw.stream.data(), tw.stream.size(), nullptr));
     if (centroids) {
@@ -1666,11 +1668,6 @@ extern "C" eoq_error_t eoq_b200_gemv_host_async(eoq_b200_weight_t *w, const void
     if (drc != EOQ_OK) return drc;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     std::lock_guard<std::mutex> lock(w->mu);
-    if (!w->xbuf.p && (w->xbuf.alloc((size_t)8 * w->K * 4) != cudaSuccess || w->ybuf.alloc((size_t)8 * w->N * 4) != cudaSuccess ||
-                       w->biasbuf.alloc((size_t)w->N * 4) != cudaSuccess)) {
-        for (DeviceBuf *b : {&w->xbuf, &w->ybuf, &w->biasbuf}) if (b->p) { cudaFree(b->p); b->p = nullptr; }
-        return EOQ_ERR_ALLOC;
-    }
     CU_TRY(cudaMemcpyAsync(w->xbuf.p, x, (size_t)batch * w->K * esz[x_dtype], cudaMemcpyHostToDevice, st));
     if (bias_host) CU_TRY(cudaMemcpyAsync(w->biasbuf.p, bias_host, (size_t)w->N * 4, cudaMemcpyHostToDevice, st));
     // A pinned (page-locked) y is device-addressable: the kernel then stores its results straight into it and the

@@ -566,6 +566,27 @@ def test_host_buffer_gemv_async_two_weights_one_sync():
         assert O.rel_l2(y.float().numpy(), ref) < TOL
 
 
+def test_first_host_buffer_gemv_allocates_nothing_and_can_be_captured():
+    """The staging of the host-buffer calls belongs to the weight from the start: an allocation would end the capture."""
+    lib = L.lib()
+    n, k = 300, 1024
+    sym, s16, packed = _int4_case(n, k, 7)
+    w = EOQWeight.from_symbols(sym, s16)
+    other = EOQWeight.from_symbols(sym, s16)
+    x, bias = torch.randn(8, k).half().pin_memory(), torch.randn(n).pin_memory()
+    y = torch.zeros(8, n).half().pin_memory()
+    stream = torch.cuda.Stream()
+    L.check(lib.eoq_b200_gemv_host(other._h, x.data_ptr(), L.F16, 8, y.data_ptr(), L.F16, None, None), "kernel loaded")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        L.check(lib.eoq_b200_gemv_host_async(w._h, x.data_ptr(), L.F16, 8, y.data_ptr(), L.F16, bias.data_ptr(), stream.cuda_stream), "captured")
+    y.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    ref = O.int4_linear(packed, s16.astype(np.float32), n, k, 128, x.float().numpy(), bias.numpy())
+    assert O.rel_l2(y.float().numpy(), ref) < TOL
+
+
 @pytest.mark.parametrize("n,k", [(96, 256), (500, 1536), (1000, 11008), (4096, 4096), (193, 4096)])
 def test_dequantised_matrix_in_every_dtype_is_the_reference_product(n, k):
     """``EOQWeight.dequantize`` (the two-tiles-per-warp kernel for the default 4-bit layout; odd numbers of row blocks,
