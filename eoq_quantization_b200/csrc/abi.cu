@@ -40,7 +40,13 @@ struct DeviceBuf {
     DeviceBuf(const DeviceBuf &) = delete;
     DeviceBuf &operator=(const DeviceBuf &) = delete;
     ~DeviceBuf() { release(); }
-    cudaError_t alloc(size_t n) { return cudaMalloc(&p, n ? n : 1); }
+    // A refused allocation is the caller's to report: left set as the runtime's last error it would fail the next launch too.
+    cudaError_t alloc(size_t n)
+    {
+        const cudaError_t e = cudaMalloc(&p, n ? n : 1);
+        if (e != cudaSuccess) { p = nullptr; (void)cudaGetLastError(); }
+        return e;
+    }
     // Out of this library's own memory pool: a model load allocates and a replaced layer releases without the driver mapping
     // and unmapping memory each time (cudaMalloc and cudaFree of the 24 MB of a layer: 0.5 to 10 ms).  The pool keeps at
     // most 256 MB that nobody uses; what is beyond goes back to the driver.
@@ -51,7 +57,7 @@ struct DeviceBuf {
         if (e == cudaSuccess) e = weight_pool(device, pool);
         if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&p, n ? n : 1, pool, nullptr);
         pooled = e == cudaSuccess;
-        if (!pooled) p = nullptr;
+        if (!pooled) { p = nullptr; (void)cudaGetLastError(); }
         return e;
     }
     void take(DeviceBuf &o)
@@ -220,19 +226,27 @@ class DeviceArena {
 
 constexpr size_t kPinnedChunk = 256u << 10, kPinnedThreads = 16, kPinnedBytes = 2 * kPinnedChunk * kPinnedThreads;
 
+std::atomic<int> g_pinned_refused{0};                    // "pinned_refused" in eoq_b200_tune: requests for staging memory are too large to be met
+
 // Page-locked staging memory (8 MB a block), kept between calls: at most two blocks, the rest is given back at once.
 class PinnedBlock {
   public:
     PinnedBlock() = default;
     PinnedBlock(const PinnedBlock &) = delete;
     PinnedBlock &operator=(const PinnedBlock &) = delete;
-    cudaError_t acquire()
+    // False where the system has no such memory to give: the caller copies without it, and the refusal is nobody's error
+    // (left set, it would be what the next launch reports).
+    bool acquire()
     {
-        {
+        const bool refused = g_pinned_refused.load() != 0;
+        if (!refused) {
             std::lock_guard<std::mutex> lock(cache().mu);
-            if (!cache().free_list.empty()) { p_ = cache().free_list.back(); cache().free_list.pop_back(); return cudaSuccess; }
+            if (!cache().free_list.empty()) { p_ = cache().free_list.back(); cache().free_list.pop_back(); return true; }
         }
-        return cudaHostAlloc(reinterpret_cast<void **>(&p_), kPinnedBytes, cudaHostAllocPortable);
+        if (cudaHostAlloc(reinterpret_cast<void **>(&p_), refused ? (size_t)1 << 60 : kPinnedBytes, cudaHostAllocPortable) == cudaSuccess) return true;
+        p_ = nullptr;
+        (void)cudaGetLastError();
+        return false;
     }
     ~PinnedBlock()
     {
@@ -256,7 +270,7 @@ cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t st)
     const size_t chunks = (bytes + kPinnedChunk - 1) / kPinnedChunk, hw = std::max(1u, std::thread::hardware_concurrency());
     const size_t threads = std::min<size_t>({kPinnedThreads / 2, hw, chunks / 4});
     PinnedBlock pinned;
-    if (threads < 2 || pinned.acquire() != cudaSuccess) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    if (threads < 2 || !pinned.acquire()) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
@@ -826,11 +840,21 @@ eoq_error_t deliver(const uint8_t *dev, uint32_t elem, size_t n, void *out, int 
         case EOQ_B200_SYM_I64: fn = elem == 1 ? convert<uint8_t, int64_t> : convert<uint16_t, int64_t>; break;
         default: return EOQ_ERR_UNSUPPORTED;
     }
+    const size_t per = kPinnedChunk / elem, chunks = (n + per - 1) / per;
     PinnedBlock pinned;
-    if (pinned.acquire() != cudaSuccess) return EOQ_ERR_ALLOC;
+    if (!pinned.acquire()) {
+        // through pageable memory, a chunk at a time (such a copy has ended when the call returns)
+        std::vector<uint8_t> chunk(std::min(n, per) * elem);
+        for (size_t lo = 0; lo < n; lo += per) {
+            const size_t cnt = std::min(per, n - lo);
+            CU_TRY(cudaMemcpyAsync(chunk.data(), dev + lo * elem, cnt * elem, cudaMemcpyDeviceToHost, st));
+            CU_TRY(cudaStreamSynchronize(st));
+            fn(chunk.data(), static_cast<uint8_t *>(out) + lo * width[out_type], cnt, shift);
+        }
+        return EOQ_OK;
+    }
     int device = 0;
     CU_TRY(cudaGetDevice(&device));
-    const size_t per = kPinnedChunk / elem, chunks = (n + per - 1) / per;
     // a thread costs some tens of microseconds to start, a chunk of 256 Ki symbols about a hundred to convert to int64
     const size_t hw = std::max(1u, std::thread::hardware_concurrency());
     const size_t threads = std::max<size_t>(1, std::min<size_t>({kPinnedThreads, hw, (chunks + 1) / 2}));
@@ -1962,6 +1986,7 @@ extern "C" int eoq_b200_tune(const char *key, int value)
     if (std::strcmp(key, "v1_lanes") == 0) { set_v1_lanes(value); return 0; }
     if (std::strcmp(key, "packed_warps") == 0) { set_packed_warps(value); return 0; }
     if (std::strcmp(key, "dequant_vec") == 0) { set_dequant_vec(value); return 0; }
+    if (std::strcmp(key, "pinned_refused") == 0) { g_pinned_refused.store(value); return 0; }
     return -1;
 }
 

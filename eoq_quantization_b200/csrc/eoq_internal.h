@@ -18,7 +18,8 @@
 //                 warp, the default; 0 = always the one-tile-per-warp kernel),
 //   "gemm_warps" (warps per CTA of the tensor-core kernel, 2..16; 0 = as many as fit),
 //   "pdl" (1 = programmatic stream serialisation for the fused kernels, the default; 0 = plain launches),
-//   "v1_lanes" (1 = the lane-per-block wire-format decoder, the default; 0 = the one-thread-per-block kernel);
+//   "v1_lanes" (1 = the lane-per-block wire-format decoder, the default; 0 = the one-thread-per-block kernel),
+//   "pinned_refused" (1 = requests for page-locked staging memory fail, as on a system that has none left; 0 = they are met);
 // eoq_b200_launch_count is the number of kernels this library has launched since it was loaded.
 extern "C" int eoq_b200_tune(const char *key, int value);
 extern "C" uint64_t eoq_b200_launch_count(void);

@@ -50,3 +50,23 @@ def test_decoded_symbols_in_every_type(a, p, n):
     for dt, shift in ((np.int64, 0), (np.int64, -a), (np.int8, -7), (np.uint8, 0), (np.int16, -3), (np.uint16, 5), (np.int32, -a)):
         got = R.decode_blocks(freq, p, d.compressed_blocks, d.block_offsets, 1024, n, dt, shift)
         assert got.dtype == dt and np.array_equal(got, (sym + shift).astype(dt)), (dt, shift)
+
+
+@pytest.mark.gpu
+def test_codec_without_page_locked_memory():
+    """Where the system has no page-locked memory to give, streams and symbols are copied without it, to the same results,
+    and the refusal does not come back as the error of a launch."""
+    rng = np.random.default_rng(5)
+    n = 3000001                                               # a stream that several threads would stage (from 2 MB on)
+    sym = rng.integers(0, 255, n)
+    d = RB.BlockedRANSEncoder(block_size=1024, precision_bits=14).encode(sym, 255)
+    assert len(d.compressed_blocks) > 2 << 20
+    freq = R._normalize_frequencies(d.freq_table, 14)[0]
+    lib = R._lib.lib()
+    assert lib.eoq_b200_tune(b"pinned_refused", 1) == 0
+    try:
+        for dt, shift in ((np.int64, 0), (np.int8, -127)):
+            got = R.decode_blocks(freq, 14, d.compressed_blocks, d.block_offsets, 1024, n, dt, shift)
+            assert np.array_equal(got, (sym + shift).astype(dt)), dt
+    finally:
+        lib.eoq_b200_tune(b"pinned_refused", 0)
