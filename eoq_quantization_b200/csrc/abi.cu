@@ -1758,6 +1758,16 @@ extern "C" eoq_error_t eoq_b200_dequant_packed(const uint8_t *d_packed, const ui
     return EOQ_OK;
 }
 
+// What a launch of the product kernel came to.  A device that has no room for any cut of it (or a driver without tensor
+// maps) is a call that is not supported, which other routes may take; everything else is a failed launch.
+static eoq_error_t product_result(int e, const char *where)
+{
+    if (e == 0) return EOQ_OK;
+    if (e == (int)cudaErrorNotSupported) return EOQ_ERR_UNSUPPORTED;
+    std::fprintf(stderr, "%s: launch failed: %s\n", where, cudaGetErrorString((cudaError_t)e));
+    return EOQ_ERR_CUDA;
+}
+
 static QmmCall packed_call(const uint8_t *d_packed, const uint16_t *d_scales_fp16, uint32_t rows, uint32_t cols, uint32_t bits, uint32_t group,
                            const void *x, int x_dtype, uint32_t batch, void *d_scratch, void *y, int y_dtype, const float *bias)
 {
@@ -1799,8 +1809,7 @@ extern "C" eoq_error_t eoq_b200_gemv_packed(const uint8_t *d_packed, const uint1
         a.row_bytes = bits == 4 ? cols / 2 : bits == 2 ? cols / 4 : cols;
         e = launch_gemv_packed(a, stream);
     }
-    if (e != 0) { std::fprintf(stderr, "eoq_b200_gemv_packed: launch failed: %s\n", cudaGetErrorString((cudaError_t)e)); return EOQ_ERR_CUDA; }
-    return EOQ_OK;
+    return product_result(e, "eoq_b200_gemv_packed");
 }
 
 extern "C" eoq_error_t eoq_b200_linear_packed(const uint8_t *d_packed, const uint16_t *d_scales_fp16, uint32_t rows, uint32_t cols,
@@ -1823,8 +1832,7 @@ extern "C" eoq_error_t eoq_b200_linear_packed(const uint8_t *d_packed, const uin
         e = launch_split_rows(x, x_dtype, cols, batch, 1, d_scratch, factors, stream);
     }
     if (e == 0) e = launch_qmm(c, stream);
-    if (e != 0) { std::fprintf(stderr, "eoq_b200_linear_packed: launch failed: %s\n", cudaGetErrorString((cudaError_t)e)); return EOQ_ERR_CUDA; }
-    return EOQ_OK;
+    return product_result(e, "eoq_b200_linear_packed");
 }
 
 // For the torch-facing front (not in the public header): whether eoq_b200_linear_packed takes the call and is to be
@@ -1857,8 +1865,7 @@ extern "C" eoq_error_t eoq_b200_linear_polar_codes(const uint8_t *d_codes, const
     c.N = rows; c.K = cols; c.M = batch; c.bits = bits; c.group = block; c.split_x = 1; c.y_dtype = y_dtype;
     int e = launch_split_rows(x, x_dtype, cols, batch, block, d_scratch, factors, stream);
     if (e == 0) e = launch_qmm(c, stream);
-    if (e != 0) { std::fprintf(stderr, "eoq_b200_linear_polar_codes: launch failed: %s\n", cudaGetErrorString((cudaError_t)e)); return EOQ_ERR_CUDA; }
-    return EOQ_OK;
+    return product_result(e, "eoq_b200_linear_polar_codes");
 }
 
 // Bytes of scratch eoq_b200_weight_linear needs in front of the activations' part: the weight's codes, two per byte.
@@ -1900,8 +1907,7 @@ extern "C" eoq_error_t eoq_b200_weight_linear(eoq_b200_weight_t *w, const void *
         c.blocked_rows = w->Npad;
         e = launch_qmm(c, stream);
     }
-    if (e != 0) { std::fprintf(stderr, "eoq_b200_weight_linear: launch failed: %s\n", cudaGetErrorString((cudaError_t)e)); return EOQ_ERR_CUDA; }
-    return EOQ_OK;
+    return product_result(e, "eoq_b200_weight_linear");
 }
 
 // For the torch-facing front (not in the public header): whether eoq_b200_weight_linear takes the call and is to be
@@ -1950,8 +1956,7 @@ extern "C" eoq_error_t eoq_b200_gemv_polar_codes(const uint8_t *d_codes, const u
         a.N = rows; a.K = cols; a.batch = batch; a.entries = 1u << bits; a.y_dtype = y_dtype; a.block_shift = shift;
         e = launch_gemv_polar_codes(a, stream);
     }
-    if (e != 0) { std::fprintf(stderr, "eoq_b200_gemv_polar_codes: launch failed: %s\n", cudaGetErrorString((cudaError_t)e)); return EOQ_ERR_CUDA; }
-    return EOQ_OK;
+    return product_result(e, "eoq_b200_gemv_polar_codes");
 }
 
 extern "C" eoq_error_t eoq_b200_weight_status(eoq_b200_weight_t *w, void *stream)

@@ -869,7 +869,7 @@ int run_variant(QmmArgs a, uint32_t most, uint32_t step, const void *packed, uin
                 if (cost < best * (n > plan.tok_tiles && plan.T ? 0.95 : 0.999)) { best = cost; plan = Plan{T, n, split, cost}; }
             }
         }
-        if (!plan.T) return (int)cudaErrorLaunchOutOfResources;
+        if (!plan.T) return (int)cudaErrorNotSupported;
         std::lock_guard<std::mutex> lock(mu);
         keys[used % 32] = key;
         plans[used % 32] = plan;
@@ -886,7 +886,7 @@ int run_variant(QmmArgs a, uint32_t most, uint32_t step, const void *packed, uin
     if (!mapped ||
         !map_2d(xmap, BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, a.K, (uint64_t)a.M * a.planes, (uint64_t)a.K * 2,
                 64, s.T, CU_TENSOR_MAP_SWIZZLE_128B))
-        return (int)cudaErrorInvalidValue;
+        return (int)cudaErrorNotSupported;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows * a.split, plan.tok_tiles);
     cfg.blockDim = dim3(threads);

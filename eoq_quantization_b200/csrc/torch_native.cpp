@@ -7,7 +7,7 @@
 //
 // Every function returns None where anything is out of the ordinary (another device current, a subclass, gradients or
 // autocast asked for, a shape or type the route does not take, no rows): the caller then runs its Python path, which
-// handles those cases and raises the errors.
+// handles those cases and raises their errors.  An error of a call that was made is raised here.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -98,11 +98,24 @@ Tensor result(const Tensor &x, int64_t N, at::ScalarType type)
 
 void *stream_of(const Tensor &x) { return c10::cuda::getCurrentCUDAStream(x.get_device()).stream(); }
 
-// A call of the C ABI: None where the library says that it does not take the arguments (the Python path reports it).
-PyObject *done(eoq_error_t rc, Tensor &&y)
+// An error of the library as the exception that the Python path raises for it.  Only "not supported" is the caller's to
+// try another route for: a launch that failed would otherwise come back as a slower call, or as garbage later.
+PyObject *failed(eoq_error_t rc, const char *where)
 {
-    if (rc != EOQ_OK) Py_RETURN_NONE;
-    return THPVariable_Wrap(std::move(y));
+    if (rc == EOQ_ERR_UNSUPPORTED) Py_RETURN_NONE;
+    PyObject *lib = PyImport_ImportModule("eoq_quantization_b200._lib");
+    PyObject *r = lib ? PyObject_CallMethod(lib, "check", "is", (int)rc, where) : nullptr;
+    Py_XDECREF(lib);
+    if (r) {
+        Py_DECREF(r);
+        PyErr_SetString(PyExc_RuntimeError, where);
+    }
+    return nullptr;
+}
+
+PyObject *done(eoq_error_t rc, Tensor &&y, const char *where)
+{
+    return rc == EOQ_OK ? THPVariable_Wrap(std::move(y)) : failed(rc, where);
 }
 
 // x @ W.T (+ bias) by the library, W written by `fill` into a dense matrix of x's type.  Where rows of a 16-bit y would not
@@ -116,7 +129,7 @@ PyObject *dense_linear(const Tensor &x, int64_t N, int64_t K, int64_t rows, PyOb
     const bool pad = x.scalar_type() != at::kFloat && N % 8 && K % 8 == 0 && (rows > 32 || N >= 2048);
     const int64_t wide = pad ? (N + 7) & ~(int64_t)7 : N;
     Tensor dense = at::detail::empty_cuda({wide, K}, x.scalar_type(), x.device(), std::nullopt);
-    if (fill(dense.data_ptr()) != EOQ_OK) Py_RETURN_NONE;
+    if (const eoq_error_t rc = fill(dense.data_ptr()); rc != EOQ_OK) return failed(rc, "dequantised copy");
     at::AutoDispatchBelowADInplaceOrView guard;
     std::optional<Tensor> b;
     if (bias != Py_None) b = THPVariable_Unpack(bias).to(x.scalar_type());
@@ -154,12 +167,12 @@ PyObject *weight_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
     if (few) {
         if (rows > 8) Py_RETURN_NONE;
         Tensor y = result(*x, N, x->scalar_type());
-        return done(eoq_b200_gemv(w, x->data_ptr(), code, (uint32_t)rows, y.data_ptr(), code, b, st), std::move(y));
+        return done(eoq_b200_gemv(w, x->data_ptr(), code, (uint32_t)rows, y.data_ptr(), code, b, st), std::move(y), "eoq_b200_gemv");
     }
     if (product) {
         Tensor y = result(*x, N, x->scalar_type());
         Tensor scratch = at::detail::empty_cuda({(int64_t)eoq_b200_weight_linear_scratch(w, (uint32_t)rows, code)}, at::kByte, x->device(), std::nullopt);
-        return done(eoq_b200_weight_linear(w, x->data_ptr(), code, (uint32_t)rows, scratch.data_ptr(), y.data_ptr(), code, b, st), std::move(y));
+        return done(eoq_b200_weight_linear(w, x->data_ptr(), code, (uint32_t)rows, scratch.data_ptr(), y.data_ptr(), code, b, st), std::move(y), "eoq_b200_weight_linear");
     }
     return dense_linear(*x, N, K, rows, a[7], [&](void *dense) { return eoq_b200_weight_decode(w, nullptr, 0, dense, code, st); });
     GUARD_END
@@ -192,7 +205,7 @@ PyObject *packed_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
         Tensor y = result(*x, N, x->scalar_type());
         return done(eoq_b200_gemv_packed(codes, scales, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)group, x->data_ptr(), code,
                                          (uint32_t)rows, nullptr, y.data_ptr(), code, b, st),
-                    std::move(y));
+                    std::move(y), "eoq_b200_gemv_packed");
     }
     if (eoq_b200_linear_packed_preferred(codes, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)group, x->data_ptr(), code, (uint32_t)rows)) {
         Tensor y = result(*x, N, x->scalar_type()), scratch;
@@ -200,7 +213,7 @@ PyObject *packed_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
         if (f32) scratch = at::detail::empty_cuda({rows, K + 1}, at::kFloat, x->device(), std::nullopt);
         return done(eoq_b200_linear_packed(codes, scales, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)group, x->data_ptr(), code,
                                            (uint32_t)rows, f32 ? scratch.data_ptr() : nullptr, y.data_ptr(), code, b, st),
-                    std::move(y));
+                    std::move(y), "eoq_b200_linear_packed");
     }
     // a few rows against whole groups per row: the entropy-coded form may take them
     if (rows <= 8 && K % 16 == 0 && group % 16 == 0 && K % group == 0) Py_RETURN_NONE;
@@ -234,12 +247,12 @@ PyObject *polar_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
         eoq_error_t rc = eoq_b200_linear_polar_codes(codes, norms, cent, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)block, x->data_ptr(), code,
                                                      (uint32_t)rows, scratch.data_ptr(), y.data_ptr(), EOQ_B200_F16,
                                                      bias ? bias->data_ptr() : nullptr, EOQ_B200_F16, stream_of(*x));
-        if (rc == EOQ_OK) return THPVariable_Wrap(std::move(y));
+        if (rc != EOQ_ERR_UNSUPPORTED) return done(rc, std::move(y), "eoq_b200_linear_polar_codes");
     }
     if (rows > (block >= 64 ? 32 : 8)) Py_RETURN_NONE;
-    if (eoq_b200_gemv_polar_codes(codes, norms, cent, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)block, x->data_ptr(), code, (uint32_t)rows,
-                                  scratch.data_ptr(), y.data_ptr(), EOQ_B200_F16, nullptr, -1, stream_of(*x)) != EOQ_OK)
-        Py_RETURN_NONE;
+    const eoq_error_t rc = eoq_b200_gemv_polar_codes(codes, norms, cent, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)block, x->data_ptr(), code,
+                                                     (uint32_t)rows, scratch.data_ptr(), y.data_ptr(), EOQ_B200_F16, nullptr, -1, stream_of(*x));
+    if (rc != EOQ_OK) return failed(rc, "eoq_b200_gemv_polar_codes");
     at::AutoDispatchBelowADInplaceOrView guard;
     if (bias) y.add_(*bias);
     return THPVariable_Wrap(std::move(y));

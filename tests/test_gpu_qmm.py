@@ -165,3 +165,13 @@ def test_packed_gemv_warp_counts(n, k):
             assert L.lib().eoq_b200_gemv_packed(packed.data_ptr(), s.data_ptr(), n, k, bits, 128, x.data_ptr(), L.F16, m, None, y.data_ptr(), L.F32,
                                                 None, _stream()) == L.EOQ_OK
             assert O.rel_l2(y.cpu().numpy(), (x.double() @ dense.T).cpu().numpy()) < 2e-6, (bits, m)
+
+
+def test_errors_of_the_library_are_raised():
+    """A call that the library refuses or fails is an exception, not a second attempt by another route."""
+    x = torch.randn(1, 256, device="cuda").half()
+    native = L.native()
+    for rows in (1, 40):                                      # a weight that is gone: the fused GEMV, the decode to a dense matrix
+        with pytest.raises(L.EOQError) as e:
+            native.weight_linear(0, x.get_device(), 96, 256, 4, 8, x.expand(rows, 256).contiguous(), None)
+        assert e.value.code == L.EOQ_ERR_NULL_PTR
