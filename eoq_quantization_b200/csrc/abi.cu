@@ -1904,6 +1904,7 @@ extern "C" eoq_error_t eoq_b200_weight_linear(eoq_b200_weight_t *w, const void *
         QmmCall c = packed_call(codes, w->scales.as<uint16_t>(), w->N, w->K, 4, w->group, x, x_dtype, batch, halves, y, y_dtype, bias);
         if (x_dtype == EOQ_B200_F32) c.tok_scale = factors;
         c.late = 1;
+        c.status = w->status_word();
         c.blocked_rows = w->Npad;
         e = launch_qmm(c, stream);
     }
@@ -1991,6 +1992,7 @@ extern "C" int eoq_b200_tune(const char *key, int value)
     if (std::strcmp(key, "v1_lanes") == 0) { set_v1_lanes(value); return 0; }
     if (std::strcmp(key, "packed_warps") == 0) { set_packed_warps(value); return 0; }
     if (std::strcmp(key, "dequant_vec") == 0) { set_dequant_vec(value); return 0; }
+    if (std::strcmp(key, "qmm_wait_us") == 0) { set_qmm_wait_us(value); return 0; }
     if (std::strcmp(key, "pinned_refused") == 0) { g_pinned_refused.store(value); return 0; }
     return -1;
 }

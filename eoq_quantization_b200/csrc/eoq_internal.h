@@ -19,6 +19,8 @@
 //   "gemm_warps" (warps per CTA of the tensor-core kernel, 2..16; 0 = as many as fit),
 //   "pdl" (1 = programmatic stream serialisation for the fused kernels, the default; 0 = plain launches),
 //   "v1_lanes" (1 = the lane-per-block wire-format decoder, the default; 0 = the one-thread-per-block kernel),
+//   "qmm_wait_us" (what a wait of the product kernel may take in microseconds, 2000000 by default; 0 = not even the time the
+//                  kernels before it need),
 //   "pinned_refused" (1 = requests for page-locked staging memory fail, as on a system that has none left; 0 = they are met);
 // eoq_b200_launch_count is the number of kernels this library has launched since it was loaded.
 extern "C" int eoq_b200_tune(const char *key, int value);
@@ -245,12 +247,14 @@ struct QmmCall {
     void *y;
     uint32_t N, K, M, bits, group;
     int bf16, split_x, y_dtype, bias_half, late;     // late: `packed` is written by the kernel before this one in the stream
+    uint32_t *status;            // device address of a word to set when a wait runs out, or null: the one qmm_status reads
     uint32_t blocked_rows;       // not 0: 4-bit codes as [K / 16][blocked_rows] words of sixteen, as the decoder leaves them
 };
 bool qmm_takes(uint32_t K, uint32_t bits, uint32_t group, const void *packed, const void *x);
 int launch_qmm(const QmmCall &c, void *stream);
 bool qmm_preferred(const QmmCall &c, double copy_us, double least_us);
 uint32_t qmm_status();
+void set_qmm_wait_us(int v);
 bool split_rows_takes(uint32_t K, uint32_t block);
 int launch_split_rows(const void *x, int x_dtype, uint32_t K, uint32_t M, uint32_t block, void *planes, float *tok_scale, void *stream);
 void count_launch();

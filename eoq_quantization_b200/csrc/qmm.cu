@@ -37,7 +37,8 @@ namespace cg = cooperative_groups;
 
 namespace eoq {
 
-__device__ uint32_t g_qmm_status = 0;      // set when a bounded wait ran out (a copy or a product that never completed)
+// Set when a bounded wait ran out (a copy or a product that never completed), unless the call has a status word of its own.
+__device__ uint32_t g_qmm_status = 0;
 
 namespace {
 
@@ -55,13 +56,63 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity)
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// Bounded: after about two seconds of polling the status word is set, and nobody waits for long any more.
-__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity)
+// Waits are bounded.  One that runs out marks the CTA, which ends the waits of all its warps, and sets the status word; the
+// warps run on with whatever is there, only that nobody requests copies any more, nor tells the barriers that count a copy's
+// bytes (an arrival beyond their count while a copy is under way would break them).  The CTA's results become NaN.  Nothing
+// of that outlives the launch but the word: later launches wait as ever, only an eighth as long (a grid of many rounds would
+// otherwise take the full limit in each).
+//   The time of a kernel before this one, which programmatic launch may leave running for as long as it likes, does not
+// count.  (A limit of 0 has no patience with them either.)
+//   The outcome of a wait is not returned for every warp to leave its loop by: that alone costs the products' warp some
+// eighty cycles a block (24 rows against 11008 x 4096: 17.9 instead of 17.0 us).  What follows a first failed attempt is a
+// function of its own, out of the loops' way: 15.9 us (inline 17.0); four rows against a polar 14336 x 4096 34.8 (37.4).
+struct Waits {
+    uint32_t mark;               // shared address of two words: the CTA has given up; the kernels before this one have ended
+    long long limit;             // clock ticks
+    uint32_t *status;
+    __device__ __forceinline__ bool stopped() const
+    {
+        uint32_t v;
+        asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(mark) : "memory");
+        return v != 0;
+    }
+    __device__ __forceinline__ void operator()(uint32_t bar, uint32_t parity) const
+    {
+        if (!bar_try(bar, parity)) slow(bar, parity, mark, limit, status);
+    }
+    // The same, and whether the CTA has not given up: asked for together, in one latency.
+    __device__ __forceinline__ bool go(uint32_t bar, uint32_t parity) const
+    {
+        uint32_t ok, stop;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%2], %3;\n\tld.volatile.shared.u32 %1, [%4];\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok), "=r"(stop) : "r"(bar), "r"(parity), "r"(mark) : "memory");
+        if (ok) return stop == 0;
+        slow(bar, parity, mark, limit, status);
+        return !stopped();
+    }
+    static __device__ __noinline__ void slow(uint32_t bar, uint32_t parity, uint32_t mark, long long limit, uint32_t *status)
+    {
+        long long t0 = clock64();
+        while (!bar_try(bar, parity)) {
+            const long long now = clock64();
+            uint32_t stop, alone;
+            asm volatile("ld.volatile.shared.v2.u32 {%0, %1}, [%2];" : "=r"(stop), "=r"(alone) : "r"(mark) : "memory");
+            if (!alone && limit) t0 = now;
+            if (!stop && now - t0 <= limit && !(now - t0 > limit / 8 && *reinterpret_cast<volatile uint32_t *>(status))) continue;
+            asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(mark), "r"(1u) : "memory");
+            *reinterpret_cast<volatile uint32_t *>(status) = 1u;
+            return;
+        }
+    }
+};
+// The last uses of a ring of n barriers, of which `used` have been made: what the copy engine still has to bring is
+// there (or does not come for some ten milliseconds) before the CTA may leave its shared memory.
+__device__ __forceinline__ void drain(uint32_t bar, uint32_t used, uint32_t n)
 {
-    if (bar_try(bar, parity)) return;
     const long long t0 = clock64();
-    while (!bar_try(bar, parity))
-        if (clock64() - t0 > 4000000000ll || *(volatile uint32_t *)&g_qmm_status) { g_qmm_status = 1u; return; }
+    for (uint32_t u = used > n ? used - n : 0u; u < used; u++)
+        while (!bar_try(bar + 8u * (u % n), (u / n) & 1u))
+            if (clock64() - t0 > 20000000ll) return;
 }
 __device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint32_t bar)
 {
@@ -221,6 +272,8 @@ struct QmmArgs {
     uint32_t nw, ns, a_base;     // stages of packed weights and of operands (A in TMEM, activations in shared memory); first A column
     uint32_t at_x, at_bar;       // shared-memory offsets
     int y_dtype, bias_half, late;   // late: the packed codes are the previous kernel's to write
+    long long limit;             // clock ticks a wait may take
+    uint32_t *status;            // word to set when one runs out, or null: g_qmm_status
 };
 
 template <int BITS, int KB>
@@ -239,7 +292,7 @@ struct Ring {
 };
 
 // barriers, in this order, eight bytes each
-enum { kWFull = 0, kWEmpty = 8, kFull = 16, kEmpty = 24, kDFull = 32, kDEmpty = 34, kSFull = 36, kSEmpty = 40, kTmemSlot = 44 };
+enum { kWFull = 0, kWEmpty = 8, kFull = 16, kEmpty = 24, kDFull = 32, kDEmpty = 34, kSFull = 36, kSEmpty = 40, kTmemSlot = 44, kDrain = 45, kMark = 46, kUsedW = 47, kUsedX = 48 };
 constexpr uint32_t kScaleRing = 4, kScaleGroups = 8, kScaleEntry = kScaleGroups * kRows * 2u;      // scales of 8 groups x 128 rows an entry
 
 // The scales of one weight row in the order of the groups, out of the ring that a warp of the CTA keeps filled.
@@ -247,6 +300,8 @@ struct ScaleReader {
     uint32_t full, empty, at, row, entry = 0;      // barrier addresses, ring address
     Ring ring;
     bool here = false;                             // this entry has been waited for
+    const Waits &wait;
+    __device__ __forceinline__ ScaleReader(const Waits &w, uint32_t f, uint32_t e, uint32_t a, uint32_t r) : full(f), empty(e), at(a), row(r), wait(w) {}
     __device__ __forceinline__ uint16_t get(uint32_t g, uint32_t lane)      // g: group, counted from the CTA's first
     {
         while ((g >> 3) > entry) {
@@ -256,7 +311,7 @@ struct ScaleReader {
             entry++;
             here = false;
         }
-        if (!here) { bar_wait(full + 8u * ring.at, ring.lap); here = true; }
+        if (!here) { wait(full + 8u * ring.at, ring.lap); here = true; }
         uint16_t v;
         asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(at + ring.at * kScaleEntry + (g & 7u) * (kRows * 2u) + row * 2u));
         return v;
@@ -278,6 +333,8 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(raw) + 1023u) & ~(uintptr_t)1023u);
     const uint32_t base = saddr(smem), bars = base + a.at_bar;
     auto bar = [&](uint32_t i) { return bars + 8u * i; };
+    const Waits wait{bars + 8u * kMark, a.limit, a.status ? a.status : &g_qmm_status};
+    auto word = [&](uint32_t i) { return reinterpret_cast<volatile uint32_t *>(smem + a.at_bar + 8u * i); };
     const uint32_t scale_ring = bars + 512u;
     uint32_t *table = reinterpret_cast<uint32_t *>(smem + a.at_bar + 512 + kScaleRing * kScaleEntry);      // polar: centroids, as {high half, low half} (fold) or fp32
     uint32_t *largest = table + 256;              // polar, scaled: the largest norm of each row (bits of a float), then the largest centroid
@@ -300,6 +357,8 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
         }
         for (uint32_t i = 0; i < kScaleRing; i++) { bar_init(bar(kSFull + i), 1); bar_init(bar(kSEmpty + i), 4 * (FOLD ? NF : NP)); }
         for (uint32_t i = 0; i < 2; i++) { bar_init(bar(kDFull + i), 1); bar_init(bar(kDEmpty + i), 4 * NF); }
+        bar_init(bar(kDrain), 1);
+        word(kMark)[0] = word(kMark)[1] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (kPol) {
@@ -352,7 +411,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
         uint32_t four;
         asm volatile("mov.b32 %0, 4;" : "=r"(four));
         // scaled: the groups of 32-column parts, counted along
-        ScaleReader sr{bar(kSFull), bar(kSEmpty), scale_ring, r};
+        ScaleReader sr(wait, bar(kSFull), bar(kSEmpty), scale_ring, r);
         uint32_t gi = 0, pos = 0;
         if (!FOLD) {
             const uint32_t c = (kb0 + set) * KB;
@@ -366,7 +425,8 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
             for (; unit < i / U::kBlocks; unit++) wr.next(a.nw);
             const uint32_t ws = wr.at, row_at = base + ws * U::kStage + r * U::kBytes;
             const uint32_t sw = BITS == 2 ? (r >> 1) & 3u : r & 7u;
-            bar_wait(bar(kWFull + ws), wr.lap);
+            wait(bar(kWFull + ws), wr.lap);
+            bool go = true;
 #pragma unroll
             for (uint32_t part = 0; part < kHalves; part++) {
                 uint32_t w[U::kWords];
@@ -431,7 +491,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
                     for (int c = 0; c < U::kWords; c++) codes_scaled<kCode, BF16>(w[c], h + c * (32 / U::kWords), c < U::kWords / 2 ? s0 : s1);
                 }
                 if (part == 0) {
-                    bar_wait(bar(kEmpty + st), ar.lap ^ 1u);
+                    go = wait.go(bar(kEmpty + st), ar.lap ^ 1u);
                     fence_after();
                 }
                 __syncwarp();
@@ -443,7 +503,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
             __syncwarp();
             // every lane's codes are in its registers, converted and stored: only now may the copy engine have the stage
             // (an arrival straight behind the shared-memory loads let it overwrite rows that were still on their way)
-            if (lane == 0) { bar_arrive(bar(kFull + st)); bar_arrive(bar(kWEmpty + ws)); }
+            if (lane == 0 && go) { bar_arrive(bar(kFull + st)); bar_arrive(bar(kWEmpty + ws)); }
 #pragma unroll
             for (int j = 0; j < NP; j++) ar.next(a.ns);
         }
@@ -453,7 +513,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
         const uint32_t lane_base = tmem + (((warp & 3u) * 32u) << 16) + set * cols;
         float *stage = reinterpret_cast<float *>(smem) + (size_t)set * cols * kRows + r;
         if (FOLD) {
-            ScaleReader sr{bar(kSFull), bar(kSEmpty), scale_ring, r};
+            ScaleReader sr(wait, bar(kSFull), bar(kSEmpty), scale_ring, r);
             float tot[TC];
 #pragma unroll
             for (int c = 0; c < TC; c++) tot[c] = 0.0f;
@@ -461,7 +521,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
             for (uint32_t s = 0; s < nseg; s++) {
                 const float sc = __half2float(__ushort_as_half(sr.get(g, lane)));
                 if (++in_group == g16 / f16) { in_group = 0; g++; }
-                bar_wait(bar(kDFull + (s & 1u)), (s >> 1) & 1u);
+                wait(bar(kDFull + (s & 1u)), (s >> 1) & 1u);
                 __syncwarp();
                 fence_after();
 #pragma unroll
@@ -489,7 +549,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
             for (int c = 0; c < TC; c++)
                 if ((uint32_t)c < cols) stage[c * kRows] = tot[c];
         } else {
-            bar_wait(bar(kDFull), 0u);
+            wait(bar(kDFull), 0u);
             __syncwarp();
             fence_after();
             for (uint32_t c = 0; c < cols; c += 16) {
@@ -512,7 +572,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
         uint32_t seg = 0, in_seg = k16_0 - seg0 * f16, acc = 0, d = tmem;
         Ring ar;
         for (uint32_t i = 0; i < nkb; i++) {
-            bar_wait(bar(kFull + ar.at), ar.lap);
+            wait(bar(kFull + ar.at), ar.lap);
             fence_after();
             const uint32_t at = tmem + a.a_base + ar.at * kACols, left = k16_n - (kb0 + i) * kB16;
             const uint64_t desc = desc0 + ((ar.at * xstage) >> 4);
@@ -525,7 +585,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
             };
             auto open = [&]() {
                 d = tmem + (seg & 1u) * a.T;
-                bar_wait(bar(kDEmpty + (seg & 1u)), ((seg >> 1) & 1u) ^ 1u);
+                wait(bar(kDEmpty + (seg & 1u)), ((seg >> 1) & 1u) ^ 1u);
                 fence_after();
             };
             auto close = [&]() {
@@ -559,9 +619,11 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
         const bool leader = elect();
         if (a.late) asm volatile("griddepcontrol.wait;" ::: "memory");
         Ring wr;
+        uint32_t used = 0;
         for (uint32_t u = u0; u < u1; u++) {
-            bar_wait(bar(kWEmpty + wr.at), wr.lap ^ 1u);
-            if (leader) {
+            const bool go = wait.go(bar(kWEmpty + wr.at), wr.lap ^ 1u);
+            if (leader && go) {
+                used++;
                 bar_expect(bar(kWFull + wr.at), U::kStage);
                 if (BITS == kBlocked4) tma_2d(base + wr.at * U::kStage, &wmap, row0, u * (U::kCols / 16), bar(kWFull + wr.at));
                 else tma_2d(base + wr.at * U::kStage, &wmap, u * U::kBytes, row0, bar(kWFull + wr.at));
@@ -569,14 +631,18 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
             __syncwarp();
             wr.next(a.nw);
         }
+        if (leader) *word(kUsedW) = used;
     } else if (warp == 4 * NP + 4 * NF + 2) {
         // ---- activation copies
         const bool leader = elect();
         asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (leader) word(kMark)[1] = 1u;
         Ring xr;
+        uint32_t used = 0;
         for (uint32_t i = 0; i < nkb; i++) {
-            bar_wait(bar(kEmpty + xr.at), xr.lap ^ 1u);
-            if (leader) {
+            const bool go = wait.go(bar(kEmpty + xr.at), xr.lap ^ 1u);
+            if (leader && go) {
+                used++;
                 bar_expect(bar(kFull + xr.at), xstage);
                 for (uint32_t p = 0; p < a.planes; p++)
 #pragma unroll
@@ -586,6 +652,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
             __syncwarp();
             xr.next(a.ns);
         }
+        if (leader) *word(kUsedX) = used;
     } else {
         // ---- scales: eight groups of 128 rows at a time, transposed on the way ([group][row])
         Ring sr;
@@ -597,7 +664,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
 #pragma unroll
                 for (uint32_t g = 0; g < kScaleGroups; g++) v[j][g] = __ldg(srow + min(grp0 + g0 + g, a.sgroups - 1u));
             }
-            bar_wait(bar(kSEmpty + sr.at), sr.lap ^ 1u);
+            wait(bar(kSEmpty + sr.at), sr.lap ^ 1u);
             const uint32_t to = scale_ring + sr.at * kScaleEntry + lane * 2u;
 #pragma unroll
             for (uint32_t j = 0; j < 4; j++)
@@ -612,6 +679,15 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
     __syncwarp();
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __syncthreads();
+    if (wait.stopped()) {                          // the same for all threads: whoever sets the mark does so before the barrier above
+        // nothing may be under way any more when tensor and shared memory are given back
+        if (warp == 4 * NP + 4 * NF) { mma_commit(bar(kDrain)); drain(bar(kDrain), 1u, 1u); }
+        if (warp == 4 * NP + 4 * NF + 1) drain(bar(kWFull), *word(kUsedW), a.nw);
+        if (warp == 4 * NP + 4 * NF + 2) drain(bar(kFull), *word(kUsedX), a.ns);
+        __syncthreads();
+        for (uint32_t e = threadIdx.x; e < a.T * kRows; e += blockDim.x) reinterpret_cast<uint32_t *>(smem)[e] = 0x7fffffffu;
+        __syncthreads();
+    }
     if (warp == 4 * NP + 4 * NF) {
         fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kTmem) : "memory");
@@ -741,6 +817,9 @@ __global__ void __launch_bounds__(512) split_rows_kernel(const void *__restrict_
         *reinterpret_cast<__half2 *>(planes + (size_t)(M + m) * K + k) = __halves2half2(la, lb);
     }
 }
+
+static std::atomic<long long> g_qmm_limit{4000000000ll};         // about two seconds
+void set_qmm_wait_us(int v) { g_qmm_limit.store(std::min(std::max(v, 0), 60000000) * 2000ll); }
 
 namespace {
 
@@ -936,6 +1015,8 @@ int qmm(const QmmCall &c, void *stream, double *cycles)
     a.N = c.N; a.K = c.K; a.M = c.M; a.group = c.group; a.sgroups = c.K / c.group; a.y_dtype = c.y_dtype;
     a.bias_half = c.bias_half;
     a.late = c.late;
+    a.limit = g_qmm_limit.load(std::memory_order_relaxed);
+    a.status = c.status;
     for (uint32_t parts = 1; a.seg == 0; parts++)              // the fewest equal parts of a group, of 32-column multiples, that are short enough
         if (c.group % (32u * parts) == 0 && c.group / parts <= 128u) a.seg = c.group / parts;
     a.planes = c.split_x ? 2u : 1u;

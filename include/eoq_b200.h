@@ -502,7 +502,9 @@ size_t eoq_b200_weight_linear_scratch(const eoq_b200_weight_t *w, uint32_t batch
 eoq_error_t eoq_b200_weight_linear(eoq_b200_weight_t *w, const void *x, int x_dtype, uint32_t batch, void *d_scratch, void *y,
                                    int y_dtype, const float *bias, void *stream);
 
-/* 0, or nonzero if a bounded wait of one of these kernels has run out on the current device since the last call (synchronises). */
+/* 0, or nonzero if a bounded wait of one of the two kernels above eoq_b200_weight_linear has run out on the current device
+ * since the last call (synchronises; what a weight's own products meet is in its eoq_b200_weight_status).  The results of
+ * such a launch are NaN; the launches after it are not affected. */
 uint32_t eoq_b200_linear_status(void);
 
 /* y = x @ W.T (+ bias) straight from PolarLinear's in-memory form (kernels/polar_engine.py:144-360: one centroid index
