@@ -5,9 +5,10 @@
 // Python, EOQLinear took 25 us of host time around a 12 us kernel (4096 x 4096, one row) and the seven packed linears
 // of a 7B-shape block 160 us around 49 us of kernels.
 //
-// Every function returns None where anything is out of the ordinary (another device current, a subclass, gradients or
-// autocast asked for, a shape or type the route does not take, no rows): the caller then runs its Python path, which
-// handles those cases and raises their errors.  An error of a call that was made is raised here.
+// Activations that are strided or misaligned are copied first, and the activations' device is made current.  Every function
+// returns None where anything else is out of the ordinary (a subclass, gradients or autocast asked for, a shape or type the
+// route does not take, no rows): the caller then runs its Python path, which handles those cases and raises their errors.
+// An error of a call that was made is raised here.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -20,6 +21,7 @@
 #include <c10/core/GradMode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -60,16 +62,33 @@ bool plain_call(const Tensor &x)
            !c10::impl::TorchDispatchModeTLS::any_modes_set();
 }
 
-// x is a dense tensor [..., K] on the current device, 16-byte aligned, of a type the kernels take; gives its rows.
-bool activations(const Tensor &x, int64_t K, int &code, int64_t &rows)
-{
-    if (!x.is_cuda() || x.layout() != at::kStrided || x.dim() < 1 || x.size(-1) != K || K <= 0 || !plain_call(x)) return false;
-    code = dtype_code(x.scalar_type());
-    if (code < 0 || !x.is_contiguous() || (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u)) return false;
-    if (x.get_device() != c10::cuda::current_device()) return false;
-    rows = x.numel() / K;
-    return rows > 0 && rows <= 0x7fffffff;
-}
+// The activations of one call as the kernels take them: [..., K] of a type they know, contiguous and 16-byte aligned, their
+// device current for as long as this lives.
+struct Activations {
+    const Tensor *x = nullptr;
+    int code = -1;
+    int64_t rows = 0;
+    bool open(PyObject *o, int64_t K)
+    {
+        const Tensor *t = tensor_of(o);
+        if (!t || !t->is_cuda() || t->layout() != at::kStrided || t->dim() < 1 || t->size(-1) != K || K <= 0 || !plain_call(*t)) return false;
+        code = dtype_code(t->scalar_type());
+        rows = t->numel() / K;
+        if (code < 0 || rows < 1 || rows > 0x7fffffff) return false;
+        if (t->get_device() != c10::cuda::current_device()) guard.emplace(t->device());
+        x = t;
+        if (!t->is_contiguous() || (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15u)) {
+            at::AutoDispatchBelowADInplaceOrView below;
+            held = t->clone(at::MemoryFormat::Contiguous);
+            x = &held;
+        }
+        return true;
+    }
+
+  private:
+    Tensor held;
+    std::optional<c10::cuda::CUDAGuard> guard;
+};
 
 bool resident(const Tensor *t, const Tensor &x, at::ScalarType type)
 {
@@ -153,12 +172,13 @@ PyObject *weight_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     if (n != 8) { PyErr_SetString(PyExc_TypeError, "weight_linear takes 8 arguments"); return nullptr; }
     GUARD_BEGIN
-    const Tensor *x = tensor_of(a[6]);
     const int64_t dev = PyLong_AsLongLong(a[1]), N = PyLong_AsLongLong(a[2]), K = PyLong_AsLongLong(a[3]);
-    int code;
-    int64_t rows;
+    Activations act;
     const float *b;
-    if (!x || !activations(*x, K, code, rows) || x->get_device() != dev || !bias_ptr(a[7], *x, N, b)) Py_RETURN_NONE;
+    if (!act.open(a[6], K) || act.x->get_device() != dev || !bias_ptr(a[7], *act.x, N, b)) Py_RETURN_NONE;
+    const Tensor *x = act.x;
+    const int code = act.code;
+    const int64_t rows = act.rows;
     eoq_b200_weight_t *w = static_cast<eoq_b200_weight_t *>(PyLong_AsVoidPtr(a[0]));
     void *st = stream_of(*x);
     const bool product = rows > 1 && eoq_b200_weight_linear_preferred(w, x->data_ptr(), code, (uint32_t)rows);
@@ -185,12 +205,14 @@ PyObject *packed_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     if (n != 8) { PyErr_SetString(PyExc_TypeError, "packed_linear takes 8 arguments"); return nullptr; }
     GUARD_BEGIN
-    const Tensor *pk = tensor_of(a[0]), *sc = tensor_of(a[1]), *x = tensor_of(a[6]);
+    const Tensor *pk = tensor_of(a[0]), *sc = tensor_of(a[1]);
     const int64_t N = PyLong_AsLongLong(a[2]), K = PyLong_AsLongLong(a[3]), bits = PyLong_AsLongLong(a[4]), group = PyLong_AsLongLong(a[5]);
-    int code;
-    int64_t rows;
+    Activations act;
     const float *b;
-    if (!x || !pk || !activations(*x, K, code, rows) || !bias_ptr(a[7], *x, N, b) || group <= 0) Py_RETURN_NONE;
+    if (!act.open(a[6], K) || !bias_ptr(a[7], *act.x, N, b) || group <= 0) Py_RETURN_NONE;
+    const Tensor *x = act.x;
+    const int code = act.code;
+    const int64_t rows = act.rows;
     const at::ScalarType pt = bits == 4 || bits == 2 ? at::kByte : at::kChar;
     const int64_t row_bytes = bits == 4 ? (K + 1) / 2 : bits == 2 ? (K + 3) / 4 : K;
     if (!resident(pk, *x, pt) || !resident(sc, *x, at::kHalf) || pk->numel() != N * row_bytes || sc->numel() < (N * K + group - 1) / group)
@@ -229,11 +251,13 @@ PyObject *polar_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     if (n != 9) { PyErr_SetString(PyExc_TypeError, "polar_linear takes 9 arguments"); return nullptr; }
     GUARD_BEGIN
-    const Tensor *cd = tensor_of(a[0]), *nr = tensor_of(a[1]), *ct = tensor_of(a[2]), *x = tensor_of(a[7]);
+    const Tensor *cd = tensor_of(a[0]), *nr = tensor_of(a[1]), *ct = tensor_of(a[2]);
     const int64_t N = PyLong_AsLongLong(a[3]), K = PyLong_AsLongLong(a[4]), bits = PyLong_AsLongLong(a[5]), block = PyLong_AsLongLong(a[6]);
-    int code;
-    int64_t rows;
-    if (!x || !activations(*x, K, code, rows) || block < 16 || (block & (block - 1)) || K % block || bits < 1 || bits > 8) Py_RETURN_NONE;
+    Activations act;
+    if (block < 16 || (block & (block - 1)) || K % block || bits < 1 || bits > 8 || !act.open(a[7], K)) Py_RETURN_NONE;
+    const Tensor *x = act.x;
+    const int code = act.code;
+    const int64_t rows = act.rows;
     if (!resident(cd, *x, at::kChar) || !resident(nr, *x, at::kHalf) || !resident(ct, *x, at::kFloat) || cd->numel() < N * K ||
         nr->numel() < N * K / block || ct->numel() < (1 << bits))
         Py_RETURN_NONE;

@@ -1,0 +1,100 @@
+"""The routes of the modules' forward calls for what a program makes of them: the same kernels, straight from the codes, whatever
+the activations' layout, the types that a cast left in the module, and the mode the call is made in.  A dense copy of the weight
+shows in the allocator's peak, an entropy-coded one in the module."""
+import numpy as np
+import pytest
+import torch
+
+from eoq_quantization_b200 import _lib as L
+from eoq_quantization_b200.core.eoq_linear import EOQLinear
+from eoq_quantization_b200.core.polar_quant import polar_quantize
+from eoq_quantization_b200.core.quantized_linear import QuantizedLinear
+from eoq_quantization_b200.core.quantized_matmul import QuantizedLinearFast
+from eoq_quantization_b200.fused import EOQWeight
+from eoq_quantization_b200.kernels.polar_engine import PolarLinear
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+N, K = 2048, 4096                                             # a dense 16-bit copy of the weight: 16 MB
+TOL = {torch.float16: 1e-3, torch.bfloat16: 8e-3, torch.float32: 1e-5}      # the result's rounding (and one of code x scale beyond 128 rows)
+ROWS = (1, 8, 24, 200)
+
+
+def _layer(kind, bias=True):
+    torch.manual_seed(3)
+    lin = torch.nn.Linear(K, N, bias=bias)
+    if kind == "packed":
+        return QuantizedLinear.from_float(lin, bits=4, block_size=128).cuda()
+    if kind == "fast":
+        return QuantizedLinearFast.from_linear(lin, bits=4, block_size=128).cuda()
+    if kind == "polar":
+        return PolarLinear.from_linear(lin.cuda(), bits=5, block_size=64)
+    q = QuantizedLinear.from_float(lin, bits=4, block_size=128).cuda()
+    return EOQLinear(EOQWeight.from_int4_packed(q.packed_weight, q.scales, K), q.bias_param)
+
+
+def _dense(layer):
+    return (layer._dense_rows(0, N) if isinstance(layer, PolarLinear) else
+            QuantizedLinear._dequantize_weight(layer) if isinstance(layer, QuantizedLinearFast) else layer._dequantize_weight()).double()
+
+
+def _taken(layer, x):
+    """(result, bytes of device memory that the call needed at its peak)."""
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    y = layer(x)
+    return y, torch.cuda.max_memory_allocated() - before
+
+
+def _check(layer, x, dense, plain, extra=0, dtype=None):
+    """The product within the result's type, without an entropy-coded copy of the weight, and without a dense one where `plain`
+    (bytes the plain call on a plain module takes) has none: at most `extra` bytes more (and two megabytes, the allocator's rounding)."""
+    y, taken = _taken(layer, x)
+    dtype = dtype or (torch.float16 if isinstance(layer, PolarLinear) else x.dtype)
+    assert y.dtype == dtype and y.shape == (*x.shape[:-1], N)
+    want = x.detach().double() @ dense.T + (0 if layer.bias is None else layer.bias.double())
+    assert O.rel_l2(y.detach().double().cpu().numpy(), want.cpu().numpy()) < max(TOL[dtype], TOL[x.dtype] if x.dtype != dtype else 0), (x.shape, x.dtype)
+    assert taken <= plain + extra + (2 << 20), (taken, plain, x.shape, x.dtype)
+    assert getattr(layer, "_eoq", None) is None
+    return y
+
+
+def _plain(layer):
+    """What the plain call takes for every number of rows and type: no dense copy up to 24 rows."""
+    took = {(m, dt): _taken(layer, torch.randn(m, K, device="cuda").to(dt))[1] for m in ROWS for dt in TOL}
+    assert max(v for (m, _), v in took.items() if m <= 24) < N * K
+    return took
+
+
+def _odd(x, how):
+    """The same values, strided or off the 16-byte grid."""
+    if how == "strided":
+        return torch.stack([x, x], dim=-1)[..., 0]
+    if how == "transposed":
+        return x.T.contiguous().T
+    return torch.cat([x.flatten(), x.flatten()[:1]])[1:].view_as(x) if how == "misaligned" else x
+
+
+@pytest.mark.parametrize("kind", ["packed", "fast", "eoq", "polar"])
+@pytest.mark.parametrize("how", ["strided", "transposed", "misaligned"])
+def test_activations_that_are_not_plain_take_the_codes_route(kind, how):
+    layer = _layer(kind)
+    dense, plain = _dense(layer), _plain(layer)
+    for rows, dt in plain:
+        x = _odd(torch.randn(rows, K, device="cuda").to(dt), how)
+        _check(layer, x, dense, plain[rows, dt], extra=x.numel() * x.element_size())          # the copy of the activations
+
+
+class _Sub(torch.Tensor):
+    pass
+
+
+def test_tensor_subclasses_take_the_codes_route():
+    layer = _layer("packed")
+    dense = _dense(layer)
+    for rows in (1, 8, 24):
+        x = torch.randn(rows, K, device="cuda").half().as_subclass(_Sub)
+        assert O.rel_l2(layer(x).as_subclass(torch.Tensor).double().cpu().numpy(),
+                        (x.as_subclass(torch.Tensor).double() @ dense.T + layer.bias_param.double()).cpu().numpy()) < 1e-3
+        assert layer._eoq is None
