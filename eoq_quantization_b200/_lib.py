@@ -50,7 +50,7 @@ EXPORTS = [
     "eoq_b200_linear_status", "eoq_b200_weight_status",
 ]
 #: exported for this project's benchmarks and tests only (declared in csrc/eoq_internal.h, not in the public header)
-INTERNAL_EXPORTS = ["eoq_b200_linear_packed_preferred", "eoq_b200_weight_linear_preferred", "eoq_b200_tune", "eoq_b200_launch_count", "eoq_b200_weight_read"]
+INTERNAL_EXPORTS = ["eoq_b200_ordered_launches", "eoq_b200_linear_packed_preferred", "eoq_b200_weight_linear_preferred", "eoq_b200_tune", "eoq_b200_launch_count", "eoq_b200_weight_read"]
 
 
 class EOQError(RuntimeError):
@@ -185,6 +185,7 @@ def lib() -> C.CDLL:
         "eoq_b200_linear_status": (C.c_uint32, []),
         "eoq_b200_weight_status": (C.c_int, [vp, vp]),
         "eoq_b200_tune": (C.c_int, [C.c_char_p, C.c_int]),
+        "eoq_b200_ordered_launches": (C.c_int, [C.c_int]),
         "eoq_b200_launch_count": (C.c_uint64, []),
         "eoq_b200_weight_read": (C.c_uint64, [vp, C.c_int, vp, C.c_uint64]),
     }

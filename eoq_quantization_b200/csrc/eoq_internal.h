@@ -23,7 +23,11 @@
 //                  kernels before it need),
 //   "pinned_refused" (1 = requests for page-locked staging memory fail, as on a system that has none left; 0 = they are met);
 // eoq_b200_launch_count is the number of kernels this library has launched since it was loaded.
+// eoq_b200_ordered_launches(on) makes the calling thread's launches wait for all that is in front of them in the stream, for
+// callers that have just written scales, norms or centroids there (the kernels read those, like all resident parts of a weight,
+// before the kernel in front has ended); returns what was set before.
 extern "C" int eoq_b200_tune(const char *key, int value);
+extern "C" int eoq_b200_ordered_launches(int on);
 extern "C" uint64_t eoq_b200_launch_count(void);
 struct eoq_b200_weight;
 extern "C" uint64_t eoq_b200_weight_read(eoq_b200_weight *w, int what, void *host, uint64_t capacity);   // test hook, see abi.cu
@@ -270,6 +274,7 @@ uint64_t launch_counter();
 void set_gemv_ctas_per_sm(int v);
 void set_gemm_warps(int v);
 void set_pdl(int v);
+bool programmatic_launches();      // whether this thread's launches may start under the kernel in front of them
 void set_gemv_pairs(int v);
 uint32_t pair_partial_slots(uint32_t nrb, uint32_t nseg);
 bool gemv_takes_pairs(const GemvArgs &a, uint32_t G, uint32_t bits, uint32_t kind);

@@ -779,6 +779,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_tiles_kernel(const GemvArgs a
 // input or write anything.  "pdl" = 0 in eoq_b200_tune falls back to plain launches.
 static std::atomic<int> g_pdl{1};
 void set_pdl(int v) { g_pdl.store(v != 0); }
+static thread_local int t_ordered = 0;           // this thread's launches wait for what is in front of them (eoq_b200_ordered_launches)
+bool programmatic_launches() { return g_pdl.load() && !t_ordered; }
+extern "C" int eoq_b200_ordered_launches(int on)
+{
+    const int was = t_ordered;
+    t_ordered = on != 0;
+    return was;
+}
 
 template <typename Kern, typename... Args>
 static cudaError_t launch_with_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)
@@ -792,7 +800,7 @@ static cudaError_t launch_with_pdl(Kern kern, dim3 grid, dim3 block, size_t smem
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = g_pdl.load() ? 1 : 0;
+    cfg.numAttrs = programmatic_launches() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 

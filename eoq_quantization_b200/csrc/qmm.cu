@@ -973,7 +973,7 @@ int run_variant(QmmArgs a, uint32_t most, uint32_t step, const void *packed, uin
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = programmatic_launches();
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = a.split; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
@@ -1089,7 +1089,7 @@ int launch_split_rows(const void *x, int x_dtype, uint32_t K, uint32_t M, uint32
     cfg.stream = reinterpret_cast<cudaStream_t>(stream);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = programmatic_launches();
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, kern, x, x_dtype, K, M, reinterpret_cast<__half *>(planes), tok_scale);

@@ -16,6 +16,7 @@
 #include <ATen/autocast_mode.h>
 #include <ATen/core/LegacyTypeDispatch.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <ATen/ops/add.h>
 #include <ATen/ops/constant_pad_nd.h>
 #include <ATen/ops/linear.h>
 #include <c10/core/GradMode.h>
@@ -32,6 +33,7 @@
 
 extern "C" int eoq_b200_linear_packed_preferred(const uint8_t *d_packed, uint32_t rows, uint32_t cols, uint32_t bits, uint32_t group,
                                                 const void *x, int x_dtype, uint32_t batch);
+extern "C" int eoq_b200_ordered_launches(int on);
 extern "C" int eoq_b200_weight_linear_preferred(const eoq_b200_weight_t *w, const void *x, int x_dtype, uint32_t batch);
 
 namespace {
@@ -95,16 +97,54 @@ bool resident(const Tensor *t, const Tensor &x, at::ScalarType type)
     return t && t->is_cuda() && t->get_device() == x.get_device() && t->scalar_type() == type && t->is_contiguous();
 }
 
-// `bias` (None or an fp32 vector of N values beside x) as the kernels take it; false if it is anything else.
-bool bias_ptr(PyObject *o, const Tensor &x, int64_t N, const float *&b)
-{
-    b = nullptr;
-    if (o == Py_None) return true;
-    const Tensor *t = tensor_of(o);
-    if (!resident(t, x, at::kFloat) || t->numel() != N) return false;
-    b = static_cast<const float *>(t->data_ptr());
-    return true;
-}
+// A parameter of the module beside x in the type that the kernels read, converted for this call where a cast of the module
+// (half(), to(bfloat16), float(), double()) left it in another one: for this call only, since nothing that a copy could be
+// kept by says that the parameter has not been written since.
+struct Parameter {
+    const Tensor *t = nullptr;
+    bool converted = false;
+    bool open(PyObject *o, const Tensor &x, at::ScalarType type)
+    {
+        t = tensor_of(o);
+        if (!t || !t->is_cuda() || t->get_device() != x.get_device() || t->layout() != at::kStrided || !t->is_floating_point()) return false;
+        if (t->scalar_type() == type && t->is_contiguous()) return true;
+        at::AutoDispatchBelowADInplaceOrView below;
+        held = t->to(type).contiguous();
+        t = &held;
+        converted = true;
+        return true;
+    }
+
+  private:
+    Tensor held;
+};
+
+// `bias` (None or a vector of N values beside x) as the kernels take it, fp32; false if it is anything else.
+struct Bias {
+    const float *p = nullptr;
+    bool open(PyObject *o, const Tensor &x, int64_t N)
+    {
+        if (o == Py_None) return true;
+        if (!value.open(o, x, at::kFloat) || value.t->numel() != N) return false;
+        p = static_cast<const float *>(value.t->data_ptr());
+        return true;
+    }
+
+  private:
+    Parameter value;
+};
+
+// While this lives the library launches its kernels one behind the other: they read scales before the kernel in front of them
+// has ended, which may be the one that is writing the converted copy.
+struct Ordered {
+    explicit Ordered(bool on) : was(on ? eoq_b200_ordered_launches(1) : -1) {}
+    ~Ordered() { if (was >= 0) eoq_b200_ordered_launches(was); }
+    Ordered(const Ordered &) = delete;
+    Ordered &operator=(const Ordered &) = delete;
+
+  private:
+    int was;
+};
 
 Tensor result(const Tensor &x, int64_t N, at::ScalarType type)
 {
@@ -174,9 +214,10 @@ PyObject *weight_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
     GUARD_BEGIN
     const int64_t dev = PyLong_AsLongLong(a[1]), N = PyLong_AsLongLong(a[2]), K = PyLong_AsLongLong(a[3]);
     Activations act;
-    const float *b;
-    if (!act.open(a[6], K) || act.x->get_device() != dev || !bias_ptr(a[7], *act.x, N, b)) Py_RETURN_NONE;
+    Bias bias;
+    if (!act.open(a[6], K) || act.x->get_device() != dev || !bias.open(a[7], *act.x, N)) Py_RETURN_NONE;
     const Tensor *x = act.x;
+    const float *b = bias.p;
     const int code = act.code;
     const int64_t rows = act.rows;
     eoq_b200_weight_t *w = static_cast<eoq_b200_weight_t *>(PyLong_AsVoidPtr(a[0]));
@@ -205,23 +246,26 @@ PyObject *packed_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     if (n != 8) { PyErr_SetString(PyExc_TypeError, "packed_linear takes 8 arguments"); return nullptr; }
     GUARD_BEGIN
-    const Tensor *pk = tensor_of(a[0]), *sc = tensor_of(a[1]);
+    const Tensor *pk = tensor_of(a[0]);
     const int64_t N = PyLong_AsLongLong(a[2]), K = PyLong_AsLongLong(a[3]), bits = PyLong_AsLongLong(a[4]), group = PyLong_AsLongLong(a[5]);
     Activations act;
-    const float *b;
-    if (!act.open(a[6], K) || !bias_ptr(a[7], *act.x, N, b) || group <= 0) Py_RETURN_NONE;
+    Bias bias;
+    Parameter sc;
+    if (group <= 0 || !act.open(a[6], K) || !bias.open(a[7], *act.x, N) || !sc.open(a[1], *act.x, at::kHalf)) Py_RETURN_NONE;
     const Tensor *x = act.x;
+    const float *b = bias.p;
+    const Ordered ordered(sc.converted);
     const int code = act.code;
     const int64_t rows = act.rows;
     const at::ScalarType pt = bits == 4 || bits == 2 ? at::kByte : at::kChar;
     const int64_t row_bytes = bits == 4 ? (K + 1) / 2 : bits == 2 ? (K + 3) / 4 : K;
-    if (!resident(pk, *x, pt) || !resident(sc, *x, at::kHalf) || pk->numel() != N * row_bytes || sc->numel() < (N * K + group - 1) / group)
+    if (!resident(pk, *x, pt) || pk->numel() != N * row_bytes || sc.t->numel() < (N * K + group - 1) / group)
         Py_RETURN_NONE;
     // two-bit codes in groups below 128 columns against a few fp32 rows stay with the entropy-coded GEMV
     if (bits == 2 && code == EOQ_B200_F32 && rows <= 8 && group % 128 && group % 16 == 0 && K % group == 0) Py_RETURN_NONE;
     void *st = stream_of(*x);
     const uint8_t *codes = static_cast<const uint8_t *>(pk->data_ptr());
-    const uint16_t *scales = static_cast<const uint16_t *>(sc->data_ptr());
+    const uint16_t *scales = static_cast<const uint16_t *>(sc.t->data_ptr());
     const bool f32 = code == EOQ_B200_F32, aligned = (reinterpret_cast<uintptr_t>(codes) & 15u) == 0;
     if (rows <= 8 && !f32 && aligned && K % 128 == 0 && group % 128 == 0 && K % group == 0) {
         Tensor y = result(*x, N, x->scalar_type());
@@ -251,35 +295,51 @@ PyObject *polar_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     if (n != 9) { PyErr_SetString(PyExc_TypeError, "polar_linear takes 9 arguments"); return nullptr; }
     GUARD_BEGIN
-    const Tensor *cd = tensor_of(a[0]), *nr = tensor_of(a[1]), *ct = tensor_of(a[2]);
+    const Tensor *cd = tensor_of(a[0]);
     const int64_t N = PyLong_AsLongLong(a[3]), K = PyLong_AsLongLong(a[4]), bits = PyLong_AsLongLong(a[5]), block = PyLong_AsLongLong(a[6]);
     Activations act;
     if (block < 16 || (block & (block - 1)) || K % block || bits < 1 || bits > 8 || !act.open(a[7], K)) Py_RETURN_NONE;
     const Tensor *x = act.x;
     const int code = act.code;
     const int64_t rows = act.rows;
-    if (!resident(cd, *x, at::kChar) || !resident(nr, *x, at::kHalf) || !resident(ct, *x, at::kFloat) || cd->numel() < N * K ||
-        nr->numel() < N * K / block || ct->numel() < (1 << bits))
+    Parameter nr, ct;
+    if (!resident(cd, *x, at::kChar) || !nr.open(a[1], *x, at::kHalf) || !ct.open(a[2], *x, at::kFloat) || cd->numel() < N * K ||
+        nr.t->numel() < N * K / block || ct.t->numel() < (1 << bits))
         Py_RETURN_NONE;
-    const Tensor *bias = a[8] == Py_None ? nullptr : tensor_of(a[8]);
-    if (a[8] != Py_None && (!resident(bias, *x, at::kHalf) || bias->numel() != N)) Py_RETURN_NONE;
+    // what the kernels read is what the module holds: wider types are rounded for the few rows that always took this route
+    if (rows > 32 && (tensor_of(a[1])->element_size() > 2 || tensor_of(a[2])->element_size() > 4)) Py_RETURN_NONE;
+    const Ordered ordered(nr.converted || ct.converted);
+    // a bias of another type than the result's is added to it, in the type that the two come to
+    const Tensor *bias = a[8] == Py_None ? nullptr : tensor_of(a[8]), *after = nullptr;
+    if (a[8] != Py_None) {
+        if (!bias || !bias->is_cuda() || bias->get_device() != x->get_device() || bias->numel() != N) Py_RETURN_NONE;
+        if (!resident(bias, *x, at::kHalf)) std::swap(bias, after);
+    }
+    auto finish = [&](Tensor &&y) {
+        if (!after) return THPVariable_Wrap(std::move(y));
+        at::AutoDispatchBelowADInplaceOrView below;
+        return THPVariable_Wrap(y.add(*after));
+    };
     const uint8_t *codes = static_cast<const uint8_t *>(cd->data_ptr());
-    const uint16_t *norms = static_cast<const uint16_t *>(nr->data_ptr());
-    const float *cent = static_cast<const float *>(ct->data_ptr());
+    const uint16_t *norms = static_cast<const uint16_t *>(nr.t->data_ptr());
+    const float *cent = static_cast<const float *>(ct.t->data_ptr());
     Tensor y = result(*x, N, at::kHalf), scratch = at::detail::empty_cuda({rows, K + 1}, at::kFloat, x->device(), std::nullopt);
     if (rows > 1 || N * K < kPolarSingleRowWeights) {
         eoq_error_t rc = eoq_b200_linear_polar_codes(codes, norms, cent, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)block, x->data_ptr(), code,
                                                      (uint32_t)rows, scratch.data_ptr(), y.data_ptr(), EOQ_B200_F16,
                                                      bias ? bias->data_ptr() : nullptr, EOQ_B200_F16, stream_of(*x));
-        if (rc != EOQ_ERR_UNSUPPORTED) return done(rc, std::move(y), "eoq_b200_linear_polar_codes");
+        if (rc == EOQ_OK) return finish(std::move(y));
+        if (rc != EOQ_ERR_UNSUPPORTED) return failed(rc, "eoq_b200_linear_polar_codes");
     }
     if (rows > (block >= 64 ? 32 : 8)) Py_RETURN_NONE;
     const eoq_error_t rc = eoq_b200_gemv_polar_codes(codes, norms, cent, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)block, x->data_ptr(), code,
                                                      (uint32_t)rows, scratch.data_ptr(), y.data_ptr(), EOQ_B200_F16, nullptr, -1, stream_of(*x));
     if (rc != EOQ_OK) return failed(rc, "eoq_b200_gemv_polar_codes");
-    at::AutoDispatchBelowADInplaceOrView guard;
-    if (bias) y.add_(*bias);
-    return THPVariable_Wrap(std::move(y));
+    if (bias) {
+        at::AutoDispatchBelowADInplaceOrView below;
+        y.add_(*bias);
+    }
+    return finish(std::move(y));
     GUARD_END
 }
 

@@ -6,6 +6,7 @@ into ``libeoq_b200.so``.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 from typing import Optional, Sequence
 
@@ -44,6 +45,18 @@ PACKED_TENSOR_ROWS = 32       # activation rows the tensor-core form of the pack
 def fused_rows(dtype: torch.dtype) -> int:
     """Activation rows up to which the fused decode + GEMV is the fastest route for this activation type."""
     return GEMV_MAX_ROWS.get(dtype, 0)
+
+
+@contextlib.contextmanager
+def _ordered_launches(on: bool):
+    """The library's launches wait for what is in front of them in the stream: for calls whose weight was converted just there
+    (the kernels read it before the kernel in front has ended)."""
+    was = _lib.lib().eoq_b200_ordered_launches(1) if on else 0
+    try:
+        yield
+    finally:
+        if on:
+            _lib.lib().eoq_b200_ordered_launches(was)
 
 
 class EOQWeight:
@@ -353,7 +366,8 @@ def gemv_packed(packed: torch.Tensor, scales: torch.Tensor, rows: int, cols: int
     b = None if bias is None else bias.to(device=x.device, dtype=torch.float32).contiguous()
     # fp32 activations on the tensor-core form: room for their two fp16 halves
     scratch = torch.empty((n, cols), dtype=torch.float32, device=x.device) if x.dtype == torch.float32 and cols % 128 == 0 and group % 128 == 0 else None
-    with torch.cuda.device(x.device):
+    converted = pk.data_ptr() != packed.data_ptr() or sc.data_ptr() != scales.data_ptr()
+    with torch.cuda.device(x.device), _ordered_launches(converted):
         _lib.check(_lib.lib().eoq_b200_gemv_packed(pk.data_ptr(), sc.data_ptr(), rows, cols, bits, group, x2.data_ptr(), _DTYPES[x.dtype], n,
                                                    scratch.data_ptr() if scratch is not None else None,
                                                    y.data_ptr(), _DTYPES[out_dtype], b.data_ptr() if b is not None else None, _stream_ptr()),
@@ -394,7 +408,8 @@ def gemv_polar_codes(codes: torch.Tensor, norms: torch.Tensor, centroids: torch.
     scratch = torch.empty((n, cols), dtype=torch.float32, device=x.device)          # the rotated activations
     y = torch.empty((n, rows), dtype=out_dtype, device=x.device)
     b = None if bias is None else bias.to(device=x.device, dtype=torch.float32).contiguous()
-    with torch.cuda.device(x.device):
+    converted = cd.data_ptr() != codes.data_ptr() or nr.data_ptr() != norms.data_ptr() or ct.data_ptr() != centroids.data_ptr()
+    with torch.cuda.device(x.device), _ordered_launches(converted):
         _lib.check(_lib.lib().eoq_b200_gemv_polar_codes(cd.data_ptr(), nr.data_ptr(), ct.data_ptr(), rows, cols, bits, block, x2.data_ptr(),
                                                         _DTYPES[x.dtype], n, scratch.data_ptr(), y.data_ptr(), _DTYPES[out_dtype],
                                                         b.data_ptr() if b is not None else None,
