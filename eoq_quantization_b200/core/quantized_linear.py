@@ -13,7 +13,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _lib
-from ..fused import (GEMM_MAX_ROWS, EOQWeight, PACKED_TENSOR_ROWS, dequant_packed, fused_rows, gemv_packed, packed_gemv_rows,
+from ..fused import (GEMM_MAX_ROWS, PLAIN, EOQWeight, PACKED_TENSOR_ROWS, call_kind, dequant_packed, fused_rows, gemv_packed, packed_gemv_rows,
                      require_cuda)
 
 
@@ -139,10 +139,11 @@ class QuantizedLinear(nn.Module):
         require_cuda(x, "QuantizedLinear.forward")
         require_cuda(self.packed_weight, "QuantizedLinear.forward")
         rows = x.numel() // max(self.in_features, 1)
-        if x.dtype in (torch.float16, torch.bfloat16, torch.float32) and \
+        plain = call_kind(x, bias) == PLAIN
+        if plain and x.dtype in (torch.float16, torch.bfloat16, torch.float32) and \
                 1 <= rows <= PACKED_TENSOR_ROWS == packed_gemv_rows(self.in_features, self.bits, self.block_size, x.dtype):
             return gemv_packed(self.packed_weight, self.scales, self.out_features, self.in_features, self.bits, self.block_size, x, bias)
-        if self._fusable() and rows >= 1 and x.dtype in (torch.float16, torch.bfloat16, torch.float32):
+        if plain and self._fusable() and rows >= 1 and x.dtype in (torch.float16, torch.bfloat16, torch.float32):
             # up to fused_rows (4 rows of 16-bit activations, 8 of fp32): fused decode + GEMV, fp32 accumulate; beyond
             # that one dequantisation amortises over enough rows for a library GEMM to win (the fused tensor-core
             # kernel would take 9..GEMM_MAX_ROWS rows of 16-bit activations if that constant were raised)

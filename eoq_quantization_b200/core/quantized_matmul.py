@@ -11,7 +11,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _lib
-from ..fused import GEMM_MAX_ROWS, EOQWeight, dequant_packed, fused_rows, gemv_packed, PACKED_TENSOR_ROWS, packed_gemv_rows, require_cuda
+from ..fused import GEMM_MAX_ROWS, WATCHED, EOQWeight, call_kind, dequant_packed, fused_rows, gemv_packed, PACKED_TENSOR_ROWS, packed_gemv_rows, require_cuda
 
 _SUPPORTED_BITS = (2, 4, 8)
 _MEMORY_THRESHOLD = 16 * 1024 * 1024
@@ -141,12 +141,13 @@ class QuantizedLinearFast(nn.Module):
                 return y
         require_cuda(x, "QuantizedLinearFast.forward")
         rows = x.numel() // max(self.in_features, 1)
-        if self.strategy == "auto" and x.dtype in (torch.float16, torch.bfloat16, torch.float32) and \
+        codes = self.strategy == "auto" and x.dtype in (torch.float16, torch.bfloat16, torch.float32) and call_kind(x, self.bias_param) != WATCHED
+        if codes and \
                 1 <= rows <= PACKED_TENSOR_ROWS == packed_gemv_rows(self.in_features, self.bits, self.block_size, x.dtype):
             # one pass over the packed codes on the tensor cores (HBM-bound), see QuantizedLinear.forward
             return gemv_packed(self.packed_weight, self.scales, self.out_features, self.in_features, self.bits, self.block_size,
                                x, self.bias_param)
-        if self.strategy == "auto" and self._fusable() and rows >= 1 and x.dtype in (torch.float16, torch.bfloat16, torch.float32):
+        if codes and self._fusable() and rows >= 1:
             # up to fused_rows (4 rows of 16-bit activations, 8 of fp32): fused decode + GEMV, fp32 accumulate; beyond
             # that one dequantisation amortises over enough rows for a library GEMM to win (the fused tensor-core
             # kernel would take 9..GEMM_MAX_ROWS rows of 16-bit activations if that constant were raised)

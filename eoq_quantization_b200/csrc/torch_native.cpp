@@ -6,8 +6,8 @@
 // of a 7B-shape block 160 us around 49 us of kernels.
 //
 // Activations that are strided or misaligned are copied first, and the activations' device is made current.  Every function
-// returns None where anything else is out of the ordinary (a subclass, gradients or autocast asked for, a shape or type the
-// route does not take, no rows): the caller then runs its Python path, which handles those cases and raises their errors.
+// returns None where anything else is out of the ordinary (a subclass, gradients, autocast or a transform of the call asked
+// for, a shape or type the route does not take, no rows): the caller then runs its Python path, which handles those cases and raises their errors.
 // An error of a call that was made is raised here.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -20,13 +20,16 @@
 #include <ATen/ops/constant_pad_nd.h>
 #include <ATen/ops/linear.h>
 #include <c10/core/GradMode.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <cstring>
+#include <optional>
 #include <vector>
 
 #include "../../include/eoq_b200.h"
@@ -57,12 +60,38 @@ int dtype_code(at::ScalarType t)
 
 const Tensor *tensor_of(PyObject *o) { return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr; }
 
-// Nothing is going to watch or rewrite this call: no gradient through x, no autocast, no dispatch mode.
-bool plain_call(const Tensor &x)
+// What torch is to make of a call besides running it: nothing; gradients with respect to one of its tensors; or something that
+// only its own operations know how to do (vmap and the other function transforms, forward-mode tangents, tracing, dispatch
+// modes, tensors that stand for others).
+enum CallKind { kPlain = 0, kGradient = 1, kWatched = 2 };
+
+CallKind kind_of(const Tensor &t)
 {
-    return !(x.requires_grad() && c10::GradMode::is_enabled()) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
-           !c10::impl::TorchDispatchModeTLS::any_modes_set();
+    // a dense CUDA tensor's keys, and nothing else
+    static const uint64_t dense = (c10::DispatchKeySet(c10::DispatchKey::CUDA) | c10::DispatchKeySet(c10::DispatchKey::AutogradCUDA) |
+                                   c10::DispatchKeySet(c10::DispatchKey::ADInplaceOrView) | c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA)).raw_repr();
+    if ((t.key_set().raw_repr() & ~dense) || t._fw_grad(0).defined()) return kWatched;
+    return t.requires_grad() && c10::GradMode::is_enabled() ? kGradient : kPlain;
 }
+
+bool thread_is_watched()
+{
+    static const uint64_t always = (c10::DispatchKeySet(c10::DispatchKey::BackendSelect) | c10::DispatchKeySet(c10::DispatchKey::ADInplaceOrView)).raw_repr();
+    return (c10::impl::tls_local_dispatch_key_set().included_.raw_repr() & ~always) || c10::impl::TorchDispatchModeTLS::any_modes_set();
+}
+
+// call_kind(tensor or None, ...): the kind of a call on these tensors, the strongest of all.  (A tensor that is not on a CUDA
+// device, or a subclass, says nothing.)
+PyObject *call_kind(PyObject *, PyObject *const *a, Py_ssize_t n)
+{
+    int kind = thread_is_watched() ? kWatched : kPlain;
+    for (Py_ssize_t i = 0; i < n; i++)
+        if (const Tensor *t = tensor_of(a[i]); t && t->is_cuda()) kind = std::max(kind, (int)kind_of(*t));
+    return PyLong_FromLong(kind);
+}
+
+// Nothing is going to watch or rewrite this call: the thread's state is the ordinary one, no autocast, x stands for itself.
+bool plain_call(const Tensor &x) { return !thread_is_watched() && !at::autocast::is_autocast_enabled(at::kCUDA) && kind_of(x) == kPlain; }
 
 // The activations of one call as the kernels take them: [..., K] of a type they know, contiguous and 16-byte aligned, their
 // device current for as long as this lives.
@@ -106,7 +135,8 @@ struct Parameter {
     bool open(PyObject *o, const Tensor &x, at::ScalarType type)
     {
         t = tensor_of(o);
-        if (!t || !t->is_cuda() || t->get_device() != x.get_device() || t->layout() != at::kStrided || !t->is_floating_point()) return false;
+        if (!t || !t->is_cuda() || t->get_device() != x.get_device() || t->layout() != at::kStrided || !t->is_floating_point() || kind_of(*t) == kWatched)
+            return false;
         if (t->scalar_type() == type && t->is_contiguous()) return true;
         at::AutoDispatchBelowADInplaceOrView below;
         held = t->to(type).contiguous();
@@ -125,7 +155,7 @@ struct Bias {
     bool open(PyObject *o, const Tensor &x, int64_t N)
     {
         if (o == Py_None) return true;
-        if (!value.open(o, x, at::kFloat) || value.t->numel() != N) return false;
+        if (!tensor_of(o) || kind_of(*tensor_of(o)) != kPlain || !value.open(o, x, at::kFloat) || value.t->numel() != N) return false;
         p = static_cast<const float *>(value.t->data_ptr());
         return true;
     }
@@ -306,13 +336,15 @@ PyObject *polar_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
     if (!resident(cd, *x, at::kChar) || !nr.open(a[1], *x, at::kHalf) || !ct.open(a[2], *x, at::kFloat) || cd->numel() < N * K ||
         nr.t->numel() < N * K / block || ct.t->numel() < (1 << bits))
         Py_RETURN_NONE;
+    if (kind_of(*tensor_of(a[1])) != kPlain || kind_of(*tensor_of(a[2])) != kPlain) Py_RETURN_NONE;
     // what the kernels read is what the module holds: wider types are rounded for the few rows that always took this route
     if (rows > 32 && (tensor_of(a[1])->element_size() > 2 || tensor_of(a[2])->element_size() > 4)) Py_RETURN_NONE;
     const Ordered ordered(nr.converted || ct.converted);
     // a bias of another type than the result's is added to it, in the type that the two come to
     const Tensor *bias = a[8] == Py_None ? nullptr : tensor_of(a[8]), *after = nullptr;
     if (a[8] != Py_None) {
-        if (!bias || !bias->is_cuda() || bias->get_device() != x->get_device() || bias->numel() != N) Py_RETURN_NONE;
+        if (!bias || !bias->is_cuda() || bias->get_device() != x->get_device() || bias->numel() != N || kind_of(*bias) != kPlain)
+            Py_RETURN_NONE;
         if (!resident(bias, *x, at::kHalf)) std::swap(bias, after);
     }
     auto finish = [&](Tensor &&y) {
@@ -481,6 +513,7 @@ PyObject *decode_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
 }
 
 PyMethodDef methods[] = {
+    {"call_kind", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(call_kind)), METH_FASTCALL, nullptr},
     {"count_symbols", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(count_symbols)), METH_FASTCALL, nullptr},
     {"encode_symbols", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(encode_symbols)), METH_FASTCALL, nullptr},
     {"decode_symbols", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(decode_symbols)), METH_FASTCALL, nullptr},

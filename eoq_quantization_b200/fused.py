@@ -42,6 +42,15 @@ GEMM_MAX_ROWS = 8       # rows up to which the tensor-core kernel would be prefe
 PACKED_TENSOR_ROWS = 32       # activation rows the tensor-core form of the packed GEMV takes per launch
 
 
+def call_kind(*tensors) -> int:
+    """What torch is to make of a call on these tensors besides running it: PLAIN, nothing; GRADIENT; or WATCHED, what only its
+    own operations can do (function transforms, forward-mode tangents, tracing, dispatch modes)."""
+    return _lib.native().call_kind(*tensors)
+
+
+PLAIN, GRADIENT, WATCHED = 0, 1, 2
+
+
 def fused_rows(dtype: torch.dtype) -> int:
     """Activation rows up to which the fused decode + GEMV is the fastest route for this activation type."""
     return GEMV_MAX_ROWS.get(dtype, 0)
@@ -260,7 +269,7 @@ class EOQWeight:
             return y
         require_cuda(x, "EOQWeight.linear")
         rows = x.numel() // max(self.cols, 1)
-        if rows >= 1 and x.dtype in _DTYPES:
+        if rows >= 1 and x.dtype in _DTYPES and (call_kind(x, bias) != WATCHED or self.kind == _lib.KIND_Q5_POLAR):
             if rows <= fused_rows(x.dtype):
                 return self.gemv(x, bias)
             if 8 < rows <= GEMM_MAX_ROWS and x.dtype != torch.float32 and self.kind == _lib.KIND_INT4_ABSMAX and self.cols % 16 == 0:

@@ -19,7 +19,7 @@ import torch.nn.functional as F
 
 from .. import _lib
 from ..core.polar_quant import _ensure_centroids, hadamard_matrix, polar_quantize
-from ..fused import EOQWeight, gemv_polar_codes, polar_codes_gemv_applies, require_cuda
+from ..fused import WATCHED, EOQWeight, call_kind, gemv_polar_codes, polar_codes_gemv_applies, require_cuda
 
 
 class PolarLinear(nn.Module):
@@ -120,7 +120,7 @@ class PolarLinear(nn.Module):
         if self.entropy_coded and self._fusable() and x2.shape[0] <= 8:
             xin = x2 if x2.dtype in (torch.float16, torch.bfloat16, torch.float32) else x2.float()
             out = self.eoq_weight().gemv(xin, out_dtype=torch.float32)
-        elif polar_codes_gemv_applies(self.in_features, self.bits, self.block_size, x2.shape[0]):
+        elif polar_codes_gemv_applies(self.in_features, self.bits, self.block_size, x2.shape[0]) and call_kind(x) != WATCHED:
             # up to 8 rows (32 with blocks of 64 columns and more): one pass over the byte codes this module keeps resident
             # (any bit width and block size the reference builds), activations rotated once per call
             xin = x2 if x2.dtype in (torch.float16, torch.bfloat16, torch.float32) else x2.float()

@@ -136,3 +136,40 @@ def test_scales_converted_for_a_call_are_complete_when_they_are_read():
         got.append(layer(x))
     for i, y in enumerate(got):
         assert torch.equal(y, want[i % 2]), i
+
+
+@pytest.mark.parametrize("kind", ["packed", "fast", "eoq", "polar"])
+def test_gradients_of_the_bias_and_of_the_activations(kind):
+    layer = _layer(kind)
+    dense = _dense(layer).float()
+    x = torch.randn(40, K, device="cuda")
+    layer.bias.requires_grad_()
+    g = torch.randn(40, N, device="cuda")
+    layer(x).backward(g.to(layer(x).dtype))
+    assert O.rel_l2(layer.bias.grad.double().cpu().numpy(), g.sum(0).double().cpu().numpy()) < 1e-3       # an fp16 bias's gradient
+    layer.bias.requires_grad_(False)
+    x.requires_grad_()
+    y = layer(x)
+    y.backward(g.to(y.dtype))
+    assert O.rel_l2(x.grad.cpu().numpy(), (g @ dense).cpu().numpy()) < (1e-3 if kind == "polar" else 1e-5)      # polar: fp16 results' gradient
+
+
+@pytest.mark.parametrize("kind", ["packed", "fast", "eoq", "polar"])
+@pytest.mark.parametrize("rows", [1, 40])
+def test_forward_mode_tangents_are_carried(kind, rows):
+    layer = _layer(kind)
+    dense = _dense(layer).float()
+    x, v = torch.randn(rows, K, device="cuda"), torch.randn(rows, K, device="cuda")
+    with torch.autograd.forward_ad.dual_level():
+        y, t = torch.autograd.forward_ad.unpack_dual(layer(torch.autograd.forward_ad.make_dual(x, v)))
+        assert t is not None and O.rel_l2(t.float().cpu().numpy(), (v @ dense.T).cpu().numpy()) < (1e-3 if kind == "polar" else 1e-5)
+        assert O.rel_l2(y.float().cpu().numpy(), layer(x).float().cpu().numpy()) < (1e-3 if kind == "polar" else 1e-5)
+
+
+@pytest.mark.parametrize("kind", ["packed", "eoq"])
+@pytest.mark.parametrize("rows", [1, 40])
+def test_vmap_runs_over_the_layers(kind, rows):
+    layer = _layer(kind)
+    x = torch.randn(3, rows, K, device="cuda")
+    y = torch.vmap(layer)(x)
+    assert O.rel_l2(y.cpu().numpy(), layer(x).cpu().numpy()) < 1e-5
