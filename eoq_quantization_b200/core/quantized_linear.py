@@ -13,8 +13,8 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _lib
-from ..fused import (GEMM_MAX_ROWS, PLAIN, EOQWeight, PACKED_TENSOR_ROWS, call_kind, dequant_packed, fused_rows, gemv_packed, packed_gemv_rows,
-                     require_cuda)
+from ..fused import (GEMM_MAX_ROWS, GRADIENT, PLAIN, EOQWeight, PACKED_TENSOR_ROWS, autocast_dtype, call_kind, dequant_packed, fused_rows,
+                     gemv_packed, packed_gemv_rows, require_cuda, with_gradient)
 
 
 class QuantizedLinear(nn.Module):
@@ -139,7 +139,14 @@ class QuantizedLinear(nn.Module):
         require_cuda(x, "QuantizedLinear.forward")
         require_cuda(self.packed_weight, "QuantizedLinear.forward")
         rows = x.numel() // max(self.in_features, 1)
-        plain = call_kind(x, bias) == PLAIN
+        dt = autocast_dtype(x)
+        if dt is not None:                      # the few rows of the fused GEMV keep their type, as they always have
+            with torch.autocast("cuda", enabled=False):
+                return self.forward(x if self._fusable() and 1 <= rows <= fused_rows(x.dtype) else x.to(dt))
+        kind = call_kind(x, bias)
+        if kind == GRADIENT:
+            return with_gradient(x, bias, lambda x, _: self.forward(x), lambda d: self._dequantize_weight().to(d), self.packed_weight, self.scales)
+        plain = kind == PLAIN
         if plain and x.dtype in (torch.float16, torch.bfloat16, torch.float32) and \
                 1 <= rows <= PACKED_TENSOR_ROWS == packed_gemv_rows(self.in_features, self.bits, self.block_size, x.dtype):
             return gemv_packed(self.packed_weight, self.scales, self.out_features, self.in_features, self.bits, self.block_size, x, bias)

@@ -11,7 +11,8 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _lib
-from ..fused import GEMM_MAX_ROWS, WATCHED, EOQWeight, call_kind, dequant_packed, fused_rows, gemv_packed, PACKED_TENSOR_ROWS, packed_gemv_rows, require_cuda
+from ..fused import (GEMM_MAX_ROWS, GRADIENT, WATCHED, EOQWeight, PACKED_TENSOR_ROWS, call_kind, dequant_packed, fused_rows, gemv_packed,
+                     packed_gemv_rows, require_cuda, with_gradient)
 
 _SUPPORTED_BITS = (2, 4, 8)
 _MEMORY_THRESHOLD = 16 * 1024 * 1024
@@ -141,7 +142,11 @@ class QuantizedLinearFast(nn.Module):
                 return y
         require_cuda(x, "QuantizedLinearFast.forward")
         rows = x.numel() // max(self.in_features, 1)
-        codes = self.strategy == "auto" and x.dtype in (torch.float16, torch.bfloat16, torch.float32) and call_kind(x, self.bias_param) != WATCHED
+        kind = call_kind(x, self.bias_param)
+        if self.strategy == "auto" and kind == GRADIENT and not torch.is_autocast_enabled("cuda"):
+            return with_gradient(x, self.bias_param, lambda x, _: self.forward(x), lambda d: fast_dequantize(
+                self.packed_weight, self.scales, self.out_features, self.in_features, self.bits, self.block_size).to(d), self.packed_weight, self.scales)
+        codes = self.strategy == "auto" and x.dtype in (torch.float16, torch.bfloat16, torch.float32) and kind != WATCHED
         if codes and \
                 1 <= rows <= PACKED_TENSOR_ROWS == packed_gemv_rows(self.in_features, self.bits, self.block_size, x.dtype):
             # one pass over the packed codes on the tensor cores (HBM-bound), see QuantizedLinear.forward

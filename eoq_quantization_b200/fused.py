@@ -51,6 +51,34 @@ def call_kind(*tensors) -> int:
 PLAIN, GRADIENT, WATCHED = 0, 1, 2
 
 
+class _Product(torch.autograd.Function):
+    """x @ W.T (+ bias) of a weight that stays as it is: forward by the layer's kernels, backward by its dequantised copy."""
+
+    @staticmethod
+    def forward(ctx, x, bias, product, dense, *held):
+        ctx.dense, ctx.bias_dtype = dense, None if bias is None else bias.dtype
+        ctx.save_for_backward(*held)
+        return product(x, bias)
+
+    @staticmethod
+    def backward(ctx, grad):
+        held = ctx.saved_tensors                # an error if what the weight is made of has been written since
+        with torch.autocast("cuda", enabled=False):
+            grad_x = grad @ ctx.dense(grad.dtype) if ctx.needs_input_grad[0] else None
+            grad_bias = grad.reshape(-1, grad.shape[-1]).sum(0).to(ctx.bias_dtype) if ctx.needs_input_grad[1] else None
+        return (grad_x, grad_bias, None, None) + (None,) * len(held)
+
+
+def with_gradient(x: torch.Tensor, bias: Optional[torch.Tensor], product, dense, *held: torch.Tensor) -> torch.Tensor:
+    """`product(x, bias)` with gradients for x and bias; `dense(dtype)` gives the weight, which is made of the tensors `held`."""
+    return _Product.apply(x, bias, product, dense, *held)
+
+
+def autocast_dtype(x: torch.Tensor) -> Optional[torch.dtype]:
+    """The type autocast wants this matrix product in, or None where it has no say."""
+    return torch.get_autocast_dtype("cuda") if x.is_cuda and x.dtype in _DTYPES and torch.is_autocast_enabled("cuda") else None
+
+
 def fused_rows(dtype: torch.dtype) -> int:
     """Activation rows up to which the fused decode + GEMV is the fastest route for this activation type."""
     return GEMV_MAX_ROWS.get(dtype, 0)
@@ -269,7 +297,14 @@ class EOQWeight:
             return y
         require_cuda(x, "EOQWeight.linear")
         rows = x.numel() // max(self.cols, 1)
-        if rows >= 1 and x.dtype in _DTYPES and (call_kind(x, bias) != WATCHED or self.kind == _lib.KIND_Q5_POLAR):
+        dt = autocast_dtype(x)
+        if dt is not None:                      # the few rows of the fused GEMV keep their type, as they always have
+            with torch.autocast("cuda", enabled=False):
+                return self.linear(x if 1 <= rows <= fused_rows(x.dtype) else x.to(dt), bias)
+        kind = call_kind(x, bias)
+        if kind == GRADIENT and self.kind != _lib.KIND_Q5_POLAR:
+            return with_gradient(x, bias, self.linear, lambda d: self.dequantize(d if d in _DTYPES else torch.float32).to(d))
+        if rows >= 1 and x.dtype in _DTYPES and (kind != WATCHED or self.kind == _lib.KIND_Q5_POLAR):
             if rows <= fused_rows(x.dtype):
                 return self.gemv(x, bias)
             if 8 < rows <= GEMM_MAX_ROWS and x.dtype != torch.float32 and self.kind == _lib.KIND_INT4_ABSMAX and self.cols % 16 == 0:

@@ -19,7 +19,7 @@ import torch.nn.functional as F
 
 from .. import _lib
 from ..core.polar_quant import _ensure_centroids, hadamard_matrix, polar_quantize
-from ..fused import WATCHED, EOQWeight, call_kind, gemv_polar_codes, polar_codes_gemv_applies, require_cuda
+from ..fused import WATCHED, EOQWeight, autocast_dtype, call_kind, gemv_polar_codes, polar_codes_gemv_applies, require_cuda
 
 
 class PolarLinear(nn.Module):
@@ -114,6 +114,9 @@ class PolarLinear(nn.Module):
                 return y
         require_cuda(x, "PolarLinear.forward")
         require_cuda(self.codes, "PolarLinear.forward")
+        if autocast_dtype(x) is not None:       # fp16 results of fp32 sums whatever autocast says
+            with torch.autocast("cuda", enabled=False):
+                return self.forward(x)
         x2 = x.reshape(-1, self.in_features)
         if self.awq_scales is not None:                       # W / s applied to x instead: (x / s) W^T
             x2 = x2.float() / self.awq_scales.float().unsqueeze(0)

@@ -173,3 +173,43 @@ def test_vmap_runs_over_the_layers(kind, rows):
     x = torch.randn(3, rows, K, device="cuda")
     y = torch.vmap(layer)(x)
     assert O.rel_l2(y.cpu().numpy(), layer(x).cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("kind", ["packed", "eoq", "polar"])
+def test_calls_under_autocast_take_the_codes_route(kind):
+    """Results of the autocast type, as torch.nn.Linear gives them, but for the few rows of the fused GEMV (and PolarLinear's fp16)."""
+    layer = _layer(kind)
+    dense, plain = _dense(layer), _plain(layer)
+    for rows, dt in plain:
+        for to in (torch.float16, torch.bfloat16):
+            few = rows <= (8 if dt == torch.float32 else 4)
+            result = torch.float16 if kind == "polar" else dt if few else to
+            with torch.autocast("cuda", dtype=to):
+                y, taken = _taken(layer, x := torch.randn(rows, K, device="cuda").to(dt))
+            assert y.dtype == result and getattr(layer, "_eoq", None) is None
+            want = x.double() @ dense.T + layer.bias.double()
+            tol = max(TOL[y.dtype], 0 if few or kind == "polar" else 2 * TOL[to])             # x is rounded to the autocast type, too
+            assert O.rel_l2(y.double().cpu().numpy(), want.cpu().numpy()) < tol, (rows, dt, to)
+            like = plain[rows, dt if few or kind == "polar" else to]
+            assert taken <= like + x.numel() * 4 + (2 << 20), (taken, like, rows, dt, to)
+
+
+@pytest.mark.parametrize("kind", ["packed", "fast", "eoq"])
+@pytest.mark.parametrize("rows", [1, 3, 24])
+def test_calls_that_want_gradients_take_the_codes_route(kind, rows):
+    layer = _layer(kind)
+    dense, plain = _dense(layer), _plain(layer)
+    for dt in TOL:
+        x = torch.randn(rows, K, device="cuda").to(dt).requires_grad_()
+        y, taken = _taken(layer, x)
+        like = _taken(layer, x.detach())[1]
+        assert y.dtype == dt and taken <= like + (2 << 20) and like < N * K and getattr(layer, "_eoq", None) is None
+        g = torch.randn(rows, N, device="cuda").to(dt)
+        y.backward(g)
+        assert x.grad.dtype == dt
+        assert O.rel_l2(x.grad.double().cpu().numpy(), (g.double() @ dense).cpu().numpy()) < TOL[dt], dt
+    if kind == "packed":
+        y = layer(x)
+        layer.scales.mul_(2)
+        with pytest.raises(RuntimeError):                     # the weight that y was made with is gone
+            y.backward(g)
