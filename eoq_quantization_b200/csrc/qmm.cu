@@ -56,6 +56,20 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity)
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
+struct QmmArgs {
+    const uint16_t *scales;      // [N][K / group] fp16 (polar: norms)
+    const float *centroids;      // polar: `entries` of them
+    const void *bias;            // [N] fp32 (bias_half: fp16), or null
+    const float *tok_scale;      // [M] factor of every activation row, or null
+    void *y;                     // [M][N]
+    uint32_t N, K, M, T, group, sgroups, seg, units, split, planes, entries;
+    uint32_t nw, ns, a_base;     // stages of packed weights and of operands (A in TMEM, activations in shared memory); first A column
+    uint32_t at_x, at_bar;       // shared-memory offsets
+    int y_dtype, bias_half, late;   // late: the packed codes are the previous kernel's to write
+    long long limit;             // clock ticks a wait may take
+    uint32_t *status;            // word to set when one runs out, or null: g_qmm_status
+};
+
 // Waits are bounded.  One that runs out marks the CTA, which ends the waits of all its warps, and sets the status word; the
 // warps run on with whatever is there, only that nobody requests copies any more, nor tells the barriers that count a copy's
 // bytes (an arrival beyond their count while a copy is under way would break them).  The CTA's results become NaN.  Nothing
@@ -65,11 +79,13 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity)
 // count.  (A limit of 0 has no patience with them either.)
 //   The outcome of a wait is not returned for every warp to leave its loop by: that alone costs the products' warp some
 // eighty cycles a block (24 rows against 11008 x 4096: 17.9 instead of 17.0 us).  What follows a first failed attempt is a
-// function of its own, out of the loops' way: 15.9 us (inline 17.0); four rows against a polar 14336 x 4096 34.8 (37.4).
+// function of its own, out of the loops' way: 16.2 us (inline 17.0); four rows against a polar 14336 x 4096 36.0 (37.5).  Not so
+// in loops that keep more in registers than a call leaves alone (`near`: the readers, and the polar producers of the variants
+// with 20 warps), which cost up to 40 % by the call (100 rows in groups of 32: 88.5 us, now 56.9).
 struct Waits {
     uint32_t mark;               // shared address of two words: the CTA has given up; the kernels before this one have ended
-    long long limit;             // clock ticks
-    uint32_t *status;
+    const QmmArgs &a;            // (read where it is needed: the readers have no registers to spare)
+    __device__ __forceinline__ uint32_t *status() const { return a.status ? a.status : &g_qmm_status; }
     __device__ __forceinline__ bool stopped() const
     {
         uint32_t v;
@@ -78,19 +94,30 @@ struct Waits {
     }
     __device__ __forceinline__ void operator()(uint32_t bar, uint32_t parity) const
     {
-        if (!bar_try(bar, parity)) slow(bar, parity, mark, limit, status);
+        if (!bar_try(bar, parity)) slow(bar, parity, mark, a.limit, status());
     }
     // The same, and whether the CTA has not given up: asked for together, in one latency.
+    template <bool NEAR = false>
     __device__ __forceinline__ bool go(uint32_t bar, uint32_t parity) const
     {
         uint32_t ok, stop;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%2], %3;\n\tld.volatile.shared.u32 %1, [%4];\n\t"
                      "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok), "=r"(stop) : "r"(bar), "r"(parity), "r"(mark) : "memory");
         if (ok) return stop == 0;
-        slow(bar, parity, mark, limit, status);
+        if (NEAR) poll(bar, parity, mark, a.limit, status());
+        else slow(bar, parity, mark, a.limit, status());
         return !stopped();
     }
+    // The same with what follows a failed attempt in its place.
+    __device__ __forceinline__ void near(uint32_t bar, uint32_t parity) const
+    {
+        if (!bar_try(bar, parity)) poll(bar, parity, mark, a.limit, status());
+    }
     static __device__ __noinline__ void slow(uint32_t bar, uint32_t parity, uint32_t mark, long long limit, uint32_t *status)
+    {
+        poll(bar, parity, mark, limit, status);
+    }
+    static __device__ __forceinline__ void poll(uint32_t bar, uint32_t parity, uint32_t mark, long long limit, uint32_t *status)
     {
         long long t0 = clock64();
         while (!bar_try(bar, parity)) {
@@ -262,20 +289,6 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16])
                    "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]) :: "memory");
 }
 
-struct QmmArgs {
-    const uint16_t *scales;      // [N][K / group] fp16 (polar: norms)
-    const float *centroids;      // polar: `entries` of them
-    const void *bias;            // [N] fp32 (bias_half: fp16), or null
-    const float *tok_scale;      // [M] factor of every activation row, or null
-    void *y;                     // [M][N]
-    uint32_t N, K, M, T, group, sgroups, seg, units, split, planes, entries;
-    uint32_t nw, ns, a_base;     // stages of packed weights and of operands (A in TMEM, activations in shared memory); first A column
-    uint32_t at_x, at_bar;       // shared-memory offsets
-    int y_dtype, bias_half, late;   // late: the packed codes are the previous kernel's to write
-    long long limit;             // clock ticks a wait may take
-    uint32_t *status;            // word to set when one runs out, or null: g_qmm_status
-};
-
 template <int BITS, int KB>
 struct Unit {                    // what one weight copy brings: 128 rows of kBytes, in blocks of KB columns (a stage of operands)
     static constexpr uint32_t kBytes = BITS == 2 ? 64u : 128u;
@@ -296,6 +309,7 @@ enum { kWFull = 0, kWEmpty = 8, kFull = 16, kEmpty = 24, kDFull = 32, kDEmpty = 
 constexpr uint32_t kScaleRing = 4, kScaleGroups = 8, kScaleEntry = kScaleGroups * kRows * 2u;      // scales of 8 groups x 128 rows an entry
 
 // The scales of one weight row in the order of the groups, out of the ring that a warp of the CTA keeps filled.
+template <bool NEAR>
 struct ScaleReader {
     uint32_t full, empty, at, row, entry = 0;      // barrier addresses, ring address
     Ring ring;
@@ -311,7 +325,11 @@ struct ScaleReader {
             entry++;
             here = false;
         }
-        if (!here) { wait(full + 8u * ring.at, ring.lap); here = true; }
+        if (!here) {
+            if (NEAR) wait.near(full + 8u * ring.at, ring.lap);
+            else wait(full + 8u * ring.at, ring.lap);
+            here = true;
+        }
         uint16_t v;
         asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(at + ring.at * kScaleEntry + (g & 7u) * (kRows * 2u) + row * 2u));
         return v;
@@ -333,7 +351,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(raw) + 1023u) & ~(uintptr_t)1023u);
     const uint32_t base = saddr(smem), bars = base + a.at_bar;
     auto bar = [&](uint32_t i) { return bars + 8u * i; };
-    const Waits wait{bars + 8u * kMark, a.limit, a.status ? a.status : &g_qmm_status};
+    const Waits wait{bars + 8u * kMark, a};
     auto word = [&](uint32_t i) { return reinterpret_cast<volatile uint32_t *>(smem + a.at_bar + 8u * i); };
     const uint32_t scale_ring = bars + 512u;
     uint32_t *table = reinterpret_cast<uint32_t *>(smem + a.at_bar + 512 + kScaleRing * kScaleEntry);      // polar: centroids, as {high half, low half} (fold) or fp32
@@ -411,7 +429,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
         uint32_t four;
         asm volatile("mov.b32 %0, 4;" : "=r"(four));
         // scaled: the groups of 32-column parts, counted along
-        ScaleReader sr(wait, bar(kSFull), bar(kSEmpty), scale_ring, r);
+        ScaleReader<false> sr(wait, bar(kSFull), bar(kSEmpty), scale_ring, r);
         uint32_t gi = 0, pos = 0;
         if (!FOLD) {
             const uint32_t c = (kb0 + set) * KB;
@@ -491,7 +509,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
                     for (int c = 0; c < U::kWords; c++) codes_scaled<kCode, BF16>(w[c], h + c * (32 / U::kWords), c < U::kWords / 2 ? s0 : s1);
                 }
                 if (part == 0) {
-                    go = wait.go(bar(kEmpty + st), ar.lap ^ 1u);
+                    go = wait.template go<(kPol && NF > 1)>(bar(kEmpty + st), ar.lap ^ 1u);
                     fence_after();
                 }
                 __syncwarp();
@@ -513,7 +531,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
         const uint32_t lane_base = tmem + (((warp & 3u) * 32u) << 16) + set * cols;
         float *stage = reinterpret_cast<float *>(smem) + (size_t)set * cols * kRows + r;
         if (FOLD) {
-            ScaleReader sr(wait, bar(kSFull), bar(kSEmpty), scale_ring, r);
+            ScaleReader<true> sr(wait, bar(kSFull), bar(kSEmpty), scale_ring, r);
             float tot[TC];
 #pragma unroll
             for (int c = 0; c < TC; c++) tot[c] = 0.0f;
@@ -521,9 +539,27 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
             for (uint32_t s = 0; s < nseg; s++) {
                 const float sc = __half2float(__ushort_as_half(sr.get(g, lane)));
                 if (++in_group == g16 / f16) { in_group = 0; g++; }
-                wait(bar(kDFull + (s & 1u)), (s >> 1) & 1u);
+                wait.near(bar(kDFull + (s & 1u)), (s >> 1) & 1u);
                 __syncwarp();
                 fence_after();
+                // 64 totals a lane and 96 registers: sixteen columns at a time.  With 32 under way the variant spilled in this loop,
+                // or did not, as the compiler happened to choose (100 rows in groups of 32: 64.2 to 75 us, now 56.9).
+                if constexpr (TC == 64) {
+#pragma unroll
+                    for (int c = 0; c < TC; c += 16) {
+                        if ((uint32_t)c >= cols) break;
+                        uint32_t v[16];
+                        tmem_ld16(lane_base + (s & 1u) * a.T + c, v);
+                        tmem_ld_wait(v);
+                        if (c + 16u >= cols) {
+                            fence_before();
+                            __syncwarp();
+                            if (lane == 0) bar_arrive(bar(kDEmpty + (s & 1u)));
+                        }
+#pragma unroll
+                        for (int j = 0; j < 16; j++) tot[c + j] = fmaf(sc, __uint_as_float(v[j]), tot[c + j]);
+                    }
+                } else {
 #pragma unroll
                 for (int c = 0; c < TC; c += 32) {
                     if ((uint32_t)c >= cols) break;
@@ -543,6 +579,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
 #pragma unroll
                         for (int j = 0; j < 16; j++) tot[c + 16 + j] = fmaf(sc, __uint_as_float(v[1][j]), tot[c + 16 + j]);
                     }
+                }
                 }
             }
 #pragma unroll
