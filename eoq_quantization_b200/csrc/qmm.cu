@@ -802,12 +802,13 @@ __global__ void __launch_bounds__(512) split_rows_kernel(const void *__restrict_
         const uint16_t b = __ldg(reinterpret_cast<const uint16_t *>(x) + i);
         return x_dtype == EOQ_B200_F16 ? __half2float(__ushort_as_half(b)) : __uint_as_float((uint32_t)b << 16);
     };
+    auto finite = [](float v) { return fabsf(v) < __int_as_float(0x7f800000) ? fabsf(v) : 0.0f; };
     float most = 0.0f;
     if (V == 0) {
         for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) {
             const float v = load(k);
             row[k] = v;
-            most = fmaxf(most, fabsf(v));
+            most = fmaxf(most, finite(v));
         }
     } else {
         constexpr int kV = V ? V : 1;
@@ -831,7 +832,7 @@ __global__ void __launch_bounds__(512) split_rows_kernel(const void *__restrict_
             for (int j = 0; j < kV; j++) {
                 v[j] *= 1.0f / (32.0f * kV);
                 row[b + 32u * j + lane] = v[j];
-                most = fmaxf(most, fabsf(v[j]));
+                most = fmaxf(most, finite(v[j]));
             }
         }
     }
@@ -841,15 +842,16 @@ __global__ void __launch_bounds__(512) split_rows_kernel(const void *__restrict_
     __syncthreads();
     most = 0.0f;
     for (uint32_t w = 0; w < nwarps; w++) most = fmaxf(most, part[w]);
-    // 2^e with 2^14 <= most 2^e < 2^15, e within what a float holds; zero rows and rows with infinities stay as they are
+    // 2^e with 2^14 <= most 2^e < 2^15, e within what a float holds, for the largest finite value; rows without one stay as they are
     int e = 0;
-    if (most > 0.0f && most < __int_as_float(0x7f800000)) e = min(120, 141 - (int)(__float_as_uint(most) >> 23));
+    if (most > 0.0f) e = min(120, 141 - (int)(__float_as_uint(most) >> 23));
     const float up = __uint_as_float((uint32_t)(127 + e) << 23);
     if (threadIdx.x == 0) tok_scale[m] = __uint_as_float((uint32_t)(127 - e) << 23);
     for (uint32_t k = threadIdx.x * 2u; k < K; k += blockDim.x * 2u) {
         const float a = row[k] * up, b = row[k + 1] * up;
         const __half ha = __float2half_rn(a), hb = __float2half_rn(b);
-        const __half la = __float2half_rn(a - __half2float(ha)), lb = __float2half_rn(b - __half2float(hb));
+        // an infinity has no remainder (and infinity less itself would make the row's results NaN)
+        const __half la = __hisinf(ha) ? __half(0) : __float2half_rn(a - __half2float(ha)), lb = __hisinf(hb) ? __half(0) : __float2half_rn(b - __half2float(hb));
         *reinterpret_cast<__half2 *>(planes + (size_t)m * K + k) = __halves2half2(ha, hb);
         *reinterpret_cast<__half2 *>(planes + (size_t)(M + m) * K + k) = __halves2half2(la, lb);
     }

@@ -175,3 +175,22 @@ def test_errors_of_the_library_are_raised():
         with pytest.raises(L.EOQError) as e:
             native.weight_linear(0, x.get_device(), 96, 256, 4, 8, x.expand(rows, 256).contiguous(), None)
         assert e.value.code == L.EOQ_ERR_NULL_PTR
+
+
+@pytest.mark.parametrize("bits,group", [(4, 128), (8, 32)])
+def test_fp32_rows_with_infinities(bits, group):
+    """A row with infinities among its values: infinite or NaN exactly where the dequantised product is, and the other rows untouched."""
+    torch.manual_seed(bits)
+    ql = QuantizedLinear.from_float(torch.nn.Linear(512, 200), bits=bits, block_size=group).cuda()
+    w = ql._dequantize_weight().double()
+    for m in (1, 12, 40, 200):
+        x = torch.randn(m, 512, device="cuda") * 1e5
+        x[0, 7] = float("inf")
+        if m > 2:
+            x[2, 100], x[2, 101] = float("inf"), float("-inf")
+        y, want = ql(x), x.double() @ w.T + ql.bias_param.double()
+        assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isinf(y), torch.isinf(want))
+        assert torch.equal(y[torch.isinf(y)].sign(), want[torch.isinf(want)].sign().float())
+        finite = [i for i in range(m) if i not in (0, 2)]
+        if finite:
+            assert O.rel_l2(y[finite].cpu().numpy(), want[finite].cpu().numpy()) < 1e-5
