@@ -957,8 +957,8 @@ def measure_llama_step(world, rank, steps, gather, with_fp16):
 
 def measure_prefill_tp(world, rank, steps):
     """Llama-70B-shape gate/up projection (28672 x 8192, INT4 g128 rANS-coded, N(0, 0.015)) row-sharded over the ranks:
-    per M, EOQWeight.linear on this rank's rows (the fused decode + tensor-core GEMM up to 128 rows of activations, decode
-    to bf16 + library GEMM beyond) followed by the all-gather of the output slices (NCCL); device time, max over ranks.  Every rank's shard is drawn from the same distribution (its own seed)."""
+    per M, EOQWeight.linear on this rank's rows (the codes decoded for the tcgen05 product, or decode to bf16 + library GEMM
+    where that is quicker) followed by the all-gather of the output slices (NCCL); device time, max over ranks.  Every rank's shard is drawn from the same distribution (its own seed)."""
     import torch
     import torch.distributed as dist
     from eoq_quantization_b200 import _lib
@@ -976,14 +976,13 @@ def measure_prefill_tp(world, rank, steps):
         sym = (np.clip(np.round(w.reshape(-1, GROUP) / sc[:, None]), -7, 7) + 7).astype(np.uint8).reshape(w.shape)
         ws.append(EOQWeight.from_symbols(sym, sc.astype(np.float16)))
         del w, sym
-    from eoq_quantization_b200.fused import GEMM_MAX_ROWS
     for m in (16, 64, 128, 256, 2048):
         x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
         full = torch.empty(world, m, n, device="cuda", dtype=torch.bfloat16) if world > 1 else None
 
         def run():
-            # EOQWeight.linear is the call a module makes: fused decode + tensor-core MMA up to GEMM_MAX_ROWS rows,
-            # one fused decode + dequantise to 16 bits and a library GEMM beyond
+            # EOQWeight.linear is the call a module makes: the codes decoded for the tcgen05 product kernel, or, where
+            # that takes longer, one fused decode + dequantise to 16 bits and a library GEMM
             ys = [wi.linear(x) for wi in ws]
             if world > 1:
                 local = ys[0] if len(ys) == 1 else torch.cat(ys, dim=1)
@@ -1032,8 +1031,9 @@ def measure_prefill_tp(world, rank, steps):
             t = torch.tensor([us], device="cuda")
             dist.all_reduce(t, op=dist.ReduceOp.MAX)
             us = float(t.item())
+        product = _lib.lib().eoq_b200_weight_linear_preferred(ws[0]._h, x.data_ptr(), _lib.BF16, m)
         res[f"M{m}"] = {"us": us, "tflops": 2.0 * m * n_total * k / us / 1e6,
-                        "path": "fused decode + tcgen05 MMA" if m <= GEMM_MAX_ROWS else "fused decode to bf16, then library GEMM",
+                        "path": "fused decode to codes, then tcgen05 product" if product else "fused decode to bf16, then library GEMM",
                         "launch": launch}
     return {"workload": "llama70b_gate_up_28672x8192_int4_g128_rans, bf16 x", "parallelism": f"row-sharded tp{world}" +
             (" + nccl all-gather of [M, rows / ranks] slices" if world > 1 else ""), "rows_per_rank": n, "per_m": res}

@@ -186,6 +186,8 @@ def lib() -> C.CDLL:
         "eoq_b200_weight_status": (C.c_int, [vp, vp]),
         "eoq_b200_tune": (C.c_int, [C.c_char_p, C.c_int]),
         "eoq_b200_ordered_launches": (C.c_int, [C.c_int]),
+        "eoq_b200_linear_packed_preferred": (C.c_int, [vp, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, vp, C.c_int, C.c_uint32]),
+        "eoq_b200_weight_linear_preferred": (C.c_int, [vp, vp, C.c_int, C.c_uint32]),
         "eoq_b200_launch_count": (C.c_uint64, []),
         "eoq_b200_weight_read": (C.c_uint64, [vp, C.c_int, vp, C.c_uint64]),
     }

@@ -27,8 +27,7 @@ class EOQLinear(nn.Module):
 
     Same call contract as ``QuantizedLinear.forward`` (core/quantized_linear.py:222-228): ``x`` of shape
     ``(..., in_features)`` in any of fp16 / bf16 / fp32, result ``(..., out_features)`` in ``x.dtype``, fp32 accumulation.
-    Up to 8 rows run the fused decode + GEMV kernel, more rows of 16-bit activations the fused decode + tensor-core
-    kernel, fp32 activations beyond 8 rows one dequantisation and a library GEMM.
+    :meth:`EOQWeight.linear` has the routes.
     """
 
     def __init__(self, weight: EOQWeight, bias: Optional[torch.Tensor] = None, bits: int = 4, block_size: int = 128):

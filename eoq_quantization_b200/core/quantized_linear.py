@@ -13,7 +13,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _lib
-from ..fused import (GEMM_MAX_ROWS, GRADIENT, PLAIN, EOQWeight, PACKED_TENSOR_ROWS, autocast_dtype, call_kind, dequant_packed, fused_rows,
+from ..fused import (GRADIENT, PLAIN, EOQWeight, PACKED_TENSOR_ROWS, autocast_dtype, call_kind, dequant_packed, fused_rows,
                      gemv_packed, packed_gemv_rows, require_cuda, with_gradient)
 
 
@@ -151,13 +151,10 @@ class QuantizedLinear(nn.Module):
                 1 <= rows <= PACKED_TENSOR_ROWS == packed_gemv_rows(self.in_features, self.bits, self.block_size, x.dtype):
             return gemv_packed(self.packed_weight, self.scales, self.out_features, self.in_features, self.bits, self.block_size, x, bias)
         if plain and self._fusable() and rows >= 1 and x.dtype in (torch.float16, torch.bfloat16, torch.float32):
-            # up to fused_rows (4 rows of 16-bit activations, 8 of fp32): fused decode + GEMV, fp32 accumulate; beyond
-            # that one dequantisation amortises over enough rows for a library GEMM to win (the fused tensor-core
-            # kernel would take 9..GEMM_MAX_ROWS rows of 16-bit activations if that constant were raised)
+            # groups that the kernels from packed codes do not take: up to fused_rows (4 rows of 16-bit activations, 8 of
+            # fp32) the fused decode + GEMV on an entropy-coded copy; beyond, one dequantisation and a library GEMM
             if rows <= fused_rows(x.dtype):
                 return self.eoq_weight().linear(x, bias)
-            if 8 < rows <= GEMM_MAX_ROWS and x.dtype != torch.float32 and self.bits == 4:          # the tensor-core kernel is built for the 4-bit layout
-                return self.eoq_weight().gemm(x, self.bias_param)
         weight = dequant_packed(self.packed_weight, self.scales, self.out_features, self.in_features, self.bits,
                                 self.block_size, dtype=x.dtype if x.dtype in (torch.float16, torch.bfloat16) else torch.float32)
         bias = self.bias_param.to(x.dtype) if self.bias_param is not None else None

@@ -1,7 +1,7 @@
 """Interface of the reference's ``core/quantized_matmul.py``: matmul against a packed
 quantised weight without the caller materialising it.  Dequantisation is the library's
-kernel; the dense product is a library GEMM; ``QuantizedLinearFast`` additionally keeps
-an entropy-coded resident copy and uses the fused decode+GEMV kernel for up to 8 rows."""
+kernel; the dense product is a library GEMM; ``QuantizedLinearFast`` with the strategy
+"auto" runs the kernels of ``QuantizedLinear``, straight from the packed codes."""
 from __future__ import annotations
 
 from typing import Optional
@@ -11,7 +11,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _lib
-from ..fused import (GEMM_MAX_ROWS, GRADIENT, WATCHED, EOQWeight, PACKED_TENSOR_ROWS, call_kind, dequant_packed, fused_rows, gemv_packed,
+from ..fused import (GRADIENT, WATCHED, EOQWeight, PACKED_TENSOR_ROWS, call_kind, dequant_packed, fused_rows, gemv_packed,
                      packed_gemv_rows, require_cuda, with_gradient)
 
 _SUPPORTED_BITS = (2, 4, 8)
@@ -153,13 +153,9 @@ class QuantizedLinearFast(nn.Module):
             return gemv_packed(self.packed_weight, self.scales, self.out_features, self.in_features, self.bits, self.block_size,
                                x, self.bias_param)
         if codes and self._fusable() and rows >= 1:
-            # up to fused_rows (4 rows of 16-bit activations, 8 of fp32): fused decode + GEMV, fp32 accumulate; beyond
-            # that one dequantisation amortises over enough rows for a library GEMM to win (the fused tensor-core
-            # kernel would take 9..GEMM_MAX_ROWS rows of 16-bit activations if that constant were raised)
+            # see QuantizedLinear.forward
             if rows <= fused_rows(x.dtype):
                 return self.eoq_weight().gemv(x, self.bias_param)
-            if 8 < rows <= GEMM_MAX_ROWS and x.dtype != torch.float32:
-                return self.eoq_weight().gemm(x, self.bias_param)
         out = quantized_matmul(x, self.packed_weight, self.scales, self.out_features, self.in_features, bits=self.bits,
                                block_size=self.block_size, strategy=self.strategy, chunk_rows=self.chunk_rows)
         if self.bias_param is not None:

@@ -3310,8 +3310,12 @@ void set_packed_warps(int v) { g_packed_warps.store(v >= 1 && v <= 16 ? v : 0); 
 // fraction of the machine.  So: the most warps, i.e. the fewest CTAs to an SM, with which the whole grid is resident (given
 // the registers the compiler gave this instantiation).  Where none is, 8 warps: rounds of eight short tiles on every SM
 // take longer than four at a time in two (14336 x 4096: 14.7 us with 4 warps, 12.0 with 8; 28672 x 4096: 25.6 with 16,
-// 21.0 with 8).  Byte codes at 7168 to 9216 x 4096: 11.3 to 12.9 us with 8 warps, 8.6 to 9.1 with 6 (and
-// 10240 x 4096 13.0 with 8, 17.2 with 5, 12.5 with 4).
+// 21.0 with 8).  Byte codes at 7168 to 9216 x 4096: 8.7 to 9.6 us with 8 warps, 7.1 to 7.3 with 6.  The smallest count but one of
+// the byte codes (5) and the smallest of the others (4) keep the grid resident with too few warps to an SM, unless rows are
+// short: byte codes with 5 / 8, 10240 x 4096 13.3 / 9.8 us, 11008 x 4096 13.4 / 9.7, 13824 x 5120 15.9 / 12.9; four bits with
+// 4 / 8, 12288 x 4096 12.4 / 9.7, 13824 x 5120 15.0 / 11.6, 10240 x 8192 23.3 / 17.7.  Over sixty shapes (1024 x 1024 to
+// 28672 x 4096, two, four and eight bits) the rule costs 1.9 % on the mean against the best count, 17 % at worst (byte codes,
+// 10240 x 8192: 4 warps 22.7 us, 8 19.3).
 template <typename Kern, typename Args>
 static cudaError_t launch_packed_mma(Kern kern, uint32_t max_warps, uint32_t tiles, uint32_t nspans, cudaStream_t st, const Args &a)
 {

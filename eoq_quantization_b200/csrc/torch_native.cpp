@@ -43,8 +43,11 @@ namespace {
 
 using at::Tensor;
 
-// A single row against a large PolarLinear is the CUDA-core kernel's: 14336 x 4096 34.0 against 37.5 us; 4096 x 4096 16.1
-// against 13.9, two rows of the former 79 against 37.7.
+// A single row against a large PolarLinear is the CUDA-core kernel's.  GEMV / product in us, blocks of 64 and of 128 columns:
+// 1024 x 4096 11.5 / 8.9, 11.2 / 8.6; 4096 x 4096 13.0 / 12.9, 13.0 / 12.0; 3072 x 8192 21.1 / 18.4, 20.9 / 17.5; 5120 x 5120
+// 18.5 / 17.9, 18.6 / 17.3; 11008 x 4096 23.4 / 31.3, 23.6 / 28.8; 4096 x 11008 27.1 / 27.8, 26.9 / 26.5; 14336 x 4096
+// 30.3 / 34.1, 30.3 / 30.1; 8192 x 8192 34.4 / 36.4, 34.3 / 32.9; 28672 x 8192 100.9 / 139.8, 101.2 / 128.4.  The line costs
+// four per cent at worst (8192 x 8192 in blocks of 128).  Two rows take the GEMV twice as long.
 constexpr int64_t kPolarSingleRowWeights = 32 << 20;
 
 // Two, and three or four, rows against an entropy-coded weight: the fused GEMV above these many weights, below them the
@@ -320,7 +323,8 @@ PyObject *packed_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
 }
 
 // polar_linear(codes, norms, centroids, N, K, bits, block, x, bias): PolarLinear.forward, fp16 results, from the byte codes.
-// One row on the CUDA cores; more, and blocks of 64, 128 or 256 columns, by the tcgen05 kernel.
+// By the tcgen05 kernel where blocks have 64, 128 or 256 columns, but for a single row against a large weight: that, and few
+// rows of other blocks, by the GEMV on the CUDA cores.
 PyObject *polar_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     if (n != 9) { PyErr_SetString(PyExc_TypeError, "polar_linear takes 9 arguments"); return nullptr; }

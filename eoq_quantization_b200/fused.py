@@ -30,15 +30,14 @@ def require_cuda(t: torch.Tensor, what: str) -> None:
                            "(there is no CPU path)")
 
 
-# Rows up to which `linear` and the reference-API modules use the fused decode + GEMV: four rows of 16-bit activations
-# (one launch), eight of fp32 activations.  Beyond, the weight is decoded once to a dense matrix (1.0 T symbols/s; a
-# 16-bit matrix stays in the 126 MB L2) for a library GEMM.  Measured, graph replay, fp16: 11008 x 4096 at 4 / 5 / 8 rows
-# 33.9 / 51.8 / 63.8 us fused (a second launch from the fifth row on) against 47.4 / 47.5 / 47.7 us decode + GEMM;
-# 4096 x 4096: 28.7 / 42.8 / 52.8 against 26.8; at 16 rows and more the fused decode + tensor-core kernel
-# (`EOQWeight.gemm`, still there to be called) loses as well, 39 against 34 us at 16 rows and 92 against 37 us at 256
-# rows on 3584 x 8192: it decodes one tile per warp through a word ring, at half the rate of the two-tiles-per-warp decoders.
+# Rows up to which the fused decode + GEMV serves a call whatever the weight's layout: four of 16-bit activations (one launch),
+# eight of fp32.  Weights that the product kernel takes leave it sooner where they are small, and go to that kernel or to one
+# decode and a library GEMM beyond (csrc/torch_native.cpp, weight_linear, has the measurements).  The fused decode + tensor-core
+# kernel (`EOQWeight.gemm`) is there to be called and loses at every number of rows: 39 against 34 us at 16 rows and 92 against
+# 37 us at 256 rows on 3584 x 8192 (decode + GEMM), since it decodes one tile per warp through a word ring, at half the rate of
+# the two-tiles-per-warp decoders.
 GEMV_MAX_ROWS = {torch.float16: 4, torch.bfloat16: 4, torch.float32: 8}
-GEMM_MAX_ROWS = 8       # rows up to which the tensor-core kernel would be preferred to decode + library GEMM: none above the GEMV's
+GEMM_MAX_ROWS = 8             # rows one call of the fused GEMV takes at most
 PACKED_TENSOR_ROWS = 32       # activation rows the tensor-core form of the packed GEMV takes per launch
 
 
@@ -288,10 +287,9 @@ class EOQWeight:
         return y.reshape(*x.shape[:-1], self.rows)
 
     def linear(self, x: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """y = x @ W.T (+ bias) in x.dtype by the fastest route built for the number of rows: up to `fused_rows` the
-        fused decode + GEMV; beyond, the weight is decoded to a dense matrix once (fused decode + dequantise kernel)
-        for a library GEMM.  (Were GEMM_MAX_ROWS raised above 8, 16-bit activations on 4-bit weights would take the
-        fused decode + tensor-core kernel, `gemm`, up to that many rows.)"""
+        """y = x @ W.T (+ bias) in x.dtype by the fastest route for the number of rows: one row, and a few against large
+        weights, by the fused decode + GEMV; more by decoding the codes for the tcgen05 product kernel, or, where that takes
+        longer (long 16-bit prompts) or does not take the layout, to a dense matrix for a library GEMM."""
         y = self._linear(*self._linear_args, GEMV_MAX_ROWS[torch.float16], GEMV_MAX_ROWS[torch.float32], x, bias)
         if y is not None:
             return y
@@ -307,8 +305,6 @@ class EOQWeight:
         if rows >= 1 and x.dtype in _DTYPES and (kind != WATCHED or self.kind == _lib.KIND_Q5_POLAR):
             if rows <= fused_rows(x.dtype):
                 return self.gemv(x, bias)
-            if 8 < rows <= GEMM_MAX_ROWS and x.dtype != torch.float32 and self.kind == _lib.KIND_INT4_ABSMAX and self.cols % 16 == 0:
-                return self.gemm(x, bias)
         dt = x.dtype if x.dtype in (torch.float16, torch.bfloat16) else torch.float32
         with self._on_device(x, "EOQWeight.linear"):
             w = self.dequantize(dt, device=x.device)

@@ -3,10 +3,12 @@
 Buffers, constructors and the result type of ``forward`` are the reference's.  Where the reference rebuilds the
 weight 64 rows at a time with torch operations (centroid look-up, inverse Hadamard, norm) and multiplies, this
 module rotates the activations once per call (H is symmetric, so x . (c H) = (x H) . c) and never materialises the
-weight: up to 32 rows of x (8 for blocks below 64 columns) are multiplied straight from the byte codes the module holds
-(any bit width and block size the reference builds; one row on the CUDA cores, several on the tensor cores), or, with ``entropy_coded = True`` and
+weight: any number of rows is multiplied straight from the byte codes the module holds, on the tcgen05 tensor cores where
+blocks have 64, 128 or 256 columns (a single row against a large layer on the CUDA cores, which also take up to 8 rows of
+blocks below 64 columns; blocks above 256 columns up to 32 rows), or, with ``entropy_coded = True`` and
 the configuration that path is built for (5-bit codes, blocks of 64), from an entropy-coded copy of the codes by
-the fused decode + GEMV kernel.  Larger batches dequantise with torch operations on the same device.
+the fused decode + GEMV kernel.  What is left (other blocks at more rows, ``awq_scales``) dequantises with torch operations
+on the same device.
 """
 from __future__ import annotations
 
@@ -39,8 +41,8 @@ class PolarLinear(nn.Module):
             self.bias = None
         self._eoq: Optional[EOQWeight] = None
         self._eoq_key = None
-        # False: forward multiplies straight from the byte codes this module holds anyway (14336 x 4096 at 5 bits: 34 / 39 /
-        # 40 us at 1 / 4 / 8 rows); True: from an entropy-coded copy (`eoq_weight()`, about 4.6 instead of 8 bits per
+        # False: forward multiplies straight from the byte codes this module holds anyway (14336 x 4096 at 5 bits: 30 / 36 /
+        # 36 us at 1 / 4 / 8 rows); True: from an entropy-coded copy (`eoq_weight()`, about 4.6 instead of 8 bits per
         # weight if the byte codes are then dropped; 48 / 64 / 116 us) where that path exists (5-bit codes, blocks of 64)
         self.entropy_coded = False
 
