@@ -110,10 +110,12 @@ class PolarLinear(nn.Module):
         """x (..., in_features) -> float16 (..., out_features), fp32 accumulation (kernels/polar_engine.py:270-340)."""
         buffers = self._buffers                 # not through nn.Module.__getattr__, which costs as much as the call
         if not self.entropy_coded and buffers["awq_scales"] is None:
+            bias = buffers["bias"] if "bias" in buffers else self.bias
+            trained = bias is not None and bias.requires_grad and torch.is_grad_enabled()        # added by torch, which then has its gradient
             y = _lib.native().polar_linear(buffers["codes"], buffers["norms"], buffers["centroids"], self.out_features, self.in_features,
-                                           self.bits, self.block_size, x, buffers["bias"] if "bias" in buffers else self.bias)
+                                           self.bits, self.block_size, x, None if trained else bias)
             if y is not None:
-                return y
+                return y + bias if trained else y
         require_cuda(x, "PolarLinear.forward")
         require_cuda(self.codes, "PolarLinear.forward")
         if autocast_dtype(x) is not None:       # fp16 results of fp32 sums whatever autocast says

@@ -143,9 +143,12 @@ def test_gradients_of_the_bias_and_of_the_activations(kind):
     layer = _layer(kind)
     dense = _dense(layer).float()
     x = torch.randn(40, K, device="cuda")
+    like = _taken(layer, x)[1]
     layer.bias.requires_grad_()
     g = torch.randn(40, N, device="cuda")
-    layer(x).backward(g.to(layer(x).dtype))
+    y, taken = _taken(layer, x)
+    assert taken <= like + (2 << 20) and like < N * K
+    y.backward(g.to(y.dtype))
     assert O.rel_l2(layer.bias.grad.double().cpu().numpy(), g.sum(0).double().cpu().numpy()) < 1e-3       # an fp16 bias's gradient
     layer.bias.requires_grad_(False)
     x.requires_grad_()
