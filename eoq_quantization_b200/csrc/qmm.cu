@@ -63,7 +63,7 @@ struct QmmArgs {
     const float *tok_scale;      // [M] factor of every activation row, or null
     void *y;                     // [M][N]
     uint32_t N, K, M, T, group, sgroups, seg, units, split, planes, entries;
-    uint32_t nw, ns, a_base;     // stages of packed weights and of operands (A in TMEM, activations in shared memory); first A column
+    uint32_t nw, ns, nd, a_base; // stages of packed weights and of operands (A in TMEM, activations in shared memory); accumulators; first A column
     uint32_t at_x, at_bar;       // shared-memory offsets
     int y_dtype, bias_half, late;   // late: the packed codes are the previous kernel's to write
     long long limit;             // clock ticks a wait may take
@@ -181,6 +181,8 @@ __device__ __forceinline__ uint32_t hmul2(uint32_t a, uint32_t b) { uint32_t r; 
 __device__ __forceinline__ uint32_t bfma2(uint32_t a, uint32_t b, uint32_t c) { uint32_t r; asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c)); return r; }
 __device__ __forceinline__ uint32_t bsub2(uint32_t a, uint32_t b) { uint32_t r; asm("sub.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) { uint32_t r; asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo)); return r; }
+// (a & b) | c in one instruction (from two immediate operands the compiler makes two, of the half-rate pipe that bounds the conversions)
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) { uint32_t r; asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(b), "r"(c)); return r; }
 __device__ __forceinline__ uint32_t dup_byte(uint32_t w, uint32_t j) { return __byte_perm(w, 0u, 0x1111u * j); }
 
 // Code pairs in their natural order, exact, from one word (4 bits: eight codes; 2 bits: sixteen; 8 bits: four).  A byte is
@@ -195,19 +197,19 @@ __device__ __forceinline__ void codes_exact(uint32_t w, uint32_t *h)
         const uint32_t u = w >> 4;
 #pragma unroll
         for (uint32_t j = 0; j < 4; j++)
-            if (BF16) h[j] = bsub2((__byte_perm(w, u, 0x4400u + 0x1111u * j) & 0x000F000Fu) | 0x43004300u, 0x43074307u);
-            else h[j] = hfma2((dup_byte(w, j) & 0x00F0000Fu) | 0x64006400u, 0x2C003C00u, 0xD470E407u);
+            if (BF16) h[j] = bsub2(and_or(__byte_perm(w, u, 0x4400u + 0x1111u * j), 0x000F000Fu, 0x43004300u), 0x43074307u);
+            else h[j] = hfma2(and_or(dup_byte(w, j), 0x00F0000Fu, 0x64006400u), 0x2C003C00u, 0xD470E407u);
     } else if (BITS == 2) {
         const uint32_t u = w >> 4;
 #pragma unroll
         for (uint32_t j = 0; j < 4; j++) {
             if (BF16) {
-                h[2 * j] = bfma2((dup_byte(w, j) & 0x000C0003u) | 0x43004300u, 0x3E803F80u, 0xC204C301u);
-                h[2 * j + 1] = bfma2((dup_byte(u, j) & 0x000C0003u) | 0x43004300u, 0x3E803F80u, 0xC204C301u);
+                h[2 * j] = bfma2(and_or(dup_byte(w, j), 0x000C0003u, 0x43004300u), 0x3E803F80u, 0xC204C301u);
+                h[2 * j + 1] = bfma2(and_or(dup_byte(u, j), 0x000C0003u, 0x43004300u), 0x3E803F80u, 0xC204C301u);
             } else {
                 const uint32_t b = dup_byte(w, j);
-                h[2 * j] = hfma2((b & 0x000C0003u) | 0x64006400u, 0x34003C00u, 0xDC04E401u);
-                h[2 * j + 1] = hfma2((b & 0x00C00030u) | 0x64006400u, 0x24002C00u, 0xCC40D410u);
+                h[2 * j] = hfma2(and_or(b, 0x000C0003u, 0x64006400u), 0x34003C00u, 0xDC04E401u);
+                h[2 * j + 1] = hfma2(and_or(b, 0x00C00030u, 0x64006400u), 0x24002C00u, 0xCC40D410u);
             }
         }
     } else {
@@ -246,13 +248,13 @@ __device__ __forceinline__ void codes_scaled(uint32_t w, uint32_t *h, uint16_t s
     if (BITS == 4) {
         const float c = -135.0f * s;
 #pragma unroll
-        for (uint32_t j = 0; j < 4; j++) h[j] = pair((__byte_perm(w, u, 0x4400u + 0x1111u * j) & 0x000F000Fu) | 0x43004300u, s, c, s, c);
+        for (uint32_t j = 0; j < 4; j++) h[j] = pair(and_or(__byte_perm(w, u, 0x4400u + 0x1111u * j), 0x000F000Fu, 0x43004300u), s, c, s, c);
     } else if (BITS == 2) {
         const float q = 0.25f * s, c0 = -129.0f * s, c1 = -33.0f * s;
 #pragma unroll
         for (uint32_t j = 0; j < 4; j++) {
-            h[2 * j] = pair((dup_byte(w, j) & 0x000C0003u) | 0x43004300u, s, c0, q, c1);
-            h[2 * j + 1] = pair((dup_byte(u, j) & 0x000C0003u) | 0x43004300u, s, c0, q, c1);
+            h[2 * j] = pair(and_or(dup_byte(w, j), 0x000C0003u, 0x43004300u), s, c0, q, c1);
+            h[2 * j + 1] = pair(and_or(dup_byte(u, j), 0x000C0003u, 0x43004300u), s, c0, q, c1);
         }
     } else {
         const uint32_t v = w ^ 0x80808080u;
@@ -305,7 +307,7 @@ struct Ring {
 };
 
 // barriers, in this order, eight bytes each
-enum { kWFull = 0, kWEmpty = 8, kFull = 16, kEmpty = 24, kDFull = 32, kDEmpty = 34, kSFull = 36, kSEmpty = 40, kTmemSlot = 44, kDrain = 45, kMark = 46, kUsedW = 47, kUsedX = 48 };
+enum { kWFull = 0, kWEmpty = 8, kFull = 16, kEmpty = 24, kDFull = 32, kDEmpty = 36, kSFull = 40, kSEmpty = 44, kTmemSlot = 48, kDrain = 49, kMark = 50, kUsedW = 51, kUsedX = 52 };
 constexpr uint32_t kScaleRing = 4, kScaleGroups = 8, kScaleEntry = kScaleGroups * kRows * 2u;      // scales of 8 groups x 128 rows an entry
 
 // The scales of one weight row in the order of the groups, out of the ring that a warp of the CTA keeps filled.
@@ -374,7 +376,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
             bar_init(bar(kFull + i), 5); bar_init(bar(kEmpty + i), 1);          // four producer warps and the activation copy
         }
         for (uint32_t i = 0; i < kScaleRing; i++) { bar_init(bar(kSFull + i), 1); bar_init(bar(kSEmpty + i), 4 * (FOLD ? NF : NP)); }
-        for (uint32_t i = 0; i < 2; i++) { bar_init(bar(kDFull + i), 1); bar_init(bar(kDEmpty + i), 4 * NF); }
+        for (uint32_t i = 0; i < 4; i++) { bar_init(bar(kDFull + i), 1); bar_init(bar(kDEmpty + i), 4 * NF); }
         bar_init(bar(kDrain), 1);
         word(kMark)[0] = word(kMark)[1] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -423,11 +425,19 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
         // ---- producers: packed codes of one row, a block of columns at a time, to the A operand in tensor memory
         const uint32_t set = warp >> 2, r = (warp & 3u) * 32u + lane;
         const uint32_t lane_base = tmem + (((warp & 3u) * 32u) << 16) + a.a_base;
-        // a code to its table entry by one byte permute and one multiply-add (of the pipe that is free; a shift and a mask are
-        // two instructions of the half-rate one, which bounds the conversion); the table repeats up to 256 entries
-        const uint32_t tab_addr = saddr(table);
         uint32_t four;
         asm volatile("mov.b32 %0, 4;" : "=r"(four));
+        // a code to its table entry in one instruction: the dot product of the word's four codes with 4 at the code's place, on
+        // top of the table's address (4 rows against 14336 x 4096 36.0 -> 32.0 us with the four accumulators of few tokens; with
+        // two reader sets, where the readers bound it, 1 % slower than a byte permute and a multiply-add: 108 rows against
+        // 13338 x 896 19.5 / 19.3); the table repeats up to 256 entries
+        const uint32_t tab_addr = saddr(table);
+        auto entry = [&](uint32_t word, uint32_t b) {
+            uint32_t off;
+            if (NF == 1) asm("dp4a.u32.u32 %0, %1, %2, %3;" : "=r"(off) : "r"(word), "r"(4u << (8 * b)), "r"(tab_addr));
+            else asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(off) : "r"(__byte_perm(word, 0u, 0x4440u + b)), "r"(four), "r"(tab_addr));
+            return off;
+        };
         // scaled: the groups of 32-column parts, counted along
         ScaleReader<false> sr(wait, bar(kSFull), bar(kSEmpty), scale_ring, r);
         uint32_t gi = 0, pos = 0;
@@ -468,9 +478,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
                         float e[4];
 #pragma unroll
                         for (int b = 0; b < 4; b++) {
-                            uint32_t off;
-                            asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(off) : "r"(__byte_perm(w[c % U::kWords], 0u, 0x4440u + b)), "r"(four), "r"(tab_addr));
-                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(e[b]) : "r"(off));
+                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(e[b]) : "r"(entry(w[c % U::kWords], b)));
                         }
 #pragma unroll
                         for (int b = 0; b < 2; b++) {
@@ -487,9 +495,7 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
                         uint32_t e[4];
 #pragma unroll
                         for (int b = 0; b < 4; b++) {
-                            uint32_t off;
-                            asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(off) : "r"(__byte_perm(w[c % U::kWords], 0u, 0x4440u + b)), "r"(four), "r"(tab_addr));
-                            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(e[b]) : "r"(off));
+                            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(e[b]) : "r"(entry(w[c % U::kWords], b)));
                         }
 #pragma unroll
                         for (int b = 0; b < 2; b++) {
@@ -536,10 +542,11 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
 #pragma unroll
             for (int c = 0; c < TC; c++) tot[c] = 0.0f;
             uint32_t g = 0, in_group = seg0 - grp0 * (g16 / f16);           // segments of group g that are behind
-            for (uint32_t s = 0; s < nseg; s++) {
+            Ring dr;
+            for (uint32_t s = 0; s < nseg; s++, dr.next(a.nd)) {
                 const float sc = __half2float(__ushort_as_half(sr.get(g, lane)));
                 if (++in_group == g16 / f16) { in_group = 0; g++; }
-                wait.near(bar(kDFull + (s & 1u)), (s >> 1) & 1u);
+                wait.near(bar(kDFull + dr.at), dr.lap);
                 __syncwarp();
                 fence_after();
                 // 64 totals a lane and 96 registers: sixteen columns at a time.  With 32 under way the variant spilled in this loop,
@@ -549,12 +556,12 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
                     for (int c = 0; c < TC; c += 16) {
                         if ((uint32_t)c >= cols) break;
                         uint32_t v[16];
-                        tmem_ld16(lane_base + (s & 1u) * a.T + c, v);
+                        tmem_ld16(lane_base + dr.at * a.T + c, v);
                         tmem_ld_wait(v);
                         if (c + 16u >= cols) {
                             fence_before();
                             __syncwarp();
-                            if (lane == 0) bar_arrive(bar(kDEmpty + (s & 1u)));
+                            if (lane == 0) bar_arrive(bar(kDEmpty + dr.at));
                         }
 #pragma unroll
                         for (int j = 0; j < 16; j++) tot[c + j] = fmaf(sc, __uint_as_float(v[j]), tot[c + j]);
@@ -564,14 +571,14 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
                 for (int c = 0; c < TC; c += 32) {
                     if ((uint32_t)c >= cols) break;
                     uint32_t v[2][16];
-                    tmem_ld16(lane_base + (s & 1u) * a.T + c, v[0]);
-                    if (c + 16u < cols) tmem_ld16(lane_base + (s & 1u) * a.T + c + 16, v[1]);
+                    tmem_ld16(lane_base + dr.at * a.T + c, v[0]);
+                    if (c + 16u < cols) tmem_ld16(lane_base + dr.at * a.T + c + 16, v[1]);
                     tmem_ld_wait(v[0]);
                     tmem_ld_wait(v[1]);
                     if (c + 32u >= cols) {              // the last read of this accumulator: the next segment may have it
                         fence_before();
                         __syncwarp();
-                        if (lane == 0) bar_arrive(bar(kDEmpty + (s & 1u)));
+                        if (lane == 0) bar_arrive(bar(kDEmpty + dr.at));
                     }
 #pragma unroll
                     for (int j = 0; j < 16; j++) tot[c + j] = fmaf(sc, __uint_as_float(v[0][j]), tot[c + j]);
@@ -606,8 +613,8 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
         const bool whole = !FOLD || f16 % kB16 == 0;
         const bool two = a.planes == 2;
         const uint32_t half16 = (a.T * 128u) >> 4;                 // the second 64 columns of a plane, in descriptor units
-        uint32_t seg = 0, in_seg = k16_0 - seg0 * f16, acc = 0, d = tmem;
-        Ring ar;
+        uint32_t in_seg = k16_0 - seg0 * f16, acc = 0, d = tmem;
+        Ring ar, dr;
         for (uint32_t i = 0; i < nkb; i++) {
             wait(bar(kFull + ar.at), ar.lap);
             fence_after();
@@ -621,13 +628,14 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
                 if (kPol) mma_ts(d, at + kHalves * 32u + j * 8u, b, idesc, 1u);
             };
             auto open = [&]() {
-                d = tmem + (seg & 1u) * a.T;
-                wait(bar(kDEmpty + (seg & 1u)), ((seg >> 1) & 1u) ^ 1u);
+                d = tmem + dr.at * a.T;
+                wait(bar(kDEmpty + dr.at), dr.lap ^ 1u);
                 fence_after();
             };
             auto close = [&]() {
-                mma_commit(bar(kDFull + (seg & 1u)));
-                seg++; in_seg = 0; acc = 0;
+                mma_commit(bar(kDFull + dr.at));
+                dr.next(a.nd);
+                in_seg = 0; acc = 0;
             };
             if (whole && left >= kB16) {
                 if (FOLD && acc == 0) open();
@@ -912,16 +920,19 @@ uint32_t resident_ctas(const void *kern, uint32_t threads, size_t smem, uint32_t
     return known.back().n;
 }
 
-struct Shape { uint32_t T, nw, ns, a_base; size_t smem; uint32_t at_x, at_bar; };
+struct Shape { uint32_t T, nw, ns, nd, a_base; size_t smem; uint32_t at_x, at_bar; };
 
 // Stages and shared memory of a kernel variant for a token tile T.  A producer set has to come by every stage on every lap
 // (its parity waits look one lap back): operand stages in multiples of the sets, weight stages in multiples of the copies
-// that a set steps over.
+// that a set steps over.  Four accumulators where tokens are few: the way from a product's commit over a reader and back takes
+// longer than two segments of products (24 rows against 11008 x 4096 in groups of 64 columns 22.1 -> 20.5 us, of 128 15.95 ->
+// 14.9, with the shorter conversions).
 void place(Shape &s, uint32_t stage_w, uint32_t unit_blocks, uint32_t sets, uint32_t planes, uint32_t a_cols, uint32_t kb, bool fold)
 {
     const size_t fixed = 512 + 1024 + 1024 + (kRows + 4) * 4 + kScaleRing * kScaleEntry, room = 226u * 1024u - fixed;
     const uint32_t xstage = s.T * 2u * kb * planes, step = std::max(1u, sets / unit_blocks);
-    s.a_base = fold ? 2 * s.T : s.T;
+    s.nd = !fold ? 1u : s.T <= 32u ? 4u : 2u;
+    s.a_base = s.nd * s.T;
     s.ns = std::min(8u, (512u - s.a_base) / a_cols) / sets * sets;
     while (s.ns > sets && room < (size_t)s.ns * xstage + std::max(4u, step) * stage_w) s.ns -= sets;
     s.nw = (uint32_t)std::min<size_t>(8, (room - (size_t)s.ns * xstage) / stage_w) / step * step;      // the rest of the room hides DRAM
@@ -948,6 +959,7 @@ int run_variant(QmmArgs a, uint32_t most, uint32_t step, const void *packed, uin
     using U = Unit<BITS, KB>;
     auto kern = qmm_kernel<BITS, BF16, FOLD, NP, NF, TC, KB>;
     constexpr uint32_t threads = (4 * NP + 4 * NF + 4) * 32, a_cols = (BITS == kPolar ? 64u : 32u) * (KB / 64);
+    constexpr bool kPol = BITS == kPolar;
     const uint32_t rows = (a.N + kRows - 1) / kRows;
     a.units = (a.K + U::kCols - 1) / U::kCols;
     auto placed = [&](uint32_t T) {
@@ -969,8 +981,8 @@ int run_variant(QmmArgs a, uint32_t most, uint32_t step, const void *packed, uin
         for (uint32_t i = 0; i < std::min(used, 32u); i++) if (keys[i] == key) plan = plans[i];
     }
     if (!plan.T) {
-        const double producers = BITS == kPolar ? FOLD ? 700.0 : 1100.0 : FOLD ? 450.0 : !BF16 ? 400.0 : BITS == 8 ? 600.0 : 660.0, products = BITS == kPolar ? 3.0 : a.planes;
-        const double fixed = BITS == kPolar && !FOLD ? 8000.0 : 4000.0;       // (a row's norms are read first, and tiles are large)
+        const double producers = kPol ? FOLD ? 700.0 : 1100.0 : FOLD ? 450.0 : !BF16 ? 400.0 : BITS == 8 ? 600.0 : 660.0, products = kPol ? 3.0 : a.planes;
+        const double fixed = kPol && !FOLD ? 8000.0 : 4000.0;       // (a row's norms are read first, and tiles are large)
         double best = 1e30;
         const uint32_t least = (a.M + most - 1) / most;
         for (uint32_t n = least; n < least + 4; n++) {
@@ -995,7 +1007,7 @@ int run_variant(QmmArgs a, uint32_t most, uint32_t step, const void *packed, uin
     }
     if (cycles) { *cycles = plan.cycles; return 0; }
     const Shape s = placed(plan.T);
-    a.T = s.T; a.nw = s.nw; a.ns = s.ns; a.a_base = s.a_base; a.at_x = s.at_x; a.at_bar = s.at_bar; a.split = plan.split;
+    a.T = s.T; a.nw = s.nw; a.ns = s.ns; a.nd = s.nd; a.a_base = s.a_base; a.at_x = s.at_x; a.at_bar = s.at_bar; a.split = plan.split;
     CUtensorMap wmap, xmap;
     const bool mapped = BITS == kBlocked4
         ? map_2d(wmap, CU_TENSOR_MAP_DATA_TYPE_INT64, packed, row_bytes / 8, a.K / 16, row_bytes, kRows, U::kCols / 16, CU_TENSOR_MAP_SWIZZLE_NONE)
