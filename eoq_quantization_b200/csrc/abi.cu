@@ -263,38 +263,6 @@ class PinnedBlock {
     uint8_t *p_ = nullptr;
 };
 
-// `bytes` of pageable host memory to the device.  The driver stages a pageable copy on one core (some 9 GB/s); from a few
-// megabytes on several threads stage it, each through two chunks of its own.  The source has been read when this returns.
-cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t st)
-{
-    const size_t chunks = (bytes + kPinnedChunk - 1) / kPinnedChunk, hw = std::max(1u, std::thread::hardware_concurrency());
-    const size_t threads = std::min<size_t>({kPinnedThreads / 2, hw, chunks / 4});
-    PinnedBlock pinned;
-    if (threads < 2 || !pinned.acquire()) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
-    int device = 0;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e != cudaSuccess) return e;
-    std::atomic<int> failed{(int)cudaSuccess};
-    parallel_for(threads, [&](size_t t) {
-        cudaEvent_t free_again[2] = {nullptr, nullptr};
-        cudaError_t r = cudaSetDevice(device);
-        for (cudaEvent_t &ev : free_again) if (r == cudaSuccess) r = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-        int slot = 0;
-        for (size_t c = t; r == cudaSuccess && c < chunks; c += threads, slot ^= 1) {
-            const size_t lo = c * kPinnedChunk, cnt = std::min(kPinnedChunk, bytes - lo);
-            r = cudaEventSynchronize(free_again[slot]);              // never recorded: complete
-            if (r != cudaSuccess) break;
-            std::memcpy(pinned.chunk(2 * t + slot), static_cast<const uint8_t *>(src) + lo, cnt);
-            r = cudaMemcpyAsync(static_cast<uint8_t *>(dst) + lo, pinned.chunk(2 * t + slot), cnt, cudaMemcpyHostToDevice, st);
-            if (r == cudaSuccess) r = cudaEventRecord(free_again[slot], st);
-        }
-        for (cudaEvent_t ev : free_again)
-            if (ev) { cudaEventSynchronize(ev); cudaEventDestroy(ev); }      // the staging memory is another call's from here on
-        if (r != cudaSuccess) failed.store((int)r);
-    }, threads);
-    return (cudaError_t)failed.load();
-}
-
 // One tensor of a decode call.
 struct V1Job {
     Payload pl;                         // validated host views of the payload
@@ -306,6 +274,9 @@ struct V1Job {
     // placement inside the arena
     size_t at_stream = 0, at_offsets = 0, at_sizes = 0, at_freq = 0, at_table = 0, at_out = 0;
     bool lanes = false;
+    // blocks checked on the device (`job_verdict` has the outcome): the offsets as they lie in the caller's memory, whatever their alignment
+    const uint8_t *raw_offsets = nullptr;
+    size_t at_raw = 0, at_verdict = 0;
 };
 
 eoq_error_t job_from_payload(const eoq_tensor_header_t *h, const uint8_t *comp, size_t comp_size, size_t out_cap, V1Job &j)
@@ -331,8 +302,11 @@ eoq_error_t decode_jobs(V1Job **jobs, size_t n, cudaStream_t st, DeviceArena &ar
     size_t meta = 0;
     for (size_t i = 0; i < n; i++) {
         V1Job &j = *jobs[i];
-        j.at_offsets = meta; meta = up(meta + (size_t)j.pl.nblocks * 4);
-        j.at_sizes = meta;   meta = up(meta + (size_t)j.pl.nblocks * 4);
+        if (j.raw_offsets) { j.at_verdict = meta; meta = up(meta + 4); }
+        else {
+            j.at_offsets = meta; meta = up(meta + (size_t)j.pl.nblocks * 4);
+            j.at_sizes = meta;   meta = up(meta + (size_t)j.pl.nblocks * 4);
+        }
         j.at_freq = meta;    meta = up(meta + (size_t)j.pl.alphabet * 4);
         V1Task t = {};
         t.nblocks = j.pl.nblocks; t.block_size = j.pl.block; t.total = j.pl.total; t.p = j.pl.p; t.alphabet = j.pl.alphabet;
@@ -351,6 +325,11 @@ eoq_error_t decode_jobs(V1Job **jobs, size_t n, cudaStream_t st, DeviceArena &ar
     for (size_t i = 0; i < n; i++) {
         V1Job &j = *jobs[i];
         j.at_stream = total; total = up(total + j.pl.stream_bytes + 16);
+        if (j.raw_offsets) {
+            j.at_raw = total;     total = up(total + (size_t)j.pl.nblocks * 4);
+            j.at_offsets = total; total = up(total + (size_t)j.pl.nblocks * 4);
+            j.at_sizes = total;   total = up(total + (size_t)j.pl.nblocks * 4);
+        }
         if (!j.dev_out) { j.at_out = total; total = up(total + (size_t)j.pl.total * j.out_elem_bytes + 32); }
     }
     if (arena.acquire(total) != cudaSuccess) return EOQ_ERR_ALLOC;
@@ -358,8 +337,11 @@ eoq_error_t decode_jobs(V1Job **jobs, size_t n, cudaStream_t st, DeviceArena &ar
     std::vector<uint8_t> blob(meta, 0);
     for (size_t i = 0; i < n; i++) {
         V1Job &j = *jobs[i];
-        std::memcpy(blob.data() + j.at_offsets, j.pl.offsets.data(), (size_t)j.pl.nblocks * 4);
-        std::memcpy(blob.data() + j.at_sizes, j.pl.sizes.data(), (size_t)j.pl.nblocks * 4);
+        if (j.raw_offsets) std::memset(blob.data() + j.at_verdict, 0xFF, 4);
+        else {
+            std::memcpy(blob.data() + j.at_offsets, j.pl.offsets.data(), (size_t)j.pl.nblocks * 4);
+            std::memcpy(blob.data() + j.at_sizes, j.pl.sizes.data(), (size_t)j.pl.nblocks * 4);
+        }
         std::memcpy(blob.data() + j.at_freq, j.freq.data(), (size_t)j.pl.alphabet * 4);
         if (!j.lanes) {
             std::vector<V1Table> table;
@@ -381,11 +363,19 @@ eoq_error_t decode_jobs(V1Job **jobs, size_t n, cudaStream_t st, DeviceArena &ar
         std::memcpy(blob.data() + at_tasks, tasks.data(), tasks.size() * sizeof(V1Task));
         std::memcpy(blob.data() + at_cta, cta_task.data(), (size_t)grid * 4);
     }
-    // pageable sources are consumed before cudaMemcpyAsync returns
+    // pageable sources are consumed before cudaMemcpyAsync returns (the driver stages them at some 27 GB/s; several threads that
+    // staged them through page-locked memory of this library's took 1.2 to 1.6 ms for 19 MB, this way takes 0.75)
     CU_TRY(cudaMemcpyAsync(d, blob.data(), meta, cudaMemcpyHostToDevice, st));
     for (size_t i = 0; i < n; i++) {
         V1Job &j = *jobs[i];
-        if (j.pl.stream_bytes) CU_TRY(upload(d + j.at_stream, j.pl.stream, j.pl.stream_bytes, st));
+        if (j.pl.stream_bytes) CU_TRY(cudaMemcpyAsync(d + j.at_stream, j.pl.stream, j.pl.stream_bytes, cudaMemcpyHostToDevice, st));
+        if (j.raw_offsets) {
+            CU_TRY(cudaMemcpyAsync(d + j.at_raw, j.raw_offsets, (size_t)j.pl.nblocks * 4, cudaMemcpyHostToDevice, st));
+            if (launch_v1_check(d + j.at_stream, j.pl.stream_bytes, reinterpret_cast<const uint32_t *>(d + j.at_raw), j.pl.nblocks,
+                                reinterpret_cast<uint32_t *>(d + j.at_offsets), reinterpret_cast<uint32_t *>(d + j.at_sizes),
+                                reinterpret_cast<uint32_t *>(d + j.at_verdict), st) != 0)
+                return EOQ_ERR_CUDA;
+        }
     }
     if (!tasks.empty()) {
         int e = launch_decode_v1_lanes(reinterpret_cast<const V1Task *>(d + at_tasks), reinterpret_cast<const uint32_t *>(d + at_cta), grid,
@@ -404,6 +394,15 @@ eoq_error_t decode_jobs(V1Job **jobs, size_t n, cudaStream_t st, DeviceArena &ar
         if (j.host_out && copy_out) CU_TRY(cudaMemcpyAsync(j.host_out, out, (size_t)j.pl.total * j.out_elem_bytes, cudaMemcpyDeviceToHost, st));
     }
     return EOQ_OK;
+}
+
+// What the checks on the device found, in the order in which the host's would have: waits for them.
+eoq_error_t job_verdict(const V1Job &j, const DeviceArena &arena, cudaStream_t st)
+{
+    uint32_t v = 0;
+    CU_TRY(cudaMemcpyAsync(&v, arena.base() + j.at_verdict, 4, cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaStreamSynchronize(st));
+    return v == ~0u ? EOQ_OK : v & 1u ? EOQ_ERR_UNSUPPORTED : EOQ_ERR_CORRUPT_STREAM;
 }
 
 eoq_error_t decode_host_to_host(const eoq_tensor_header_t *h, const uint8_t *comp, size_t comp_size, void *output,
@@ -756,7 +755,7 @@ extern "C" void eoq_cuda_batch_destroy(eoq_cuda_batch_ctx_t *ctx)
 // Validates a blocked stream on the host, as the reference's decoders do block by block, and makes it a job.
 static eoq_error_t blocked_job(const uint32_t *freq, uint32_t alphabet, uint32_t precision_bits, const uint8_t *data, size_t data_len,
                                const uint32_t *offsets, uint32_t num_blocks, uint32_t block_size, uint32_t num_symbols,
-                               int out_elem_bytes, V1Job &job)
+                               int out_elem_bytes, V1Job &job, bool check_on_device = false)
 {
     if (!freq || !data || !offsets) return EOQ_ERR_NULL_PTR;
     if (alphabet == 0 || block_size == 0) return EOQ_ERR_INVALID_HEADER;
@@ -769,8 +768,9 @@ static eoq_error_t blocked_job(const uint32_t *freq, uint32_t alphabet, uint32_t
     std::vector<uint32_t> f(freq, freq + alphabet), cdf(alphabet + 1, 0);
     for (uint32_t s = 0; s < alphabet; s++) { sum += f[s]; cdf[s + 1] = cdf[s] + f[s]; }
     if (sum != (1ull << precision_bits)) return EOQ_ERR_INVALID_HEADER;
-    std::vector<uint32_t> sizes(num_blocks);
-    for (uint32_t b = 0; b < num_blocks; b++) {
+    // (a look at the first byte of every block of a cold 19 MB stream takes 1.5 ms here, a few microseconds on the device)
+    std::vector<uint32_t> sizes(check_on_device ? 0 : num_blocks);
+    for (uint32_t b = 0; b < (uint32_t)sizes.size(); b++) {
         const uint64_t lo = offsets[b], hi = b + 1 < num_blocks ? offsets[b + 1] : data_len;
         if (hi < lo || hi > data_len) return EOQ_ERR_CORRUPT_STREAM;
         sizes[b] = (uint32_t)(hi - lo);
@@ -779,7 +779,8 @@ static eoq_error_t blocked_job(const uint32_t *freq, uint32_t alphabet, uint32_t
     }
     job.pl.alphabet = alphabet; job.pl.p = precision_bits; job.pl.block = block_size; job.pl.total = num_symbols;
     job.pl.nblocks = num_blocks; job.pl.stream = data; job.pl.stream_bytes = (uint32_t)data_len;
-    job.pl.offsets.assign(offsets, offsets + num_blocks);
+    if (check_on_device) job.raw_offsets = reinterpret_cast<const uint8_t *>(offsets);
+    else job.pl.offsets.assign(offsets, offsets + num_blocks);
     job.pl.sizes = std::move(sizes);
     job.freq = std::move(f);
     job.cdf = std::move(cdf);
@@ -894,13 +895,14 @@ extern "C" eoq_error_t eoq_b200_decode_blocked_as(const uint32_t *freq, uint32_t
     if (out_type < EOQ_B200_SYM_I8 || out_type > EOQ_B200_SYM_I64 || out_type == EOQ_B200_SYM_U32) return EOQ_ERR_UNSUPPORTED;
     V1Job job;
     eoq_error_t rc = blocked_job(freq, alphabet, precision_bits, data, data_len, offsets, num_blocks, block_size, num_symbols,
-                                 alphabet <= 256 ? 1 : 2, job);
+                                 alphabet <= 256 ? 1 : 2, job, have_device());
     if (rc != EOQ_OK) return rc;
     if (!have_device()) return EOQ_ERR_CUDA;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     V1Job *one = &job;
     DeviceArena arena;
     rc = decode_jobs(&one, 1, st, arena, false);
+    if (rc == EOQ_OK) rc = job_verdict(job, arena, st);
     if (rc == EOQ_OK) rc = deliver(arena.base() + job.at_out, job.out_elem_bytes, num_symbols, out, out_type, shift, st);
     if (rc != EOQ_OK) return rc;
     CU_TRY(cudaStreamSynchronize(st));
@@ -1116,14 +1118,14 @@ eoq_error_t upload_weight(const TiledWeights &tw, const uint16_t *scales, const 
     w->table.p = base + at_table; w->tiles.p = base + at_tiles; w->scales.p = base + at_scales; w->counters.p = base + at_counters;
     w->xbuf.p = base + at_x; w->ybuf.p = base + at_y; w->biasbuf.p = base + at_bias;
     if (built) w->stream.take(*built);
-    else CU_TRY(upload(w->stream.p, tw.stream.data(), tw.stream.size(), nullptr));
+    else CU_TRY(cudaMemcpyAsync(w->stream.p, tw.stream.data(), tw.stream.size(), cudaMemcpyHostToDevice, nullptr));
     if (centroids) {
         w->centroids.p = base + at_cent;
         CU_TRY(cudaMemcpyAsync(w->centroids.p, centroids, 32 * 4, cudaMemcpyHostToDevice, nullptr));
     }
     CU_TRY(cudaMemcpyAsync(w->table.p, tw.table.data(), tw.table.size() * 4, cudaMemcpyHostToDevice, nullptr));
     CU_TRY(cudaMemcpyAsync(w->tiles.p, tw.tiles.data(), tw.tiles.size() * sizeof(TileDesc), cudaMemcpyHostToDevice, nullptr));
-    CU_TRY(upload(w->scales.p, scales, w->scale_bytes, nullptr));
+    CU_TRY(cudaMemcpyAsync(w->scales.p, scales, w->scale_bytes, cudaMemcpyHostToDevice, nullptr));
     if (pairs_layout) {
         w->scales_t.p = base + at_scales_t;
         w->pair_partials.p = base + at_partials;
@@ -1366,18 +1368,26 @@ extern "C" eoq_error_t eoq_b200_weight_from_rans(const uint8_t *c, size_t size, 
     if ((uint64_t)32 + (uint64_t)a * 4 + (uint64_t)nb * 4 + dsz > size) return EOQ_ERR_CORRUPT_STREAM;
     if ((uint64_t)opts->rows * opts->cols != n) return EOQ_ERR_INVALID_HEADER;
     if (a == 0 || a > 256) return EOQ_ERR_UNSUPPORTED;
-    std::vector<uint32_t> raw(a), freq, cdf, offs(nb);
+    std::vector<uint32_t> raw(a), freq, cdf;
     std::memcpy(raw.data(), c + 32, (size_t)a * 4);
-    std::memcpy(offs.data(), c + 32 + (size_t)a * 4, (size_t)nb * 4);
     eoq_error_t rc = normalize_reference(raw.data(), a, p, freq, cdf);
     if (rc != EOQ_OK) return rc;
     if (!have_device()) return EOQ_ERR_CUDA;
     // decoded into device memory and encoded into tiles there: the symbols never visit the host
     DeviceArena sym;
     if (sym.acquire(n) != cudaSuccess) return EOQ_ERR_ALLOC;
-    rc = eoq_b200_decode_blocked(freq.data(), a, p, c + 32 + (size_t)a * 4 + (size_t)nb * 4, dsz, offs.data(), nb, bs, n,
-                                 sym.base(), 1, 1, nullptr);
-    if (rc != EOQ_OK) return rc;
+    if (n) {
+        V1Job job;
+        rc = blocked_job(freq.data(), a, p, c + 32 + (size_t)a * 4 + (size_t)nb * 4, dsz, reinterpret_cast<const uint32_t *>(c + 32 + (size_t)a * 4), nb, bs, n, 1,
+                         job, true);
+        if (rc != EOQ_OK) return rc;
+        job.dev_out = sym.base();
+        V1Job *one = &job;
+        DeviceArena arena;
+        rc = decode_jobs(&one, 1, nullptr, arena);
+        if (rc == EOQ_OK) rc = job_verdict(job, arena, nullptr);
+        if (rc != EOQ_OK) { cudaStreamSynchronize(nullptr); return rc; }
+    }
     return weight_from_device_symbols(sym.base(), scales_fp16, opts, out);
 }
 

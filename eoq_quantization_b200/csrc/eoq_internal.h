@@ -205,6 +205,10 @@ static_assert(sizeof(V1Task) % 4 == 0 && sizeof(V1Task) <= 256 * 4, "copied into
 bool   v1_task_prepare(V1Task &t);
 size_t v1_task_smem(const V1Task &t, uint32_t warps);
 uint32_t v1_plan_ctas(V1Task *tasks, uint32_t ntasks, uint32_t &warps_per_cta, size_t &smem);
+// Blocks of a wire-format stream on the device: their sizes from the offsets, those that are not well-formed emptied.  *verdict (all
+// ones before) becomes the least of 2 x block (out of order or bounds) and 2 x block + 1 (a state wider than 32 bits).
+int launch_v1_check(const uint8_t *stream, uint32_t bytes, const uint32_t *raw, uint32_t nblocks, uint32_t *offsets, uint32_t *sizes, uint32_t *verdict,
+                    void *st);
 int launch_decode_v1_lanes(const V1Task *d_tasks, const uint32_t *d_cta_task, uint32_t grid, uint32_t warps_per_cta, size_t smem,
                            void *stream);
 int launch_decode_v1_syminfo(const uint8_t *d_stream, const uint32_t *d_offsets, const uint32_t *d_sizes,

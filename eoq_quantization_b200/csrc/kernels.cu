@@ -2720,6 +2720,31 @@ int launch_decode_v1_lanes_single(V1Task t, void *stream)
     return (int)cudaGetLastError();
 }
 
+__global__ void __launch_bounds__(256) v1_check_kernel(const uint8_t *__restrict__ stream, uint32_t bytes, const uint32_t *__restrict__ raw, uint32_t nblocks,
+                                                       uint32_t *__restrict__ offsets, uint32_t *__restrict__ sizes, uint32_t *__restrict__ verdict)
+{
+    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= nblocks) return;
+    const uint32_t lo = raw[b], hi = b + 1u < nblocks ? raw[b + 1u] : bytes;
+    bool corrupt = hi < lo || hi > bytes, wide = false;
+    if (!corrupt && hi > lo) {
+        const uint32_t len = stream[lo];
+        corrupt = 1u + len > hi - lo;
+        wide = len > 4u;
+    }
+    const bool bad = corrupt || wide;
+    offsets[b] = bad ? 0u : lo;
+    sizes[b] = bad ? 0u : hi - lo;
+    if (bad) atomicMin(verdict, 2u * b + (corrupt ? 0u : 1u));
+}
+
+int launch_v1_check(const uint8_t *stream, uint32_t bytes, const uint32_t *raw, uint32_t nblocks, uint32_t *offsets, uint32_t *sizes, uint32_t *verdict, void *st)
+{
+    v1_check_kernel<<<(nblocks + 255u) / 256u, 256, 0, reinterpret_cast<cudaStream_t>(st)>>>(stream, bytes, raw, nblocks, offsets, sizes, verdict);
+    g_launches++;
+    return (int)cudaGetLastError();
+}
+
 int launch_decode_v1_lanes(const V1Task *d_tasks, const uint32_t *d_cta_task, uint32_t grid, uint32_t warps_per_cta, size_t smem, void *stream)
 {
     static std::mutex mu;
