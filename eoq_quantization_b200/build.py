@@ -14,7 +14,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libeoq_b200.so")
 NATIVE = os.path.join(HERE, "_native.so")
-SOURCES = ["abi.cu", "kernels.cu", "qmm.cu", "rans_host.cpp", "wire_host.cpp"]
+SOURCES = ["abi.cu", "kernels.cu", "qmm.cu", "wire_encode.cu", "rans_host.cpp", "wire_host.cpp"]
 HEADERS = ["eoq_internal.h", os.path.join("..", "..", "include", "eoq_b200.h")]
 
 

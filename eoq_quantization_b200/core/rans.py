@@ -32,6 +32,15 @@ def count_symbols(symbols: np.ndarray, alphabet_size: int, shift: int = 0, clamp
     return np.array(counts, dtype=np.int64), lo, hi
 
 
+def stage_symbols(symbols: np.ndarray, alphabet_size: int, shift: int = 0, clamp: bool = False):
+    """(staged, int64 counts): the array on the device, counted there, to be handed to `encode_blocks` or `encode_container`
+    beside it; or (None, None) where the host counts and encodes (short arrays, no device in use, symbols outside the alphabet)."""
+    if not readable(symbols) or not 0 < alphabet_size <= 4096:
+        return None, None
+    got = _lib.native().stage_symbols(symbols, _ELEMENTS[symbols.dtype], shift, int(clamp), alphabet_size)
+    return (None, None) if got is None else (got[0], np.array(got[1], dtype=np.int64))
+
+
 def compute_frequency_table(symbols: np.ndarray, alphabet_size: int) -> np.ndarray:
     """Histogram of symbol values (core/rans.py:32-55); ValueError if out of range."""
     symbols = np.asarray(symbols).ravel()
@@ -99,14 +108,14 @@ def _check_precision(p: int) -> None:
         raise ValueError(f"precision_bits must be in [8, 20], got {p}")
 
 
-def encode_blocks(freq_norm: np.ndarray, precision_bits: int, symbols: np.ndarray, block_size: int):
-    """Host encoder of the library -> (bytes, offsets), wire format of core/rans.py:210-276."""
+def encode_blocks(freq_norm: np.ndarray, precision_bits: int, symbols: np.ndarray, block_size: int, staged=None):
+    """Encoder of the library (on the device for `staged` symbols) -> (bytes, offsets), wire format of core/rans.py:210-276."""
     sym = np.asarray(symbols).ravel()
     if sym.size == 0:
         return b"", []
     f = np.ascontiguousarray(freq_norm, dtype=np.uint32)
     if precision_bits <= 16 and readable(sym):
-        return _native(_lib.native().encode_symbols(sym, _ELEMENTS[sym.dtype], 0, 0, f, precision_bits, block_size, None, None),
+        return _native(_lib.native().encode_symbols(sym, _ELEMENTS[sym.dtype], 0, 0, f, precision_bits, block_size, None, None, staged),
                        "eoq_b200_wire_encode")
     sym = np.ascontiguousarray(sym.astype(np.uint32))
     nb = (sym.size + block_size - 1) // block_size
@@ -120,14 +129,14 @@ def encode_blocks(freq_norm: np.ndarray, precision_bits: int, symbols: np.ndarra
 
 
 def encode_container(symbols: np.ndarray, shift: int, freq_norm: np.ndarray, precision_bits: int, block_size: int, head: bytes,
-                     counts: np.ndarray) -> bytes:
+                     counts: np.ndarray, staged=None) -> bytes:
     """A whole `RANS` container (core/rans_blocked.py:176-214) of value + shift, clipped to the alphabet: `head` up to the
     data size, the counts, the offsets and the blocks."""
     table = np.asarray(counts).astype("<u4")
     if symbols.size == 0:
         return head + b"\0\0\0\0" + table.tobytes()
     return _native(_lib.native().encode_symbols(symbols, _ELEMENTS[symbols.dtype], shift, 1, np.ascontiguousarray(freq_norm, dtype=np.uint32),
-                                                precision_bits, block_size, head, table), "eoq_b200_wire_encode")
+                                                precision_bits, block_size, head, table, staged), "eoq_b200_wire_encode")
 
 
 def decode_blocks(freq_norm: np.ndarray, precision_bits: int, data: bytes, offsets, block_size: int, n: int,

@@ -10,7 +10,7 @@ from typing import Callable, Dict, Optional, Tuple
 import numpy as np
 import torch
 
-from .rans import RANSEncoder, _normalize_frequencies, count_symbols, decode_blocks, encode_container, readable
+from .rans import RANSEncoder, _normalize_frequencies, count_symbols, decode_blocks, encode_container, readable, stage_symbols
 from .rans_blocked import (BlockedRANSDecoder, BlockedRANSEncoder, container_head, deserialize_blocked_rans,  # noqa: F401
                            open_container, serialize_blocked_rans)  # noqa: F401
 from .utils import QuantizedTensor, dequantize, quantize_absmax
@@ -42,10 +42,12 @@ def compress_tensor_rans(name: str, codes: torch.Tensor, scales: torch.Tensor, b
     alphabet = 2 * qmax + 1
     block, precision = 256, 14
     # counted and encoded where they lie, code + qmax clipped to the alphabet on the way
-    counts = count_symbols(flat, alphabet, qmax, True)[0] if n else np.zeros(alphabet, np.int64)
+    staged, counts = stage_symbols(flat, alphabet, qmax, True) if n else (None, np.zeros(alphabet, np.int64))
+    if n and staged is None:
+        counts = count_symbols(flat, alphabet, qmax, True)[0]
     enc = RANSEncoder(counts, precision_bits=precision)
     head = container_head(n, block, (n + block - 1) // block, alphabet, precision)
-    rans_bytes = encode_container(flat, qmax, enc.freq, precision, block, head, counts)
+    rans_bytes = encode_container(flat, qmax, enc.freq, precision, block, head, counts, staged)
     scales_bytes = scales.detach().cpu().float().numpy().astype(np.float16).tobytes()
     return CompressedTensorData(name=name, shape=shape, bits=bits, block_size=block_size, scales_bytes=scales_bytes,
                                 rans_bytes=rans_bytes, n_elements=n, original_size=n * 2,

@@ -11,7 +11,7 @@ from dataclasses import dataclass
 import numpy as np
 
 from .rans import (RANSDecoder, RANSEncoder, _normalize_frequencies, compute_frequency_table, decode_blocks,
-                   encode_blocks, estimate_compressed_size)  # noqa: F401
+                   encode_blocks, estimate_compressed_size, stage_symbols)  # noqa: F401
 
 
 @dataclass
@@ -52,9 +52,11 @@ class BlockedRANSEncoder:
     def encode(self, symbols: np.ndarray, alphabet_size: int) -> BlockedRANSData:
         symbols = np.asarray(symbols).ravel()
         n = len(symbols)
-        freq = compute_frequency_table(symbols, alphabet_size)
+        staged, freq = stage_symbols(symbols, alphabet_size)
+        if staged is None:
+            freq = compute_frequency_table(symbols, alphabet_size)
         enc = RANSEncoder(freq, precision_bits=self.precision_bits)
-        data, offsets = encode_blocks(enc.freq, self.precision_bits, symbols, self.block_size)
+        data, offsets = encode_blocks(enc.freq, self.precision_bits, symbols, self.block_size, staged)
         return BlockedRANSData(compressed_blocks=data, block_offsets=offsets, freq_table=freq, num_symbols=n,
                                block_size=self.block_size, num_blocks=(n + self.block_size - 1) // self.block_size,
                                alphabet_size=alphabet_size, precision_bits=self.precision_bits)

@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <memory>
 #include <mutex>
@@ -262,6 +263,54 @@ class PinnedBlock {
     static Cache &cache() { static Cache *c = new Cache(); return *c; }      // never destroyed: no CUDA call after main
     uint8_t *p_ = nullptr;
 };
+
+// `bytes` that have to be made on the way to the device, through page-locked memory: `fill(lo, cnt, chunk)` puts bytes
+// [lo, lo + cnt) into a chunk of it.  A few threads fill, this one hands the chunks to the copy engine in order and frees their
+// slots.  Complete when this returns.  False from a fill: its error, cudaErrorInvalidValue.
+template <typename Fill>
+cudaError_t upload_filled(PinnedBlock &pinned, void *dst, size_t bytes, cudaStream_t st, size_t threads, Fill &&fill)
+{
+    constexpr size_t kSlots = kPinnedBytes / kPinnedChunk, kAhead = kSlots / 2;
+    const size_t chunks = (bytes + kPinnedChunk - 1) / kPinnedChunk;
+    auto size_of = [&](size_t c) { return std::min(kPinnedChunk, bytes - c * kPinnedChunk); };
+    auto copy = [&](size_t c) {
+        return cudaMemcpyAsync(static_cast<uint8_t *>(dst) + c * kPinnedChunk, pinned.chunk(c % kSlots), size_of(c), cudaMemcpyHostToDevice, st);
+    };
+    cudaError_t e = cudaSuccess;
+    cudaEvent_t done[2] = {nullptr, nullptr};            // behind every kAhead chunks, in turn
+    for (cudaEvent_t &ev : done) if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    std::atomic<size_t> next{0}, freed{kSlots};          // chunk to fill next; chunks below this have a slot
+    std::unique_ptr<std::atomic<int>[]> filled(new std::atomic<int>[chunks]);
+    for (size_t c = 0; c < chunks; c++) filled[c].store(0, std::memory_order_relaxed);
+    std::atomic<bool> stop{false};
+    auto work = [&] {
+        for (size_t c; !stop.load(std::memory_order_relaxed) && (c = next.fetch_add(1)) < chunks;) {
+            while (c >= freed.load(std::memory_order_acquire)) { if (stop.load(std::memory_order_relaxed)) return; std::this_thread::yield(); }
+            filled[c].store(fill(c * kPinnedChunk, size_of(c), pinned.chunk(c % kSlots)) ? 1 : -1, std::memory_order_release);
+        }
+    };
+    std::vector<std::thread> pool;
+    if (threads > 1) for (size_t t = 0; t < threads; t++) pool.emplace_back(work);
+    for (size_t c = 0; e == cudaSuccess && c < chunks; c++) {
+        if (pool.empty()) filled[c].store(fill(c * kPinnedChunk, size_of(c), pinned.chunk(c % kSlots)) ? 1 : -1, std::memory_order_relaxed);
+        int f;
+        while (!(f = filled[c].load(std::memory_order_acquire))) std::this_thread::yield();
+        if (f < 0) { e = cudaErrorInvalidValue; break; }
+        e = copy(c);
+        if (e == cudaSuccess && (c + 1) % kAhead == 0) {
+            // the half of the slots that was handed over before this one
+            const size_t half = (c + 1) / kAhead;
+            e = cudaEventRecord(done[half & 1], st);
+            if (e == cudaSuccess && half > 1) { e = cudaEventSynchronize(done[(half - 1) & 1]); freed.store(kSlots + (half - 1) * kAhead, std::memory_order_release); }
+        }
+    }
+    stop.store(true);
+    for (std::thread &t : pool) t.join();
+    cudaError_t last = cudaEventRecord(done[0], st);     // the staging memory is another call's from here on
+    if (last == cudaSuccess) last = cudaEventSynchronize(done[0]);
+    for (cudaEvent_t ev : done) if (ev) cudaEventDestroy(ev);
+    return e != cudaSuccess ? e : last;
+}
 
 // One tensor of a decode call.
 struct V1Job {
@@ -905,6 +954,202 @@ extern "C" eoq_error_t eoq_b200_decode_blocked_as(const uint32_t *freq, uint32_t
     if (rc == EOQ_OK) rc = job_verdict(job, arena, st);
     if (rc == EOQ_OK) rc = deliver(arena.base() + job.at_out, job.out_elem_bytes, num_symbols, out, out_type, shift, st);
     if (rc != EOQ_OK) return rc;
+    CU_TRY(cudaStreamSynchronize(st));
+    return EOQ_OK;
+}
+
+// -- symbols of a host array staged on the device, counted and encoded there (for the torch-facing front; not in the public header) --
+//
+// Used where the process has a context on the device already (encoding alone makes none), the array is long enough for the
+// copies to be worth it (64 Ki symbols: 0.33 ms on the host's threads, 0.1 here) and the alphabet fits shared memory.  On a
+// stream of its own: whatever else is under way on the device is not waited for.  Nothing is accepted or refused here that
+// the host encoder does not accept or refuse: what this one does not take, an array with symbols outside the alphabet among it, goes there.
+namespace {
+
+constexpr size_t kStageSymbols = 1u << 16;
+
+bool context_is_active(int dev)
+{
+    typedef CUresult (*StateFn)(CUdevice, unsigned int *, int *);
+    static StateFn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuDevicePrimaryCtxGetState", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
+        (void)cudaGetLastError();
+        return reinterpret_cast<StateFn>(p);
+    }();
+    unsigned int flags = 0;
+    int active = 0;
+    return fn && fn(dev, &flags, &active) == CUDA_SUCCESS && active;
+}
+
+// Streams kept between calls, a few a device; the others are destroyed.
+class SideStream {
+  public:
+    SideStream() = default;
+    SideStream(const SideStream &) = delete;
+    SideStream &operator=(const SideStream &) = delete;
+    bool acquire(int dev)
+    {
+        dev_ = dev;
+        {
+            std::lock_guard<std::mutex> lock(cache().mu);
+            auto &v = cache().free_list;
+            for (size_t i = 0; i < v.size(); i++)
+                if (v[i].first == dev) { st_ = v[i].second; v.erase(v.begin() + i); return true; }
+        }
+        if (cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking) == cudaSuccess) return true;
+        st_ = nullptr;
+        return false;
+    }
+    ~SideStream()
+    {
+        if (!st_) return;
+        std::lock_guard<std::mutex> lock(cache().mu);
+        if (cache().free_list.size() < 4) cache().free_list.emplace_back(dev_, st_);
+        else cudaStreamDestroy(st_);
+    }
+    cudaStream_t get() const { return st_; }
+
+  private:
+    struct Cache { std::mutex mu; std::vector<std::pair<int, cudaStream_t>> free_list; };
+    static Cache &cache() { static Cache *c = new Cache(); return *c; }      // never destroyed: no CUDA call after main
+    cudaStream_t st_ = nullptr;
+    int dev_ = 0;
+};
+
+// Allocations and waits of this thread are allowed although a stream of it may be recording: they have no part in the recording.
+struct BesideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+struct OnDevice {
+    int was = -1;
+    explicit OnDevice(int dev) { if (cudaGetDevice(&was) != cudaSuccess || (was != dev && cudaSetDevice(dev) != cudaSuccess)) was = -1; else if (was == dev) was = -1; }
+    ~OnDevice() { if (was >= 0) cudaSetDevice(was); }
+};
+
+}  // namespace
+
+struct eoq_b200_symbols {
+    SideStream stream;               // given back last
+    DeviceArena sym, work;
+    int dev = 0, wide = 0, shift = 0;
+    bool moved = false, is_signed = false, clamp = false;        // the bytes are the caller's: value + shift, clamped or not, is the symbol
+    uint32_t n = 0, alphabet = 0, nblocks = 0;
+    size_t at_counts = 0, at_table = 0, at_offsets = 0, at_out = 0, bytes = 0;
+    ~eoq_b200_symbols()
+    {
+        BesideCapture beside;
+        if (stream.get()) cudaStreamSynchronize(stream.get());      // the arenas are another call's from here on
+        (void)cudaGetLastError();
+    }
+};
+
+extern "C" void eoq_b200_symbols_free(eoq_b200_symbols *s) { delete s; }
+
+// The staged array, or null: the host encodes.
+extern "C" eoq_b200_symbols *eoq_b200_symbols_stage(const void *symbols, int elem, size_t n, int64_t shift, int clamp, uint32_t alphabet)
+{
+    if (!symbols || n < kStageSymbols || n > (1u << 28) || alphabet == 0 || alphabet > 4096u || elem < EOQ_B200_SYM_I8 || elem > EOQ_B200_SYM_I64) return nullptr;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || !context_is_active(dev)) { (void)cudaGetLastError(); return nullptr; }
+    BesideCapture beside;
+    std::unique_ptr<eoq_b200_symbols> s(new eoq_b200_symbols());
+    s->dev = dev; s->n = (uint32_t)n; s->alphabet = alphabet; s->wide = alphabet > 256u;
+    const size_t width = s->wide ? 2 : 1;
+    s->at_counts = (n * width + 255) & ~(size_t)255;
+    s->at_table = s->at_counts + (((size_t)alphabet * 8 + 8 + 255) & ~(size_t)255);
+    PinnedBlock pinned;
+    if (!s->stream.acquire(dev) || s->sym.acquire(s->at_table + (size_t)alphabet * 16) != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
+    cudaStream_t st = s->stream.get();
+    uint8_t *to = s->sym.base();
+    // Bytes that hold a symbol as it will be kept go up as they are, and the device moves and clamps them; other types are
+    // narrowed on the way into the staging memory (a core reads some 1 G of them a second).
+    const bool as_is = !s->wide && (elem == EOQ_B200_SYM_I8 || elem == EOQ_B200_SYM_U8) && shift > -(1 << 24) && shift < (1 << 24);
+    cudaError_t e = cudaSuccess;
+    if (as_is) {
+        e = cudaMemcpyAsync(to, symbols, n, cudaMemcpyHostToDevice, st);
+    } else if (!pinned.acquire()) {
+        return nullptr;
+    } else {
+        const size_t bytes = n * width, hw = std::max(1u, std::thread::hardware_concurrency());
+        const size_t threads = std::min<size_t>({kPinnedThreads / 2, hw, (bytes + kPinnedChunk - 1) / kPinnedChunk});
+        e = upload_filled(pinned, to, bytes, st, threads, [&](size_t lo, size_t cnt, uint8_t *chunk) {
+            return wire_narrow(symbols, elem, lo / width, cnt / width, shift, clamp != 0, alphabet, chunk);
+        });
+    }
+    if (e != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
+    if (as_is) { s->moved = true; s->is_signed = elem == EOQ_B200_SYM_I8; s->shift = (int)shift; s->clamp = clamp != 0; }
+    return s.release();
+}
+
+// Counts of the symbols; EOQ_ERR_UNSUPPORTED where one is outside the alphabet (and not to be clamped).
+extern "C" eoq_error_t eoq_b200_symbols_count(eoq_b200_symbols *s, uint64_t *counts)
+{
+    BesideCapture beside;
+    OnDevice on(s->dev);
+    cudaStream_t st = s->stream.get();
+    unsigned long long *d = reinterpret_cast<unsigned long long *>(s->sym.base() + s->at_counts);
+    CU_TRY(cudaMemsetAsync(d, 0, (size_t)s->alphabet * 8 + 8, st));
+    unsigned long long *outside = d + s->alphabet;
+    if (s->moved && launch_wire_move(s->sym.base(), s->is_signed, s->shift, s->n, s->alphabet, outside, st) != 0) return EOQ_ERR_CUDA;
+    s->moved = false;
+    std::vector<uint64_t> got((size_t)s->alphabet + 1);
+    if (launch_wire_count(s->sym.base(), s->wide, s->n, s->alphabet, d, st) != 0) return EOQ_ERR_CUDA;
+    CU_TRY(cudaMemcpyAsync(got.data(), d, got.size() * 8, cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaStreamSynchronize(st));
+    std::memcpy(counts, got.data(), (size_t)s->alphabet * 8);
+    return got.back() && !s->clamp ? EOQ_ERR_UNSUPPORTED : EOQ_OK;
+}
+
+extern "C" eoq_error_t eoq_b200_symbols_encode(eoq_b200_symbols *s, const uint32_t *freq, uint32_t alphabet, uint32_t p, uint32_t block, size_t *bytes)
+{
+    if (!s || !freq || !bytes) return EOQ_ERR_NULL_PTR;
+    if (p < 1 || block == 0) return EOQ_ERR_INVALID_HEADER;
+    if (p > 16 || alphabet != s->alphabet) return EOQ_ERR_UNSUPPORTED;
+    std::vector<uint32_t> table;
+    if (!wire_table(freq, alphabet, p, table)) return EOQ_ERR_INVALID_HEADER;
+    BesideCapture beside;
+    OnDevice on(s->dev);
+    cudaStream_t st = s->stream.get();
+    WireEncodeArgs a = {};
+    a.sym = s->sym.base(); a.n = s->n; a.alphabet = alphabet; a.p = p; a.block = std::min(block, s->n);
+    a.nblocks = s->nblocks = (uint32_t)(((uint64_t)s->n + block - 1) / block);
+    a.words = a.block / 2u + 1u;                       // two bytes a symbol at most
+    auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+    const size_t scratch = (size_t)((a.nblocks + 31u) / 32u) * 128u * a.words, most = (size_t)s->n * 2 + (size_t)a.nblocks * 8;
+    if (scratch > (2ull << 30)) return EOQ_ERR_UNSUPPORTED;         // few, long blocks: the host's
+    const size_t at_record = up(scratch), at_sizes = up(at_record + (size_t)a.nblocks * 16);
+    s->at_offsets = up(at_sizes + (size_t)a.nblocks * 4);
+    const size_t at_total = up(s->at_offsets + (size_t)a.nblocks * 4);
+    s->at_out = at_total + 256;
+    if (s->work.acquire(s->at_out + most) != cudaSuccess) { (void)cudaGetLastError(); return EOQ_ERR_UNSUPPORTED; }
+    uint8_t *d = s->work.base();
+    a.table = reinterpret_cast<const uint4 *>(s->sym.base() + s->at_table);
+    a.scratch = reinterpret_cast<uint32_t *>(d); a.record = reinterpret_cast<uint4 *>(d + at_record); a.sizes = reinterpret_cast<uint32_t *>(d + at_sizes);
+    unsigned long long *total = reinterpret_cast<unsigned long long *>(d + at_total), sum = 0;
+    CU_TRY(cudaMemcpyAsync(s->sym.base() + s->at_table, table.data(), table.size() * 4, cudaMemcpyHostToDevice, st));
+    if (launch_wire_encode(a, s->wide, reinterpret_cast<uint32_t *>(d + s->at_offsets), total, d + s->at_out, st) != 0) return EOQ_ERR_CUDA;
+    CU_TRY(cudaMemcpyAsync(&sum, total, 8, cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaStreamSynchronize(st));
+    if (sum > 0xFFFFFFFFull) return EOQ_ERR_OVERFLOW;
+    *bytes = s->bytes = (size_t)sum;
+    return EOQ_OK;
+}
+
+// The encoded bytes (as many as eoq_b200_symbols_encode said) and the blocks' offsets.
+extern "C" eoq_error_t eoq_b200_symbols_fetch(eoq_b200_symbols *s, uint8_t *data, uint32_t *offsets)
+{
+    if (!s || !data || !offsets || !s->work.base()) return EOQ_ERR_NULL_PTR;
+    BesideCapture beside;
+    OnDevice on(s->dev);
+    cudaStream_t st = s->stream.get();
+    const eoq_error_t rc = deliver(s->work.base() + s->at_out, 1, s->bytes, data, EOQ_B200_SYM_U8, 0, st);
+    if (rc != EOQ_OK) return rc;
+    CU_TRY(cudaMemcpyAsync(offsets, s->work.base() + s->at_offsets, (size_t)s->nblocks * 4, cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
     return EOQ_OK;
 }

@@ -217,6 +217,23 @@ int launch_decode_v1_syminfo(const uint8_t *d_stream, const uint32_t *d_offsets,
 int launch_decode_v1_resume(const uint8_t *d_block, uint32_t stream_end, const V1Table *d_table,
                             uint32_t *d_state_pos /* [2]: state, pos */, uint8_t *d_out, uint32_t count,
                             uint32_t p, void *stream);
+// The wire format's encoder on the device (wire_encode.cu).  Symbols of one byte (wide: two) below `alphabet`, 16-byte aligned.
+struct WireEncodeArgs {
+    const void *sym;
+    const uint4 *table;          // per symbol: reciprocal (two words), frequency, cumulative
+    uint32_t *scratch;           // [blocks of 32][words][32]
+    uint4 *record;               // per block: state, words, the bytes short of a word, how many
+    uint32_t *sizes;
+    uint32_t n, alphabet, p, block, nblocks, words;
+};
+int launch_wire_move(uint8_t *sym, int is_signed, int shift, uint32_t n, uint32_t alphabet, unsigned long long *outside, void *stream);
+int launch_wire_count(const void *sym, int wide, uint32_t n, uint32_t alphabet, unsigned long long *counts, void *stream);
+int launch_wire_encode(const WireEncodeArgs &a, int wide, uint32_t *offsets, unsigned long long *total, uint8_t *out, void *stream);
+// Symbols [lo, lo + n) of a host array (value + shift, below `alphabet` by clamping) to bytes, or with alphabets above 256 to
+// two bytes each (wire_host.cpp); false where one was outside and clamping was not asked for.
+bool wire_narrow(const void *symbols, int elem, size_t lo, size_t n, int64_t shift, bool clamp, uint32_t alphabet, void *out);
+// Reciprocal, frequency and cumulative frequency of every symbol (wire_host.cpp); false for a table that is none.
+bool wire_table(const uint32_t *freq, uint32_t alphabet, uint32_t p, std::vector<uint32_t> &words);
 // GEMV on QuantizedLinear's in-memory form (packed codes, fp16 scales): see gemv_packed_kernel.
 struct PackedGemvArgs {
     const uint8_t *packed;      // [N][row_bytes]

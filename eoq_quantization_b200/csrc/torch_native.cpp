@@ -36,6 +36,12 @@
 
 extern "C" int eoq_b200_linear_packed_preferred(const uint8_t *d_packed, uint32_t rows, uint32_t cols, uint32_t bits, uint32_t group,
                                                 const void *x, int x_dtype, uint32_t batch);
+struct eoq_b200_symbols;
+extern "C" eoq_b200_symbols *eoq_b200_symbols_stage(const void *symbols, int elem, size_t n, int64_t shift, int clamp, uint32_t alphabet);
+extern "C" eoq_error_t eoq_b200_symbols_count(eoq_b200_symbols *s, uint64_t *counts);
+extern "C" eoq_error_t eoq_b200_symbols_encode(eoq_b200_symbols *s, const uint32_t *freq, uint32_t alphabet, uint32_t p, uint32_t block, size_t *bytes);
+extern "C" eoq_error_t eoq_b200_symbols_fetch(eoq_b200_symbols *s, uint8_t *data, uint32_t *offsets);
+extern "C" void eoq_b200_symbols_free(eoq_b200_symbols *s);
 extern "C" int eoq_b200_ordered_launches(int on);
 extern "C" int eoq_b200_weight_linear_preferred(const eoq_b200_weight_t *w, const void *x, int x_dtype, uint32_t batch);
 
@@ -418,11 +424,63 @@ PyObject *count_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
     GUARD_END
 }
 
-// encode_symbols(array, type, shift, clamp, freq, precision, block_size, head, table): with head None (bytes, [offsets]), else the
+constexpr const char *kStaged = "eoq_b200.symbols";
+
+void free_staged(PyObject *c) { eoq_b200_symbols_free(static_cast<eoq_b200_symbols *>(PyCapsule_GetPointer(c, kStaged))); }
+
+// stage_symbols(array, type, shift, clamp, alphabet) -> (staged, [counts]): the array on the device, for one encode_symbols call
+// in front of which it is counted there; or None: count_symbols and encode_symbols take the array.
+PyObject *stage_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
+{
+    if (n != 5) { PyErr_SetString(PyExc_TypeError, "stage_symbols takes 5 arguments"); return nullptr; }
+    GUARD_BEGIN
+    Buffer sym(a[0]);
+    if (!sym.ok) return nullptr;
+    const int type = (int)PyLong_AsLong(a[1]), clamp = (int)PyLong_AsLong(a[3]);
+    const int64_t shift = PyLong_AsLongLong(a[2]), alphabet = PyLong_AsLongLong(a[4]);
+    if (PyErr_Occurred()) return nullptr;
+    if (alphabet < 1 || alphabet > 4096) Py_RETURN_NONE;
+    eoq_b200_symbols *s = nullptr;
+    std::vector<uint64_t> counts((size_t)alphabet);
+    eoq_error_t rc = EOQ_OK;
+    Py_BEGIN_ALLOW_THREADS
+    s = eoq_b200_symbols_stage(sym.v.buf, type, (size_t)(sym.v.len / sym.v.itemsize), shift, clamp, (uint32_t)alphabet);
+    if (s) rc = eoq_b200_symbols_count(s, counts.data());
+    if (s && rc != EOQ_OK) { eoq_b200_symbols_free(s); s = nullptr; }
+    Py_END_ALLOW_THREADS
+    if (!s) Py_RETURN_NONE;
+    PyObject *staged = PyCapsule_New(s, kStaged, free_staged);
+    if (!staged) { eoq_b200_symbols_free(s); return nullptr; }
+    PyObject *list = PyList_New((Py_ssize_t)alphabet);
+    if (!list) { Py_DECREF(staged); return nullptr; }
+    for (int64_t i = 0; i < alphabet; i++) PyList_SET_ITEM(list, i, PyLong_FromUnsignedLongLong(counts[(size_t)i]));
+    return Py_BuildValue("NN", staged, list);
+    GUARD_END
+}
+
+// What encode_symbols encoded, on the host or (staged) on the device, until it has been fetched.
+struct Encoded {
+    eoq_b200_wire_t *wire = nullptr;
+    eoq_b200_symbols *staged = nullptr;
+    size_t bytes = 0;
+    Encoded() = default;
+    Encoded(const Encoded &) = delete;
+    Encoded &operator=(const Encoded &) = delete;
+    ~Encoded() { if (wire) eoq_b200_wire_take(wire, nullptr, nullptr); }
+    eoq_error_t fetch(uint8_t *data, uint32_t *offsets)
+    {
+        if (staged) return eoq_b200_symbols_fetch(staged, data, offsets);
+        eoq_b200_wire_take(wire, data, offsets);
+        wire = nullptr;
+        return EOQ_OK;
+    }
+};
+
+// encode_symbols(array, type, shift, clamp, freq, precision, block_size, head, table, staged): with head None (bytes, [offsets]), else the
 // container in one piece: head, u32 data size, table, u32 offsets, data; or an error code.
 PyObject *encode_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
-    if (n != 9) { PyErr_SetString(PyExc_TypeError, "encode_symbols takes 9 arguments"); return nullptr; }
+    if (n != 10) { PyErr_SetString(PyExc_TypeError, "encode_symbols takes 10 arguments"); return nullptr; }
     GUARD_BEGIN
     Buffer sym(a[0]);
     if (!sym.ok) return nullptr;
@@ -433,33 +491,43 @@ PyObject *encode_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
     if (PyErr_Occurred()) return nullptr;
     const int64_t count = sym.v.len / sym.v.itemsize, alphabet = freq.v.len / 4;
     if (count < 1 || count > 0xFFFFFFFFll || block < 1 || block > 0xFFFFFFFFll || p < 1 || p > 16) return codec_error(EOQ_ERR_UNSUPPORTED);
-    eoq_b200_wire_t *w = nullptr;
-    size_t bytes = 0;
+    Encoded w;
+    if (a[9] != Py_None) {
+        w.staged = static_cast<eoq_b200_symbols *>(PyCapsule_GetPointer(a[9], kStaged));
+        if (!w.staged) return nullptr;
+    }
     eoq_error_t rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = eoq_b200_wire_encode(sym.v.buf, type, (uint32_t)count, shift, clamp, static_cast<const uint32_t *>(freq.v.buf), (uint32_t)alphabet, (uint32_t)p,
-                              (uint32_t)block, &w, &bytes);
+    rc = EOQ_ERR_UNSUPPORTED;
+    if (w.staged) rc = eoq_b200_symbols_encode(w.staged, static_cast<const uint32_t *>(freq.v.buf), (uint32_t)alphabet, (uint32_t)p, (uint32_t)block, &w.bytes);
+    if (rc == EOQ_ERR_UNSUPPORTED) {
+        w.staged = nullptr;
+        rc = eoq_b200_wire_encode(sym.v.buf, type, (uint32_t)count, shift, clamp, static_cast<const uint32_t *>(freq.v.buf), (uint32_t)alphabet, (uint32_t)p,
+                                  (uint32_t)block, &w.wire, &w.bytes);
+    }
     Py_END_ALLOW_THREADS
     if (rc != EOQ_OK) return codec_error(rc);
+    const size_t bytes = w.bytes;
     const int64_t nb = (count + block - 1) / block;
     if (a[7] == Py_None) {
         PyObject *data = PyBytes_FromStringAndSize(nullptr, (Py_ssize_t)bytes);
         PyObject *list = data ? PyList_New((Py_ssize_t)nb) : nullptr;
-        if (!list) { Py_XDECREF(data); eoq_b200_wire_take(w, nullptr, nullptr); return nullptr; }
+        if (!list) { Py_XDECREF(data); return nullptr; }
         std::vector<uint32_t> offs((size_t)nb);
         uint8_t *to = reinterpret_cast<uint8_t *>(PyBytes_AS_STRING(data));
         Py_BEGIN_ALLOW_THREADS
-        eoq_b200_wire_take(w, to, offs.data());
+        rc = w.fetch(to, offs.data());
         Py_END_ALLOW_THREADS
+        if (rc != EOQ_OK) { Py_DECREF(data); Py_DECREF(list); return codec_error(rc); }
         for (int64_t b = 0; b < nb; b++) PyList_SET_ITEM(list, b, PyLong_FromUnsignedLong(offs[(size_t)b]));
         return Py_BuildValue("NN", data, list);
     }
     // container: head, data size, table, offsets, data
     Buffer head(a[7]), table(a[8]);
-    if (!head.ok || !table.ok) { eoq_b200_wire_take(w, nullptr, nullptr); return nullptr; }
+    if (!head.ok || !table.ok) return nullptr;
     const size_t at_table = (size_t)head.v.len + 4, at_offs = at_table + (size_t)table.v.len, at_data = at_offs + 4 * (size_t)nb;
     PyObject *whole = PyBytes_FromStringAndSize(nullptr, (Py_ssize_t)(at_data + bytes));
-    if (!whole) { eoq_b200_wire_take(w, nullptr, nullptr); return nullptr; }
+    if (!whole) return nullptr;
     uint8_t *to = reinterpret_cast<uint8_t *>(PyBytes_AS_STRING(whole));
     const uint32_t size32 = (uint32_t)bytes;
     std::memcpy(to, head.v.buf, (size_t)head.v.len);
@@ -467,9 +535,10 @@ PyObject *encode_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
     std::memcpy(to + at_table, table.v.buf, (size_t)table.v.len);
     std::vector<uint32_t> offs((size_t)nb);
     Py_BEGIN_ALLOW_THREADS
-    eoq_b200_wire_take(w, to + at_data, offs.data());
+    rc = w.fetch(to + at_data, offs.data());
     std::memcpy(to + at_offs, offs.data(), 4 * (size_t)nb);
     Py_END_ALLOW_THREADS
+    if (rc != EOQ_OK) { Py_DECREF(whole); return codec_error(rc); }
     return whole;
     GUARD_END
 }
@@ -519,6 +588,7 @@ PyObject *decode_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
 PyMethodDef methods[] = {
     {"call_kind", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(call_kind)), METH_FASTCALL, nullptr},
     {"count_symbols", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(count_symbols)), METH_FASTCALL, nullptr},
+    {"stage_symbols", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(stage_symbols)), METH_FASTCALL, nullptr},
     {"encode_symbols", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(encode_symbols)), METH_FASTCALL, nullptr},
     {"decode_symbols", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(decode_symbols)), METH_FASTCALL, nullptr},
     {"weight_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(weight_linear)), METH_FASTCALL, nullptr},

@@ -198,6 +198,61 @@ static bool by_type(const void *sym, int elem, int64_t shift, bool clamp, uint32
     return false;
 }
 
+template <typename T, typename D>
+static bool narrow(const T *p, size_t n, int64_t shift, bool clamp, int64_t top, D *out)
+{
+    bool outside = false;
+    if (sizeof(T) <= 2 && shift > -(1 << 24) && shift < (1 << 24)) {
+        const int32_t s = (int32_t)shift, t = (int32_t)top;
+        for (size_t i = 0; i < n; i++) {
+            const int32_t v = (int32_t)p[i] + s, c = v < 0 ? 0 : v > t ? t : v;
+            outside |= c != v;
+            out[i] = (D)c;
+        }
+    } else if (!clamp) {
+        // (no compare in the loop, which the compiler then vectorises: bits above the result's, and a second look at the results)
+        uint64_t high = 0;
+        D most = 0;
+        for (size_t i = 0; i < n; i++) {
+            const uint64_t v = (uint64_t)((int64_t)p[i] + shift);
+            high |= v;
+            out[i] = (D)v;
+        }
+        for (size_t i = 0; i < n; i++) most = std::max(most, out[i]);
+        return (high >> (8 * sizeof(D))) == 0 && (int64_t)most <= top;
+    } else {
+        for (size_t i = 0; i < n; i++) {
+            const int64_t v = (int64_t)p[i] + shift, c = v < 0 ? 0 : v > top ? top : v;
+            outside |= c != v;
+            out[i] = (D)c;
+        }
+    }
+    return clamp || !outside;
+}
+
+bool wire_narrow(const void *symbols, int elem, size_t lo, size_t n, int64_t shift, bool clamp, uint32_t alphabet, void *out)
+{
+    bool fine = false;
+    by_type(symbols, elem, shift, clamp, alphabet, [&](auto src) {
+        fine = alphabet <= 256 ? narrow(src.p + lo, n, shift, clamp, src.top, static_cast<uint8_t *>(out))
+                               : narrow(src.p + lo, n, shift, clamp, src.top, static_cast<uint16_t *>(out));
+    });
+    return fine;
+}
+
+bool wire_table(const uint32_t *freq, uint32_t alphabet, uint32_t p, std::vector<uint32_t> &words)
+{
+    words.resize((size_t)alphabet * 4);
+    uint64_t sum = 0;
+    for (uint32_t s = 0; s < alphabet; s++) {
+        if (freq[s] == 0 || freq[s] > 1u << p) return false;
+        const uint64_t m = (1ull << 48) / freq[s] + 1;
+        words[4 * s] = (uint32_t)m; words[4 * s + 1] = (uint32_t)(m >> 32); words[4 * s + 2] = freq[s]; words[4 * s + 3] = (uint32_t)sum;
+        sum += freq[s];
+    }
+    return sum == 1ull << p;
+}
+
 }  // namespace eoq
 
 using namespace eoq;
