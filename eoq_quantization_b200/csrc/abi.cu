@@ -2101,6 +2101,12 @@ extern "C" int eoq_b200_linear_packed_preferred(const uint8_t *d_packed, uint32_
                          (double)rows * cols / 1.2e6, 5.5) ? 1 : 0;
 }
 
+// Above 64 rows, and above 32 against weights of which several CTAs share the columns anyway (from 8192 rows on a block of 64
+// columns costs some 1300 cycles when rotated, 900 to 1500 when not, by the rows).  14336 x 4096 has not been split, so it goes like
+// 11008 x 4096: 64 rows 42.0 us / rotated 45.6, 80 rows 48.4 / 46.3, 512 rows 127 / 94.8; 4096 x 4096, 40 rows 16.9 / 16.6, 200
+// rows 30.2 / 21.2; 1024 x 4096, 40 rows 12.0 / 9.0.
+static bool polar_rotates(uint32_t rows, uint32_t batch) { return batch > 64u || (batch > 32u && rows <= 8192u); }
+
 extern "C" eoq_error_t eoq_b200_linear_polar_codes(const uint8_t *d_codes, const uint16_t *d_norms_fp16, const float *d_centroids,
                                                    uint32_t rows, uint32_t cols, uint32_t bits, uint32_t block, const void *x, int x_dtype,
                                                    uint32_t batch, void *d_scratch, void *y, int y_dtype, const void *bias, int bias_dtype,
@@ -2118,7 +2124,13 @@ extern "C" eoq_error_t eoq_b200_linear_polar_codes(const uint8_t *d_codes, const
     c.packed = d_codes; c.scales = d_norms_fp16; c.centroids = d_centroids; c.bias = bias; c.x = d_scratch; c.tok_scale = factors; c.y = y;
     c.bias_half = bias_dtype == EOQ_B200_F16;
     c.N = rows; c.K = cols; c.M = batch; c.bits = bits; c.group = block; c.split_x = 1; c.y_dtype = y_dtype;
-    int e = launch_split_rows(x, x_dtype, cols, batch, block, d_scratch, factors, stream);
+    // many 16-bit rows against blocks of 64: the weight is rotated on its way to the products instead of the activations, which
+    // then are one fp16 plane (bf16 ones brought to fp16's range a row at a time) and need two products of a pair, not three
+    c.rotate = block == 64 && polar_rotates(rows, batch) && x_dtype != EOQ_B200_F32 && (x_dtype != EOQ_B200_F16 || (reinterpret_cast<uintptr_t>(x) & 15u) == 0);
+    if (c.rotate) c.split_x = 0;
+    if (c.rotate && x_dtype == EOQ_B200_F16) { c.x = x; c.tok_scale = nullptr; }
+    int e = 0;
+    if (c.x == d_scratch) e = launch_split_rows(x, x_dtype, cols, batch, c.rotate ? 1 : block, d_scratch, factors, stream);
     if (e == 0) e = launch_qmm(c, stream);
     return product_result(e, "eoq_b200_linear_polar_codes");
 }

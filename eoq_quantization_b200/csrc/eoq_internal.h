@@ -273,6 +273,7 @@ struct QmmCall {
     uint32_t N, K, M, bits, group;
     int bf16, split_x, y_dtype, bias_half, late;     // late: `packed` is written by the kernel before this one in the stream
     uint32_t *status;            // device address of a word to set when a wait runs out, or null: the one qmm_status reads
+    int rotate;                  // polar, blocks of 64: x is not rotated, the kernel rotates the weight; one fp16 plane
     uint32_t blocked_rows;       // not 0: 4-bit codes as [K / 16][blocked_rows] words of sixteen, as the decoder leaves them
 };
 bool qmm_takes(uint32_t K, uint32_t bits, uint32_t group, const void *packed, const void *x);

@@ -17,7 +17,8 @@
 //           runs over all of K: for many tokens (up to 256 a CTA), where reading accumulators back would cost more.
 //
 // Warp roles: producers (four warps per set, one per TMEM lane quadrant; the sets take blocks of columns in turn), readers
-// (fold and epilogue, the same quadrants), and one warp each to issue the MMAs, the weight copies and the activation
+// (fold, the same quadrants; at the end of `scaled` both take the accumulator to shared memory: 200 bf16 rows in groups of 128
+// against 11008 x 4096 34.3 us with the readers alone, 31.6), and one warp each to issue the MMAs, the weight copies and the activation
 // copies and to fetch the scales.  Few row tiles: the columns are split over the CTAs of a cluster, which add their
 // totals up through distributed shared memory, so there is no scratch in global memory and the order of the additions
 // is fixed.
@@ -44,6 +45,7 @@ namespace {
 
 constexpr uint32_t kRows = 128;
 constexpr int kPolar = 5;                  // "BITS" of the byte codes that go through a centroid table
+constexpr int kPolarRot = 7;               // the same in blocks of 64, rotated here: every 64 values of a row times the Hadamard matrix
 constexpr int kBlocked4 = 6;               // "BITS" of 4-bit codes in [K / 16][rows] words of sixteen
 
 __device__ __forceinline__ uint32_t saddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -267,6 +269,14 @@ __device__ __forceinline__ void codes_scaled(uint32_t w, uint32_t *h, uint16_t s
     }
 }
 
+// two fp32 in a register pair
+__device__ __forceinline__ uint64_t pack2(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float low2(uint64_t v) { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return a; }
+__device__ __forceinline__ float high2(uint64_t v) { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return b; }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) { uint64_t r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+
 __device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t (&r)[32])
 {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
@@ -343,7 +353,8 @@ __global__ void __launch_bounds__((4 * NP + 4 * NF + 4) * 32, 1)
 qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap)
 {
     using U = Unit<BITS, KB>;
-    constexpr bool kPol = BITS == kPolar;
+    constexpr bool kRot = BITS == kPolarRot, kPol = BITS == kPolar || kRot;
+    static_assert(!kRot || (!FOLD && KB == 64), "a thread rotates one block of 64 columns");
     constexpr int kCode = kPol ? 8 : BITS == kBlocked4 ? 4 : BITS;
     constexpr uint32_t kHalves = KB / 64;                         // 64-column parts of a block
     constexpr uint32_t kACols = (kPol ? 64u : 32u) * kHalves;     // TMEM columns of a block (polar: high and low halves)
@@ -408,8 +419,20 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
         if (warp < 4 * NP) {
             const uint16_t *norms = a.scales + (size_t)min(row0 + r, a.N - 1u) * a.sgroups + grp0;
             float most = 0.0f;
+            auto larger = [&](uint32_t bits) { most = fmaxf(most, fabsf(__half2float(__ushort_as_half((uint16_t)bits)))); };
+            if (((reinterpret_cast<uintptr_t>(a.scales) | a.sgroups * 2u | grp0 * 2u | ngroups * 2u) & 15u) == 0) {
+                // eight a load (64 norms a row one at a time: 7 of the 187 us of 512 rows against 14336 x 4096)
+#pragma unroll 4
+                for (uint32_t g = (warp >> 2) * 8u; g < ngroups; g += NP * 8u) {
+                    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(norms + g));
+                    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int i = 0; i < 4; i++) { larger(w[i] & 0xFFFFu); larger(w[i] >> 16); }
+                }
+            } else {
 #pragma unroll 16
-            for (uint32_t g = warp >> 2; g < ngroups; g += NP) most = fmaxf(most, fabsf(__half2float(__ushort_as_half(__ldg(norms + g)))));
+                for (uint32_t g = warp >> 2; g < ngroups; g += NP) larger(__ldg(norms + g));
+            }
             atomicMax(largest + r, __float_as_uint(most));
             if (threadIdx.x < 256u) atomicMax(largest + kRows, table[threadIdx.x] & 0x7fffffffu);
         }
@@ -470,7 +493,39 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
                     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[4 * c]), "=r"(w[4 * c + 1]), "=r"(w[4 * c + 2]), "=r"(w[4 * c + 3]) : "r"(at));
                 }
                 uint32_t h[32], lo[kPol ? 32 : 1];
-                if (kPol && !FOLD) {
+                if constexpr (kRot) {
+                    // the block's values, a fast Walsh-Hadamard transform of them in registers (pairs of neighbours a register
+                    // pair), times norm / 64, as two fp16 halves
+                    const float sc = __half2float(__ushort_as_half(sr.get(gi, lane))) * up * (1.0f / 64.0f);
+                    gi += NP;
+                    uint64_t e[32];
+#pragma unroll
+                    for (int c = 0; c < 16; c++) {
+                        float f[4];
+#pragma unroll
+                        for (int b = 0; b < 4; b++) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f[b]) : "r"(entry(w[c % U::kWords], b)));
+                        e[2 * c] = pack2(f[0] + f[1], f[0] - f[1]);
+                        e[2 * c + 1] = pack2(f[2] + f[3], f[2] - f[3]);
+                    }
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1)
+#pragma unroll
+                        for (int c = 0; c < 32; c++)
+                            if (!(c & d)) { const uint64_t s = e[c], t = e[c | d]; e[c] = add2(s, t); e[c | d] = sub2(s, t); }
+                    const uint64_t sc2 = pack2(sc, sc);
+#pragma unroll
+                    for (int c = 0; c < 32; c++) {
+                        const uint64_t v = mul2(e[c], sc2);
+                        const __half2 hi = __floats2half2_rn(low2(v), high2(v));
+                        h[c] = *reinterpret_cast<const uint32_t *>(&hi);
+                        // what the halves left, each in one multiply-add of an fp16 with an fp32 (-1 x half + value)
+                        float l0, l1;
+                        asm("{.reg .b16 a, b, m;\n\tmov.b32 {a, b}, %2;\n\tmov.b16 m, 0xBC00;\n\tfma.rn.f32.f16 %0, a, m, %3;\n\tfma.rn.f32.f16 %1, b, m, %4;}"
+                            : "=f"(l0), "=f"(l1) : "r"(h[c]), "f"(low2(v)), "f"(high2(v)));
+                        const __half2 rest = __floats2half2_rn(l0, l1);
+                        lo[c] = *reinterpret_cast<const uint32_t *>(&rest);
+                    }
+                } else if (kPol && !FOLD) {
                     const float sc = __half2float(__ushort_as_half(sr.get(gi, lane))) * up;
                     for (pos += part + 1 == kHalves ? 64u + KB * (NP - 1) : 64u; pos >= a.group; pos -= a.group) gi++;
 #pragma unroll
@@ -592,18 +647,6 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
 #pragma unroll
             for (int c = 0; c < TC; c++)
                 if ((uint32_t)c < cols) stage[c * kRows] = tot[c];
-        } else {
-            wait(bar(kDFull), 0u);
-            __syncwarp();
-            fence_after();
-            for (uint32_t c = 0; c < cols; c += 16) {
-                uint32_t v[16];
-                tmem_ld16(lane_base + c, v);
-                tmem_ld_wait(v);
-#pragma unroll
-                for (int j = 0; j < 16; j++) stage[(c + j) * kRows] = kPol ? __uint_as_float(v[j]) * down : __uint_as_float(v[j]);
-            }
-            fence_before();
         }
     } else if (warp == 4 * NP + 4 * NF) {
         // ---- products.  This warp's instructions are what a block costs when tokens are few: one barrier and one commit a
@@ -722,6 +765,21 @@ qmm_kernel(const QmmArgs a, const __grid_constant__ CUtensorMap wmap, const __gr
         }
     }
     __syncwarp();
+    if (!FOLD && warp < 4 * NP + 4 * NF) {
+        // totals to shared memory, [token][row]: sixteen tokens at a time, the producers' warps among the takers
+        const uint32_t r = (warp & 3u) * 32u + lane;
+        wait(bar(kDFull), 0u);
+        __syncwarp();
+        fence_after();
+        for (uint32_t c = (warp >> 2) * 16u; c < a.T; c += (NP + NF) * 16u) {
+            uint32_t v[16];
+            tmem_ld16(tmem + (((warp & 3u) * 32u) << 16) + c, v);
+            tmem_ld_wait(v);
+#pragma unroll
+            for (int j = 0; j < 16; j++) reinterpret_cast<float *>(smem)[(size_t)(c + j) * kRows + r] = kPol ? __uint_as_float(v[j]) * down : __uint_as_float(v[j]);
+        }
+        fence_before();
+    }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __syncthreads();
     if (wait.stopped()) {                          // the same for all threads: whoever sets the mark does so before the barrier above
@@ -958,8 +1016,8 @@ int run_variant(QmmArgs a, uint32_t most, uint32_t step, const void *packed, uin
 {
     using U = Unit<BITS, KB>;
     auto kern = qmm_kernel<BITS, BF16, FOLD, NP, NF, TC, KB>;
-    constexpr uint32_t threads = (4 * NP + 4 * NF + 4) * 32, a_cols = (BITS == kPolar ? 64u : 32u) * (KB / 64);
-    constexpr bool kPol = BITS == kPolar;
+    constexpr uint32_t threads = (4 * NP + 4 * NF + 4) * 32, a_cols = (BITS == kPolar || BITS == kPolarRot ? 64u : 32u) * (KB / 64);
+    constexpr bool kPol = BITS == kPolar || BITS == kPolarRot;
     const uint32_t rows = (a.N + kRows - 1) / kRows;
     a.units = (a.K + U::kCols - 1) / U::kCols;
     auto placed = [&](uint32_t T) {
@@ -981,7 +1039,7 @@ int run_variant(QmmArgs a, uint32_t most, uint32_t step, const void *packed, uin
         for (uint32_t i = 0; i < std::min(used, 32u); i++) if (keys[i] == key) plan = plans[i];
     }
     if (!plan.T) {
-        const double producers = kPol ? FOLD ? 700.0 : 1100.0 : FOLD ? 450.0 : !BF16 ? 400.0 : BITS == 8 ? 600.0 : 660.0, products = kPol ? 3.0 : a.planes;
+        const double producers = BITS == kPolarRot ? 1250.0 : kPol ? FOLD ? 700.0 : 1100.0 : FOLD ? 450.0 : !BF16 ? 400.0 : BITS == 8 ? 600.0 : 660.0, products = BITS == kPolar ? 3.0 : kPol ? 2.0 : a.planes;
         const double fixed = kPol && !FOLD ? 8000.0 : 4000.0;       // (a row's norms are read first, and tiles are large)
         double best = 1e30;
         const uint32_t least = (a.M + most - 1) / most;
@@ -1056,6 +1114,12 @@ int run_scaled(const QmmArgs &a, const void *packed, uint64_t row_bytes, const v
 // time brought to their range, and a CTA takes 256 tokens: a block costs 1100 cycles whatever the tokens up to some 160, so
 // fewer, larger tiles pay.  14336 x 4096, 64 columns a block, 128 tokens 55 us / 52, 256 tokens 100 / 82.  Both leave 22
 // bits of each factor.
+//   Blocks of 64 columns against 16-bit activations (c.rotate): the producers rotate the weight's blocks in registers, where
+// the other two want rotated activations of two halves each.  The activations are exact then, and a pair takes two
+// products, not three.  What bounds it: instruction slots and the multiply-add pipe of the producers (some 600 instructions a
+// block and warp), then the tensor pipe.  512 tokens against 14336 x 4096 187 -> 139 us, 11008 x 4096 127 -> 94.8 (97.8 before
+// the remainders came from one mixed multiply-add each; look-ups by byte permutes instead of dot products 103), with a third
+// less error (4096 columns, fp32 results: 1.88e-6 -> 1.27e-6).
 constexpr uint32_t kPolarFold = 112;
 
 int qmm(const QmmCall &c, void *stream, double *cycles)
@@ -1074,6 +1138,7 @@ int qmm(const QmmCall &c, void *stream, double *cycles)
     a.entries = c.centroids ? 1u << c.bits : 1u;
     const bool bf = c.bf16 && !c.split_x;
     const uint64_t row_bytes = c.blocked_rows ? (uint64_t)c.blocked_rows * 8 : c.centroids ? c.K : c.bits == 4 ? c.K / 2 : c.bits == 2 ? c.K / 4 : c.K;
+    if (c.rotate) return run_variant<kPolarRot, false, false, 2, 1, 32, 64>(a, 256, 16, c.packed, row_bytes, c.x, st, cycles);
     if (c.centroids && c.M > kPolarFold) return run_variant<kPolar, false, false, 2, 1, 32, 64>(a, 256, 16, c.packed, row_bytes, c.x, st, cycles);
     if (c.centroids) return run_fold<kPolar, false>(a, c.packed, row_bytes, c.x, st, cycles);
     const bool fold = c.split_x || c.M <= 128u;
