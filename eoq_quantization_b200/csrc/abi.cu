@@ -2067,6 +2067,10 @@ extern "C" eoq_error_t eoq_b200_gemv_packed(const uint8_t *d_packed, const uint1
     return product_result(e, "eoq_b200_gemv_packed");
 }
 
+// For the torch-facing front (not in the public header): whether up to eight rows of 16-bit activations are to go to
+// eoq_b200_gemv_packed's tensor-core form.
+extern "C" int eoq_b200_gemv_packed_preferred(uint32_t cols, uint32_t bits, uint32_t group) { return packed_mma_takes(cols, bits, group) ? 1 : 0; }
+
 extern "C" eoq_error_t eoq_b200_linear_packed(const uint8_t *d_packed, const uint16_t *d_scales_fp16, uint32_t rows, uint32_t cols,
                                               uint32_t bits, uint32_t group, const void *x, int x_dtype, uint32_t batch, void *d_scratch,
                                               void *y, int y_dtype, const float *bias, void *stream)

@@ -3131,12 +3131,20 @@ __device__ __forceinline__ void mma_m16n8k16_first(float (&c)[4], uint32_t a0, u
                      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
 }
 
+// (a & b) | c in one instruction: from two immediate operands the compiler makes two, of the half-rate pipe that bounds the kernel
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c)
+{
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
+}
+
 // two codes, already sitting in the low bits of the two halves of v, to two exact signed 16-bit floats
 template <bool BF16>
 __device__ __forceinline__ uint32_t codes_to_pair(uint32_t v, uint32_t mask, uint32_t q)
 {
     const uint32_t magic = BF16 ? 0x43004300u : 0x64006400u;
-    const uint32_t biased = (v & mask) | magic, off = magic | q | (q << 16);
+    const uint32_t biased = and_or(v, mask, magic), off = magic | q | (q << 16);
     uint32_t r;
     if (BF16) asm("sub.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(biased), "r"(off));
     else asm("sub.f16x2 %0, %1, %2;" : "=r"(r) : "r"(biased), "r"(off));
@@ -3149,7 +3157,7 @@ template <bool BF16>
 __device__ __forceinline__ uint32_t scaled_pair(uint32_t v, uint32_t mask, uint32_t mul, uint32_t sub)
 {
     static_assert(!BF16, "a bf16 mantissa has no room above bit 6");
-    const uint32_t biased = (v & mask) | 0x64006400u;
+    const uint32_t biased = and_or(v, mask, 0x64006400u);
     uint32_t r;
     asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(biased), "r"(mul | (mul << 16)), "r"(sub | (sub << 16)));
     return r;
@@ -3209,49 +3217,62 @@ __device__ __forceinline__ void unpack_span(const uint32_t (&w)[BITS], uint32_t 
 // rotation).  Lanes whose activation row does not exist read zeros from a constant block instead of branching.
 __device__ const uint4 kZeroBlock[4] = {};
 
-template <int BITS, bool BF16>
+//
+// U: columns of a unit whose scale is applied on its own, the largest of 128, 64 and 32 that divides a group.  A span stays 128
+// columns; of its 128 / U units a lane takes an equal part of each (32 columns in all), so that a unit's products are a run of
+// the span's, and loads it in pieces of as many bytes as lie together.
+template <int BITS, bool BF16, int U>
 __global__ void __launch_bounds__(BITS == 8 ? 256 : 512, BITS == 8 ? 3 : 2) gemv_packed_mma_kernel(const PackedGemvArgs a)
 {
+    static_assert(BITS != 2 || U >= 64, "a unit of 32 two-bit codes is no whole word of a lane");
+    constexpr int kUnits = 128 / U;                                // of a span
     static_assert(BITS == 2 || BITS == 4 || BITS == 8, "two or four bits packed, or one code per byte");
     constexpr int kRows = 2;                                       // a lane's weight rows: g and g + 8 of the tile
     constexpr int kDepth = 2;                                      // register sets of weights: kDepth - 1 spans requested ahead
     __shared__ float red[kMmaMaxWarps][16][8];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5, g = lane >> 2, t = lane & 3u;
     const uint32_t row0 = blockIdx.x * 16u;
-    const uint32_t sgroups = a.K / a.group, nspans = a.K >> 7, gspans = a.group >> 7;
+    const uint32_t sgroups = a.K / a.group, nspans = a.K >> 7, gunits = a.group / U;
     const uint8_t *pw[kRows];
     const uint16_t *ps[kRows];
 #pragma unroll
     for (int r = 0; r < kRows; r++) {
         const uint32_t row = min(row0 + r * 8u + g, a.N - 1u);
-        pw[r] = a.packed + (size_t)row * a.row_bytes + t * (4u * BITS);
+        pw[r] = a.packed + (size_t)row * a.row_bytes + t * (4u * BITS / kUnits);
         ps[r] = a.scales + (size_t)row * sgroups;
     }
     // a lane's 64 bytes of activation row g per span, or the zero block with no stride where that row does not exist
     const bool has = g < a.batch;
-    const uint16_t *xr = has ? reinterpret_cast<const uint16_t *>(a.x) + (size_t)g * a.K + t * 32u : reinterpret_cast<const uint16_t *>(kZeroBlock);
+    const uint16_t *xr = has ? reinterpret_cast<const uint16_t *>(a.x) + (size_t)g * a.K + t * (U / 4u) : reinterpret_cast<const uint16_t *>(kZeroBlock);
     const uint32_t xstep = has ? 128u : 0u;
     float tot[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 
-    auto load_span = [&](uint32_t s, uint32_t (&w)[kRows][BITS], uint16_t (&sc)[kRows]) {
+    auto load_span = [&](uint32_t s, uint32_t (&w)[kRows][BITS], uint16_t (&sc)[kRows][kUnits]) {
         if (s >= nspans) return;
-        const uint32_t off = s * (16u * BITS), gi = gspans == 1u ? s : s / gspans;
+        constexpr int kWords = BITS / kUnits;                      // of a lane's part of a unit
 #pragma unroll
-        for (int r = 0; r < kRows; r++) {
-            if (BITS == 2) {
-                const uint2 v = __ldg(reinterpret_cast<const uint2 *>(pw[r] + off));
-                w[r][0] = v.x; w[r][1] = v.y;
-            } else {
+        for (int r = 0; r < kRows; r++)
 #pragma unroll
-                for (int h = 0; h < BITS / 4; h++) {
-                    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(pw[r] + off) + h);
-                    w[r][4 * h] = v.x; w[r][4 * h + 1] = v.y; w[r][4 * h + 2] = v.z; w[r][4 * h + 3] = v.w;
+            for (int u = 0; u < kUnits; u++) {
+                const uint8_t *p = pw[r] + s * (16u * BITS) + u * (U * BITS / 8);
+                if constexpr (kWords == 1) {
+                    w[r][u] = __ldg(reinterpret_cast<const uint32_t *>(p));
+                } else if constexpr (kWords == 2) {
+                    const uint2 v = __ldg(reinterpret_cast<const uint2 *>(p));
+                    w[r][2 * u] = v.x; w[r][2 * u + 1] = v.y;
+                } else {
+#pragma unroll
+                    for (int h = 0; h < kWords / 4; h++) {
+                        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p) + h);
+                        uint32_t *d = &w[r][u * kWords + 4 * h];
+                        d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+                    }
                 }
+                const uint32_t at = s * kUnits + u;
+                sc[r][u] = __ldg(ps[r] + (gunits == 1u ? at : at / gunits));
             }
-            sc[r] = __ldg(ps[r] + gi);
-        }
     };
-    auto compute_span = [&](uint32_t s, const uint32_t (&w)[kRows][BITS], const uint16_t (&sc)[kRows]) {
+    auto compute_span = [&](uint32_t s, const uint32_t (&w)[kRows][BITS], const uint16_t (&sc)[kRows][kUnits]) {
         uint32_t h0[16], h1[16];
         unpack_span<BITS, BF16>(w[0], h0);
         unpack_span<BITS, BF16>(w[1], h1);
@@ -3260,7 +3281,8 @@ __global__ void __launch_bounds__(BITS == 8 ? 256 : 512, BITS == 8 ? 3 : 2) gemv
             uint32_t q[16];
 #pragma unroll
             for (int h = 0; h < 4; h++) {
-                const uint4 v = __ldg(reinterpret_cast<const uint4 *>(src) + h);
+                const int unit = h * kUnits / 4;                   // pieces of eight columns, 4 / kUnits a unit
+                const uint4 v = __ldg(reinterpret_cast<const uint4 *>(src + (has ? unit * U : 0)) + (h - unit * 4 / kUnits));
                 q[4 * h] = v.x; q[4 * h + 1] = v.y; q[4 * h + 2] = v.z; q[4 * h + 3] = v.w;
             }
 #pragma unroll
@@ -3277,26 +3299,31 @@ __global__ void __launch_bounds__(BITS == 8 ? 256 : 512, BITS == 8 ? 3 : 2) gemv
             }
         };
         uint32_t xp[16];
-        float c[4], d[4];
         load_xp(xr + s * xstep, xp);
-        // two accumulators: consecutive instructions do not wait for one another
-        mma_m16n8k16_first<BF16>(c, h0[0], h1[0], h0[1], h1[1], xp[0], xp[1]);
-        mma_m16n8k16_first<BF16>(d, h0[2], h1[2], h0[3], h1[3], xp[2], xp[3]);
 #pragma unroll
-        for (int m = 2; m < 8; m += 2) {
-            mma_m16n8k16<BF16>(c, h0[2 * m], h1[2 * m], h0[2 * m + 1], h1[2 * m + 1], xp[2 * m], xp[2 * m + 1]);
-            mma_m16n8k16<BF16>(d, h0[2 * m + 2], h1[2 * m + 2], h0[2 * m + 3], h1[2 * m + 3], xp[2 * m + 2], xp[2 * m + 3]);
+        for (int u = 0; u < kUnits; u++) {
+            constexpr int kProducts = 8 / kUnits;
+            const int f = u * kProducts;
+            float c[4], d[4];
+            // two accumulators: consecutive instructions do not wait for one another
+            mma_m16n8k16_first<BF16>(c, h0[2 * f], h1[2 * f], h0[2 * f + 1], h1[2 * f + 1], xp[2 * f], xp[2 * f + 1]);
+            mma_m16n8k16_first<BF16>(d, h0[2 * f + 2], h1[2 * f + 2], h0[2 * f + 3], h1[2 * f + 3], xp[2 * f + 2], xp[2 * f + 3]);
+#pragma unroll
+            for (int m = f + 2; m < f + kProducts; m += 2) {
+                mma_m16n8k16<BF16>(c, h0[2 * m], h1[2 * m], h0[2 * m + 1], h1[2 * m + 1], xp[2 * m], xp[2 * m + 1]);
+                mma_m16n8k16<BF16>(d, h0[2 * m + 2], h1[2 * m + 2], h0[2 * m + 3], h1[2 * m + 3], xp[2 * m + 2], xp[2 * m + 3]);
+            }
+            const float fa = half_bits_to_float(sc[0][u]), fb = half_bits_to_float(sc[1][u]);
+            tot[0] = fmaf(fa, c[0] + d[0], tot[0]); tot[1] = fmaf(fa, c[1] + d[1], tot[1]);
+            tot[2] = fmaf(fb, c[2] + d[2], tot[2]); tot[3] = fmaf(fb, c[3] + d[3], tot[3]);
         }
-        const float fa = half_bits_to_float(sc[0]), fb = half_bits_to_float(sc[1]);
-        tot[0] = fmaf(fa, c[0] + d[0], tot[0]); tot[1] = fmaf(fa, c[1] + d[1], tot[1]);
-        tot[2] = fmaf(fb, c[2] + d[2], tot[2]); tot[3] = fmaf(fb, c[3] + d[3], tot[3]);
     };
 
     // The weights and scales do not depend on the kernel before this one in the stream, the activations may: the
     // first span's weight loads are in flight before the dependency wait (programmatic dependent launch).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     uint32_t wbuf[kDepth][kRows][BITS];
-    uint16_t sbuf[kDepth][kRows];
+    uint16_t sbuf[kDepth][kRows][kUnits];
 #pragma unroll
     for (int d = 0; d < kDepth - 1; d++) load_span(warp + d * nwarps, wbuf[d], sbuf[d]);
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -3318,6 +3345,16 @@ __global__ void __launch_bounds__(BITS == 8 ? 256 : 512, BITS == 8 ? 3 : 2) gemv
         for (uint32_t w = 0; w < nwarps; w++) v += red[w][r][b];
         if (row < a.N && b < a.batch) store_y(a.y, (size_t)b * a.N + row, v + (a.bias ? __ldg(a.bias + row) : 0.0f), a.y_dtype);
     }
+}
+
+// Whole spans a row, whole units a group.  Against the product kernel, which took groups that are not whole spans before (1 and 8
+// rows, us): four bits in groups of 64, 4096 x 4096 9.2 -> 5.5 and 9.5 -> 5.6, 11008 x 4096 21.5 -> 11.3 and 21.5 -> 12.4, 4096 x
+// 11008 17.2 -> 11.2 and 17.4 -> 11.5; in groups of 32, 11008 x 4096 35.3 -> 16.5 and 35.3 -> 17.8; bytes in groups of 64, 4096 x
+// 4096 9.2 -> 7.1, 11008 x 4096 22.1 -> 13.3, but 4096 x 11008 16.6 -> 16.8 (bf16 17.9 -> 20.4): a few long rows of bytes, whose
+// columns that kernel spreads over more SMs, stay there.
+bool packed_mma_takes(uint32_t K, uint32_t bits, uint32_t group)
+{
+    return K % 128u == 0 && K % group == 0 && group % (bits == 2 ? 64u : 32u) == 0 && (group % 128u == 0 || bits == 4 || bits == 2 || K <= 8192u);
 }
 
 // bits: 2 and 4 as packed by QuantizedLinear (low bits first, code + qmax), anything else one signed code per byte.
@@ -3377,13 +3414,17 @@ static cudaError_t launch_packed_mma(Kern kern, uint32_t max_warps, uint32_t til
 int launch_gemv_packed(const PackedGemvArgs &a, void *stream)
 {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (a.batch <= 8 && a.x_dtype != EOQ_B200_F32 && a.K % 128u == 0 && a.group % 128u == 0 && (reinterpret_cast<uintptr_t>(a.x) & 15u) == 0) {
-        const uint32_t tiles = (a.N + 15u) / 16u, nspans = a.K >> 7;
+    if (packed_mma_takes(a.K, a.bits, a.group) && a.batch <= 8 && a.x_dtype != EOQ_B200_F32 && (reinterpret_cast<uintptr_t>(a.x) & 15u) == 0) {
+        const uint32_t tiles = (a.N + 15u) / 16u, nspans = a.K >> 7, max_warps = a.bits == 4 || a.bits == 2 ? 16u : 8u;
         const bool bf = a.x_dtype == EOQ_B200_BF16;
-        cudaError_t e;
-        if (a.bits == 4) e = bf ? launch_packed_mma(gemv_packed_mma_kernel<4, true>, 16u, tiles, nspans, st, a) : launch_packed_mma(gemv_packed_mma_kernel<4, false>, 16u, tiles, nspans, st, a);
-        else if (a.bits == 2) e = bf ? launch_packed_mma(gemv_packed_mma_kernel<2, true>, 16u, tiles, nspans, st, a) : launch_packed_mma(gemv_packed_mma_kernel<2, false>, 16u, tiles, nspans, st, a);
-        else e = bf ? launch_packed_mma(gemv_packed_mma_kernel<8, true>, 8u, tiles, nspans, st, a) : launch_packed_mma(gemv_packed_mma_kernel<8, false>, 8u, tiles, nspans, st, a);
+        void (*kern)(PackedGemvArgs) = nullptr;
+#define EOQ_PACKED_MMA(B, U) (bf ? gemv_packed_mma_kernel<B, true, U> : gemv_packed_mma_kernel<B, false, U>)
+        const uint32_t unit = a.group % 128u == 0 ? 128u : a.group % 64u == 0 ? 64u : 32u;
+        if (a.bits == 4) kern = unit == 128u ? EOQ_PACKED_MMA(4, 128) : unit == 64u ? EOQ_PACKED_MMA(4, 64) : EOQ_PACKED_MMA(4, 32);
+        else if (a.bits == 2) kern = unit == 128u ? EOQ_PACKED_MMA(2, 128) : EOQ_PACKED_MMA(2, 64);
+        else kern = unit == 128u ? EOQ_PACKED_MMA(8, 128) : unit == 64u ? EOQ_PACKED_MMA(8, 64) : EOQ_PACKED_MMA(8, 32);
+#undef EOQ_PACKED_MMA
+        const cudaError_t e = launch_packed_mma(kern, max_warps, tiles, nspans, st, a);
         g_launches++;
         return (int)e;
     }
