@@ -161,6 +161,22 @@ __device__ __forceinline__ uint32_t rans_step(const uint32_t *tab, uint32_t &x, 
     return e;
 }
 
+// The same step, written out, and the entry as it is.
+__device__ __forceinline__ uint32_t rans_step_entry(uint32_t tab_addr, uint32_t &x, uint32_t mask, uint32_t p, uint32_t bias_mask)
+{
+    uint32_t e;
+    asm("{\n\t.reg .b32 s, q, f, b;\n\t"
+        "and.b32 s, %0, %2;\n\t"
+        "mad.lo.u32 s, s, 4, %3;\n\t"
+        "ld.shared.u32 %1, [s];\n\t"
+        "shr.u32 q, %0, %4;\n\t"
+        "shr.u32 f, %1, 23;\n\t"
+        "and.b32 b, %1, %5;\n\t"
+        "mad.lo.u32 %0, f, q, b;\n\t}"
+        : "+r"(x), "=r"(e) : "r"(mask), "r"(tab_addr), "r"(p), "r"(bias_mask));
+    return e;
+}
+
 // The same step with the INT4 fields of the entry turned into float bit patterns, written out
 // instruction by instruction so that a step is exactly: AND, IMAD (address), LDS, 2 x SHR, AND, IMAD
 // (state), and one LOP3 per field ((e & mask) | exponent, exponent in a register).
@@ -2091,25 +2107,40 @@ __global__ void __launch_bounds__(512, 1) dequant_pairs_kernel(const DecodeArgs 
             for (int half = 0; half < 2; half++) {
                 float v[2][G][8];
                 uint32_t word[2][G];                                 // kPack: eight codes
+                uint32_t run[2][G];                                  // ... of which the last few, not yet in their place
 #pragma unroll
                 for (int k = 0; k < 2; k++)
 #pragma unroll
-                    for (int j = 0; j < G; j++) word[k][j] = 0u;
+                    for (int j = 0; j < G; j++) word[k][j] = run[k][j] = 0u;
 #pragma unroll
                 for (int s = 0; s < 8; s++) {
                     uint32_t u[2][3];
+                    if constexpr (kPack) {
+                        // The half-rate integer pipe bounds this form (55 % of all cycles with a logic instruction, a shift and
+                        // another logic instruction a code).  A code is masked in its field, and multiply-adds, of another pipe,
+                        // line up as many codes above it as the register has room for; such a run is moved to its place at once:
+                        // 11008 x 4096 22.3 -> 17.6 us.
+#pragma unroll
+                        for (int k = 0; k < 2; k++) {
+                            const uint32_t e = rans_step_entry(tab_addr, ch[k].x, mask, p, F::kBiasMask);
+#pragma unroll
+                            for (int j = 0; j < G; j++) {
+                                const int bit = F::field_bit(j), most = (32 - bit) / 4, at = s % most, first = s - at;
+                                const uint32_t code = e & (15u << bit);
+                                run[k][j] = at == 0 ? code : code * (1u << (4 * at)) + run[k][j];
+                                if (at == most - 1 || s == 7) {
+                                    const uint32_t r = run[k][j];
+                                    word[k][j] |= 4 * first >= bit ? r << (4 * first - bit) : r >> (bit - 4 * first);
+                                }
+                            }
+                            staged_renorm(ch[k].x, ch[k].w, ch[k].addr, c64, c1);
+                        }
+                        continue;
+                    }
                     rans_step_int4<F0::kMask, F1::kMask, F2::kMask>(tab_addr, ch[0].x, mask, p, F::kBiasMask, magic0, magic1, magic2, u[0][0], u[0][1], u[0][2]);
                     rans_step_int4<F0::kMask, F1::kMask, F2::kMask>(tab_addr, ch[1].x, mask, p, F::kBiasMask, magic0, magic1, magic2, u[1][0], u[1][1], u[1][2]);
 #pragma unroll
                     for (int k = 0; k < 2; k++) {
-                        if (kPack) {
-#pragma unroll
-                            for (int j = 0; j < G; j++) {
-                                const int bit = F::field_bit(j), to = 4 * s;
-                                word[k][j] |= (to >= bit ? u[k][j] << (to - bit) : u[k][j] >> (bit - to)) & (15u << to);
-                            }
-                            continue;
-                        }
                         v[k][0][s] = (__uint_as_float(u[k][0]) - F0::kOffset) * sc[k][0];
                         v[k][1][s] = (__uint_as_float(u[k][1]) - F1::kOffset) * sc[k][1];
                         v[k][2][s] = (__uint_as_float(u[k][2]) - F2::kOffset) * sc[k][2];
