@@ -216,6 +216,13 @@ class DeviceArena {
         else cudaFree(cur_.p);
         cur_ = Block();
     }
+    // gives the memory back to the device where it is more than `keep`
+    void release_beyond(size_t keep)
+    {
+        if (!cur_.p || cur_.cap <= keep) return;
+        cudaFree(cur_.p);
+        cur_ = Block();
+    }
     uint8_t *base() const { return static_cast<uint8_t *>(cur_.p); }
 
   private:
@@ -1044,6 +1051,8 @@ struct eoq_b200_symbols {
     {
         BesideCapture beside;
         if (stream.get()) cudaStreamSynchronize(stream.get());      // the arenas are another call's from here on
+        sym.release_beyond(256u << 20);                             // a process that encoded a large array once does not keep its scratch
+        work.release_beyond(256u << 20);
         (void)cudaGetLastError();
     }
 };
