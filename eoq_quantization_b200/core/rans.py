@@ -1,6 +1,6 @@
 """Single-stream rANS front end with the interface of the reference's
-``core/rans.py``: table helpers on the host, encoding in the library's host
-encoder, decoding on the GPU."""
+``core/rans.py``: table helpers on the host, encoding in the library (on the
+device where long arrays are staged there, else on the host), decoding on the GPU."""
 from __future__ import annotations
 
 import ctypes as C

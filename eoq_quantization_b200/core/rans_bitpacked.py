@@ -1,5 +1,5 @@
 """Bridge between the absmax quantiser and the rANS coder: interface of the reference's
-``core/rans_bitpacked.py``.  Compression runs in the library's host encoder; decompression
+``core/rans_bitpacked.py``.  Compression runs in the library's encoder; decompression
 decodes on the GPU."""
 from __future__ import annotations
 

@@ -809,6 +809,9 @@ extern "C" void eoq_cuda_batch_destroy(eoq_cuda_batch_ctx_t *ctx)
 // =========================================================================
 
 // Validates a blocked stream on the host, as the reference's decoders do block by block, and makes it a job.
+// Blocks up to which the checks stay on the host: some 9 ns a block, against one more copy, launch and wait, 20 us.
+constexpr uint32_t kHostChecks = 4096;
+
 static eoq_error_t blocked_job(const uint32_t *freq, uint32_t alphabet, uint32_t precision_bits, const uint8_t *data, size_t data_len,
                                const uint32_t *offsets, uint32_t num_blocks, uint32_t block_size, uint32_t num_symbols,
                                int out_elem_bytes, V1Job &job, bool check_on_device = false)
@@ -824,7 +827,8 @@ static eoq_error_t blocked_job(const uint32_t *freq, uint32_t alphabet, uint32_t
     std::vector<uint32_t> f(freq, freq + alphabet), cdf(alphabet + 1, 0);
     for (uint32_t s = 0; s < alphabet; s++) { sum += f[s]; cdf[s + 1] = cdf[s] + f[s]; }
     if (sum != (1ull << precision_bits)) return EOQ_ERR_INVALID_HEADER;
-    // (a look at the first byte of every block of a cold 19 MB stream takes 1.5 ms here, a few microseconds on the device)
+    // (a look at the first byte of each of 176 K blocks of a cold 19 MB stream takes 1.5 ms here, a few microseconds on the device)
+    check_on_device = check_on_device && num_blocks > kHostChecks;
     std::vector<uint32_t> sizes(check_on_device ? 0 : num_blocks);
     for (uint32_t b = 0; b < (uint32_t)sizes.size(); b++) {
         const uint64_t lo = offsets[b], hi = b + 1 < num_blocks ? offsets[b + 1] : data_len;
@@ -958,10 +962,13 @@ extern "C" eoq_error_t eoq_b200_decode_blocked_as(const uint32_t *freq, uint32_t
     V1Job *one = &job;
     DeviceArena arena;
     rc = decode_jobs(&one, 1, st, arena, false);
-    if (rc == EOQ_OK) rc = job_verdict(job, arena, st);
+    // (the checks' outcome is asked for last: waiting for it first would keep the threads of `deliver` from starting under the decoder,
+    // 0.2 ms; a stream that is refused leaves whatever was decoded in `out`)
     if (rc == EOQ_OK) rc = deliver(arena.base() + job.at_out, job.out_elem_bytes, num_symbols, out, out_type, shift, st);
+    if (rc == EOQ_OK && job.raw_offsets) rc = job_verdict(job, arena, st);
+    const cudaError_t e = cudaStreamSynchronize(st);                  // the arena is another call's from here on
     if (rc != EOQ_OK) return rc;
-    CU_TRY(cudaStreamSynchronize(st));
+    CU_TRY(e);
     return EOQ_OK;
 }
 
@@ -1632,15 +1639,20 @@ extern "C" eoq_error_t eoq_b200_weight_from_rans(const uint8_t *c, size_t size, 
     if (sym.acquire(n) != cudaSuccess) return EOQ_ERR_ALLOC;
     if (n) {
         V1Job job;
-        rc = blocked_job(freq.data(), a, p, c + 32 + (size_t)a * 4 + (size_t)nb * 4, dsz, reinterpret_cast<const uint32_t *>(c + 32 + (size_t)a * 4), nb, bs, n, 1,
+        const uint8_t *offsets = c + 32 + (size_t)a * 4;             // of any alignment: read on the host only from a copy
+        std::vector<uint32_t> aligned(nb <= kHostChecks ? nb : 0);
+        if (!aligned.empty()) std::memcpy(aligned.data(), offsets, aligned.size() * 4);
+        rc = blocked_job(freq.data(), a, p, offsets + (size_t)nb * 4, dsz, aligned.empty() ? reinterpret_cast<const uint32_t *>(offsets) : aligned.data(), nb, bs, n, 1,
                          job, true);
         if (rc != EOQ_OK) return rc;
         job.dev_out = sym.base();
         V1Job *one = &job;
         DeviceArena arena;
         rc = decode_jobs(&one, 1, nullptr, arena);
-        if (rc == EOQ_OK) rc = job_verdict(job, arena, nullptr);
-        if (rc != EOQ_OK) { cudaStreamSynchronize(nullptr); return rc; }
+        if (rc == EOQ_OK && job.raw_offsets) rc = job_verdict(job, arena, nullptr);
+        const cudaError_t e = cudaStreamSynchronize(nullptr);
+        if (rc != EOQ_OK) return rc;
+        CU_TRY(e);
     }
     return weight_from_device_symbols(sym.base(), scales_fp16, opts, out);
 }

@@ -470,6 +470,8 @@ eoq_error_t eoq_b200_dequant_packed(const uint8_t *d_packed, const uint16_t *d_s
  * to the remainder; the codes are exact, so the products carry about 2^-22),
  * which one extra small launch writes into d_scratch (batch * cols * 4 bytes,
  * 16-byte aligned, the caller's; NULL: fp32 activations take the general form).
+ * Up to eight 16-bit rows run there with groups that are multiples of 32 (2 bits: of 64)
+ * as well, but for byte codes of more than 8192 columns.
  * More rows than the form in use takes: EOQ_ERR_UNSUPPORTED. */
 eoq_error_t eoq_b200_gemv_packed(const uint8_t *d_packed, const uint16_t *d_scales_fp16, uint32_t rows, uint32_t cols,
                                  uint32_t bits, uint32_t group, const void *x, int x_dtype, uint32_t batch, void *d_scratch,
@@ -487,7 +489,8 @@ eoq_error_t eoq_b200_linear_packed(const uint8_t *d_packed, const uint16_t *d_sc
                                    void *y, int y_dtype, const float *bias, void *stream);
 
 /* The same from PolarLinear's byte codes (see eoq_b200_gemv_polar_codes), any number of activation rows, blocks of 64, 128
- * or 256 columns; rotated activations and centroids as two fp16 halves each.  bias: NULL, fp32 or fp16.  d_scratch:
+ * or 256 columns; rotated activations and centroids as two fp16 halves each, or (many 16-bit rows against blocks of 64)
+ * the activations as they are and the rotated weight as two halves.  bias: NULL, fp32 or fp16.  d_scratch:
  * batch * (cols + 1) * 4 bytes. */
 eoq_error_t eoq_b200_linear_polar_codes(const uint8_t *d_codes, const uint16_t *d_norms_fp16, const float *d_centroids,
                                         uint32_t rows, uint32_t cols, uint32_t bits, uint32_t block, const void *x, int x_dtype,

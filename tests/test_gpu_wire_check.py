@@ -12,21 +12,23 @@ from eoq_quantization_b200.core.rans_blocked import BlockedRANSEncoder, serializ
 from eoq_quantization_b200.fused import EOQWeight
 
 pytestmark = pytest.mark.gpu
-N, K, BLOCK = 96, 512, 256
+N, K = 96, 512
 
 
-def _stream():
+def _stream(block=256):
     sym = np.random.default_rng(3).integers(0, 15, N * K)
-    data = BlockedRANSEncoder(BLOCK, 14).encode(sym, 15)
+    data = BlockedRANSEncoder(block, 14).encode(sym, 15)
     return sym, data
 
 
 @pytest.mark.parametrize("what", ["fine", "order", "past the end", "last past the end", "state longer than the block", "wide state", "both"])
-@pytest.mark.parametrize("at", [0, 7, N * K // BLOCK - 1])
-def test_corrupt_blocks_give_the_hosts_codes(what, at):
-    sym, data = _stream()
+@pytest.mark.parametrize("at", [0, 7, -1])
+@pytest.mark.parametrize("block", [256, 12, 8])                # 192 and 4096 blocks (checked on the host), 6144
+def test_corrupt_blocks_give_the_hosts_codes(what, at, block):
+    sym, data = _stream(block)
     offs, raw = np.array(data.block_offsets, np.uint32), bytearray(data.compressed_blocks)
     nb = len(offs)
+    at = nb - 1 if at < 0 else at
     if what == "order":
         offs[at] = offs[min(at + 1, nb - 1)] + (5 if at + 1 < nb else len(raw))
     elif what == "past the end":
@@ -41,9 +43,9 @@ def test_corrupt_blocks_give_the_hosts_codes(what, at):
             raw[offs[nb // 2]] = 255
     lib, freq = L.lib(), np.ascontiguousarray(_normalize_frequencies(data.freq_table, 14)[0], dtype=np.uint32)
     buf, out = np.frombuffer(bytes(raw), np.uint8), np.zeros(N * K, np.uint8)
-    want = lib.eoq_b200_decode_blocked(freq.ctypes.data, 15, 14, buf.ctypes.data, buf.size, offs.ctypes.data, nb, BLOCK, N * K, out.ctypes.data, 1, 0, None)
+    want = lib.eoq_b200_decode_blocked(freq.ctypes.data, 15, 14, buf.ctypes.data, buf.size, offs.ctypes.data, nb, block, N * K, out.ctypes.data, 1, 0, None)
     assert (want == L.EOQ_OK) == (what == "fine")
-    got = L.native().decode_symbols(freq, 14, bytes(raw), offs, BLOCK, np.zeros(N * K, np.int64), 6, 0)
+    got = L.native().decode_symbols(freq, 14, bytes(raw), offs, block, np.zeros(N * K, np.int64), 6, 0)
     assert (0 if got is None else got) == want
     # the container, at an address off every boundary
     data.compressed_blocks, data.block_offsets = bytes(raw), offs.tolist()
