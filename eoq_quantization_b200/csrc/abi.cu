@@ -319,6 +319,39 @@ cudaError_t upload_filled(PinnedBlock &pinned, void *dst, size_t bytes, cudaStre
     return e != cudaSuccess ? e : last;
 }
 
+// `bytes` of pageable host memory to the device by several threads, each through two chunks of its own.  The source has been
+// read when this returns.  For decodes whose symbols threads deliver to the host afterwards (a 7 MB container: 0.1 to 0.2 ms less
+// in all than behind one copy by the driver); streams that stay on the device go by the driver's.
+cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t st)
+{
+    const size_t chunks = (bytes + kPinnedChunk - 1) / kPinnedChunk, hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t threads = std::min<size_t>({kPinnedThreads / 2, hw, chunks / 4});
+    PinnedBlock pinned;
+    if (threads < 2 || !pinned.acquire()) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    std::atomic<int> failed{(int)cudaSuccess};
+    parallel_for(threads, [&](size_t t) {
+        cudaEvent_t free_again[2] = {nullptr, nullptr};
+        cudaError_t r = cudaSetDevice(device);
+        for (cudaEvent_t &ev : free_again) if (r == cudaSuccess) r = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        int slot = 0;
+        for (size_t c = t; r == cudaSuccess && c < chunks; c += threads, slot ^= 1) {
+            const size_t lo = c * kPinnedChunk, cnt = std::min(kPinnedChunk, bytes - lo);
+            r = cudaEventSynchronize(free_again[slot]);              // never recorded: complete
+            if (r != cudaSuccess) break;
+            std::memcpy(pinned.chunk(2 * t + slot), static_cast<const uint8_t *>(src) + lo, cnt);
+            r = cudaMemcpyAsync(static_cast<uint8_t *>(dst) + lo, pinned.chunk(2 * t + slot), cnt, cudaMemcpyHostToDevice, st);
+            if (r == cudaSuccess) r = cudaEventRecord(free_again[slot], st);
+        }
+        for (cudaEvent_t ev : free_again)
+            if (ev) { cudaEventSynchronize(ev); cudaEventDestroy(ev); }      // the staging memory is another call's from here on
+        if (r != cudaSuccess) failed.store((int)r);
+    }, threads);
+    return (cudaError_t)failed.load();
+}
+
 // One tensor of a decode call.
 struct V1Job {
     Payload pl;                         // validated host views of the payload
@@ -424,7 +457,7 @@ eoq_error_t decode_jobs(V1Job **jobs, size_t n, cudaStream_t st, DeviceArena &ar
     CU_TRY(cudaMemcpyAsync(d, blob.data(), meta, cudaMemcpyHostToDevice, st));
     for (size_t i = 0; i < n; i++) {
         V1Job &j = *jobs[i];
-        if (j.pl.stream_bytes) CU_TRY(cudaMemcpyAsync(d + j.at_stream, j.pl.stream, j.pl.stream_bytes, cudaMemcpyHostToDevice, st));
+        if (j.pl.stream_bytes) CU_TRY(j.dev_out ? cudaMemcpyAsync(d + j.at_stream, j.pl.stream, j.pl.stream_bytes, cudaMemcpyHostToDevice, st) : upload(d + j.at_stream, j.pl.stream, j.pl.stream_bytes, st));
         if (j.raw_offsets) {
             CU_TRY(cudaMemcpyAsync(d + j.at_raw, j.raw_offsets, (size_t)j.pl.nblocks * 4, cudaMemcpyHostToDevice, st));
             if (launch_v1_check(d + j.at_stream, j.pl.stream_bytes, reinterpret_cast<const uint32_t *>(d + j.at_raw), j.pl.nblocks,
