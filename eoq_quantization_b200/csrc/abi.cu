@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <memory>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <unistd.h>
 
@@ -297,7 +298,11 @@ cudaError_t upload_filled(PinnedBlock &pinned, void *dst, size_t bytes, cudaStre
         }
     };
     std::vector<std::thread> pool;
-    if (threads > 1) for (size_t t = 0; t < threads; t++) pool.emplace_back(work);
+    pool.reserve(threads);
+    if (threads > 1 && e == cudaSuccess) {
+        // (where the system gives no more threads, those that there are fill, or this one)
+        try { for (size_t t = 0; t < threads; t++) pool.emplace_back(work); } catch (const std::system_error &) {}
+    }
     for (size_t c = 0; e == cudaSuccess && c < chunks; c++) {
         if (pool.empty()) filled[c].store(fill(c * kPinnedChunk, size_of(c), pinned.chunk(c % kSlots)) ? 1 : -1, std::memory_order_relaxed);
         int f;

@@ -45,6 +45,11 @@ def test_what_is_not_staged_and_calls_beside_a_recording():
     assert R.stage_symbols(sym, 15)[0] is None and R.stage_symbols(sym, 15, 0, True)[0] is not None
     with pytest.raises(ValueError, match="got range"):
         BlockedRANSEncoder().encode(sym, 15)
+    # bytes go up as they are and are looked at there
+    low = np.zeros(70001, np.int8)
+    low[70000], low[3] = 20, -9
+    assert R.stage_symbols(low, 15)[0] is None
+    assert R.stage_symbols(low, 15, 7, True)[1].tolist() == R.count_symbols(low, 15, 7, True)[0].tolist()
     sym = np.random.default_rng(0).integers(0, 15, 1 << 17)
     want = BlockedRANSEncoder().encode(sym, 15).compressed_blocks
     x, graph = torch.ones(8, device="cuda"), torch.cuda.CUDAGraph()
