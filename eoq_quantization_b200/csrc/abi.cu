@@ -847,7 +847,8 @@ extern "C" void eoq_cuda_batch_destroy(eoq_cuda_batch_ctx_t *ctx)
 // =========================================================================
 
 // Validates a blocked stream on the host, as the reference's decoders do block by block, and makes it a job.
-// Blocks up to which the checks stay on the host: some 9 ns a block, against one more copy, launch and wait, 20 us.
+// Blocks up to which the checks stay on the host: some 5 ns a block, against one more copy, launch and wait, some 14 us. Decodes
+// to int8 of blocks of 256, host's checks and device's: 2048 blocks 180 and 192 us, 5154 347 and 314, 65536 2111 and 1806.
 constexpr uint32_t kHostChecks = 4096;
 
 static eoq_error_t blocked_job(const uint32_t *freq, uint32_t alphabet, uint32_t precision_bits, const uint8_t *data, size_t data_len,
