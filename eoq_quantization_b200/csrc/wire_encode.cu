@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(1024) wire_scan_kernel(const uint32_t *__restr
 // [1 B state length][state, big-endian][bytes] of every block to its place, a warp a block.
 __global__ void __launch_bounds__(256) wire_gather_kernel(const WireEncodeArgs a, const uint32_t *__restrict__ offsets, uint8_t *__restrict__ out)
 {
-    const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    const uint32_t b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31u;      // (threads of all blocks can be more than 2^32)
     if (b >= a.nblocks) return;
     const uint4 r = a.record[b];
     const uint32_t *words = a.scratch + (size_t)(b >> 5) * 32u * a.words + (b & 31u);

@@ -1,9 +1,12 @@
 """The wire format's encoder on the device gives the host encoder's bytes: symbol types and alphabets on either side of a byte,
 blocks that end off every boundary, tables from a few slots to 2^16, arrays around the length that is staged."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
+from eoq_quantization_b200 import _lib as L
 from eoq_quantization_b200.core import rans as R
 from eoq_quantization_b200.core.rans_blocked import BlockedRANSDecoder, BlockedRANSEncoder
 from oracle import oracle as O
@@ -59,3 +62,31 @@ def test_what_is_not_staged_and_calls_beside_a_recording():
         y = y * 2
     graph.replay()
     assert got == want and y.tolist() == [4.0] * 8
+
+
+def test_more_than_two_to_the_27_blocks():
+    torch.zeros(1, device="cuda")
+    n = (1 << 27) + 77
+    sym, lib = np.ones(n, np.uint8), L.lib()
+    sym[:1000] = 0
+    freq = np.array([100, 156], np.uint32)
+    lib.eoq_b200_symbols_stage.restype, lib.eoq_b200_symbols_stage.argtypes = C.c_void_p, [C.c_void_p, C.c_int, C.c_size_t, C.c_int64, C.c_int, C.c_uint32]
+    s = C.c_void_p(lib.eoq_b200_symbols_stage(sym.ctypes.data, R._ELEMENTS[sym.dtype], n, 0, 0, 2))
+    assert s.value
+    counts, size, want = np.zeros(2, np.uint64), C.c_size_t(), C.c_size_t()
+    try:
+        assert lib.eoq_b200_symbols_count(s, C.c_void_p(counts.ctypes.data)) == L.EOQ_OK and counts.tolist() == [1000, n - 1000]
+        assert lib.eoq_b200_symbols_encode(s, C.c_void_p(freq.ctypes.data), 2, 8, 1, C.byref(size)) == L.EOQ_OK
+        got, at = np.zeros(size.value, np.uint8), np.zeros(n, np.uint32)
+        assert lib.eoq_b200_symbols_fetch(s, C.c_void_p(got.ctypes.data), C.c_void_p(at.ctypes.data)) == L.EOQ_OK
+    finally:
+        lib.eoq_b200_symbols_free(s)
+    # every block is one symbol: a zero's bytes, then a one's for all the others
+    h = C.c_void_p()
+    assert lib.eoq_b200_wire_encode(sym[999:].ctypes.data, R._ELEMENTS[sym.dtype], 2, 0, 0, freq.ctypes.data, 2, 8, 1, C.byref(h), C.byref(want)) == L.EOQ_OK
+    pair, offs = np.zeros(want.value, np.uint8), np.zeros(2, np.uint32)
+    lib.eoq_b200_wire_take(h, pair.ctypes.data, offs.ctypes.data)
+    zero, one = pair[:offs[1]], pair[offs[1]:]
+    assert np.array_equal(at, np.where(np.arange(n) < 1000, np.arange(n) * len(zero), 1000 * len(zero) + (np.arange(n) - 1000) * len(one)))
+    assert np.array_equal(got[:1000 * len(zero)].reshape(1000, -1), np.tile(zero, (1000, 1)))
+    assert (got[1000 * len(zero):].reshape(-1, len(one)) == one).all()
