@@ -2106,7 +2106,7 @@ extern "C" eoq_error_t eoq_b200_gemv_packed(const uint8_t *d_packed, const uint1
     const uint32_t per16 = bits == 4 ? 32u : bits == 2 ? 64u : 16u;
     if (cols % per16 || group % 8u || cols % group || (reinterpret_cast<uintptr_t>(d_packed) & 15u)) return EOQ_ERR_UNSUPPORTED;
     const bool f32 = x_dtype == EOQ_B200_F32;
-    // rows of the tensor-core forms: 32 where a group is whole 128-column spans, 8 otherwise
+    // rows: 32 where a group is whole 128-column spans and the product kernel may take them, 8 otherwise
     const bool wide = cols % 128u == 0 && group % 128u == 0 &&
                       (f32 ? d_scratch && (reinterpret_cast<uintptr_t>(d_scratch) & 15u) == 0 : (reinterpret_cast<uintptr_t>(x) & 15u) == 0);
     if (batch > (wide ? 32u : 8u)) return EOQ_ERR_UNSUPPORTED;
@@ -2129,7 +2129,7 @@ extern "C" eoq_error_t eoq_b200_gemv_packed(const uint8_t *d_packed, const uint1
 
 // For the torch-facing front (not in the public header): whether up to eight rows of 16-bit activations are to go to
 // eoq_b200_gemv_packed's tensor-core form.
-extern "C" int eoq_b200_gemv_packed_preferred(uint32_t cols, uint32_t bits, uint32_t group) { return packed_mma_takes(cols, bits, group) ? 1 : 0; }
+extern "C" int eoq_b200_gemv_packed_preferred(uint32_t rows, uint32_t cols, uint32_t bits, uint32_t group) { return group && packed_mma_preferred(rows, cols, bits, group) ? 1 : 0; }
 
 extern "C" eoq_error_t eoq_b200_linear_packed(const uint8_t *d_packed, const uint16_t *d_scales_fp16, uint32_t rows, uint32_t cols,
                                               uint32_t bits, uint32_t group, const void *x, int x_dtype, uint32_t batch, void *d_scratch,

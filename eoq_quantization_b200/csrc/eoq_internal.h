@@ -260,6 +260,7 @@ void set_packed_warps(int v);
 void set_dequant_vec(int v);
 int launch_gemv_packed(const PackedGemvArgs &a, void *stream);
 bool packed_mma_takes(uint32_t K, uint32_t bits, uint32_t group);      // whether its tensor-core form takes the weight
+bool packed_mma_preferred(uint32_t N, uint32_t K, uint32_t bits, uint32_t group);      // ... and is quicker than the product kernel
 int launch_dequant_packed(const uint8_t *packed, const uint16_t *scales, uint32_t K, uint32_t row_bytes, uint32_t bits,
                           uint32_t group, uint32_t row_lo, uint32_t row_hi, void *out, int out_dtype, void *stream);
 // Activations x quantised weights on the tensor cores (qmm.cu).  x: [M][K] of 16-bit values, or with split_x two fp16

@@ -3378,21 +3378,35 @@ __global__ void __launch_bounds__(BITS == 8 ? 256 : 512, BITS == 8 ? 3 : 2) gemv
     }
 }
 
-// Whole spans a row, whole units a group.  Against the product kernel, which took groups that are not whole spans before (1 and 8
-// rows, us): four bits in groups of 64, 4096 x 4096 9.2 -> 5.5 and 9.5 -> 5.6, 11008 x 4096 21.5 -> 11.3 and 21.5 -> 12.4, 4096 x
-// 11008 17.2 -> 11.2 and 17.4 -> 11.5; in groups of 32, 11008 x 4096 35.3 -> 16.5 and 35.3 -> 17.8; bytes in groups of 64, 4096 x
-// 4096 9.2 -> 7.1, 11008 x 4096 22.1 -> 13.3, but 4096 x 11008 16.6 -> 16.8 (bf16 17.9 -> 20.4): a few long rows of bytes, whose
-// columns that kernel spreads over more SMs, stay there.
+// Whole spans a row, whole units a group; byte codes in groups that are not whole spans up to 8192 columns.
 bool packed_mma_takes(uint32_t K, uint32_t bits, uint32_t group)
 {
     return K % 128u == 0 && K % group == 0 && group % (bits == 2 ? 64u : 32u) == 0 && (group % 128u == 0 || bits == 4 || bits == 2 || K <= 8192u);
 }
 
+// Against the product kernel, for groups that are not whole spans (us at one fp16 row, this kernel / that one, a different weight
+// in every launch).  A CTA here goes over all columns of sixteen rows, that one spreads a few row tiles' columns over many SMs, so few
+// rows of many columns are its: groups of 64, bytes 512 x 2048 2.7 / 3.7, 512 x 5120 6.2 / 5.0, 2048 x 8192 13.4 / 10.2, 3072 x 4096 7.5 /
+// 8.4, 4096 x 8192 14.1 / 14.3 (bf16 17.8 / 15.0), 5120 x 8192 14.3 / 17.9; four bits 1024 x 6144 6.4 / 6.4, 1024 x 11008 11.9 / 9.5, 2048 x
+// 11008 12.0 / 12.1, 2048 x 28672 29.3 / 26.8, 3072 x 28672 30.3 / 32.9; two bits 1024 x 14336 13.7 / 10.4.  Groups of 32 cross in
+// the same places.  Not its although it is a little quicker there: calls so short that its launch on the host takes longer (bytes 512 x
+// 4096 4.9 / 4.5, launched one by one 6.5 / 7.3), and weights that it only wins from HBM (two bits 1024 x 11008 10.2 / 9.6, from the L2 9.0 /
+// 9.6; bytes 14336 x 5120 24.3 / 23.8, 19.3 / 23.2).
+bool packed_mma_preferred(uint32_t N, uint32_t K, uint32_t bits, uint32_t group)
+{
+    if (!packed_mma_takes(K, bits, group)) return false;
+    if (group % 128u == 0) return true;
+    if (bits == 4 || bits == 2) {       // the crossing moves up between 1536 and 2048 rows, to 11008 columns (two bits: 14336)
+        const uint32_t more = N > 1536u ? N - 1536u : 0u;
+        return N > 2048u || K <= (bits == 4 ? 6144u + more * 19u / 2u : 11008u + more * 13u / 2u);
+    }
+    return N > 4096u || K <= 3072u || (K <= 4096u && (N <= 1024u || N >= 3072u));
+}
+
 // bits: 2 and 4 as packed by QuantizedLinear (low bits first, code + qmax), anything else one signed code per byte.
 // K a multiple of the group and of the columns in sixteen bytes (32 nibbles, 64 two-bit codes, 16 bytes), the group a
 // multiple of 8, packed rows 16-byte aligned: checked by the caller.
-// Up to eight activation rows; the tensor-core form for 16-bit ones, 16-byte aligned, against scale groups of whole
-// 128-column spans.
+// Up to eight activation rows; the tensor-core form for 16-bit ones, 16-byte aligned, where packed_mma_takes has the weight.
 static std::atomic<int> g_packed_warps{0};              // 0 = by shape; "packed_warps" in eoq_b200_tune
 void set_packed_warps(int v) { g_packed_warps.store(v >= 1 && v <= 16 ? v : 0); }
 

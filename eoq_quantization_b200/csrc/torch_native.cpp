@@ -43,7 +43,7 @@ extern "C" eoq_error_t eoq_b200_symbols_encode(eoq_b200_symbols *s, const uint32
 extern "C" eoq_error_t eoq_b200_symbols_fetch(eoq_b200_symbols *s, uint8_t *data, uint32_t *offsets);
 extern "C" void eoq_b200_symbols_free(eoq_b200_symbols *s);
 extern "C" int eoq_b200_ordered_launches(int on);
-extern "C" int eoq_b200_gemv_packed_preferred(uint32_t cols, uint32_t bits, uint32_t group);
+extern "C" int eoq_b200_gemv_packed_preferred(uint32_t rows, uint32_t cols, uint32_t bits, uint32_t group);
 extern "C" int eoq_b200_weight_linear_preferred(const eoq_b200_weight_t *w, const void *x, int x_dtype, uint32_t batch);
 
 namespace {
@@ -280,8 +280,8 @@ PyObject *weight_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
 }
 
 // packed_linear(packed, scales, N, K, bits, group, x, bias): QuantizedLinear.forward.  Up to eight rows of 16-bit
-// activations against rows of whole 128-column spans by the warp-level tensor-core GEMV, otherwise by the tcgen05 kernel
-// where it takes the shape and is the quicker one, else by a dequantised copy and a library GEMM.
+// activations against rows of whole 128-column spans by the warp-level tensor-core GEMV where it is quicker than the tcgen05
+// kernel, otherwise by that where it takes the shape and is the quicker one, else by a dequantised copy and a library GEMM.
 PyObject *packed_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     if (n != 8) { PyErr_SetString(PyExc_TypeError, "packed_linear takes 8 arguments"); return nullptr; }
@@ -307,7 +307,7 @@ PyObject *packed_linear(PyObject *, PyObject *const *a, Py_ssize_t n)
     const uint8_t *codes = static_cast<const uint8_t *>(pk->data_ptr());
     const uint16_t *scales = static_cast<const uint16_t *>(sc.t->data_ptr());
     const bool f32 = code == EOQ_B200_F32, aligned = (reinterpret_cast<uintptr_t>(codes) & 15u) == 0;
-    if (rows <= 8 && !f32 && aligned && K % group == 0 && eoq_b200_gemv_packed_preferred((uint32_t)K, (uint32_t)bits, (uint32_t)group)) {
+    if (rows <= 8 && !f32 && aligned && K % group == 0 && eoq_b200_gemv_packed_preferred((uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)group)) {
         Tensor y = result(*x, N, x->scalar_type());
         return done(eoq_b200_gemv_packed(codes, scales, (uint32_t)N, (uint32_t)K, (uint32_t)bits, (uint32_t)group, x->data_ptr(), code,
                                          (uint32_t)rows, nullptr, y.data_ptr(), code, b, st),
