@@ -2168,8 +2168,16 @@ extern "C" int eoq_b200_linear_packed_preferred(const uint8_t *d_packed, uint32_
 // Above 64 rows, and above 32 against weights of which several CTAs share the columns anyway (from 8192 rows on a block of 64
 // columns costs some 1300 cycles when rotated, 900 to 1500 when not, by the rows).  14336 x 4096 has not been split, so it goes like
 // 11008 x 4096: 64 rows 42.0 us / rotated 45.6, 80 rows 48.4 / 46.3, 512 rows 127 / 94.8; 4096 x 4096, 40 rows 16.9 / 16.6, 200
-// rows 30.2 / 21.2; 1024 x 4096, 40 rows 12.0 / 9.0.
-static bool polar_rotates(uint32_t rows, uint32_t batch) { return batch > 64u || (batch > 32u && rows <= 8192u); }
+// rows 30.2 / 21.2; 1024 x 4096, 40 rows 12.0 / 9.0.  But not 113 to 128 rows (the other form's tile of 128 tokens, without its folds)
+// where row tiles are many and long, 12288 x 4096 45.3 / 47.1, 14336 x 8192 94.1 / 97.6, 28672 x 8192 176 / 211 (11008 x 8192 86.2 / 84.1, 14336 x 2048
+// 26.2 / 25.5, 18944 x 8192 101.0 / 101.5), and up to 144 where they are most, 28672 x 4096 101.8 / 104.4, 28672 x 8192 186 / 215 (24576 x 8192 161.7 /
+// 162.8, 20480 x 8192 154.1 / 156.1, 18944 x 8192 106.3 / 102.4, 28672 x 11008 253 / 243).
+static bool polar_rotates(uint32_t rows, uint32_t cols, uint32_t batch)
+{
+    if (batch > 112u && cols >= 4096u && (batch <= 128u ? rows >= 12288u : batch <= 144u && rows > 24576u && cols <= 8192u)) return false;
+    return batch > 64u || (batch > 32u && rows <= 8192u);
+}
+extern "C" int eoq_b200_polar_rotates(uint32_t rows, uint32_t cols, uint32_t batch) { return polar_rotates(rows, cols, batch) ? 1 : 0; }      // (for the tests)
 
 extern "C" eoq_error_t eoq_b200_linear_polar_codes(const uint8_t *d_codes, const uint16_t *d_norms_fp16, const float *d_centroids,
                                                    uint32_t rows, uint32_t cols, uint32_t bits, uint32_t block, const void *x, int x_dtype,
@@ -2190,7 +2198,7 @@ extern "C" eoq_error_t eoq_b200_linear_polar_codes(const uint8_t *d_codes, const
     c.N = rows; c.K = cols; c.M = batch; c.bits = bits; c.group = block; c.split_x = 1; c.y_dtype = y_dtype;
     // many 16-bit rows against blocks of 64: the weight is rotated on its way to the products instead of the activations, which
     // then are one fp16 plane (bf16 ones brought to fp16's range a row at a time) and need two products of a pair, not three
-    c.rotate = block == 64 && polar_rotates(rows, batch) && x_dtype != EOQ_B200_F32 && (x_dtype != EOQ_B200_F16 || (reinterpret_cast<uintptr_t>(x) & 15u) == 0);
+    c.rotate = block == 64 && polar_rotates(rows, cols, batch) && x_dtype != EOQ_B200_F32 && (x_dtype != EOQ_B200_F16 || (reinterpret_cast<uintptr_t>(x) & 15u) == 0);
     if (c.rotate) c.split_x = 0;
     if (c.rotate && x_dtype == EOQ_B200_F16) { c.x = x; c.tok_scale = nullptr; }
     int e = 0;

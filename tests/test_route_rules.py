@@ -23,3 +23,10 @@ def _rule(name, n):
     (8, 128, 512, 28672, 1), (4, 256, 256, 28672, 1), (8, 64, 11008, 8320, 0), (2, 32, 4096, 4096, 0), (4, 48, 4096, 4608, 0), (4, 64, 4096, 4160, 0)])
 def test_a_few_rows_of_16_bit_activations(bits, group, n, k, warp_level):
     assert _rule("eoq_b200_gemv_packed_preferred", 4)(n, k, bits, group) == warp_level
+
+
+@pytest.mark.parametrize("n,k,rows,rotated", [
+    (8192, 4096, 32, 0), (8192, 4096, 33, 1), (8193, 4096, 64, 0), (8193, 4096, 65, 1), (28672, 8192, 112, 1), (12288, 4096, 113, 0), (12288, 4096, 128, 0),
+    (12288, 4096, 129, 1), (11008, 8192, 128, 1), (14336, 2048, 128, 1), (28672, 8192, 144, 0), (28672, 8192, 145, 1), (20480, 8192, 144, 1), (28672, 11008, 144, 1)])
+def test_polar_rows_that_rotate_the_weight(n, k, rows, rotated):
+    assert _rule("eoq_b200_polar_rotates", 3)(n, k, rows) == rotated
