@@ -32,12 +32,13 @@ def count_symbols(symbols: np.ndarray, alphabet_size: int, shift: int = 0, clamp
     return np.array(counts, dtype=np.int64), lo, hi
 
 
-def stage_symbols(symbols: np.ndarray, alphabet_size: int, shift: int = 0, clamp: bool = False):
+def stage_symbols(symbols: np.ndarray, alphabet_size: int, shift: int = 0, clamp: bool = False, block_size: int = 0):
     """(staged, int64 counts): the array on the device, counted there, to be handed to `encode_blocks` or `encode_container`
-    beside it; or (None, None) where the host counts and encodes (short arrays, no device in use, symbols outside the alphabet)."""
+    beside it; or (None, None) where the host counts and encodes (short arrays, few long blocks where `block_size` is given, no
+    device in use, symbols outside the alphabet)."""
     if not readable(symbols) or not 0 < alphabet_size <= 4096:
         return None, None
-    got = _lib.native().stage_symbols(symbols, _ELEMENTS[symbols.dtype], shift, int(clamp), alphabet_size)
+    got = _lib.native().stage_symbols(symbols, _ELEMENTS[symbols.dtype], shift, int(clamp), alphabet_size, block_size)
     return (None, None) if got is None else (got[0], np.array(got[1], dtype=np.int64))
 
 

@@ -42,7 +42,7 @@ def compress_tensor_rans(name: str, codes: torch.Tensor, scales: torch.Tensor, b
     alphabet = 2 * qmax + 1
     block, precision = 256, 14
     # counted and encoded where they lie, code + qmax clipped to the alphabet on the way
-    staged, counts = stage_symbols(flat, alphabet, qmax, True) if n else (None, np.zeros(alphabet, np.int64))
+    staged, counts = stage_symbols(flat, alphabet, qmax, True, block) if n else (None, np.zeros(alphabet, np.int64))
     if n and staged is None:
         counts = count_symbols(flat, alphabet, qmax, True)[0]
     enc = RANSEncoder(counts, precision_bits=precision)

@@ -52,7 +52,7 @@ class BlockedRANSEncoder:
     def encode(self, symbols: np.ndarray, alphabet_size: int) -> BlockedRANSData:
         symbols = np.asarray(symbols).ravel()
         n = len(symbols)
-        staged, freq = stage_symbols(symbols, alphabet_size)
+        staged, freq = stage_symbols(symbols, alphabet_size, block_size=self.block_size)
         if staged is None:
             freq = compute_frequency_table(symbols, alphabet_size)
         enc = RANSEncoder(freq, precision_bits=self.precision_bits)

@@ -1014,12 +1014,19 @@ extern "C" eoq_error_t eoq_b200_decode_blocked_as(const uint32_t *freq, uint32_t
 // -- symbols of a host array staged on the device, counted and encoded there (for the torch-facing front; not in the public header) --
 //
 // Used where the process has a context on the device already (encoding alone makes none), the array is long enough for the
-// copies to be worth it (64 Ki symbols: 0.33 ms on the host's threads, 0.1 here) and the alphabet fits shared memory.  On a
+// copies to be worth it (64 Ki symbols in blocks of 256, the whole call: 0.22 ms on the host's sixteen cores, 0.16 here), its blocks are short
+// enough (eoq_b200_symbols_preferred) and the alphabet fits shared memory.  On a
 // stream of its own: whatever else is under way on the device is not waited for.  Nothing is accepted or refused here that
 // the host encoder does not accept or refuse: what this one does not take, an array with symbols outside the alphabet among it, goes there.
 namespace {
 
 constexpr size_t kStageSymbols = 1u << 16;
+
+// A block is one chain, 0.073 us a symbol, while what the device saves with short chains grows as about n^(2/3): 0.03 ms x
+// (n / 32 Ki)^(2/3).  Whole calls, device / host's sixteen cores, us, fifteen symbols: 64 Ki symbols in blocks of 512 199 / 221, 1024
+// 235 / 220, in one 4820 / 390; 256 Ki in blocks of 1024 222 / 390, 4096 470 / 430; 1 Mi in blocks of 4096 546 / 789, 16384 1540 / 900, in one
+// 75600 / 5240; 4 Mi in blocks of 4096 895 / 1650, 16384 2110 / 1740; 16 Mi in blocks of 16384 3280 / 4750, 65536 7090 / 6300.
+bool chains_are_short(double n, double block) { const double b = std::min(n, block); return 16.0 * b * b * b <= n * n; }
 
 bool context_is_active(int dev)
 {
@@ -1104,6 +1111,9 @@ struct eoq_b200_symbols {
 };
 
 extern "C" void eoq_b200_symbols_free(eoq_b200_symbols *s) { delete s; }
+
+// Whether n symbols in blocks of `block` are encoded sooner on the device than on the host's cores.
+extern "C" int eoq_b200_symbols_preferred(size_t n, uint64_t block) { return n >= kStageSymbols && chains_are_short((double)n, (double)block) ? 1 : 0; }
 
 // The staged array, or null: the host encodes.
 extern "C" eoq_b200_symbols *eoq_b200_symbols_stage(const void *symbols, int elem, size_t n, int64_t shift, int clamp, uint32_t alphabet)

@@ -37,6 +37,7 @@
 extern "C" int eoq_b200_linear_packed_preferred(const uint8_t *d_packed, uint32_t rows, uint32_t cols, uint32_t bits, uint32_t group,
                                                 const void *x, int x_dtype, uint32_t batch);
 struct eoq_b200_symbols;
+extern "C" int eoq_b200_symbols_preferred(size_t n, uint64_t block);
 extern "C" eoq_b200_symbols *eoq_b200_symbols_stage(const void *symbols, int elem, size_t n, int64_t shift, int clamp, uint32_t alphabet);
 extern "C" eoq_error_t eoq_b200_symbols_count(eoq_b200_symbols *s, uint64_t *counts);
 extern "C" eoq_error_t eoq_b200_symbols_encode(eoq_b200_symbols *s, const uint32_t *freq, uint32_t alphabet, uint32_t p, uint32_t block, size_t *bytes);
@@ -429,23 +430,24 @@ constexpr const char *kStaged = "eoq_b200.symbols";
 
 void free_staged(PyObject *c) { eoq_b200_symbols_free(static_cast<eoq_b200_symbols *>(PyCapsule_GetPointer(c, kStaged))); }
 
-// stage_symbols(array, type, shift, clamp, alphabet) -> (staged, [counts]): the array on the device, for one encode_symbols call
-// in front of which it is counted there; or None: count_symbols and encode_symbols take the array.
+// stage_symbols(array, type, shift, clamp, alphabet, block size or 0) -> (staged, [counts]): the array on the device, for one
+// encode_symbols call in front of which it is counted there; or None: count_symbols and encode_symbols take the array.
 PyObject *stage_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
-    if (n != 5) { PyErr_SetString(PyExc_TypeError, "stage_symbols takes 5 arguments"); return nullptr; }
+    if (n != 6) { PyErr_SetString(PyExc_TypeError, "stage_symbols takes 6 arguments"); return nullptr; }
     GUARD_BEGIN
     Buffer sym(a[0]);
     if (!sym.ok) return nullptr;
     const int type = (int)PyLong_AsLong(a[1]), clamp = (int)PyLong_AsLong(a[3]);
-    const int64_t shift = PyLong_AsLongLong(a[2]), alphabet = PyLong_AsLongLong(a[4]);
+    const int64_t shift = PyLong_AsLongLong(a[2]), alphabet = PyLong_AsLongLong(a[4]), block = PyLong_AsLongLong(a[5]);
     if (PyErr_Occurred()) return nullptr;
-    if (alphabet < 1 || alphabet > 4096) Py_RETURN_NONE;
+    const size_t count = (size_t)(sym.v.len / sym.v.itemsize);
+    if (alphabet < 1 || alphabet > 4096 || block < 0 || (block && !eoq_b200_symbols_preferred(count, (uint64_t)block))) Py_RETURN_NONE;
     eoq_b200_symbols *s = nullptr;
     std::vector<uint64_t> counts((size_t)alphabet);
     eoq_error_t rc = EOQ_OK;
     Py_BEGIN_ALLOW_THREADS
-    s = eoq_b200_symbols_stage(sym.v.buf, type, (size_t)(sym.v.len / sym.v.itemsize), shift, clamp, (uint32_t)alphabet);
+    s = eoq_b200_symbols_stage(sym.v.buf, type, count, shift, clamp, (uint32_t)alphabet);
     if (s) rc = eoq_b200_symbols_count(s, counts.data());
     if (s && rc != EOQ_OK) { eoq_b200_symbols_free(s); s = nullptr; }
     Py_END_ALLOW_THREADS

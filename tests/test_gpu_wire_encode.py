@@ -64,6 +64,17 @@ def test_what_is_not_staged_and_calls_beside_a_recording():
     assert got == want and y.tolist() == [4.0] * 8
 
 
+@pytest.mark.parametrize("n,short,long", [(1 << 16, 645, 646), (70001, 256, 70001)])
+def test_few_long_blocks_are_the_hosts_and_give_the_same_bytes(n, short, long):
+    torch.zeros(1, device="cuda")
+    sym = np.minimum(np.abs(np.random.default_rng(n).standard_normal(n) * 3).astype(np.int64), 14)
+    for block, on_device in ((short, True), (long, False)):
+        staged, _ = R.stage_symbols(sym, 15, block_size=block)
+        assert (staged is not None) == on_device
+        data, want = BlockedRANSEncoder(block, 14).encode(sym, 15), O.encode_blocked(sym, 15, block, 14)
+        assert data.compressed_blocks == bytes(want.compressed_blocks) and list(data.block_offsets) == list(want.block_offsets)
+
+
 def test_more_than_two_to_the_27_blocks():
     torch.zeros(1, device="cuda")
     n = (1 << 27) + 77

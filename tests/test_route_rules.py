@@ -30,3 +30,12 @@ def test_a_few_rows_of_16_bit_activations(bits, group, n, k, warp_level):
     (12288, 4096, 129, 1), (11008, 8192, 128, 1), (14336, 2048, 128, 1), (28672, 8192, 144, 0), (28672, 8192, 145, 1), (20480, 8192, 144, 1), (28672, 11008, 144, 1)])
 def test_polar_rows_that_rotate_the_weight(n, k, rows, rotated):
     assert _rule("eoq_b200_polar_rotates", 3)(n, k, rows) == rotated
+
+
+@pytest.mark.parametrize("n,block,on_device", [
+    (65535, 256, 0), (1 << 16, 1, 1), (1 << 16, 256, 1), (1 << 16, 645, 1), (1 << 16, 646, 0), (1 << 16, 1 << 16, 0), (1 << 18, 1024, 1), (1 << 18, 4096, 0),
+    (1 << 20, 4096, 1), (1 << 20, 16384, 0), (1 << 20, 1 << 40, 0), (1 << 24, 16384, 1), (1 << 24, 65536, 0), (1 << 24, 1 << 24, 0)])
+def test_blocks_that_are_encoded_on_the_device(n, block, on_device):
+    fn = L.lib().eoq_b200_symbols_preferred
+    fn.restype, fn.argtypes = C.c_int, [C.c_size_t, C.c_uint64]
+    assert fn(n, block) == on_device
