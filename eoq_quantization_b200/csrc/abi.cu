@@ -10,6 +10,7 @@
 #include <cstring>
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <exception>
 #include <memory>
 #include <mutex>
 #include <system_error>
@@ -1017,10 +1018,16 @@ extern "C" eoq_error_t eoq_b200_decode_blocked_as(const uint32_t *freq, uint32_t
 // copies to be worth it (64 Ki symbols in blocks of 256, the whole call: 0.22 ms on the host's sixteen cores, 0.16 here), its blocks are short
 // enough (eoq_b200_symbols_preferred) and the alphabet fits shared memory.  On a
 // stream of its own: whatever else is under way on the device is not waited for.  Nothing is accepted or refused here that
-// the host encoder does not accept or refuse: what this one does not take, an array with symbols outside the alphabet among it, goes there.
+// the host encoder does not accept or refuse: what this one does not take, an array with symbols outside the alphabet among it,
+// goes there, and so does an array with which any call to the device fails.
 namespace {
 
 constexpr size_t kStageSymbols = 1u << 16;
+
+// "symbols_refused" in eoq_b200_tune: the step of a device encode that fails as if the device had nothing to give.
+enum { kRefuseStage = 1, kRefuseCount, kRefuseScratch, kRefuseEncode, kRefuseFetch };
+std::atomic<int> g_symbols_refused{0};
+bool refused(int step) { return g_symbols_refused.load(std::memory_order_relaxed) == step; }
 
 // A block is one chain, 0.073 us a symbol, while what the device saves with short chains grows as about n^(2/3): 0.03 ms x
 // (n / 32 Ki)^(2/3).  Whole calls, device / host's sixteen cores, us, fifteen symbols: 64 Ki symbols in blocks of 512 199 / 221, 1024
@@ -1117,7 +1124,7 @@ extern "C" int eoq_b200_symbols_preferred(size_t n, uint64_t block) { return n >
 
 // The staged array, or null: the host encodes.
 extern "C" eoq_b200_symbols *eoq_b200_symbols_stage(const void *symbols, int elem, size_t n, int64_t shift, int clamp, uint32_t alphabet)
-{
+try {
     if (!symbols || n < kStageSymbols || n > (1u << 28) || alphabet == 0 || alphabet > 4096u || elem < EOQ_B200_SYM_I8 || elem > EOQ_B200_SYM_I64) return nullptr;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || !context_is_active(dev)) { (void)cudaGetLastError(); return nullptr; }
@@ -1128,7 +1135,7 @@ extern "C" eoq_b200_symbols *eoq_b200_symbols_stage(const void *symbols, int ele
     s->at_counts = (n * width + 255) & ~(size_t)255;
     s->at_table = s->at_counts + (((size_t)alphabet * 8 + 8 + 255) & ~(size_t)255);
     PinnedBlock pinned;
-    if (!s->stream.acquire(dev) || s->sym.acquire(s->at_table + (size_t)alphabet * 16) != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
+    if (refused(kRefuseStage) || !s->stream.acquire(dev) || s->sym.acquire(s->at_table + (size_t)alphabet * 16) != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
     cudaStream_t st = s->stream.get();
     uint8_t *to = s->sym.base();
     // Bytes that hold a symbol as it will be kept go up as they are, and the device moves and clamps them; other types are
@@ -1149,15 +1156,16 @@ extern "C" eoq_b200_symbols *eoq_b200_symbols_stage(const void *symbols, int ele
     if (e != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
     if (as_is) { s->moved = true; s->is_signed = elem == EOQ_B200_SYM_I8; s->shift = (int)shift; s->clamp = clamp != 0; }
     return s.release();
-}
+} catch (const std::exception &) { return nullptr; }
 
 // Counts of the symbols; EOQ_ERR_UNSUPPORTED where one is outside the alphabet (and not to be clamped).
 extern "C" eoq_error_t eoq_b200_symbols_count(eoq_b200_symbols *s, uint64_t *counts)
-{
+try {
     BesideCapture beside;
     OnDevice on(s->dev);
     cudaStream_t st = s->stream.get();
     unsigned long long *d = reinterpret_cast<unsigned long long *>(s->sym.base() + s->at_counts);
+    if (refused(kRefuseCount)) return EOQ_ERR_CUDA;
     CU_TRY(cudaMemsetAsync(d, 0, (size_t)s->alphabet * 8 + 8, st));
     unsigned long long *outside = d + s->alphabet;
     if (s->moved && launch_wire_move(s->sym.base(), s->is_signed, s->shift, s->n, s->alphabet, outside, st) != 0) return EOQ_ERR_CUDA;
@@ -1168,10 +1176,10 @@ extern "C" eoq_error_t eoq_b200_symbols_count(eoq_b200_symbols *s, uint64_t *cou
     CU_TRY(cudaStreamSynchronize(st));
     std::memcpy(counts, got.data(), (size_t)s->alphabet * 8);
     return got.back() && !s->clamp ? EOQ_ERR_UNSUPPORTED : EOQ_OK;
-}
+} catch (const std::exception &) { return EOQ_ERR_ALLOC; }
 
 extern "C" eoq_error_t eoq_b200_symbols_encode(eoq_b200_symbols *s, const uint32_t *freq, uint32_t alphabet, uint32_t p, uint32_t block, size_t *bytes)
-{
+try {
     if (!s || !freq || !bytes) return EOQ_ERR_NULL_PTR;
     if (p < 1 || block == 0) return EOQ_ERR_INVALID_HEADER;
     if (p > 16 || alphabet != s->alphabet) return EOQ_ERR_UNSUPPORTED;
@@ -1191,24 +1199,25 @@ extern "C" eoq_error_t eoq_b200_symbols_encode(eoq_b200_symbols *s, const uint32
     s->at_offsets = up(at_sizes + (size_t)a.nblocks * 4);
     const size_t at_total = up(s->at_offsets + (size_t)a.nblocks * 4);
     s->at_out = at_total + 256;
-    if (s->work.acquire(s->at_out + most) != cudaSuccess) { (void)cudaGetLastError(); return EOQ_ERR_UNSUPPORTED; }
+    if (refused(kRefuseScratch) || s->work.acquire(s->at_out + most) != cudaSuccess) { (void)cudaGetLastError(); return EOQ_ERR_UNSUPPORTED; }
     uint8_t *d = s->work.base();
     a.table = reinterpret_cast<const uint4 *>(s->sym.base() + s->at_table);
     a.scratch = reinterpret_cast<uint32_t *>(d); a.record = reinterpret_cast<uint4 *>(d + at_record); a.sizes = reinterpret_cast<uint32_t *>(d + at_sizes);
     unsigned long long *total = reinterpret_cast<unsigned long long *>(d + at_total), sum = 0;
     CU_TRY(cudaMemcpyAsync(s->sym.base() + s->at_table, table.data(), table.size() * 4, cudaMemcpyHostToDevice, st));
-    if (launch_wire_encode(a, s->wide, reinterpret_cast<uint32_t *>(d + s->at_offsets), total, d + s->at_out, st) != 0) return EOQ_ERR_CUDA;
+    if (refused(kRefuseEncode) || launch_wire_encode(a, s->wide, reinterpret_cast<uint32_t *>(d + s->at_offsets), total, d + s->at_out, st) != 0) return EOQ_ERR_CUDA;
     CU_TRY(cudaMemcpyAsync(&sum, total, 8, cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
     if (sum > 0xFFFFFFFFull) return EOQ_ERR_OVERFLOW;
     *bytes = s->bytes = (size_t)sum;
     return EOQ_OK;
-}
+} catch (const std::exception &) { return EOQ_ERR_ALLOC; }
 
 // The encoded bytes (as many as eoq_b200_symbols_encode said) and the blocks' offsets.
 extern "C" eoq_error_t eoq_b200_symbols_fetch(eoq_b200_symbols *s, uint8_t *data, uint32_t *offsets)
-{
+try {
     if (!s || !data || !offsets || !s->work.base()) return EOQ_ERR_NULL_PTR;
+    if (refused(kRefuseFetch)) return EOQ_ERR_CUDA;
     BesideCapture beside;
     OnDevice on(s->dev);
     cudaStream_t st = s->stream.get();
@@ -1217,7 +1226,7 @@ extern "C" eoq_error_t eoq_b200_symbols_fetch(eoq_b200_symbols *s, uint8_t *data
     CU_TRY(cudaMemcpyAsync(offsets, s->work.base() + s->at_offsets, (size_t)s->nblocks * 4, cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
     return EOQ_OK;
-}
+} catch (const std::exception &) { return EOQ_ERR_ALLOC; }
 
 extern "C" eoq_error_t eoq_b200_encode_blocked(const uint32_t *freq, uint32_t alphabet, uint32_t precision_bits,
                                                const uint32_t *symbols, uint32_t num_symbols, uint32_t block_size,
@@ -2343,6 +2352,7 @@ extern "C" int eoq_b200_tune(const char *key, int value)
     if (std::strcmp(key, "dequant_vec") == 0) { set_dequant_vec(value); return 0; }
     if (std::strcmp(key, "qmm_wait_us") == 0) { set_qmm_wait_us(value); return 0; }
     if (std::strcmp(key, "pinned_refused") == 0) { g_pinned_refused.store(value); return 0; }
+    if (std::strcmp(key, "symbols_refused") == 0) { g_symbols_refused.store(value); return 0; }
     return -1;
 }
 

@@ -499,50 +499,54 @@ PyObject *encode_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
         w.staged = static_cast<eoq_b200_symbols *>(PyCapsule_GetPointer(a[9], kStaged));
         if (!w.staged) return nullptr;
     }
-    eoq_error_t rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = EOQ_ERR_UNSUPPORTED;
-    if (w.staged) rc = eoq_b200_symbols_encode(w.staged, static_cast<const uint32_t *>(freq.v.buf), (uint32_t)alphabet, (uint32_t)p, (uint32_t)block, &w.bytes);
-    if (rc == EOQ_ERR_UNSUPPORTED) {
-        w.staged = nullptr;
-        rc = eoq_b200_wire_encode(sym.v.buf, type, (uint32_t)count, shift, clamp, static_cast<const uint32_t *>(freq.v.buf), (uint32_t)alphabet, (uint32_t)p,
-                                  (uint32_t)block, &w.wire, &w.bytes);
-    }
-    Py_END_ALLOW_THREADS
-    if (rc != EOQ_OK) return codec_error(rc);
-    const size_t bytes = w.bytes;
     const int64_t nb = (count + block - 1) / block;
-    if (a[7] == Py_None) {
-        PyObject *data = PyBytes_FromStringAndSize(nullptr, (Py_ssize_t)bytes);
-        PyObject *list = data ? PyList_New((Py_ssize_t)nb) : nullptr;
-        if (!list) { Py_XDECREF(data); return nullptr; }
-        std::vector<uint32_t> offs((size_t)nb);
-        uint8_t *to = reinterpret_cast<uint8_t *>(PyBytes_AS_STRING(data));
-        Py_BEGIN_ALLOW_THREADS
-        rc = w.fetch(to, offs.data());
-        Py_END_ALLOW_THREADS
-        if (rc != EOQ_OK) { Py_DECREF(data); Py_DECREF(list); return codec_error(rc); }
-        for (int64_t b = 0; b < nb; b++) PyList_SET_ITEM(list, b, PyLong_FromUnsignedLong(offs[(size_t)b]));
-        return Py_BuildValue("NN", data, list);
+    std::optional<Buffer> head, table;
+    size_t at_table = 0, at_offs = 0, at_data = 0;
+    if (a[7] != Py_None) {
+        head.emplace(a[7]);
+        table.emplace(a[8]);
+        if (!head->ok || !table->ok) return nullptr;
+        at_table = (size_t)head->v.len + 4; at_offs = at_table + (size_t)table->v.len; at_data = at_offs + 4 * (size_t)nb;
     }
-    // container: head, data size, table, offsets, data
-    Buffer head(a[7]), table(a[8]);
-    if (!head.ok || !table.ok) return nullptr;
-    const size_t at_table = (size_t)head.v.len + 4, at_offs = at_table + (size_t)table.v.len, at_data = at_offs + 4 * (size_t)nb;
-    PyObject *whole = PyBytes_FromStringAndSize(nullptr, (Py_ssize_t)(at_data + bytes));
-    if (!whole) return nullptr;
-    uint8_t *to = reinterpret_cast<uint8_t *>(PyBytes_AS_STRING(whole));
-    const uint32_t size32 = (uint32_t)bytes;
-    std::memcpy(to, head.v.buf, (size_t)head.v.len);
-    std::memcpy(to + head.v.len, &size32, 4);
-    std::memcpy(to + at_table, table.v.buf, (size_t)table.v.len);
     std::vector<uint32_t> offs((size_t)nb);
-    Py_BEGIN_ALLOW_THREADS
-    rc = w.fetch(to + at_data, offs.data());
-    std::memcpy(to + at_offs, offs.data(), 4 * (size_t)nb);
-    Py_END_ALLOW_THREADS
-    if (rc != EOQ_OK) { Py_DECREF(whole); return codec_error(rc); }
-    return whole;
+    // on the device where the symbols are staged, and whatever goes wrong there, on the host, which has all that it takes
+    for (;;) {
+        eoq_error_t rc;
+        Py_BEGIN_ALLOW_THREADS
+        rc = w.staged ? eoq_b200_symbols_encode(w.staged, static_cast<const uint32_t *>(freq.v.buf), (uint32_t)alphabet, (uint32_t)p, (uint32_t)block, &w.bytes)
+                      : eoq_b200_wire_encode(sym.v.buf, type, (uint32_t)count, shift, clamp, static_cast<const uint32_t *>(freq.v.buf), (uint32_t)alphabet,
+                                             (uint32_t)p, (uint32_t)block, &w.wire, &w.bytes);
+        Py_END_ALLOW_THREADS
+        PyObject *whole = nullptr;                     // the container, or the blocks' bytes alone
+        if (rc == EOQ_OK) {
+            whole = PyBytes_FromStringAndSize(nullptr, (Py_ssize_t)(at_data + w.bytes));
+            if (!whole) return nullptr;
+            uint8_t *to = reinterpret_cast<uint8_t *>(PyBytes_AS_STRING(whole));
+            Py_BEGIN_ALLOW_THREADS
+            rc = w.fetch(to + at_data, offs.data());
+            Py_END_ALLOW_THREADS
+        }
+        if (rc != EOQ_OK) {
+            Py_XDECREF(whole);
+            if (!w.staged) return codec_error(rc);
+            w.staged = nullptr;
+            continue;
+        }
+        if (!head) {
+            PyObject *list = PyList_New((Py_ssize_t)nb);
+            if (!list) { Py_DECREF(whole); return nullptr; }
+            for (int64_t b = 0; b < nb; b++) PyList_SET_ITEM(list, b, PyLong_FromUnsignedLong(offs[(size_t)b]));
+            return Py_BuildValue("NN", whole, list);
+        }
+        // head, data size, table, offsets, data
+        uint8_t *to = reinterpret_cast<uint8_t *>(PyBytes_AS_STRING(whole));
+        const uint32_t size32 = (uint32_t)w.bytes;
+        std::memcpy(to, head->v.buf, (size_t)head->v.len);
+        std::memcpy(to + head->v.len, &size32, 4);
+        std::memcpy(to + at_table, table->v.buf, (size_t)table->v.len);
+        std::memcpy(to + at_offs, offs.data(), 4 * (size_t)nb);
+        return whole;
+    }
     GUARD_END
 }
 

@@ -8,6 +8,7 @@ import torch
 
 from eoq_quantization_b200 import _lib as L
 from eoq_quantization_b200.core import rans as R
+from eoq_quantization_b200.core.rans_bitpacked import compress_tensor_rans
 from eoq_quantization_b200.core.rans_blocked import BlockedRANSDecoder, BlockedRANSEncoder
 from oracle import oracle as O
 
@@ -73,6 +74,21 @@ def test_few_long_blocks_are_the_hosts_and_give_the_same_bytes(n, short, long):
         assert (staged is not None) == on_device
         data, want = BlockedRANSEncoder(block, 14).encode(sym, 15), O.encode_blocked(sym, 15, block, 14)
         assert data.compressed_blocks == bytes(want.compressed_blocks) and list(data.block_offsets) == list(want.block_offsets)
+
+
+@pytest.mark.parametrize("step", [1, 2, 3, 4, 5])
+def test_what_the_device_refuses_the_host_encodes(step):
+    torch.zeros(1, device="cuda")
+    codes = torch.from_numpy(np.random.default_rng(step).integers(-7, 8, 1 << 17).astype(np.int8))
+    sym = codes.numpy().astype(np.int64) + 7
+    want, record = BlockedRANSEncoder().encode(sym, 15), compress_tensor_rans("w", codes, torch.ones(1024), 4, 128, (1 << 17,))
+    try:
+        assert L.lib().eoq_b200_tune(b"symbols_refused", step) == 0
+        got, again = BlockedRANSEncoder().encode(sym, 15), compress_tensor_rans("w", codes, torch.ones(1024), 4, 128, (1 << 17,))
+    finally:
+        L.lib().eoq_b200_tune(b"symbols_refused", 0)
+    assert got.compressed_blocks == want.compressed_blocks and list(got.block_offsets) == list(want.block_offsets)
+    assert again.rans_bytes == record.rans_bytes and np.array_equal(got.freq_table, want.freq_table)
 
 
 def test_more_than_two_to_the_27_blocks():
