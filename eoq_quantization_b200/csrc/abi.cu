@@ -927,6 +927,17 @@ void convert(const void *src, void *dst, size_t n, int64_t shift)
 
 typedef void (*ConvertFn)(const void *, void *, size_t, int64_t);
 
+// This thread's rule for calls beside a stream that is recording (relaxed: allocations and waits are allowed although a stream may be,
+// since they have no part in the recording), as long as this lives.
+struct CaptureMode {
+    cudaStreamCaptureMode mode;
+    explicit CaptureMode(cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed) : mode(m) { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~CaptureMode() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    CaptureMode(const CaptureMode &) = delete;
+    CaptureMode &operator=(const CaptureMode &) = delete;
+    static cudaStreamCaptureMode current() { return CaptureMode().mode; }
+};
+
 // Symbols (1 or 2 bytes each on the device, complete on `st`) to `out`, of the type EOQ_B200_SYM_* names.
 eoq_error_t deliver(const uint8_t *dev, uint32_t elem, size_t n, void *out, int out_type, int64_t shift, cudaStream_t st)
 {
@@ -960,7 +971,9 @@ eoq_error_t deliver(const uint8_t *dev, uint32_t elem, size_t n, void *out, int 
     const size_t hw = std::max(1u, std::thread::hardware_concurrency());
     const size_t threads = std::max<size_t>(1, std::min<size_t>({kPinnedThreads, hw, (chunks + 1) / 2}));
     std::atomic<int> failed{0};
+    const cudaStreamCaptureMode mode = CaptureMode::current();              // a thread starts with one of its own
     parallel_for(threads, [&](size_t t) {
+        const CaptureMode as_the_caller(mode);
         cudaEvent_t done[2] = {nullptr, nullptr};
         bool ok = cudaSetDevice(device) == cudaSuccess && cudaEventCreateWithFlags(&done[0], cudaEventDisableTiming) == cudaSuccess &&
                   cudaEventCreateWithFlags(&done[1], cudaEventDisableTiming) == cudaSuccess;
@@ -1085,13 +1098,6 @@ class SideStream {
     int dev_ = 0;
 };
 
-// Allocations and waits of this thread are allowed although a stream of it may be recording: they have no part in the recording.
-struct BesideCapture {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    ~BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
-
 struct OnDevice {
     int was = -1;
     explicit OnDevice(int dev) { if (cudaGetDevice(&was) != cudaSuccess || (was != dev && cudaSetDevice(dev) != cudaSuccess)) was = -1; else if (was == dev) was = -1; }
@@ -1109,7 +1115,7 @@ struct eoq_b200_symbols {
     size_t at_counts = 0, at_table = 0, at_offsets = 0, at_out = 0, bytes = 0;
     ~eoq_b200_symbols()
     {
-        BesideCapture beside;
+        const CaptureMode beside;
         if (stream.get()) cudaStreamSynchronize(stream.get());      // the arenas are another call's from here on
         sym.release_beyond(256u << 20);                             // a process that encoded a large array once does not keep its scratch
         work.release_beyond(256u << 20);
@@ -1128,7 +1134,7 @@ try {
     if (!symbols || n < kStageSymbols || n > (1u << 28) || alphabet == 0 || alphabet > 4096u || elem < EOQ_B200_SYM_I8 || elem > EOQ_B200_SYM_I64) return nullptr;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || !context_is_active(dev)) { (void)cudaGetLastError(); return nullptr; }
-    BesideCapture beside;
+    const CaptureMode beside;
     std::unique_ptr<eoq_b200_symbols> s(new eoq_b200_symbols());
     s->dev = dev; s->n = (uint32_t)n; s->alphabet = alphabet; s->wide = alphabet > 256u;
     const size_t width = s->wide ? 2 : 1;
@@ -1161,7 +1167,7 @@ try {
 // Counts of the symbols; EOQ_ERR_UNSUPPORTED where one is outside the alphabet (and not to be clamped).
 extern "C" eoq_error_t eoq_b200_symbols_count(eoq_b200_symbols *s, uint64_t *counts)
 try {
-    BesideCapture beside;
+    const CaptureMode beside;
     OnDevice on(s->dev);
     cudaStream_t st = s->stream.get();
     unsigned long long *d = reinterpret_cast<unsigned long long *>(s->sym.base() + s->at_counts);
@@ -1185,7 +1191,7 @@ try {
     if (p > 16 || alphabet != s->alphabet) return EOQ_ERR_UNSUPPORTED;
     std::vector<uint32_t> table;
     if (!wire_table(freq, alphabet, p, table)) return EOQ_ERR_INVALID_HEADER;
-    BesideCapture beside;
+    const CaptureMode beside;
     OnDevice on(s->dev);
     cudaStream_t st = s->stream.get();
     WireEncodeArgs a = {};
@@ -1218,7 +1224,7 @@ extern "C" eoq_error_t eoq_b200_symbols_fetch(eoq_b200_symbols *s, uint8_t *data
 try {
     if (!s || !data || !offsets || !s->work.base()) return EOQ_ERR_NULL_PTR;
     if (refused(kRefuseFetch)) return EOQ_ERR_CUDA;
-    BesideCapture beside;
+    const CaptureMode beside;
     OnDevice on(s->dev);
     cudaStream_t st = s->stream.get();
     const eoq_error_t rc = deliver(s->work.base() + s->at_out, 1, s->bytes, data, EOQ_B200_SYM_U8, 0, st);

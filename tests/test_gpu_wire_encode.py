@@ -76,6 +76,20 @@ def test_few_long_blocks_are_the_hosts_and_give_the_same_bytes(n, short, long):
         assert data.compressed_blocks == bytes(want.compressed_blocks) and list(data.block_offsets) == list(want.block_offsets)
 
 
+def test_threads_that_fetch_beside_a_recording():
+    torch.zeros(1, device="cuda")
+    sym = np.random.default_rng(1).integers(0, 15, 1 << 23).astype(np.int8)             # 4 MB of blocks: several threads
+    want = BlockedRANSEncoder().encode(sym, 15).compressed_blocks
+    for size in (1 << 23, (1 << 23) - 5):                                               # and once with scratch that is there already
+        x, graph = torch.ones(8, device="cuda"), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            y = x + 1
+            got = BlockedRANSEncoder().encode(sym[:size], 15).compressed_blocks
+            y = y * 2
+        graph.replay()
+        assert (size < 1 << 23 or got == want) and y.tolist() == [4.0] * 8
+
+
 @pytest.mark.parametrize("step", [1, 2, 3, 4, 5])
 def test_what_the_device_refuses_the_host_encodes(step):
     torch.zeros(1, device="cuda")
