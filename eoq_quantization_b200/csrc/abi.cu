@@ -358,6 +358,52 @@ cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t st)
     return (cudaError_t)failed.load();
 }
 
+// Status words (of resident weights, of a decode's checks): 64 bytes each of page-locked memory that the device can address, dealt out of
+// pages (a page-locked allocation per weight, and its release, took 1.5 ms each).  A page whose words have all come
+// back is given back unless it is the only one.
+class StatusWords {
+  public:
+    static cudaError_t take(uint32_t **host, uint32_t **dev)
+    {
+        std::lock_guard<std::mutex> lock(mu());
+        Page *page = nullptr;
+        for (Page &p : pages()) if (p.used != ~0ull) { page = &p; break; }
+        if (!page) {
+            Page fresh;
+            cudaError_t e = cudaHostAlloc(reinterpret_cast<void **>(&fresh.host), 64 * 64, cudaHostAllocPortable | cudaHostAllocMapped);
+            if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&fresh.dev), fresh.host, 0);
+            if (e != cudaSuccess) return e;
+            pages().push_back(fresh);
+            page = &pages().back();
+        }
+        int slot = 0;
+        while ((page->used >> slot) & 1) slot++;
+        page->used |= 1ull << slot;
+        *host = reinterpret_cast<uint32_t *>(page->host + 64 * slot);
+        *dev = reinterpret_cast<uint32_t *>(page->dev + 64 * slot);
+        std::memset(*host, 0, 64);
+        return cudaSuccess;
+    }
+    static void give(uint32_t *word)
+    {
+        if (!word) return;
+        std::lock_guard<std::mutex> lock(mu());
+        uint8_t *at = reinterpret_cast<uint8_t *>(word);
+        for (size_t i = 0; i < pages().size(); i++) {
+            Page &p = pages()[i];
+            if (at < p.host || at >= p.host + 64 * 64) continue;
+            p.used &= ~(1ull << ((at - p.host) / 64));
+            if (p.used == 0 && pages().size() > 1) { cudaFreeHost(p.host); pages().erase(pages().begin() + i); }
+            return;
+        }
+    }
+
+  private:
+    struct Page { uint8_t *host = nullptr, *dev = nullptr; uint64_t used = 0; };
+    static std::mutex &mu() { static std::mutex *m = new std::mutex(); return *m; }
+    static std::vector<Page> &pages() { static std::vector<Page> *v = new std::vector<Page>(); return *v; }
+};
+
 // One tensor of a decode call.
 struct V1Job {
     Payload pl;                         // validated host views of the payload
@@ -372,6 +418,16 @@ struct V1Job {
     // blocks checked on the device (`job_verdict` has the outcome): the offsets as they lie in the caller's memory, whatever their alignment
     const uint8_t *raw_offsets = nullptr;
     size_t at_raw = 0, at_verdict = 0;
+    uint32_t *verdict = nullptr;        // page-locked, complete once `checked` is; without such memory null both
+    cudaEvent_t checked = nullptr;
+    V1Job() = default;
+    V1Job(const V1Job &) = delete;
+    V1Job &operator=(const V1Job &) = delete;
+    ~V1Job()
+    {
+        if (checked) cudaEventDestroy(checked);
+        StatusWords::give(verdict);
+    }
 };
 
 eoq_error_t job_from_payload(const eoq_tensor_header_t *h, const uint8_t *comp, size_t comp_size, size_t out_cap, V1Job &j)
@@ -470,6 +526,15 @@ eoq_error_t decode_jobs(V1Job **jobs, size_t n, cudaStream_t st, DeviceArena &ar
                                 reinterpret_cast<uint32_t *>(d + j.at_offsets), reinterpret_cast<uint32_t *>(d + j.at_sizes),
                                 reinterpret_cast<uint32_t *>(d + j.at_verdict), st) != 0)
                 return EOQ_ERR_CUDA;
+            uint32_t *unused;
+            if (g_pinned_refused.load() == 0 && StatusWords::take(&j.verdict, &unused) == cudaSuccess &&
+                cudaEventCreateWithFlags(&j.checked, cudaEventDisableTiming) == cudaSuccess) {
+                CU_TRY(cudaMemcpyAsync(j.verdict, d + j.at_verdict, 4, cudaMemcpyDeviceToHost, st));
+                CU_TRY(cudaEventRecord(j.checked, st));
+            } else {
+                j.checked = nullptr;
+                (void)cudaGetLastError();
+            }
         }
     }
     if (!tasks.empty()) {
@@ -491,12 +556,18 @@ eoq_error_t decode_jobs(V1Job **jobs, size_t n, cudaStream_t st, DeviceArena &ar
     return EOQ_OK;
 }
 
-// What the checks on the device found, in the order in which the host's would have: waits for them.
+// What the checks on the device found, in the order in which the host's would have: waits for them, and not for the decoder behind
+// them (but where there is no page-locked memory).
 eoq_error_t job_verdict(const V1Job &j, const DeviceArena &arena, cudaStream_t st)
 {
     uint32_t v = 0;
-    CU_TRY(cudaMemcpyAsync(&v, arena.base() + j.at_verdict, 4, cudaMemcpyDeviceToHost, st));
-    CU_TRY(cudaStreamSynchronize(st));
+    if (j.checked) {
+        CU_TRY(cudaEventSynchronize(j.checked));
+        v = *static_cast<volatile uint32_t *>(j.verdict);
+    } else {
+        CU_TRY(cudaMemcpyAsync(&v, arena.base() + j.at_verdict, 4, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaStreamSynchronize(st));
+    }
     return v == ~0u ? EOQ_OK : v & 1u ? EOQ_ERR_UNSUPPORTED : EOQ_ERR_CORRUPT_STREAM;
 }
 
@@ -847,11 +918,14 @@ extern "C" void eoq_cuda_batch_destroy(eoq_cuda_batch_ctx_t *ctx)
 // Part 2: Python-facing codec entry points and the fused path
 // =========================================================================
 
-// Validates a blocked stream on the host, as the reference's decoders do block by block, and makes it a job.
 // Blocks up to which the checks stay on the host: some 5 ns a block, against one more copy, launch and wait, some 14 us. Decodes
 // to int8 of blocks of 256, host's checks and device's: 2048 blocks 180 and 192 us, 5154 347 and 314, 65536 2111 and 1806.
+// (And from 2^30 blocks on, where a verdict would not hold the block's number.)
 constexpr uint32_t kHostChecks = 4096;
+static bool checks_on_device(uint32_t num_blocks) { return num_blocks > kHostChecks && num_blocks < (1u << 30); }
 
+// Validates a blocked stream, as the reference's decoders do block by block, and makes it a job: on the host, but for the blocks where
+// `check_on_device` and there are many.
 static eoq_error_t blocked_job(const uint32_t *freq, uint32_t alphabet, uint32_t precision_bits, const uint8_t *data, size_t data_len,
                                const uint32_t *offsets, uint32_t num_blocks, uint32_t block_size, uint32_t num_symbols,
                                int out_elem_bytes, V1Job &job, bool check_on_device = false)
@@ -868,7 +942,7 @@ static eoq_error_t blocked_job(const uint32_t *freq, uint32_t alphabet, uint32_t
     for (uint32_t s = 0; s < alphabet; s++) { sum += f[s]; cdf[s + 1] = cdf[s] + f[s]; }
     if (sum != (1ull << precision_bits)) return EOQ_ERR_INVALID_HEADER;
     // (a look at the first byte of each of 176 K blocks of a cold 19 MB stream takes 1.5 ms here, a few microseconds on the device)
-    check_on_device = check_on_device && num_blocks > kHostChecks;
+    check_on_device = check_on_device && checks_on_device(num_blocks);
     std::vector<uint32_t> sizes(check_on_device ? 0 : num_blocks);
     for (uint32_t b = 0; b < (uint32_t)sizes.size(); b++) {
         const uint64_t lo = offsets[b], hi = b + 1 < num_blocks ? offsets[b + 1] : data_len;
@@ -1015,10 +1089,8 @@ extern "C" eoq_error_t eoq_b200_decode_blocked_as(const uint32_t *freq, uint32_t
     V1Job *one = &job;
     DeviceArena arena;
     rc = decode_jobs(&one, 1, st, arena, false);
-    // (the checks' outcome is asked for last: waiting for it first would keep the threads of `deliver` from starting under the decoder,
-    // 0.2 ms; a stream that is refused leaves whatever was decoded in `out`)
+    if (rc == EOQ_OK && job.raw_offsets) rc = job_verdict(job, arena, st);      // a stream that is refused leaves `out` alone
     if (rc == EOQ_OK) rc = deliver(arena.base() + job.at_out, job.out_elem_bytes, num_symbols, out, out_type, shift, st);
-    if (rc == EOQ_OK && job.raw_offsets) rc = job_verdict(job, arena, st);
     const cudaError_t e = cudaStreamSynchronize(st);                  // the arena is another call's from here on
     if (rc != EOQ_OK) return rc;
     CU_TRY(e);
@@ -1294,52 +1366,6 @@ extern "C" eoq_error_t eoq_b200_encode_blocked(const uint32_t *freq, uint32_t al
 }
 
 // -- resident weights ---------------------------------------------------------
-
-// Status words of the resident weights: 64 bytes each of page-locked memory that the device can address, dealt out of
-// pages (a page-locked allocation per weight, and its release, took 1.5 ms each).  A page whose words have all come
-// back is given back unless it is the only one.
-class StatusWords {
-  public:
-    static cudaError_t take(uint32_t **host, uint32_t **dev)
-    {
-        std::lock_guard<std::mutex> lock(mu());
-        Page *page = nullptr;
-        for (Page &p : pages()) if (p.used != ~0ull) { page = &p; break; }
-        if (!page) {
-            Page fresh;
-            cudaError_t e = cudaHostAlloc(reinterpret_cast<void **>(&fresh.host), 64 * 64, cudaHostAllocPortable | cudaHostAllocMapped);
-            if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&fresh.dev), fresh.host, 0);
-            if (e != cudaSuccess) return e;
-            pages().push_back(fresh);
-            page = &pages().back();
-        }
-        int slot = 0;
-        while ((page->used >> slot) & 1) slot++;
-        page->used |= 1ull << slot;
-        *host = reinterpret_cast<uint32_t *>(page->host + 64 * slot);
-        *dev = reinterpret_cast<uint32_t *>(page->dev + 64 * slot);
-        std::memset(*host, 0, 64);
-        return cudaSuccess;
-    }
-    static void give(uint32_t *word)
-    {
-        if (!word) return;
-        std::lock_guard<std::mutex> lock(mu());
-        uint8_t *at = reinterpret_cast<uint8_t *>(word);
-        for (size_t i = 0; i < pages().size(); i++) {
-            Page &p = pages()[i];
-            if (at < p.host || at >= p.host + 64 * 64) continue;
-            p.used &= ~(1ull << ((at - p.host) / 64));
-            if (p.used == 0 && pages().size() > 1) { cudaFreeHost(p.host); pages().erase(pages().begin() + i); }
-            return;
-        }
-    }
-
-  private:
-    struct Page { uint8_t *host = nullptr, *dev = nullptr; uint64_t used = 0; };
-    static std::mutex &mu() { static std::mutex *m = new std::mutex(); return *m; }
-    static std::vector<Page> &pages() { static std::vector<Page> *v = new std::vector<Page>(); return *v; }
-};
 
 struct eoq_b200_weight {
     int device = 0;
@@ -1704,7 +1730,7 @@ extern "C" eoq_error_t eoq_b200_weight_from_rans(const uint8_t *c, size_t size, 
     if (n) {
         V1Job job;
         const uint8_t *offsets = c + 32 + (size_t)a * 4;             // of any alignment: read on the host only from a copy
-        std::vector<uint32_t> aligned(nb <= kHostChecks ? nb : 0);
+        std::vector<uint32_t> aligned(checks_on_device(nb) ? 0 : nb);
         if (!aligned.empty()) std::memcpy(aligned.data(), offsets, aligned.size() * 4);
         rc = blocked_job(freq.data(), a, p, offsets + (size_t)nb * 4, dsz, aligned.empty() ? reinterpret_cast<const uint32_t *>(offsets) : aligned.data(), nb, bs, n, 1,
                          job, true);

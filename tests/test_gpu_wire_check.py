@@ -58,6 +58,29 @@ def test_corrupt_blocks_give_the_hosts_codes(what, at, block):
         assert np.array_equal(EOQWeight(h.value, L.KIND_INT4_ABSMAX).decode_symbols().cpu().numpy().ravel(), sym)
 
 
+@pytest.mark.parametrize("pinned_refused", [0, 1])
+@pytest.mark.parametrize("what", ["order", "state longer than the block", "wide state"])
+@pytest.mark.parametrize("block", [12, 8])                     # 4096 blocks (checked on the host), 6144
+def test_a_refused_stream_leaves_the_result_alone(block, what, pinned_refused):
+    sym, data = _stream(block)
+    offs, raw = np.array(data.block_offsets, np.uint32), bytearray(data.compressed_blocks)
+    if what == "order":
+        offs[-2] = offs[-1] + 1
+    else:
+        raw[offs[-1]] = 255 if what == "state longer than the block" else 5
+    freq = np.ascontiguousarray(_normalize_frequencies(data.freq_table, 14)[0], dtype=np.uint32)
+    try:
+        L.lib().eoq_b200_tune(b"pinned_refused", pinned_refused)
+        for dtype, code in ((np.int8, 0), (np.int64, 6)):
+            out = np.full(N * K, 77, dtype)
+            got = L.native().decode_symbols(freq, 14, bytes(raw), offs, block, out, code, 0)
+            assert got == (L.EOQ_ERR_UNSUPPORTED if what == "wide state" else L.EOQ_ERR_CORRUPT_STREAM) and (out == 77).all()
+            assert L.native().decode_symbols(freq, 14, data.compressed_blocks, np.array(data.block_offsets, np.uint32), block, out, code, 0) is None
+            assert np.array_equal(out, sym)
+    finally:
+        L.lib().eoq_b200_tune(b"pinned_refused", 0)
+
+
 @pytest.mark.parametrize("offset", [0, 4, 8, 5])
 def test_tiles_from_symbols_of_any_alignment(offset):
     sym, _ = _stream()
