@@ -1197,6 +1197,8 @@ struct eoq_b200_symbols {
 
 extern "C" void eoq_b200_symbols_free(eoq_b200_symbols *s) { delete s; }
 
+extern "C" size_t eoq_b200_symbols_size(const eoq_b200_symbols *s) { return s ? s->n : 0; }
+
 // Whether n symbols in blocks of `block` are encoded sooner on the device than on the host's cores.
 extern "C" int eoq_b200_symbols_preferred(size_t n, uint64_t block) { return n >= kStageSymbols && chains_are_short((double)n, (double)block) ? 1 : 0; }
 

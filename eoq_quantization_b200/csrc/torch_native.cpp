@@ -43,6 +43,7 @@ extern "C" eoq_error_t eoq_b200_symbols_count(eoq_b200_symbols *s, uint64_t *cou
 extern "C" eoq_error_t eoq_b200_symbols_encode(eoq_b200_symbols *s, const uint32_t *freq, uint32_t alphabet, uint32_t p, uint32_t block, size_t *bytes);
 extern "C" eoq_error_t eoq_b200_symbols_fetch(eoq_b200_symbols *s, uint8_t *data, uint32_t *offsets);
 extern "C" void eoq_b200_symbols_free(eoq_b200_symbols *s);
+extern "C" size_t eoq_b200_symbols_size(const eoq_b200_symbols *s);
 extern "C" int eoq_b200_ordered_launches(int on);
 extern "C" int eoq_b200_gemv_packed_preferred(uint32_t rows, uint32_t cols, uint32_t bits, uint32_t group);
 extern "C" int eoq_b200_weight_linear_preferred(const eoq_b200_weight_t *w, const void *x, int x_dtype, uint32_t batch);
@@ -498,6 +499,7 @@ PyObject *encode_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
     if (a[9] != Py_None) {
         w.staged = static_cast<eoq_b200_symbols *>(PyCapsule_GetPointer(a[9], kStaged));
         if (!w.staged) return nullptr;
+        if (eoq_b200_symbols_size(w.staged) != (size_t)count) w.staged = nullptr;      // another array's: as many offsets as that one has blocks
     }
     const int64_t nb = (count + block - 1) / block;
     std::optional<Buffer> head, table;

@@ -76,6 +76,16 @@ def test_few_long_blocks_are_the_hosts_and_give_the_same_bytes(n, short, long):
         assert data.compressed_blocks == bytes(want.compressed_blocks) and list(data.block_offsets) == list(want.block_offsets)
 
 
+def test_an_array_beside_another_ones_staged_symbols():
+    torch.zeros(1, device="cuda")
+    sym = np.random.default_rng(2).integers(0, 15, 1 << 17).astype(np.uint8)
+    staged, counts = R.stage_symbols(sym, 15)
+    freq = R.RANSEncoder(counts, 14).freq
+    for other in (sym[:70000], np.concatenate([sym, sym])):
+        assert R.encode_blocks(freq, 14, other, 256, staged) == R.encode_blocks(freq, 14, other, 256)
+    assert R.encode_blocks(freq, 14, sym, 256, staged) == R.encode_blocks(freq, 14, sym, 256)
+
+
 def test_threads_that_fetch_beside_a_recording():
     torch.zeros(1, device="cuda")
     sym = np.random.default_rng(1).integers(0, 15, 1 << 23).astype(np.int8)             # 4 MB of blocks: several threads
