@@ -225,6 +225,13 @@ class DeviceArena {
         cudaFree(cur_.p);
         cur_ = Block();
     }
+    // what is kept between calls, back to the device
+    static void trim()
+    {
+        std::lock_guard<std::mutex> lock(cache().mu);
+        for (const Block &b : cache().free_list) cudaFree(b.p);
+        cache().free_list.clear();
+    }
     uint8_t *base() const { return static_cast<uint8_t *>(cur_.p); }
 
   private:
@@ -264,6 +271,12 @@ class PinnedBlock {
         std::lock_guard<std::mutex> lock(cache().mu);
         if (cache().free_list.size() < 2) cache().free_list.push_back(p_);
         else cudaFreeHost(p_);
+    }
+    static void trim()
+    {
+        std::lock_guard<std::mutex> lock(cache().mu);
+        for (uint8_t *p : cache().free_list) cudaFreeHost(p);
+        cache().free_list.clear();
     }
     uint8_t *chunk(size_t i) const { return p_ + i * kPinnedChunk; }
 
@@ -1102,7 +1115,8 @@ extern "C" eoq_error_t eoq_b200_decode_blocked_as(const uint32_t *freq, uint32_t
 // Used where the process has a context on the device already (encoding alone makes none), the array is long enough for the
 // copies to be worth it (64 Ki symbols in blocks of 256, the whole call: 0.22 ms on the host's sixteen cores, 0.16 here), its blocks are short
 // enough (eoq_b200_symbols_preferred) and the alphabet fits shared memory.  On a
-// stream of its own: whatever else is under way on the device is not waited for.  Nothing is accepted or refused here that
+// stream of its own: whatever else is under way on the device is not waited for, but where scratch is allocated or given back (a larger
+// array than before, one that wants more than 256 MB: cudaMalloc and cudaFree wait for the device).  Nothing is accepted or refused here that
 // the host encoder does not accept or refuse: what this one does not take, an array with symbols outside the alphabet among it,
 // goes there, and so does an array with which any call to the device fails.
 namespace {
@@ -2386,6 +2400,7 @@ extern "C" int eoq_b200_tune(const char *key, int value)
     if (std::strcmp(key, "dequant_vec") == 0) { set_dequant_vec(value); return 0; }
     if (std::strcmp(key, "qmm_wait_us") == 0) { set_qmm_wait_us(value); return 0; }
     if (std::strcmp(key, "pinned_refused") == 0) { g_pinned_refused.store(value); return 0; }
+    if (std::strcmp(key, "release_scratch") == 0) { DeviceArena::trim(); PinnedBlock::trim(); return 0; }
     if (std::strcmp(key, "symbols_refused") == 0) { g_symbols_refused.store(value); return 0; }
     return -1;
 }

@@ -429,7 +429,13 @@ PyObject *count_symbols(PyObject *, PyObject *const *a, Py_ssize_t n)
 
 constexpr const char *kStaged = "eoq_b200.symbols";
 
-void free_staged(PyObject *c) { eoq_b200_symbols_free(static_cast<eoq_b200_symbols *>(PyCapsule_GetPointer(c, kStaged))); }
+void free_staged(PyObject *c)
+{
+    eoq_b200_symbols *s = static_cast<eoq_b200_symbols *>(PyCapsule_GetPointer(c, kStaged));
+    Py_BEGIN_ALLOW_THREADS             // may wait for the device
+    eoq_b200_symbols_free(s);
+    Py_END_ALLOW_THREADS
+}
 
 // stage_symbols(array, type, shift, clamp, alphabet, block size or 0) -> (staged, [counts]): the array on the device, for one
 // encode_symbols call in front of which it is counted there; or None: count_symbols and encode_symbols take the array.

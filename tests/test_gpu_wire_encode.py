@@ -1,6 +1,7 @@
 """The wire format's encoder on the device gives the host encoder's bytes: symbol types and alphabets on either side of a byte,
 blocks that end off every boundary, tables from a few slots to 2^16, arrays around the length that is staged."""
 import ctypes as C
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
@@ -74,6 +75,31 @@ def test_few_long_blocks_are_the_hosts_and_give_the_same_bytes(n, short, long):
         assert (staged is not None) == on_device
         data, want = BlockedRANSEncoder(block, 14).encode(sym, 15), O.encode_blocked(sym, 15, block, 14)
         assert data.compressed_blocks == bytes(want.compressed_blocks) and list(data.block_offsets) == list(want.block_offsets)
+
+
+def test_scratch_is_bounded_and_given_back():
+    torch.zeros(1, device="cuda")
+    lib = L.lib()
+    assert lib.eoq_b200_tune(b"release_scratch", 0) == 0
+    before = torch.cuda.mem_get_info()[0]
+    BlockedRANSEncoder().encode(np.zeros(1 << 23, np.uint8), 15)                        # some 50 MB
+    kept = before - torch.cuda.mem_get_info()[0]
+    assert 0 < kept <= 64 << 20
+    big, at_first = np.zeros(80 << 20, np.uint8), BlockedRANSEncoder().encode(np.zeros(1 << 17, np.uint8), 15).compressed_blocks
+    BlockedRANSEncoder().encode(big, 15)                                                # more than 256 MB of scratch: not kept
+    assert before - torch.cuda.mem_get_info()[0] <= 256 << 20
+    assert lib.eoq_b200_tune(b"release_scratch", 0) == 0
+    assert before - torch.cuda.mem_get_info()[0] <= 4 << 20                             # (the side stream and its kernels stay)
+    assert BlockedRANSEncoder().encode(np.zeros(1 << 17, np.uint8), 15).compressed_blocks == at_first
+
+
+def test_two_threads_encode_at_once():
+    torch.zeros(1, device="cuda")
+    arrays = [np.random.default_rng(i).integers(0, 15, (1 << 18) + 1000 * i).astype(t) for i, t in enumerate((np.uint8, np.int64, np.int32))]
+    want = [BlockedRANSEncoder().encode(a, 15).compressed_blocks for a in arrays]
+    with ThreadPoolExecutor(3) as pool:
+        for _ in range(8):
+            assert list(pool.map(lambda a: BlockedRANSEncoder().encode(a, 15).compressed_blocks, arrays)) == want
 
 
 def test_an_array_beside_another_ones_staged_symbols():
