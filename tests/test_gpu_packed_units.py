@@ -37,3 +37,22 @@ def test_units_of_a_span(bits, n, k, group):
             if m <= 8 and packed_gemv_applies(k, bits, group, dt, m):
                 y = gemv_packed(layer.packed_weight, layer.scales, n, k, bits, group, x, layer.bias_param, out_dtype=torch.float32)
                 assert O.rel_l2(y.cpu().numpy(), want.cpu().numpy()) < 1e-6, (dt, m)
+
+
+@pytest.mark.parametrize("bits,group", [(4, 64), (4, 32), (2, 64), (8, 64), (8, 32)])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_rows_that_are_not_finite(bits, group, dt):
+    n, k, m = 40, 256, 8
+    g = torch.Generator(device="cuda").manual_seed(bits + group)
+    qmax = (1 << (bits - 1)) - 1
+    c = torch.randint(-qmax, qmax + 1, (n, k), generator=g, device="cuda")
+    packed = c.to(torch.int8) if bits == 8 else sum((c + qmax)[:, i::8 // bits].to(torch.uint8) << (bits * i) for i in range(8 // bits)).to(torch.uint8)
+    scales, x = (torch.rand(n, k // group, generator=g, device="cuda") + 0.1).half(), torch.randn(m, k, generator=g, device="cuda").to(dt)
+    want = gemv_packed(packed, scales, n, k, bits, group, x, out_dtype=torch.float32)
+    x[1, 7], x[4, group], x[6, 255] = float("inf"), float("-inf"), float("nan")
+    y = gemv_packed(packed, scales, n, k, bits, group, x, out_dtype=torch.float32)
+    assert torch.equal(y[[0, 2, 3, 5, 7]], want[[0, 2, 3, 5, 7]]) and torch.isnan(y[6]).all()
+    inf = float("inf")
+    for row, col, sign in ((1, 7, 1), (4, group, -1)):            # a zero code times infinity is NaN, others take its sign
+        expect = torch.where(c[:, col] == 0, torch.full((n,), float("nan"), device="cuda"), sign * torch.sign(c[:, col]) * inf)
+        assert torch.equal(torch.nan_to_num(y[row], 123.0), torch.nan_to_num(expect, 123.0))
