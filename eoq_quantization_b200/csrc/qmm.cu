@@ -1116,8 +1116,8 @@ int run_scaled(const QmmArgs &a, const void *packed, uint64_t row_bytes, const v
 // bits of each factor.
 //   Blocks of 64 columns against 16-bit activations (c.rotate): the producers rotate the weight's blocks in registers, where
 // the other two want rotated activations of two halves each.  The activations are exact then, and a pair takes two
-// products, not three.  What bounds it: instruction slots and the multiply-add pipe of the producers (some 600 instructions a
-// block and warp), then the tensor pipe.  512 tokens against 14336 x 4096 187 -> 139 us, 11008 x 4096 127 -> 94.8 (97.8 before
+// products, not three.  What bounds it, 512 tokens against 14336 x 4096: the tensor pipe, busy 66 % of an SM's active
+// cycles, beside the producers (instruction slots 49 %, multiply-add pipe 41 %); SMs are active 68 % of the time, for 224 CTAs are a round and a half.  512 tokens against 14336 x 4096 187 -> 139 us, 11008 x 4096 127 -> 94.8 (97.8 before
 // the remainders came from one mixed multiply-add each; look-ups by byte permutes instead of dot products 103), with a third
 // less error (4096 columns, fp32 results: 1.88e-6 -> 1.27e-6).
 constexpr uint32_t kPolarFold = 112;

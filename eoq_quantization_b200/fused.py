@@ -366,7 +366,7 @@ def dequant_packed(packed: torch.Tensor, scales: torch.Tensor, rows: int, cols: 
 
 def packed_gemv_rows(cols: int, bits: int, group: int, dtype: torch.dtype = torch.float16) -> int:
     """Activation rows `gemv_packed` takes for this shape: 32 on its tensor-core form (scale groups of whole 128-column
-    spans; fp32 activations go in as two fp16 halves each), 8 on the general form, 0 if it does not apply."""
+    spans; fp32 activations go in as two fp16 halves each), 8 on the forms for other groups, 0 if it does not apply."""
     if not (2 <= bits <= 8 and group > 0 and cols % group == 0):
         return 0
     if dtype in _DTYPES and cols % 128 == 0 and group % 128 == 0:

@@ -199,14 +199,14 @@ void eoq_cuda_batch_destroy(eoq_cuda_batch_ctx_t *ctx);
  * core/rans_bitpacked.py:126-154.  `freq` is the NORMALISED table (sum 2^p, all
  * >= 1; the caller normalises as core/rans.py:85-153 does).  `data`/`offsets`
  * are host pointers.  out_elem_bytes is 1 or 2.  If out_on_device is nonzero
- * `out` is a device pointer and the call is asynchronous on `stream`. */
+ * `out` is a device pointer.  Complete when the call returns. */
 eoq_error_t eoq_b200_decode_blocked(const uint32_t *freq, uint32_t alphabet, uint32_t precision_bits,
                                     const uint8_t *data, size_t data_len, const uint32_t *offsets,
                                     uint32_t num_blocks, uint32_t block_size, uint32_t num_symbols,
                                     void *out, int out_elem_bytes, int out_on_device, void *stream);
 
 /* The same with a host array of another integer type as the result: out[i] = (type)(symbol + shift), out_type one of
- * EOQ_B200_SYM_* below (not U32). */
+ * EOQ_B200_SYM_* below (not U32).  A stream that is refused leaves `out` alone. */
 eoq_error_t eoq_b200_decode_blocked_as(const uint32_t *freq, uint32_t alphabet, uint32_t precision_bits, const uint8_t *data,
                                        size_t data_len, const uint32_t *offsets, uint32_t num_blocks, uint32_t block_size,
                                        uint32_t num_symbols, void *out, int out_type, int64_t shift, void *stream);
